@@ -215,7 +215,7 @@ __device__ __forceinline__ void der_bulk(const ModelDev &m, const double *r, dou
 template <>
 __device__ __forceinline__ void der_bulk<CHGB_MODEL_LANDAU>(const ModelDev &m, const double *r, double *d) {
     double op = r[0];
-    d[0] = fma(-m.epsilon, op, (op * op) * op);
+    d[0] = op * fma(op, op, -m.epsilon);   // two FP64 instructions, two roundings
 }
 
 // f' of simple_wertheim for a given X(rho), src/models/SimpleWertheim.cpp:40-53
@@ -316,6 +316,15 @@ __device__ __forceinline__ double bulk_fe<CHGB_MODEL_SALEH>(const ModelDev &m, c
     double fe2 = log(X_2B) - X_2B / 2.0 + 0.5;
     double bonding = r[0] * m.sv0 * fe1 + r[1] * m.sv1 * fe2 + r[2] * m.half * (fe1 + fe2);
     return f_ref + bonding;
+}
+
+// Programmatic dependent launch: wait for the stream's previous kernel (its
+// writes have landed), then let the next kernel's CTAs be placed on the SMs
+// this grid no longer needs.  Without the launch attribute the wait returns at
+// once.
+__device__ __forceinline__ void pdl_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 
 struct KArr {

@@ -663,10 +663,6 @@ constexpr int STX = 32, STY = 8, SPX = STX + 2, SPY = STY + 2, SPP = SPX * SPY;
 // returns at once.  (Measured on GB300: 2D N=1024 split step 25.9 -> 25.1 us,
 // N=256 4.5 -> 4.2 us; the 3D N=256 step is unchanged.  The fused kernels,
 // whose single wave would then hold idle waiting CTAs, do not use it.)
-__device__ __forceinline__ void pdl_begin() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
-}
 
 template <int DIMS, int S>
 __device__ __forceinline__ void split_load_plane(double (*dst)[SPP], const double *__restrict__ src, const Geom &g,

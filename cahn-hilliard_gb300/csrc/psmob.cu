@@ -207,6 +207,8 @@ int psmob_create(const chgb_params &p, const Geom &g, const ModelDev &m, PsMob *
         psmob_destroy(s);
         return r;
     }
+    // the GMRES solve captures its passes into conditional graph bodies: plain launches there
+    spectral_set_pdl(s->eng, !p.use_gmres);
     s->hat = spectral_hat_size(s->eng);
     s->hall = s->hat * s->S;
     s->constant = p.mobility_type == CHGB_MOBILITY_CONSTANT;

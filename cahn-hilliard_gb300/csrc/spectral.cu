@@ -26,12 +26,12 @@
 // inv) + COL_y(inv).  1D: ROW + an elementwise update.
 // The real r2c/c2r of a row of L = 2M values is a complex FFT of length M on
 // the even/odd packing z[n] = x[2n] + i x[2n+1] plus one pre/post-processing
-// sweep.  FFT passes are Stockham autosort, radix 4 (one radix-2 pass first
-// when log2 of the length is odd), twiddles from one exactly symmetric
-// table W[q] = exp(-2 pi i q / N).  The transforms run in 64-bit block
-// floating point (bfp.cuh): each line is converted to fixed point with one
-// exponent, transformed with integer arithmetic and converted back; the state,
-// f' and the mode update stay FP64.
+// sweep.  The transforms run in 64-bit block floating point (bfp.cuh): each
+// line is converted to fixed point with one exponent, transformed with integer
+// arithmetic and converted back; the state, f' and the mode update stay FP64.
+// A line's values live in registers, four or eight to a thread, from the load
+// of the row or column to the store of its transform; they cross between
+// threads through shared memory once per radix-4 or radix-8 pass.
 #include <cmath>
 #include <vector>
 
@@ -49,162 +49,32 @@ cudaError_t bc_read_spectral(unsigned long long *first) { return bc_read_tu(firs
 namespace {
 
 // ---------------------------------------------------------------------------
-// Fixed-point (block floating point) Stockham FFT of one line, bfp.cuh.
+// Pseudospectral line transforms, bfp.cuh.
 // ---------------------------------------------------------------------------
-constexpr int FX_NAN_SCALE = 1 << 30;   // output scale of a line that held a NaN or an infinity
 
-__device__ __forceinline__ double2 fx_out(fx2 v, int sh) {
-    if(sh == FX_NAN_SCALE) return make_double2(__longlong_as_double(0x7FF8000000000000ll),
-                                               __longlong_as_double(0x7FF8000000000000ll));
-    return fx_store(v, sh);
-}
+// The CTA's share of a row pass: `lines` = rows * S lines of length M = 2^lgM,
+// one after another, T = max(1, M / E) threads each; a column pass: C lines,
+// interleaved in groups of at most FX_MAX_INTERLEAVE.
+constexpr int FX_MAX_INTERLEAVE = 8;
+constexpr int FX_MAX_WARPS = 32;
+constexpr int FX_E_SMALL = 4;
 
-// One pass of fx_fft_line: radix 2 (R == 2, the first pass of an odd log2 L)
-// or radix 4, Ns the length of the sub-transforms already formed.  in_d /
-// out_d: the pass reads FP64 values (scaled by 2^sh_in into fixed point) /
-// writes FP64 values (scaled back by 2^-sh_out) instead of fixed point; the
-// template flags IN_D / OUT_D say whether that conversion code is compiled at
-// all.  One body serves the first, middle and last passes of a line: with
-// small boxes every SM runs a kernel's code about once, and instruction
-// fetch, not arithmetic, is what a longer unrolled body costs.  DIR = -1
-// forward (twiddles w), +1 inverse (conj w).
-template <int DIR, int R, bool IN_D, bool OUT_D>
-__device__ __forceinline__ void fx_pass(const void *src_, void *dst_, int L, int Ns, int lane, int tpl,
-                                        const int4 *__restrict__ tw, int wstep, int sh_in, int sh_out, bool in_d,
-                                        bool out_d) {
-    const double2 *srcd = static_cast<const double2 *>(src_);
-    const fx2 *srcf = static_cast<const fx2 *>(src_);
-    double2 *dstd = static_cast<double2 *>(dst_);
-    fx2 *dstf = static_cast<fx2 *>(dst_);
-    if(R == 2) {
-        for(int j = lane; j < L / 2; j += tpl) {
-            if(!CHGB_BC(104, 2 * j + 1, L)) continue;
-            fx2 v0, v1;
-            if(IN_D && in_d) {
-                v0 = fx_load(srcd[j], sh_in);
-                v1 = fx_load(srcd[j + L / 2], sh_in);
-            }
-            else {
-                v0 = srcf[j];
-                v1 = srcf[j + L / 2];
-            }
-            const fx2 r0 = fx_add(v0, v1), r1 = fx_sub(v0, v1);
-            if(OUT_D && out_d) {
-                dstd[2 * j] = fx_out(r0, sh_out);
-                dstd[2 * j + 1] = fx_out(r1, sh_out);
-            }
-            else {
-                dstf[2 * j] = r0;
-                dstf[2 * j + 1] = r1;
-            }
-        }
-        return;
-    }
-    const int Q = L / 4;
-    const int tstride = (Q / Ns) * wstep;
-    for(int j = lane; j < Q; j += tpl) {
-        const int k = j & (Ns - 1);
-        if(!CHGB_BC(105, j + 3 * Q, L) || !CHGB_BC(105, (j - k) * 4 + k + 3 * Ns, L)) continue;
-        fx2 v0, v1, v2, v3;
-        if(IN_D && in_d) {
-            v0 = fx_load(srcd[j], sh_in);
-            v1 = fx_load(srcd[j + Q], sh_in);
-            v2 = fx_load(srcd[j + 2 * Q], sh_in);
-            v3 = fx_load(srcd[j + 3 * Q], sh_in);
-        }
-        else {
-            v0 = srcf[j];
-            v1 = srcf[j + Q];
-            v2 = srcf[j + 2 * Q];
-            v3 = srcf[j + 3 * Q];
-        }
-        fx2 s0, d0, s1, d1;
-        if(Ns > 1) {
-            const int m = k * tstride;
-            const fx2 t2 = fx_cmul<(DIR > 0)>(v2, tw[2 * m]);
-            s0 = fx_add(v0, t2);
-            d0 = fx_sub(v0, t2);
-            const fx2 t1 = fx_cmul<(DIR > 0)>(v1, tw[m]);
-            const fx2 t3 = fx_cmul<(DIR > 0)>(v3, tw[3 * m]);
-            s1 = fx_add(t1, t3);
-            d1 = fx_sub(t1, t3);
-        }
-        else {
-            s0 = fx_add(v0, v2);
-            d0 = fx_sub(v0, v2);
-            s1 = fx_add(v1, v3);
-            d1 = fx_sub(v1, v3);
-        }
-        const fx2 mi_d1 = fx2{d1.y, -d1.x};   // -i * d1
-        const int o = (j - k) * 4 + k;
-        const fx2 r0 = fx_add(s0, s1), r2 = fx_sub(s0, s1);
-        const fx2 r1 = DIR < 0 ? fx_add(d0, mi_d1) : fx_sub(d0, mi_d1);
-        const fx2 r3 = DIR < 0 ? fx_sub(d0, mi_d1) : fx_add(d0, mi_d1);
-        if(OUT_D && out_d) {
-            dstd[o] = fx_out(r0, sh_out);
-            dstd[o + Ns] = fx_out(r1, sh_out);
-            dstd[o + 2 * Ns] = fx_out(r2, sh_out);
-            dstd[o + 3 * Ns] = fx_out(r3, sh_out);
-        }
-        else {
-            dstf[o] = r0;
-            dstf[o + Ns] = r1;
-            dstf[o + 2 * Ns] = r2;
-            dstf[o + 3 * Ns] = r3;
-        }
-    }
-}
+inline int fx_line_threads(int L, int E) { return L > E ? L / E : 1; }
 
-// Fixed-point Stockham FFT of line li (length L >= 2, 16-byte elements, LS
-// elements between lines) in the shared buffers a/b, the counterpart of
-// fft_line.  The input is FP64 (IN_D, scaled by 2^sh_in) or fixed point; the
-// output FP64 (OUT_D, scaled by 2^-sh_out; FX_NAN_SCALE writes NaN) or fixed
-// point.  Every thread of the block must call it (it synchronises after each
-// pass).  Returns the buffer holding the result.
-template <int DIR, bool IN_D, bool OUT_D>
-__device__ void *fx_fft_line(void *a, void *b, int L, int log2L, int LS, int li, int lane, int tpl, bool active,
-                             const int4 *__restrict__ tw, int wstep, int sh_in, int sh_out) {
-    char *in = static_cast<char *>(a), *out = static_cast<char *>(b);
-    const size_t off = (size_t) li * LS * 16;
-    const int passes = (log2L & 1) + log2L / 2;
-    int p = 0, Ns = 1;
-    if(log2L & 1) {
-        if(active)
-            fx_pass<DIR, 2, IN_D, OUT_D>(in + off, out + off, L, 1, lane, tpl, tw, wstep, sh_in, sh_out, true,
-                                         passes == 1);
-        char *t = in;
-        in = out;
-        out = t;
-        Ns = 2;
-        p = 1;
-        __syncthreads();
-    }
-    for(; Ns < L; Ns *= 4, p++) {
-        if(active)
-            fx_pass<DIR, 4, IN_D, OUT_D>(in + off, out + off, L, Ns, lane, tpl, tw, wstep, sh_in, sh_out, p == 0,
-                                         p == passes - 1);
-        char *t = in;
-        in = out;
-        out = t;
-        __syncthreads();
-    }
-    return in;
-}
-
-// Largest exponent field over elements [0, n) of line li (lines LS apart) of
-// an FP64 buffer, reduced over the line's threads into sm_e[li] (see
-// fx_line_max); the caller synchronises before reading it.
-__device__ __forceinline__ void fx_line_exponent(const double2 *buf, int n, int LS, int li, int lane, int tpl,
-                                                 bool active, int *sm_e) {
-    int e = 0;
-    if(active) {
-        const double2 *src = buf + (size_t) li * LS;
-        for(int j = lane; j < n; j += tpl) {
-            const double2 v = src[j];
-            e = max(e, max(fx_expo(v.x), fx_expo(v.y)));
-        }
-    }
-    fx_line_max(e, tpl, li, lane, active, sm_e);
+template <int E>
+__device__ __forceinline__ FxLine fx_line(int lg, int lgC, bool whole_block) {
+    constexpr int lgE = E == 8 ? 3 : 2;
+    FxLine ln;
+    ln.lg = lg;
+    ln.lgC = lgC;
+    const int lgT = lg > lgE ? lg - lgE : 0;
+    ln.T = 1 << lgT;
+    ln.c = threadIdx.x & ((1 << lgC) - 1);
+    ln.lane = (threadIdx.x >> lgC) & (ln.T - 1);
+    const int nthr = blockDim.x, wbase = threadIdx.x & ~31;
+    // 0: the barriers are the block's
+    ln.warp_mask = whole_block || lgT + lgC > 5 ? 0u : nthr - wbase >= 32 ? 0xffffffffu : (1u << (nthr - wbase)) - 1u;
+    return ln;
 }
 
 enum { ROW_IN_REAL = 0, ROW_IN_HAT = 1 };
@@ -212,180 +82,307 @@ enum { ROW_IN_REAL = 0, ROW_IN_HAT = 1 };
 // g <- (M - M0[s]) (g / N^d) (FLUX_DM) or M (g / N^d) (FLUX_M).
 enum { FLUX_NONE = 0, FLUX_DM = 1, FLUX_M = 2 };
 
-// ROW kernel: `lines` = rows_per_cta * S lines per CTA, line li -> species
-// li % S of row blockIdx.x * rows_per_cta + li / S.  Half-spectrum rows live at
-// work[s * hat + row * H]; real rows at real[s * bins + row * N].  The shared
-// memory holds two buffers of lines * (M + 1) 16-byte elements, then 2 * lines
-// ints for the lines' exponents.  The transforms run in fixed point
-// (fx_fft_line); f' and the stored values are FP64.  Headroom: the c2r
-// pre-processing and the r2c post-processing each grow magnitudes by up to 4,
-// so both transforms take G = log2 M + 3.  FLUX: the mobility stage applied to
-// the real row between the two transforms (mob, M0 as psm_flux_kernel's).
-template <int KIND, int IN, bool FPRIME, bool WRITE_REAL, bool R2C, int FLUX = FLUX_NONE>
-__device__ __forceinline__ void row_body(double2 *__restrict__ work, const double *__restrict__ real_in,
-                                         double *__restrict__ real_out, int N, int M, int log2M, int rows_per_cta,
-                                         int tpl, long long bins, long long hat, const int4 *__restrict__ twf,
-                                         const ModelDev &m, long long row0, double2 *sm2,
-                                         const double *__restrict__ mob = nullptr,
-                                         const double *__restrict__ M0 = nullptr) {
-    constexpr int S = NSpecies<KIND>::value;
-    const int LS = M + 1;
-    const int lines = rows_per_cta * S;
-    double2 *A = sm2;
-    double2 *B = sm2 + lines * LS;
-    int *sm_e = reinterpret_cast<int *>(sm2 + 2 * lines * LS);   // [0, lines): c2r input, [lines, 2 lines): r2c input
-    const int li = threadIdx.x / tpl, lane = threadIdx.x - li * tpl;
-    const bool active = li < lines;
-    const int s = active ? li % S : 0;
-    const long long row = row0 + (active ? li / S : 0);
-    const int H = M + 1;
-    const int G = log2M + 3;
-    if(active && lane == 0) {
-        sm_e[li] = 0;
-        sm_e[lines + li] = 0;
-    }
-    double2 *cur;
-
-    if(IN == ROW_IN_REAL) {
-        if(active && CHGB_BC(106, row * N + N - 1, bins)) {
-            const double2 *src = reinterpret_cast<const double2 *>(real_in + s * bins + row * N);
-            for(int n = lane; n < M; n += tpl) A[li * LS + n] = src[n];
+// c2r of one row from its half spectrum src[0..M] to the packed real row
+// z[n] = x[2n] + i x[2n+1], n = lane + i T, in r[i].  The pre-processing
+//     Z[k] = (X[k] + conj X[M-k]) + i conj(w^k) (X[k] - conj X[M-k])
+// takes the modes k and M - k together: with T = conj(w^k) (X[k] - conj X[M-k])
+// and E = X[k] + conj X[M-k], Z[k] = E + i T and Z[M-k] = conj(E - i T), one
+// twiddle product for two modes.  The imaginary parts of the k = 0 and k = M
+// bins do not reach the real row (FFTW's c2r contract; they are not round-off
+// zeros when the spectrum is i k times a field).  Headroom G = log2 M + 3.
+template <int E>
+__device__ __forceinline__ void fx_row_c2r(double2 (&r)[E], const double2 *__restrict__ src, bool active,
+                                           const FxLine &ln, fx2 *&cur, fx2 *&oth, const int4 *__restrict__ twf,
+                                           int *sm_w) {
+    const int M = 1 << ln.lg, np = min(E, M) / 2;
+    double2 xa[E / 2], xb[E / 2], xm = make_double2(0.0, 0.0);
+    int mag = 0;
+#pragma unroll
+    for(int i = 0; i < E / 2; i++) {
+        const int k = ln.lane + i * ln.T;
+        xa[i] = xb[i] = make_double2(0.0, 0.0);
+        if(active && i < np) {
+            xa[i] = src[k];
+            xb[i] = src[M - k];
+            if(k == 0) xa[i].y = xb[i].y = 0.0;
         }
-        __syncthreads();
-        cur = A;
+        mag = max(mag, max(max(fx_mag(xa[i].x), fx_mag(xa[i].y)), max(fx_mag(xb[i].x), fx_mag(xb[i].y))));
+    }
+    if(ln.lane == 0 && active) {
+        xm = src[M / 2];
+        mag = max(mag, max(fx_mag(xm.x), fx_mag(xm.y)));
+    }
+    mag = fx_line_max(mag, 1, ln.T, sm_w);
+    const FxScale s = fx_line_scale(mag, ln.lg + 3);
+    double2 all[E + 1];
+#pragma unroll
+    for(int i = 0; i < E / 2; i++) {
+        all[i] = xa[i];
+        all[E / 2 + i] = xb[i];
+    }
+    all[E] = xm;
+    fx_scale_by(all, s.odd, s.pre);
+    // stored with real and imaginary parts swapped: the inverse transform
+    const int a0 = ln.at(ln.lane);
+#pragma unroll
+    for(int i = 0; i < E / 2; i++) {
+        if(i < np) {
+            const int k = ln.lane + i * ln.T;
+            const fx2 a = fx_in(all[i], s), b = fx_in(all[E / 2 + i], s);
+            const fx2 e = fx2{a.x + b.x, a.y - b.y};
+            const fx2 t = fx_cmul<true>(fx2{a.x - b.x, a.y + b.y}, __ldg(&twf[k]));
+            cur[a0 + i * ln.step(ln.T)] = fx2{e.y + t.x, e.x - t.y};
+            if(k > 0) cur[ln.at(M - k)] = fx2{t.x - e.y, e.x + t.y};
+        }
+    }
+    if(ln.lane == 0 && M > 1) {
+        const fx2 a = fx_in(all[E], s);
+        cur[ln.at(M / 2)] = fx2{-2 * a.y, 2 * a.x};
+    }
+    ln.sync();
+    fx2 v[E];
+#pragma unroll
+    for(int i = 0; i < E; i++) v[i] = (i < M) ? cur[a0 + i * ln.step(ln.T)] : fx2{0, 0};
+    fx_swap_buf(cur, oth);
+    fx_fft(v, ln, cur, oth, twf, ln.lg + 1);
+#pragma unroll
+    for(int i = 0; i < E; i++) r[i] = fx_out(fx_swap(v[i]), s);
+    fx_scale_by(r, s.odd, s.post);
+}
+
+// r2c of one packed real row r[i] to its half spectrum dst[0..M], the
+// post-processing X[k] = (a + t) / 2, X[M-k] = conj(a - t) / 2 with
+// a = Z[k] + conj Z[M-k], t = w^k (-i) (Z[k] - conj Z[M-k]), two modes to a
+// product as above; the halving is folded into the output scale.
+template <int E>
+__device__ __forceinline__ void fx_row_r2c(double2 (&r)[E], double2 *__restrict__ dst, bool active,
+                                           const FxLine &ln, fx2 *&cur, fx2 *&oth, const int4 *__restrict__ twf,
+                                           int *sm_w) {
+    const int M = 1 << ln.lg, np = min(E, M) / 2;
+    int mag = 0;
+#pragma unroll
+    for(int i = 0; i < E; i++)
+        if(i < M) mag = max(mag, max(fx_mag(r[i].x), fx_mag(r[i].y)));
+    mag = fx_line_max(mag, 1, ln.T, sm_w);
+    FxScale s = fx_line_scale(mag, ln.lg + 3);
+    fx_scale_by(r, s.odd, s.pre);
+    fx2 v[E];
+#pragma unroll
+    for(int i = 0; i < E; i++) v[i] = (i < M) ? fx_in(r[i], s) : fx2{0, 0};
+    fx_fft(v, ln, cur, oth, twf, ln.lg + 1);
+    const int a0 = ln.at(ln.lane);
+#pragma unroll
+    for(int i = 0; i < E; i++)
+        if(i < M) cur[a0 + i * ln.step(ln.T)] = v[i];
+    ln.sync();
+    s.sh += 1;
+    double2 x[E + 1];
+#pragma unroll
+    for(int i = 0; i < E / 2; i++) {
+        x[i] = x[E / 2 + i] = make_double2(0.0, 0.0);
+        if(i < np) {
+            const int k = ln.lane + i * ln.T;
+            const fx2 zk = v[i], zc = cur[k ? ln.at(M - k) : a0];
+            const fx2 a = fx2{zk.x + zc.x, zk.y - zc.y};
+            const fx2 t = fx_cmul<false>(fx2{zk.y + zc.y, zc.x - zk.x}, __ldg(&twf[k]));
+            x[i] = fx_out(fx2{a.x + t.x, a.y + t.y}, s);
+            x[E / 2 + i] = fx_out(fx2{a.x - t.x, t.y - a.y}, s);
+            if(k == 0) x[i].y = x[E / 2 + i].y = 0.0;
+        }
+    }
+    x[E] = make_double2(0.0, 0.0);
+    if(ln.lane == 0) {
+        const fx2 z = cur[ln.at(M / 2)];
+        x[E] = fx_out(fx2{2 * z.x, -2 * z.y}, s);
+    }
+    fx_scale_by(x, s.odd, s.post);
+    if(active) {
+#pragma unroll
+        for(int i = 0; i < E / 2; i++) {
+            if(i < np) {
+                const int k = ln.lane + i * ln.T;
+                dst[k] = x[i];
+                dst[M - k] = x[E / 2 + i];
+            }
+        }
+        if(ln.lane == 0) dst[M / 2] = x[E];
+    }
+    fx_swap_buf(cur, oth);
+}
+
+// f'(rho) of a line's cells in registers.  The formula of one cell inlines
+// once, not eight times: the values of the longer models go through the
+// thread's own slots of shared memory in a loop.
+template <int KIND, int E>
+__device__ __forceinline__ void row_fprime(double2 (&r)[E], const ModelDev &m, const FxLine &ln, fx2 *&cur, fx2 *&oth,
+                                           int s, int line_size, bool active) {
+    const int ne = min(E, 1 << ln.lg), a0 = ln.at(ln.lane), as = ln.step(ln.T);
+    if constexpr(KIND == CHGB_MODEL_LANDAU) {
+#pragma unroll
+        for(int i = 0; i < E; i++) {
+            der_bulk<KIND>(m, &r[i].x, &r[i].x);
+            der_bulk<KIND>(m, &r[i].y, &r[i].y);
+        }
     }
     else {
-        int e = 0;
-        if(active && CHGB_BC(107, row * H + H - 1, hat)) {
-            // c2r of a half spectrum: the imaginary parts of the k = 0 and k = M
-            // bins do not reach the real row (FFTW's c2r contract; they are
-            // not round-off zeros when the spectrum is i k times a field)
-            const double2 *src = work + s * hat + row * H;
-            for(int k = lane; k < H; k += tpl) {
-                double2 v = src[k];
-                if(k == 0 || k == M) v.y = 0.0;
-                B[li * LS + k] = v;
-                e = max(e, max(fx_expo(v.x), fx_expo(v.y)));
-            }
-        }
-        __syncthreads();
-        fx_line_max(e, tpl, li, lane, active, sm_e);
-        __syncthreads();
-        const int emax = active ? sm_e[li] : 0;
-        const int sh = fx_scale(emax, G);
-        // c2r pre-processing in fixed point:
-        //   Z[k] = (X[k] + conj X[M-k]) + i conj(w^k) (X[k] - conj X[M-k])
-        if(active) {
-            const double2 *X = B + li * LS;
-            fx2 *Z = reinterpret_cast<fx2 *>(A + li * LS);
-            for(int k = lane; k < M; k += tpl) {
-                const fx2 xk = fx_load(X[k], sh);
-                fx2 xc = fx_load(X[M - k], sh);
-                xc.y = -xc.y;
-                const fx2 e2 = fx_add(xk, xc);
-                const fx2 t = fx_cmul<true>(fx_sub(xk, xc), twf[k]);
-                Z[k] = fx2{e2.x - t.y, e2.y + t.x};
-            }
-        }
-        __syncthreads();
-        cur = static_cast<double2 *>(
-            fx_fft_line<+1, false, true>(A, B, M, log2M, LS, li, lane, tpl, active, twf, 2, 0,
-                                         emax == 2047 ? FX_NAN_SCALE : sh));
-    }
-    double2 *other = (cur == A) ? B : A;
-
-    if(WRITE_REAL && active && CHGB_BC(106, row * N + N - 1, bins)) {
-        double2 *dst = reinterpret_cast<double2 *>(real_out + s * bins + row * N);
-        for(int n = lane; n < M; n += tpl) dst[n] = cur[li * LS + n];
-    }
-    if(FLUX != FLUX_NONE) {
-        if(active) {
-            const double2 *mrow = reinterpret_cast<const double2 *>(mob + s * bins + row * N);
-            const double inv_bins = 1.0 / (double) bins;   // exact: N^d is a power of two
-            const double m0 = (FLUX == FLUX_DM) ? M0[s] : 0.0;
-            for(int n = lane; n < M; n += tpl) {
-                double2 v = cur[li * LS + n];
-                const double2 mm = mrow[n];
-                const double g0 = v.x * inv_bins, g1 = v.y * inv_bins;
-                if(FLUX == FLUX_DM) {
-                    v.x = (mm.x - m0) * g0;
-                    v.y = (mm.y - m0) * g1;
-                }
-                else {
-                    v.x = mm.x * g0;
-                    v.y = mm.y * g1;
-                }
-                cur[li * LS + n] = v;
-            }
-        }
-        __syncthreads();
-    }
-    if(FPRIME) {
-        // f'(rho) of the row's cells; species-0 lines do the work for all species
-        if(active && s == 0) {
-            for(int n = lane; n < M; n += tpl) {
-                double r0[S], r1[S], d0[S], d1[S];
+        double2 *A = reinterpret_cast<double2 *>(cur);
 #pragma unroll
-                for(int q = 0; q < S; q++) {
-                    double2 v = cur[(li + q) * LS + n];
-                    r0[q] = v.x;
-                    r1[q] = v.y;
+        for(int i = 0; i < E; i++)
+            if(i < ne) A[a0 + i * as] = r[i];
+        if constexpr(KIND == CHGB_MODEL_SIMPLE_WERTHEIM) {
+#pragma unroll 1
+            for(int i = 0; i < ne; i++) {
+                double2 v = A[a0 + i * as];
+                der_bulk<KIND>(m, &v.x, &v.x);
+                der_bulk<KIND>(m, &v.y, &v.y);
+                A[a0 + i * as] = v;
+            }
+        }
+        else {
+            // der_bulk<CHGB_MODEL_SALEH>, term by term, each species' line its own:
+            // the first two lines form the log X of their pairs in their second
+            // buffer, the linker's adds them up in its own, then every line adds
+            // its logarithm and writes f' over that
+            double2 *B = reinterpret_cast<double2 *>(oth);
+            __syncthreads();
+            if(active && s < 2) {
+                const double2 *R2 = A + (2 - s) * line_size;
+                const double delta = s == 0 ? m.dAA : m.dBB, sv = s == 0 ? m.sv0 : m.sv1;
+#pragma unroll 1
+                for(int i = 0; i < ne; i++) {
+                    const int p = a0 + i * as;
+                    const double2 o = A[p], c = R2[p];
+                    B[p] = make_double2(saleh_log_X(delta, sv, o.x, m.half, c.x, m.logtab),
+                                        saleh_log_X(delta, sv, o.y, m.half, c.y, m.logtab));
                 }
-                der_bulk<KIND>(m, r0, d0);
-                der_bulk<KIND>(m, r1, d1);
+            }
+            __syncthreads();
+            if(active && s == 2) {
+#pragma unroll 1
+                for(int i = 0; i < ne; i++) {
+                    const int p = a0 + i * as;
+                    const double2 l0 = B[p - 2 * line_size], l1 = B[p - line_size];
+                    B[p] = make_double2(l0.x + l1.x, l0.y + l1.y);
+                }
+            }
+            __syncthreads();
+            if(active) {
+                const double2 *R = A - s * line_size;
+                const double v = s == 0 ? m.sv0 : s == 1 ? m.sv1 : m.half;
+#pragma unroll 1
+                for(int i = 0; i < ne; i++) {
+                    const int p = a0 + i * as;
+                    const double2 r0 = R[p], r1 = R[p + line_size], r2 = R[p + 2 * line_size], o = A[p], l = B[p];
+                    double2 d;
 #pragma unroll
-                for(int q = 0; q < S; q++) cur[(li + q) * LS + n] = make_double2(d0[q], d1[q]);
+                    for(int h = 0; h < 2; h++) {
+                        const double rho_tot = ((0. + (h ? r0.y : r0.x)) + (h ? r1.y : r1.x)) + (h ? r2.y : r2.x);
+                        const double b2 = m.two_B2 * rho_tot, b3 = 3.0 * m.B3 * (rho_tot * rho_tot);
+                        const double own = h ? o.y : o.x;
+                        const double f = (own != 0.) ? ((tab_log(own, m.logtab) + b2) + b3) + v * (h ? l.y : l.x) : 0.0;
+                        if(h) d.y = f;
+                        else d.x = f;
+                    }
+                    B[p] = d;
+                }
             }
+            // the other lines may still read this one's A: the next exchange writes B first
+            A = B;
+            fx_swap_buf(cur, oth);
         }
-        __syncthreads();
-    }
-    if(R2C) {
-        fx_line_exponent(cur, M, LS, li, lane, tpl, active, sm_e + lines);
-        __syncthreads();
-        const int emax = active ? sm_e[lines + li] : 0;
-        const int sh = fx_scale(emax, G);
-        const fx2 *Z = static_cast<const fx2 *>(
-                           fx_fft_line<-1, true, false>(cur, other, M, log2M, LS, li, lane, tpl, active, twf, 2, sh, 0)) +
-                       li * LS;
-        // post-processing: X[k] = (a + w^k (-i b)) / 2 with a = Zk + conj Z_{M-k},
-        // b = Zk - conj Z_{M-k}; the halving is folded into the output scale
-        if(active && CHGB_BC(107, row * H + H - 1, hat)) {
-            const int sh_out = emax == 2047 ? FX_NAN_SCALE : sh + 1;
-            double2 *dst = work + s * hat + row * H;
-            for(int k = lane; k <= M; k += tpl) {
-                const fx2 zk = Z[k == M ? 0 : k];
-                fx2 zc = Z[k == 0 ? 0 : M - k];
-                zc.y = -zc.y;
-                const fx2 a = fx_add(zk, zc), bb = fx_sub(zk, zc);
-                const fx2 t = fx_cmul<false>(fx2{bb.y, -bb.x}, twf[k]);
-                double2 xk = fx_out(fx_add(a, t), sh_out);
-                if(k == 0 || k == M) xk.y = 0.0;
-                dst[k] = xk;
-            }
-        }
+#pragma unroll
+        for(int i = 0; i < E; i++)
+            if(i < ne) r[i] = A[a0 + i * as];
     }
 }
 
-template <int KIND, int IN, bool FPRIME, bool WRITE_REAL, bool R2C, int FLUX = FLUX_NONE>
-__global__ void __launch_bounds__(1024) row_kernel(double2 *__restrict__ work, const double *__restrict__ real_in,
-                                                   double *__restrict__ real_out, int N, int M, int log2M,
-                                                   int rows_per_cta, int tpl, long long bins, long long hat,
-                                                   const int4 *__restrict__ twf, ModelDev m,
-                                                   const double *__restrict__ mob, const double *__restrict__ M0) {
-    extern __shared__ double2 sm2[];
-    row_body<KIND, IN, FPRIME, WRITE_REAL, R2C, FLUX>(work, real_in, real_out, N, M, log2M, rows_per_cta, tpl, bins,
-                                                      hat, twf, m, (long long) blockIdx.x * rows_per_cta, sm2, mob, M0);
+// ROW pass: line li of the CTA is species li % S of row row0 + li / S.
+// Half-spectrum rows live at work[s * hat + row * H]; real rows at
+// real[s * bins + row * N].  The shared memory holds two buffers of the CTA's
+// blockDim / T lines.  The transforms run in fixed point; f' and the stored
+// values are FP64.  FLUX: the mobility stage
+// applied to the real row between the two transforms (mob, M0 as
+// psm_flux_kernel's).
+template <int KIND, int E, int IN, bool FPRIME, bool WRITE_REAL, bool R2C, int FLUX = FLUX_NONE>
+__device__ __forceinline__ void row_body(double2 *__restrict__ work, const double *__restrict__ real_in,
+                                         double *__restrict__ real_out, int lgM, int rows_per_cta, long long bins,
+                                         long long hat, const int4 *__restrict__ twf, const ModelDev &m,
+                                         long long row0, fx2 *sm, const double *__restrict__ mob = nullptr,
+                                         const double *__restrict__ M0 = nullptr) {
+    constexpr int S = NSpecies<KIND>::value;
+    __shared__ int sm_w[2][FX_MAX_WARPS];
+    const FxLine ln = fx_line<E>(lgM, 0, S > 1);
+    const int M = 1 << lgM, N = 2 * M, H = M + 1;
+    const int LS = fx_line_size(M), lines = rows_per_cta * S;
+    const int li = threadIdx.x / ln.T, nl = blockDim.x / ln.T;
+    const int s = li % S;
+    const long long row = row0 + li / S;
+    const bool active = li < lines && CHGB_BC(106, row * N + N - 1, bins) && CHGB_BC(107, row * H + H - 1, hat);
+    fx2 *cur = sm + li * LS, *oth = sm + (nl + li) * LS;
+    double2 r[E];
+
+    if constexpr(IN == ROW_IN_REAL) {
+        const double2 *src = reinterpret_cast<const double2 *>(real_in + s * bins + row * N);
+#pragma unroll
+        for(int i = 0; i < E; i++)
+            r[i] = (active && i < M) ? src[ln.lane + i * ln.T] : make_double2(0.0, 0.0);
+    }
+    else {
+        fx_row_c2r(r, work + s * hat + row * H, active, ln, cur, oth, twf, sm_w[0]);
+    }
+    if constexpr(WRITE_REAL) {
+        double2 *dst = reinterpret_cast<double2 *>(real_out + s * bins + row * N);
+#pragma unroll
+        for(int i = 0; i < E; i++)
+            if(active && i < M) dst[ln.lane + i * ln.T] = r[i];
+    }
+    if constexpr(FLUX != FLUX_NONE) {
+        const double2 *mrow = reinterpret_cast<const double2 *>(mob + s * bins + row * N);
+        const double inv_bins = 1.0 / (double) bins;   // exact: N^d is a power of two
+        const double m0 = (FLUX == FLUX_DM && active) ? M0[s] : 0.0;
+#pragma unroll
+        for(int i = 0; i < E; i++) {
+            if(active && i < M) {
+                const double2 mm = mrow[ln.lane + i * ln.T];
+                const double g0 = r[i].x * inv_bins, g1 = r[i].y * inv_bins;
+                if(FLUX == FLUX_DM) r[i] = make_double2((mm.x - m0) * g0, (mm.y - m0) * g1);
+                else r[i] = make_double2(mm.x * g0, mm.y * g1);
+            }
+        }
+    }
+    if constexpr(FPRIME) row_fprime<KIND, E>(r, m, ln, cur, oth, s, LS, active);
+    if constexpr(R2C) fx_row_r2c(r, work + s * hat + row * H, active, ln, cur, oth, twf, sm_w[1]);
+}
+
+// Threads of a row CTA: at most 256 a line (E = 8: N = 4096; E = 4: N = 2048).
+template <int KIND>
+struct RowThreads {
+    static constexpr int value = 256 * NSpecies<KIND>::value;
+};
+
+template <int KIND, int E, int IN, bool FPRIME, bool WRITE_REAL, bool R2C, int FLUX = FLUX_NONE>
+__global__ void __launch_bounds__(RowThreads<KIND>::value) row_kernel(double2 *__restrict__ work,
+                                                                      const double *__restrict__ real_in,
+                                                                      double *__restrict__ real_out, int lgM,
+                                                                      int rows_per_cta, long long bins, long long hat,
+                                                                      const int4 *__restrict__ twf, ModelDev m,
+                                                                      const double *__restrict__ mob,
+                                                                      const double *__restrict__ M0) {
+    extern __shared__ fx2 sm2[];
+    pdl_begin();
+    row_body<KIND, E, IN, FPRIME, WRITE_REAL, R2C, FLUX>(work, real_in, real_out, lgM, rows_per_cta, bins, hat, twf, m,
+                                                      (long long) blockIdx.x * rows_per_cta, sm2, mob, M0);
 }
 
 // Batched row pass of one time step: CTA b takes rows items[b].y.. of replica items[b].x.
 template <int KIND>
 __global__ void __launch_bounds__(256) row_batch_kernel(const PsBatchRep *__restrict__ reps,
                                                         const int2 *__restrict__ items) {
-    extern __shared__ double2 sm2[];
+    extern __shared__ fx2 sm2[];
     const int2 it = items[blockIdx.x];
     const PsBatchRep &r = reps[it.x];
-    row_body<KIND, ROW_IN_HAT, true, false, true>(r.work, nullptr, nullptr, r.N, r.M, r.log2M, r.row_rpc, r.row_tpl,
-                                                  r.bins, r.hat, r.twf, r.m, it.y, sm2);
+    row_body<KIND, FX_E_SMALL, ROW_IN_HAT, true, false, true>(r.work, nullptr, nullptr, r.log2N - 1, r.row_rpc, r.bins, r.hat,
+                                                  r.twf, r.m, it.y, sm2);
 }
 
 enum { COL_FWD = 0, COL_INV = 1, COL_STEP = 2, COL_INIT = 3, COL_GRAD_INV = 4, COL_FWD_DIV = 5, COL_FWD_MU = 6,
@@ -409,56 +406,58 @@ struct ColOps {
     double two_k, dt, Ssplit, k0, inv_bins;   // inv_bins = 1 / N^d, exact (a power of two)
 };
 
-// (column, position) of element e of a CTA's ncols lines stored position-major
-// (e = pos * ncols + c): a mask and a shift when ncols is a power of two (every
-// CTA but a ragged last one, lg = log2 ncols), integer division otherwise.
-__device__ __forceinline__ void col_split(int e, int ncols, int lg, int &c, int &pos) {
-    if(lg >= 0) {
-        c = e & (ncols - 1);
-        pos = e >> lg;
+// One transform of a column line: r[i] = values at positions lane + i T, INV
+// the unnormalised inverse.  Headroom G = log2 L + 1.
+template <bool INV, int E>
+__device__ __forceinline__ void fx_col_fft(double2 (&r)[E], const FxLine &ln, int C, fx2 *&cur, fx2 *&oth,
+                                           const int4 *__restrict__ twf, int *sm_w) {
+    const int L = 1 << ln.lg;
+    int mag = 0;
+#pragma unroll
+    for(int i = 0; i < E; i++)
+        if(i < L) mag = max(mag, max(fx_mag(r[i].x), fx_mag(r[i].y)));
+    mag = fx_line_max(mag, C, ln.T * C, sm_w);
+    const FxScale s = fx_line_scale(mag, ln.lg + 1);
+    fx_scale_by(r, s.odd, s.pre);
+    fx2 v[E];
+#pragma unroll
+    for(int i = 0; i < E; i++) {
+        v[i] = (i < L) ? fx_in(r[i], s) : fx2{0, 0};
+        if(INV) v[i] = fx_swap(v[i]);
     }
-    else {
-        c = e % ncols;
-        pos = e / ncols;
-    }
+    fx_fft(v, ln, cur, oth, twf, ln.lg);
+#pragma unroll
+    for(int i = 0; i < E; i++) r[i] = fx_out(INV ? fx_swap(v[i]) : v[i], s);
+    fx_scale_by(r, s.odd, s.post);
 }
 
-__device__ __forceinline__ int col_log2(int ncols) { return (ncols & (ncols - 1)) == 0 ? __ffs(ncols) - 1 : -1; }
-
 // COL pass: C lines (adjacent half-spectrum columns kx0..) of one species and
-// one plane per CTA; element pos of line li at
-//   off = species * hat + plane * plane_stride + (kx0 + li) + pos * elem_stride.
-// The shared memory holds two buffers of C * L elements, then 2 * C ints for
-// the lines' exponents.  Transforms in fixed point, G = log2 L + 1.
-template <int MODE>
+// one plane per CTA, in groups of at most FX_MAX_INTERLEAVE interleaved lines;
+// element pos of column kx at
+//   off = species * hat + plane * plane_stride + kx + pos * elem_stride.
+// The shared memory holds two buffers of C lines.
+template <int MODE, int E>
 __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
-                                         const double *__restrict__ alpha, const double *__restrict__ beta, int L,
-                                         int log2L, int H, int C, int tpl, long long elem_stride,
-                                         long long plane_stride, long long hat, const int4 *__restrict__ twf,
-                                         int wstep, double scale, int kx0, long long plane, long long species,
-                                         double2 *sm2, const ColOps &ops = ColOps()) {
-    const int LS = L;
-    double2 *A = sm2;
-    double2 *B = sm2 + C * LS;
-    int *sm_e = reinterpret_cast<int *>(sm2 + 2 * C * LS);
-    const int li = threadIdx.x / tpl, lane = threadIdx.x - li * tpl;
-    const long long base = species * hat + plane * plane_stride + kx0;
-    const int ncols = min(C, H - kx0);
-    const int lg = col_log2(ncols);
-    const bool active = li < ncols;
-    const int nthr = blockDim.x;
-    const int G = log2L + 1;
-    if(active && lane == 0) {
-        sm_e[li] = 0;
-        sm_e[C + li] = 0;
-    }
-
-    // coalesced load: consecutive threads take adjacent columns of one row
-    for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-        int c, pos;
-        col_split(e, ncols, lg, c, pos);
-        const long long off = base + c + pos * elem_stride;
-        if(!CHGB_BC(101, off - species * hat, hat) || !CHGB_BC(102, c * LS + pos, C * LS)) continue;
+                                         const double *__restrict__ alpha, const double *__restrict__ beta, int lgL,
+                                         int H, int lgC, long long elem_stride, long long plane_stride, long long hat,
+                                         const int4 *__restrict__ twf, double scale, int kx0, long long plane,
+                                         long long species, fx2 *sm, const ColOps &ops = ColOps()) {
+    __shared__ int sm_w[2][FX_MAX_WARPS * FX_MAX_INTERLEAVE];
+    const int lgI = min(lgC, 3), I = 1 << lgI;   // interleaved lines of a group
+    const FxLine ln = fx_line<E>(lgL, lgI, false);
+    const int L = 1 << lgL, LS = fx_line_size(L) << lgI;
+    const int group = threadIdx.x / (ln.T << lgI), groups = 1 << (lgC - lgI);
+    const int kx = kx0 + (group << lgI) + ln.c;
+    const bool active = group < groups && kx < H;
+    fx2 *cur = sm + group * LS, *oth = sm + (blockDim.x / (ln.T << lgI) + group) * LS;
+    const long long off0 = species * hat + plane * plane_stride + kx + ln.lane * elem_stride;
+    const long long dT = ln.T * elem_stride;
+    double2 r[E];
+#pragma unroll
+    for(int i = 0; i < E; i++) {
+        r[i] = make_double2(0.0, 0.0);
+        const long long off = off0 + i * dT;
+        if(!active || i >= L || !CHGB_BC(101, off - species * hat, hat)) continue;
         double2 v;
         if(MODE == COL_GRAD_INV) {
             v = mul_ik(ops.kd[off], ops.src[off]);
@@ -474,78 +473,47 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
             const double m0 = ops.M0[species];
             const double denom = 1.0 + ops.dt * m0 * (ops.Ssplit * k2 + 2.0 * ops.k0 * k4);
             const double cc = ops.dt * m0 * k2;
-            const double2 r = ops.rho[off], f = ops.fder[off];
-            double ar = r.x, ai = r.y;
+            const double2 q = ops.rho[off], f = ops.fder[off];
+            double ar = q.x, ai = q.y;
             if(ops.with_div) {
                 const double2 d = ops.div_in[off];
-                ar = r.x + ops.dt * d.x;
-                ai = r.y + ops.dt * d.y;
+                ar = q.x + ops.dt * d.x;
+                ai = q.y + ops.dt * d.y;
             }
-            const double nr = (ar - cc * (f.x - ops.Ssplit * r.x)) / denom;
-            const double ni = (ai - cc * (f.y - ops.Ssplit * r.y)) / denom;
+            const double nr = (ar - cc * (f.x - ops.Ssplit * q.x)) / denom;
+            const double ni = (ai - cc * (f.y - ops.Ssplit * q.y)) / denom;
             ops.rho[off] = make_double2(nr, ni);
             v = make_double2(nr * ops.inv_bins, ni * ops.inv_bins);
         }
         else {
             v = work[off];
         }
-        A[c * LS + pos] = v;
+        r[i] = v;
     }
-    __syncthreads();
-    fx_line_exponent(A, L, LS, li, lane, tpl, active, sm_e);
-    __syncthreads();
-    int emax = active ? sm_e[li] : 0;
-    int sh = fx_scale(emax, G);
-    double2 *cur;
-    if(MODE == COL_INV || MODE == COL_GRAD_INV || MODE == COL_UPD_INV) {
-        cur = static_cast<double2 *>(fx_fft_line<+1, true, true>(A, B, L, log2L, LS, li, lane, tpl, active, twf,
-                                                                 wstep, sh, emax == 2047 ? FX_NAN_SCALE : sh));
-    }
-    else {
-        cur = static_cast<double2 *>(fx_fft_line<-1, true, true>(A, B, L, log2L, LS, li, lane, tpl, active, twf,
-                                                                 wstep, sh, emax == 2047 ? FX_NAN_SCALE : sh));
-    }
-    if(MODE == COL_INIT) {
-        for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-            int c, pos;
-            col_split(e, ncols, lg, c, pos);
-            if(!CHGB_BC(101, base + c + pos * elem_stride - species * hat, hat) || !CHGB_BC(102, c * LS + pos, C * LS))
-                continue;
-            double2 v = cur[c * LS + pos];
-            psi_hat[base + c + pos * elem_stride] = make_double2(v.x * scale, v.y * scale);
-        }
-        return;
-    }
-    if(MODE == COL_STEP) {
-        for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-            int c, pos;
-            col_split(e, ncols, lg, c, pos);
-            long long off = base + c + pos * elem_stride;
-            if(!CHGB_BC(101, off - species * hat, hat) || !CHGB_BC(102, c * LS + pos, C * LS)) continue;
-            double2 ph = psi_hat[off];
-            double al = alpha[off], be = beta[off];
-            double2 f = cur[c * LS + pos];
-            double2 nv = make_double2(fma(al, ph.x, -be * f.x), fma(al, ph.y, -be * f.y));
+    constexpr bool INV = MODE == COL_INV || MODE == COL_GRAD_INV || MODE == COL_UPD_INV;
+    fx_col_fft<INV>(r, ln, I, cur, oth, twf, sm_w[0]);
+    if constexpr(MODE == COL_STEP) {
+#pragma unroll
+        for(int i = 0; i < E; i++) {
+            const long long off = off0 + i * dT;
+            if(!active || i >= L || !CHGB_BC(101, off - species * hat, hat)) continue;
+            const double2 ph = psi_hat[off];
+            const double al = alpha[off], be = beta[off];
+            const double2 nv = make_double2(fma(al, ph.x, -be * r[i].x), fma(al, ph.y, -be * r[i].y));
             psi_hat[off] = nv;
-            cur[c * LS + pos] = nv;
+            r[i] = nv;
         }
-        __syncthreads();
-        fx_line_exponent(cur, L, LS, li, lane, tpl, active, sm_e + C);
-        __syncthreads();
-        emax = active ? sm_e[C + li] : 0;
-        sh = fx_scale(emax, G);
-        double2 *other = (cur == A) ? B : A;
-        cur = static_cast<double2 *>(fx_fft_line<+1, true, true>(cur, other, L, log2L, LS, li, lane, tpl, active,
-                                                                 twf, wstep, sh,
-                                                                 emax == 2047 ? FX_NAN_SCALE : sh));
+        fx_col_fft<true>(r, ln, I, cur, oth, twf, sm_w[1]);
     }
-    for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-        int c, pos;
-        col_split(e, ncols, lg, c, pos);
-        const long long off = base + c + pos * elem_stride;
-        if(!CHGB_BC(101, off - species * hat, hat) || !CHGB_BC(102, c * LS + pos, C * LS)) continue;
-        double2 f = cur[c * LS + pos];
-        if(MODE == COL_FWD_DIV) {
+#pragma unroll
+    for(int i = 0; i < E; i++) {
+        const long long off = off0 + i * dT;
+        if(!active || i >= L || !CHGB_BC(101, off - species * hat, hat)) continue;
+        double2 f = r[i];
+        if(MODE == COL_INIT) {
+            psi_hat[off] = make_double2(f.x * scale, f.y * scale);
+        }
+        else if(MODE == COL_FWD_DIV) {
             if(ops.use_dealias) {
                 const double D = ops.dealias[off];
                 f.x *= D;
@@ -564,8 +532,8 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
             work[off] = f;
             if(MODE == COL_FWD_MU) {
                 const double t = ops.two_k * ops.q2[off];
-                const double2 r = ops.rho[off];
-                double2 v = make_double2(f.x + t * r.x, f.y + t * r.y);
+                const double2 q = ops.rho[off];
+                double2 v = make_double2(f.x + t * q.x, f.y + t * q.y);
                 if(ops.use_dealias) {
                     const double D = ops.dealias[off];
                     v.x *= D;
@@ -577,26 +545,27 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(1024) col_kernel(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
-                                                   const double *__restrict__ alpha, const double *__restrict__ beta,
-                                                   int L, int log2L, int H, int C, int tpl, long long elem_stride,
-                                                   long long plane_stride, long long hat,
-                                                   const int4 *__restrict__ twf, int wstep, double scale, ColOps ops) {
-    extern __shared__ double2 sm2[];
-    col_body<MODE>(work, psi_hat, alpha, beta, L, log2L, H, C, tpl, elem_stride, plane_stride, hat, twf, wstep, scale,
-                   blockIdx.x * C, blockIdx.y, blockIdx.z, sm2, ops);
+template <int MODE, int E>
+__global__ void __launch_bounds__(512, E == 4 ? 2 : 1) col_kernel(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
+                                                  const double *__restrict__ alpha, const double *__restrict__ beta,
+                                                  int lgL, int H, int lgC, long long elem_stride,
+                                                  long long plane_stride, long long hat,
+                                                  const int4 *__restrict__ twf, double scale, ColOps ops) {
+    extern __shared__ fx2 sm2[];
+    pdl_begin();
+    col_body<MODE, E>(work, psi_hat, alpha, beta, lgL, H, lgC, elem_stride, plane_stride, hat, twf, scale,
+                   (int) blockIdx.x << lgC, blockIdx.y, blockIdx.z, sm2, ops);
 }
 
 // Batched 2D column pass (forward, update, inverse) of one time step:
 // CTA b takes columns items[b].z.. of species items[b].y of replica items[b].x.
 __global__ void __launch_bounds__(256) col_batch_kernel(const PsBatchRep *__restrict__ reps,
                                                         const int4 *__restrict__ items) {
-    extern __shared__ double2 sm2[];
+    extern __shared__ fx2 sm2[];
     const int4 it = items[blockIdx.x];
     const PsBatchRep &r = reps[it.x];
-    col_body<COL_STEP>(r.work, r.psi_hat, r.alpha, r.beta, r.N, r.log2N, r.H, r.col_C, r.col_tpl, r.H, 0, r.hat, r.twf,
-                       1, 0.0, it.z, 0, it.y, sm2);
+    col_body<COL_STEP, FX_E_SMALL>(r.work, r.psi_hat, r.alpha, r.beta, r.log2N, r.H, r.log2C, r.H, 0, r.hat, r.twf, 0.0, it.z, 0,
+                       it.y, sm2);
 }
 
 // 1D: elementwise init (psi_t = F[rho] / N) or update on the half spectrum.
@@ -633,16 +602,18 @@ struct SpectralState {
     int H = 0;
     long long hat = 0;       // complex values per species
     double2 *psi_hat = nullptr, *work = nullptr;
-    int4 *twf = nullptr;      // the twiddles in fixed point (bfp.cuh): limbs of round(w 2^61)
+    int4 *twf = nullptr;      // the twiddles in fixed point (bfp.cuh): limbs of round(w 2^62)
     double *alpha = nullptr, *beta = nullptr;
     const double *real_buf = nullptr;  // the handle's real-space density buffer
     bool real_valid = false;  // the real buffer holds the current rho
     bool hat_valid = false;   // work holds the x-half-spectrum rows of the current rho
-    // launch shapes
-    int row_rpc = 1, row_tpl = 1, row_threads = 1;
+    // launch shapes: rows per row CTA, log2 of the columns per column CTA
+    int row_rpc = 1, row_threads = 1;
     size_t row_smem = 0;
-    int col_C = 1, col_tpl = 1, col_threads = 1;
+    int lgC = 0, col_threads = 1;
     size_t col_smem = 0;
+    bool pdl = true;          // programmatic dependent launch of the passes
+    int E = 8;                // values per thread of the line transforms
 };
 
 // Wave-vector tables of src/integrators/PseudospectralCPU.cpp:32-86, folded
@@ -702,16 +673,18 @@ static void build_tables(const SpectralState &s, std::vector<double> &alpha, std
     }
 }
 
-// One fixed-point twiddle component: W = round(v 2^61) as limbs (W >> 31, W mod 2^31).
+// One fixed-point twiddle component: W = round(v 2^62) = hi 2^32 + lo, both
+// signed (bfp.cuh).  lo = -2^31 becomes -2^31 + 1: the kernels negate limbs.
 static void fx_limbs(long double v, int &hi, int &lo) {
-    const long long W = llroundl(v * 2305843009213693952.0L);   // 2^61
-    hi = (int) (W >> 31);
-    lo = (int) (W & 0x7FFFFFFFll);
+    const long long W = llroundl(v * 4611686018427387904.0L);   // 2^62
+    lo = (int) (uint32_t) (W & 0xFFFFFFFFll);
+    hi = (int) ((W - lo) >> 32);
+    if(lo == INT32_MIN) lo = -INT32_MAX;
 }
 
 // W[q] = exp(-2 pi i q / N), q < N, in fixed point for the transforms of
 // bfp.cuh: built from one octant in long double so that the table is exactly
-// symmetric (W[N/4] = -i, W[N/2] = -1 exactly), then rounded to 2^-61.
+// symmetric (W[N/4] = -i, W[N/2] = -1 exactly), then rounded to 2^-62.
 static void build_twiddles(int N, std::vector<int4> &wf) {
     wf.resize(N);
     for(int q = 0; q < N; q++) {
@@ -756,13 +729,26 @@ static void build_twiddles(int N, std::vector<int4> &wf) {
 
 static void tune_col_shape(SpectralState *s);
 
-// Dynamic shared memory limit of every column-pass kernel.
-static void set_col_smem(size_t smem) {
-    for(const void *f : {(const void *) col_kernel<COL_FWD>, (const void *) col_kernel<COL_INV>,
-                         (const void *) col_kernel<COL_STEP>, (const void *) col_kernel<COL_INIT>,
-                         (const void *) col_kernel<COL_GRAD_INV>, (const void *) col_kernel<COL_FWD_DIV>,
-                         (const void *) col_kernel<COL_FWD_MU>, (const void *) col_kernel<COL_UPD_INV>})
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+// Values per thread of a box's line transforms: four where the box has too few
+// lines to fill the GPU's schedulers eight values to a thread (a shorter chain
+// for each warp), eight where it has not (fewer twiddle products and
+// exchanges).  Measured on GB300, us per pass: 2D N=256 Saleh (50 steps) 1406
+// with four, 1775 with eight; 3D N=128 (27 steps) 2618 with eight.
+static int fx_elems(const Geom &g) { return g.dims == 2 && g.N <= 1024 ? FX_E_SMALL : 8; }
+
+// Columns per CTA of the column passes.
+static void set_col_shape(SpectralState *s, int C) {
+    s->lgC = ilog2(C);
+    s->col_threads = C * fx_line_threads(s->g.N, s->E);
+    s->col_smem = sizeof(fx2) * 2 * (size_t) C * fx_line_size(s->g.N);
+}
+
+// Let a kernel take `smem` bytes of dynamic shared memory.  The limit is one of
+// the kernel, not of a handle: it is only ever set to the largest a CTA can
+// have beside the kernels' static arrays, so that no handle lowers another's.
+static cudaError_t allow_smem(const void *f, size_t smem) {
+    if(smem <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
 }
 
 int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, SpectralState **out, std::string &err) {
@@ -801,47 +787,54 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
         err = "table upload failed";
         return CHGB_ERR_CUDA;
     }
-    // launch shapes
+    s->E = fx_elems(g);
+    s->pdl = g.dims == 3;
+    // launch shapes.  A CTA takes at least a warp's worth of lines, then more up
+    // to 128 threads while ~2 CTAs per SM are left: small boxes want their few
+    // lines spread over as many SMs as possible
+    constexpr long long kSpreadCtas = 2 * 152;
     const int M = g.N / 2;
     const long long rows = (long long) g.bins / g.N;
-    s->row_tpl = std::max(1, std::min(M / 4, 256));
-    // rows per CTA: up to 128 threads, but never below ~2 CTAs per SM -- the
-    // FP64 pipe of each SM is the shared resource, so small boxes want their
-    // few rows spread over as many SMs as possible (2D N=256: 256 one-warp
-    // CTAs rather than 64 four-warp ones)
-    constexpr long long kSpreadCtas = 2 * 152;
+    const int row_T = fx_line_threads(M, s->E);
     s->row_rpc = 1;
-    while(s->row_rpc * 2 * s->row_tpl * g.S <= 128 && s->row_rpc * 2 <= rows &&
-          rows / (s->row_rpc * 2) >= kSpreadCtas)
+    while(s->row_rpc * 2 * row_T * g.S <= 128 && s->row_rpc * 2 <= rows &&
+          (s->row_rpc * row_T * g.S < 32 || rows / (s->row_rpc * 2) >= kSpreadCtas))
         s->row_rpc *= 2;
-    s->row_threads = s->row_rpc * g.S * s->row_tpl;
-    s->row_smem = sizeof(double2) * 2 * (size_t) s->row_rpc * g.S * (M + 1) + sizeof(int) * 2 * s->row_rpc * g.S;
-    const int L = g.N;
-    s->col_tpl = std::max(1, std::min(L / 4, 256));
-    // columns per CTA: the same rule (2D N=256: 129 CTAs of one column each)
+    s->row_threads = s->row_rpc * g.S * row_T;
+    s->row_smem = sizeof(fx2) * 2 * (size_t) (s->row_threads / row_T) * fx_line_size(M);
+    const int col_T = fx_line_threads(g.N, s->E);
     const long long col_lines = (long long) s->H * (g.dims == 3 ? g.N : 1) * g.S;
-    s->col_C = 1;
-    while(s->col_C * 2 * s->col_tpl <= 256 && s->col_C * 2 <= 8 && col_lines / (s->col_C * 2) >= kSpreadCtas)
-        s->col_C *= 2;
-    s->col_threads = s->col_C * s->col_tpl;
-    s->col_smem = sizeof(double2) * 2 * (size_t) s->col_C * L + sizeof(int) * 2 * s->col_C;
+    int C = 1;
+    while(C * 2 * col_T <= 256 && C * 2 <= FX_MAX_INTERLEAVE &&
+          (C * col_T < 32 || col_lines / (C * 2) >= kSpreadCtas))
+        C *= 2;
+    set_col_shape(s, C);
     // shared-memory attributes, once
-    auto setattr = [&](const void *f, size_t smem) {
-        if(smem > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
-    };
-#define SETROW(K)                                                                                   \
-    setattr((const void *) row_kernel<K, ROW_IN_REAL, false, false, true>, s->row_smem);            \
-    setattr((const void *) row_kernel<K, ROW_IN_REAL, true, false, true>, s->row_smem);             \
-    setattr((const void *) row_kernel<K, ROW_IN_HAT, true, false, true>, s->row_smem);              \
-    setattr((const void *) row_kernel<K, ROW_IN_HAT, false, true, false>, s->row_smem);             \
-    setattr((const void *) row_kernel<K, ROW_IN_HAT, true, true, true>, s->row_smem);              \
-    setattr((const void *) row_kernel<K, ROW_IN_HAT, false, false, true, FLUX_DM>, s->row_smem);    \
-    setattr((const void *) row_kernel<K, ROW_IN_HAT, false, false, true, FLUX_M>, s->row_smem);
-    SETROW(CHGB_MODEL_LANDAU)
-    SETROW(CHGB_MODEL_SIMPLE_WERTHEIM)
-    SETROW(CHGB_MODEL_SALEH)
+    auto setattr = [](const void *f, size_t smem) { allow_smem(f, smem); };
+#define SETROW(K, E)                                                                            \
+    setattr((const void *) row_kernel<K, E, ROW_IN_REAL, false, false, true>, s->row_smem);     \
+    setattr((const void *) row_kernel<K, E, ROW_IN_REAL, true, false, true>, s->row_smem);      \
+    setattr((const void *) row_kernel<K, E, ROW_IN_HAT, true, false, true>, s->row_smem);       \
+    setattr((const void *) row_kernel<K, E, ROW_IN_HAT, false, true, false>, s->row_smem);      \
+    setattr((const void *) row_kernel<K, E, ROW_IN_HAT, true, true, true>, s->row_smem);        \
+    setattr((const void *) row_kernel<K, E, ROW_IN_HAT, false, false, true, FLUX_DM>, s->row_smem); \
+    setattr((const void *) row_kernel<K, E, ROW_IN_HAT, false, false, true, FLUX_M>, s->row_smem);
+    SETROW(CHGB_MODEL_LANDAU, 8)
+    SETROW(CHGB_MODEL_SIMPLE_WERTHEIM, 8)
+    SETROW(CHGB_MODEL_SALEH, 8)
+    SETROW(CHGB_MODEL_LANDAU, 4)
+    SETROW(CHGB_MODEL_SIMPLE_WERTHEIM, 4)
+    SETROW(CHGB_MODEL_SALEH, 4)
 #undef SETROW
-    if(s->col_smem > 48 * 1024) set_col_smem(s->col_smem);
+    for(const void *f : {(const void *) col_kernel<COL_FWD, 8>, (const void *) col_kernel<COL_INV, 8>,
+                         (const void *) col_kernel<COL_STEP, 8>, (const void *) col_kernel<COL_INIT, 8>,
+                         (const void *) col_kernel<COL_GRAD_INV, 8>, (const void *) col_kernel<COL_FWD_DIV, 8>,
+                         (const void *) col_kernel<COL_FWD_MU, 8>, (const void *) col_kernel<COL_UPD_INV, 8>,
+                         (const void *) col_kernel<COL_FWD, 4>, (const void *) col_kernel<COL_INV, 4>,
+                         (const void *) col_kernel<COL_STEP, 4>, (const void *) col_kernel<COL_INIT, 4>,
+                         (const void *) col_kernel<COL_GRAD_INV, 4>, (const void *) col_kernel<COL_FWD_DIV, 4>,
+                         (const void *) col_kernel<COL_FWD_MU, 4>, (const void *) col_kernel<COL_UPD_INV, 4>})
+        setattr(f, 224 * 1024);   // whatever shape the timing below picks
     cudaError_t e = cudaGetLastError();
     if(e != cudaSuccess) {
         spectral_destroy(s);
@@ -863,29 +856,45 @@ void spectral_destroy(SpectralState *s) {
     delete s;
 }
 
+void spectral_set_pdl(SpectralState *s, bool on) { s->pdl = s->pdl && on; }
+
 namespace {
+
+// A pass as a programmatic dependent launch (pdl_begin in the kernels): the
+// next pass's CTAs are placed while the last ones of this pass drain.
+template <typename... Params, typename... Args>
+cudaError_t launch_pass(const SpectralState *s, void (*kernel)(Params...), dim3 grid, int threads, size_t smem,
+                        cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned) threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = s->pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
+dim3 row_grid(const SpectralState *s) { return dim3((unsigned) ((long long) s->g.bins / s->g.N / s->row_rpc)); }
 
 template <int KIND, int IN, bool FPRIME, bool WRITE_REAL, bool R2C>
 cudaError_t launch_row_kind(SpectralState *s, const double *real_in, double *real_out, cudaStream_t st) {
-    const int M = s->g.N / 2;
-    const long long rows = (long long) s->g.bins / s->g.N;
-    dim3 grid((unsigned) (rows / s->row_rpc));
-    row_kernel<KIND, IN, FPRIME, WRITE_REAL, R2C><<<grid, s->row_threads, s->row_smem, st>>>(
-        s->work, real_in, real_out, s->g.N, M, ilog2(M), s->row_rpc, s->row_tpl, s->g.bins, s->hat, s->twf, s->m,
-        nullptr, nullptr);
-    return cudaGetLastError();
+    auto kernel = s->E == 8 ? row_kernel<KIND, 8, IN, FPRIME, WRITE_REAL, R2C>
+                            : row_kernel<KIND, 4, IN, FPRIME, WRITE_REAL, R2C>;
+    return launch_pass(s, kernel, row_grid(s), s->row_threads, s->row_smem, st, s->work, real_in, real_out, ilog2(s->g.N) - 1, s->row_rpc, s->g.bins, s->hat, s->twf, s->m,
+                       nullptr, nullptr);
 }
 
 // Row pass of the variable-mobility flux: c2r of work's rows, the flux stage, r2c back into work.
 template <int KIND, int FLUX>
 cudaError_t launch_row_flux_kind(SpectralState *s, const double *mob, const double *M0, cudaStream_t st) {
-    const int M = s->g.N / 2;
-    const long long rows = (long long) s->g.bins / s->g.N;
-    dim3 grid((unsigned) (rows / s->row_rpc));
-    row_kernel<KIND, ROW_IN_HAT, false, false, true, FLUX><<<grid, s->row_threads, s->row_smem, st>>>(
-        s->work, nullptr, nullptr, s->g.N, M, ilog2(M), s->row_rpc, s->row_tpl, s->g.bins, s->hat, s->twf, s->m, mob,
-        M0);
-    return cudaGetLastError();
+    auto kernel = s->E == 8 ? row_kernel<KIND, 8, ROW_IN_HAT, false, false, true, FLUX>
+                            : row_kernel<KIND, 4, ROW_IN_HAT, false, false, true, FLUX>;
+    return launch_pass(s, kernel, row_grid(s), s->row_threads, s->row_smem, st, s->work, nullptr, nullptr, ilog2(s->g.N) - 1, s->row_rpc, s->g.bins, s->hat,
+                       s->twf, s->m, mob, M0);
 }
 
 template <int FLUX>
@@ -929,11 +938,11 @@ cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps
         plane_stride = H;
         planes = N;
     }
-    dim3 grid((unsigned) ((H + s->col_C - 1) / s->col_C), (unsigned) planes, (unsigned) s->g.S);
-    col_kernel<MODE><<<grid, s->col_threads, s->col_smem, st>>>(s->work, s->psi_hat, s->alpha, s->beta, N, ilog2(N),
-                                                               H, s->col_C, s->col_tpl, elem_stride, plane_stride,
-                                                               s->hat, s->twf, 1, 1.0 / (double) s->g.bins, ops);
-    return cudaGetLastError();
+    const int C = 1 << s->lgC;
+    auto kernel = s->E == 8 ? col_kernel<MODE, 8> : col_kernel<MODE, 4>;
+    return launch_pass(s, kernel, dim3((unsigned) ((H + C - 1) / C), (unsigned) planes, (unsigned) s->g.S),
+                       s->col_threads, s->col_smem, st, s->work, s->psi_hat, s->alpha, s->beta, ilog2(N), H, s->lgC,
+                       elem_stride, plane_stride, s->hat, s->twf, 1.0 / (double) s->g.bins, ops);
 }
 
 }  // namespace
@@ -958,29 +967,17 @@ static void tune_col_shape(SpectralState *s) {
         if(st) cudaStreamDestroy(st);
         return;
     }
-    const int L = s->g.N, axis = s->g.dims - 1;
+    const int axis = s->g.dims - 1;
     const long long nd = s->hat * s->g.S * 2;   // doubles of psi_hat / work
-    const int C0 = s->col_C, T0 = s->col_threads;
-    const size_t M0 = s->col_smem;
-    int bestC = C0, bestT = T0;
-    size_t bestM = M0;
+    const int C0 = 1 << s->lgC;
+    int bestC = C0;
     float best = 0.0f;
     bool ok = launch_fill_noise(reinterpret_cast<double *>(s->psi_hat), 0.0, 1e-2, nd, st) == cudaSuccess &&
               launch_fill_noise(reinterpret_cast<double *>(s->work), 0.0, 1e-2, nd, st) == cudaSuccess;
-    for(int C : {1, 2, 4}) {
+    for(int C : {1, 2, 4, 8}) {
         if(!ok) break;
-        const int threads = C * s->col_tpl;
-        const size_t smem = sizeof(double2) * 2 * (size_t) C * L + sizeof(int) * 2 * C;
-        if(threads > 1024 || smem > 227 * 1024) continue;
-        if(smem > 48 * 1024 &&
-           cudaFuncSetAttribute(col_kernel<COL_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) !=
-               cudaSuccess) {
-            cudaGetLastError();
-            continue;
-        }
-        s->col_C = C;
-        s->col_threads = threads;
-        s->col_smem = smem;
+        set_col_shape(s, C);
+        if(s->col_threads > 512 || s->col_threads < 32 || s->col_smem > 224 * 1024) continue;
         cudaError_t e = launch_col<COL_STEP>(s, axis, st);   // warm-up
         if(e == cudaSuccess) e = cudaEventRecord(ev0, st);
         for(int r = 0; r < 5 && e == cudaSuccess; r++) e = launch_col<COL_STEP>(s, axis, st);
@@ -995,14 +992,9 @@ static void tune_col_shape(SpectralState *s) {
         if(best == 0.0f || ms < best) {
             best = ms;
             bestC = C;
-            bestT = threads;
-            bestM = smem;
         }
     }
-    s->col_C = bestC;
-    s->col_threads = bestT;
-    s->col_smem = bestM;
-    if(bestM > 48 * 1024) set_col_smem(bestM);
+    set_col_shape(s, bestC);
     cudaMemsetAsync(s->psi_hat, 0, sizeof(double) * nd, st);
     cudaMemsetAsync(s->work, 0, sizeof(double) * nd, st);
     cudaStreamSynchronize(st);
@@ -1123,29 +1115,24 @@ void spectral_batch_rep(const SpectralState *s, PsBatchRep *r, size_t *row_smem,
     r->twf = s->twf;
     r->m = s->m;
     r->N = N;
-    r->M = M;
-    r->log2M = ilog2(M);
     r->log2N = ilog2(N);
     r->H = s->H;
     r->bins = s->g.bins;
     r->hat = s->hat;
-    r->row_tpl = std::max(1, std::min(M / 4, 64));
+    const int row_T = fx_line_threads(M, FX_E_SMALL), col_T = fx_line_threads(N, FX_E_SMALL);
     r->row_rpc = 1;
-    while(r->row_rpc * 2 * r->row_tpl * S <= PS_BATCH_THREADS && r->row_rpc * 2 <= N) r->row_rpc *= 2;
-    r->col_tpl = std::max(1, std::min(N / 4, 64));
-    r->col_C = std::max(1, std::min(PS_BATCH_THREADS / r->col_tpl, 16));
-    *row_smem = sizeof(double2) * 2 * (size_t) r->row_rpc * S * (M + 1) + sizeof(int) * 2 * r->row_rpc * S;
-    *col_smem = sizeof(double2) * 2 * (size_t) r->col_C * N + sizeof(int) * 2 * r->col_C;
+    while(r->row_rpc * 2 * row_T * S <= PS_BATCH_THREADS && r->row_rpc * 2 <= N) r->row_rpc *= 2;
+    r->col_C = std::max(1, std::min(PS_BATCH_THREADS / col_T, 16));
+    r->log2C = ilog2(r->col_C);
+    *row_smem = sizeof(fx2) * 2 * (size_t) (PS_BATCH_THREADS / row_T) * fx_line_size(M);
+    *col_smem = sizeof(fx2) * 2 * (size_t) (PS_BATCH_THREADS / col_T) * fx_line_size(N);
 }
 
 namespace {
 template <int KIND>
 cudaError_t configure_kind(size_t row_smem, size_t col_smem) {
-    cudaError_t e = cudaSuccess;
-    if(row_smem > 48 * 1024)
-        e = cudaFuncSetAttribute(row_batch_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) row_smem);
-    if(e == cudaSuccess && col_smem > 48 * 1024)
-        e = cudaFuncSetAttribute(col_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) col_smem);
+    cudaError_t e = allow_smem((const void *) row_batch_kernel<KIND>, row_smem);
+    if(e == cudaSuccess) e = allow_smem((const void *) col_batch_kernel, col_smem);
     return e;
 }
 }  // namespace
@@ -1206,8 +1193,13 @@ namespace {
 
 // Sum over the block; the result is valid in thread 0.
 __device__ __forceinline__ double block_sum(double v, double *red) {
-    for(int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    const int n = min(32, (int) blockDim.x - w * 32);
+    const unsigned mask = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+    for(int o = 16; o > 0; o >>= 1) {
+        const double t = __shfl_down_sync(mask, v, o);
+        if(lane + o < n) v += t;
+    }
     __syncthreads();
     if(lane == 0) red[w] = v;
     __syncthreads();
@@ -1219,91 +1211,34 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
 
 // Row pass of the adjoint step: work rows (x half spectrum of beta lam_hat after
 // the inverse y transform) -> C2R -> B lam; geps += <B lam, psi_n>; * f''(psi_n) -> R2C.
-__global__ void __launch_bounds__(1024) row_adj_kernel(double2 *__restrict__ work, const double *__restrict__ psi_n,
-                                                      int N, int M, int log2M, int rows_per_cta, int tpl,
-                                                      const int4 *__restrict__ twf, double eps,
-                                                      double *__restrict__ geps) {
-    extern __shared__ double2 sm2[];
+__global__ void __launch_bounds__(256) row_adj_kernel(double2 *__restrict__ work, const double *__restrict__ psi_n,
+                                                     int lgM, int rows_per_cta, const int4 *__restrict__ twf,
+                                                     double eps, double *__restrict__ geps) {
+    extern __shared__ fx2 sm2[];
     __shared__ double red[32];
-    const int LS = M + 1, H = M + 1;
-    const int lines = rows_per_cta;
-    double2 *A = sm2;
-    double2 *B = sm2 + lines * LS;
-    int *sm_e = reinterpret_cast<int *>(sm2 + 2 * lines * LS);   // exponents: c2r input, r2c input
-    const int li = threadIdx.x / tpl, lane = threadIdx.x - li * tpl;
-    const bool active = li < lines;
-    const long long row = (long long) blockIdx.x * rows_per_cta + (active ? li : 0);
-    const int G = log2M + 3;
-    if(active && lane == 0) {
-        sm_e[li] = 0;
-        sm_e[lines + li] = 0;
-    }
-    int e = 0;
-    if(active) {
-        const double2 *src = work + row * H;
-        for(int k = lane; k < H; k += tpl) {
-            const double2 v = src[k];
-            B[li * LS + k] = v;
-            e = max(e, max(fx_expo(v.x), fx_expo(v.y)));
-        }
-    }
-    __syncthreads();
-    fx_line_max(e, tpl, li, lane, active, sm_e);
-    __syncthreads();
-    int emax = active ? sm_e[li] : 0;
-    int sh = fx_scale(emax, G);
-    // c2r pre-processing in fixed point, as the forward row pass
-    if(active) {
-        const double2 *X = B + li * LS;
-        fx2 *Z = reinterpret_cast<fx2 *>(A + li * LS);
-        for(int k = lane; k < M; k += tpl) {
-            const fx2 xk = fx_load(X[k], sh);
-            fx2 xc = fx_load(X[M - k], sh);
-            xc.y = -xc.y;
-            const fx2 e2 = fx_add(xk, xc);
-            const fx2 t = fx_cmul<true>(fx_sub(xk, xc), twf[k]);
-            Z[k] = fx2{e2.x - t.y, e2.y + t.x};
-        }
-    }
-    __syncthreads();
-    double2 *cur = static_cast<double2 *>(fx_fft_line<+1, false, true>(A, B, M, log2M, LS, li, lane, tpl, active, twf,
-                                                                       2, 0, emax == 2047 ? FX_NAN_SCALE : sh));
-    double2 *other = (cur == A) ? B : A;
+    __shared__ int sm_w[2][FX_MAX_WARPS];
+    constexpr int E = FX_E_SMALL;
+    const FxLine ln = fx_line<E>(lgM, 0, false);
+    const int M = 1 << lgM, N = 2 * M, LS = fx_line_size(M);
+    const int li = threadIdx.x / ln.T, nl = blockDim.x / ln.T;
+    const long long row = (long long) blockIdx.x * rows_per_cta + li;
+    fx2 *cur = sm2 + li * LS, *oth = sm2 + (nl + li) * LS;
+    double2 r[E];
+    fx_row_c2r(r, work + row * (M + 1), true, ln, cur, oth, twf, sm_w[0]);
     double acc = 0.0;
-    if(active) {
-        const double2 *pr = reinterpret_cast<const double2 *>(psi_n + row * N);
-        for(int n = lane; n < M; n += tpl) {
-            double2 b = cur[li * LS + n];
-            double2 p = pr[n];
+    const double2 *pr = reinterpret_cast<const double2 *>(psi_n + row * N);
+#pragma unroll
+    for(int i = 0; i < E; i++) {
+        if(i < M) {
+            const double2 b = r[i], p = pr[ln.lane + i * ln.T];
             acc = fma(b.x, p.x, acc);
             acc = fma(b.y, p.y, acc);
-            cur[li * LS + n] = make_double2(b.x * fma(3.0 * p.x, p.x, -eps), b.y * fma(3.0 * p.y, p.y, -eps));
+            r[i] = make_double2(b.x * fma(3.0 * p.x, p.x, -eps), b.y * fma(3.0 * p.y, p.y, -eps));
         }
     }
-    double t = block_sum(acc, red);
+    const double t = block_sum(acc, red);
     if(threadIdx.x == 0) geps[blockIdx.x] += t;
-    __syncthreads();
-    fx_line_exponent(cur, M, LS, li, lane, tpl, active, sm_e + lines);
-    __syncthreads();
-    emax = active ? sm_e[lines + li] : 0;
-    sh = fx_scale(emax, G);
-    const fx2 *Z = static_cast<const fx2 *>(
-                       fx_fft_line<-1, true, false>(cur, other, M, log2M, LS, li, lane, tpl, active, twf, 2, sh, 0)) +
-                   li * LS;
-    if(active) {
-        const int sh_out = emax == 2047 ? FX_NAN_SCALE : sh + 1;
-        double2 *dst = work + row * H;
-        for(int k = lane; k <= M; k += tpl) {
-            const fx2 zk = Z[k == M ? 0 : k];
-            fx2 zc = Z[k == 0 ? 0 : M - k];
-            zc.y = -zc.y;
-            const fx2 a = fx_add(zk, zc), bb = fx_sub(zk, zc);
-            const fx2 tt = fx_cmul<false>(fx2{bb.y, -bb.x}, twf[k]);
-            double2 xk = fx_out(fx_add(a, tt), sh_out);
-            if(k == 0 || k == M) xk.y = 0.0;
-            dst[k] = xk;
-        }
-    }
+    fx_row_r2c(r, work + row * (M + 1), true, ln, cur, oth, twf, sm_w[1]);
 }
 
 enum { ADJ_A = 1, ADJ_B = 2, ADJ_BA = 3 };
@@ -1312,100 +1247,66 @@ enum { ADJ_A = 1, ADJ_B = 2, ADJ_BA = 3 };
 // update) and/or A part (gradient sums with psi_next = psi_t_{n+1} and
 // psi_cur = psi_t_n, then beta * lam_hat and the inverse y FFT into work).
 template <int MODE>
-__global__ void __launch_bounds__(1024) col_adj_kernel(double2 *__restrict__ work, double2 *__restrict__ lam,
-                                                      const double *__restrict__ alpha, const double *__restrict__ beta,
-                                                      const double *__restrict__ tk, const double *__restrict__ tm1,
-                                                      const double *__restrict__ tm2,
-                                                      const double2 *__restrict__ psi_next,
-                                                      const double2 *__restrict__ psi_cur, int L, int log2L, int H,
-                                                      int C, int tpl, const int4 *__restrict__ twf,
-                                                      double *__restrict__ gk, double *__restrict__ gm) {
-    extern __shared__ double2 sm2[];
+__global__ void __launch_bounds__(256) col_adj_kernel(double2 *__restrict__ work, double2 *__restrict__ lam,
+                                                     const double *__restrict__ alpha, const double *__restrict__ beta,
+                                                     const double *__restrict__ tk, const double *__restrict__ tm1,
+                                                     const double *__restrict__ tm2,
+                                                     const double2 *__restrict__ psi_next,
+                                                     const double2 *__restrict__ psi_cur, int lgL, int H, int lgC,
+                                                     const int4 *__restrict__ twf, double *__restrict__ gk,
+                                                     double *__restrict__ gm) {
+    extern __shared__ fx2 sm2[];
     __shared__ double red[32];
-    const int LS = L;
-    double2 *A = sm2;
-    double2 *B = sm2 + C * LS;
-    int *sm_e = reinterpret_cast<int *>(sm2 + 2 * C * LS);   // exponents: forward input, inverse input
-    const int li = threadIdx.x / tpl, lane = threadIdx.x - li * tpl;
-    const int kx0 = blockIdx.x * C;
-    const int ncols = min(C, H - kx0);
-    const int lg = col_log2(ncols);
-    const bool active = li < ncols;
-    const int nthr = blockDim.x;
-    const int G = log2L + 1;
-    if(active && lane == 0) {
-        sm_e[li] = 0;
-        sm_e[C + li] = 0;
-    }
-    double2 *cur = A;
+    __shared__ int sm_w[2][FX_MAX_WARPS * FX_MAX_INTERLEAVE];
+    const int C = 1 << lgC;   // at most FX_MAX_INTERLEAVE: one group
+    constexpr int E = FX_E_SMALL;
+    const FxLine ln = fx_line<E>(lgL, lgC, false);
+    const int L = 1 << lgL;
+    const int kx = blockIdx.x * C + ln.c;
+    const bool active = kx < H;
+    fx2 *cur = sm2, *oth = sm2 + (fx_line_size(L) << lgC);
+    const long long off0 = kx + (long long) ln.lane * H, dT = (long long) ln.T * H;
+    double2 r[E];
+#pragma unroll
+    for(int i = 0; i < E; i++)
+        r[i] = (active && i < L) ? ((MODE & ADJ_B) ? work : lam)[off0 + i * dT] : make_double2(0.0, 0.0);
     if(MODE & ADJ_B) {
-        for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-            int c, pos;
-            col_split(e, ncols, lg, c, pos);
-            A[c * LS + pos] = work[kx0 + c + (long long) pos * H];
+        fx_col_fft<false>(r, ln, C, cur, oth, twf, sm_w[0]);
+#pragma unroll
+        for(int i = 0; i < E; i++) {
+            if(active && i < L) {
+                const long long off = off0 + i * dT;
+                const double2 l = lam[off];
+                const double al = alpha[off];
+                r[i] = make_double2(fma(al, l.x, -r[i].x), fma(al, l.y, -r[i].y));
+                lam[off] = r[i];
+            }
         }
-        __syncthreads();
-        fx_line_exponent(A, L, LS, li, lane, tpl, active, sm_e);
-        __syncthreads();
-        const int emax = active ? sm_e[li] : 0;
-        const int sh = fx_scale(emax, G);
-        cur = static_cast<double2 *>(fx_fft_line<-1, true, true>(A, B, L, log2L, LS, li, lane, tpl, active, twf, 1,
-                                                                 sh, emax == 2047 ? FX_NAN_SCALE : sh));
-        for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-            int c, pos;
-            col_split(e, ncols, lg, c, pos);
-            long long off = kx0 + c + (long long) pos * H;
-            double2 q = cur[c * LS + pos];
-            double2 l = lam[off];
-            double al = alpha[off];
-            double2 nv = make_double2(fma(al, l.x, -q.x), fma(al, l.y, -q.y));
-            lam[off] = nv;
-            cur[c * LS + pos] = nv;
-        }
-        __syncthreads();
-    }
-    else {
-        for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-            int c, pos;
-            col_split(e, ncols, lg, c, pos);
-            A[c * LS + pos] = lam[kx0 + c + (long long) pos * H];
-        }
-        __syncthreads();
     }
     if(MODE & ADJ_A) {
         double ak = 0.0, am = 0.0;
-        for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-            int c, pos;
-            col_split(e, ncols, lg, c, pos);
-            int kx = kx0 + c;
-            long long off = kx + (long long) pos * H;
-            double2 l = cur[c * LS + pos];
-            double2 pn = psi_next[off], pc = psi_cur[off];
-            double w = (kx == 0 || kx == L / 2) ? 1.0 : 2.0;
-            double dn = fma(l.x, pn.x, l.y * pn.y);
-            double dc = fma(l.x, pc.x, l.y * pc.y);
-            ak = fma(w * tk[off], dn, ak);
-            am = fma(w, fma(tm1[off], dn, -tm2[off] * dc), am);
-            double be = beta[off];
-            cur[c * LS + pos] = make_double2(be * l.x, be * l.y);
+        const double w = (kx == 0 || kx == L / 2) ? 1.0 : 2.0;
+#pragma unroll
+        for(int i = 0; i < E; i++) {
+            if(active && i < L) {
+                const long long off = off0 + i * dT;
+                const double2 l = r[i], pn = psi_next[off], pc = psi_cur[off];
+                const double dn = fma(l.x, pn.x, l.y * pn.y);
+                const double dc = fma(l.x, pc.x, l.y * pc.y);
+                ak = fma(w * tk[off], dn, ak);
+                am = fma(w, fma(tm1[off], dn, -tm2[off] * dc), am);
+                const double be = beta[off];
+                r[i] = make_double2(be * l.x, be * l.y);
+            }
         }
         double t = block_sum(ak, red);
         if(threadIdx.x == 0) gk[blockIdx.x] += t;
         t = block_sum(am, red);
         if(threadIdx.x == 0) gm[blockIdx.x] += t;
-        __syncthreads();
-        fx_line_exponent(cur, L, LS, li, lane, tpl, active, sm_e + C);
-        __syncthreads();
-        const int emax = active ? sm_e[C + li] : 0;
-        const int sh = fx_scale(emax, G);
-        double2 *other = (cur == A) ? B : A;
-        cur = static_cast<double2 *>(fx_fft_line<+1, true, true>(cur, other, L, log2L, LS, li, lane, tpl, active, twf,
-                                                                 1, sh, emax == 2047 ? FX_NAN_SCALE : sh));
-        for(int e = threadIdx.x; e < ncols * L; e += nthr) {
-            int c, pos;
-            col_split(e, ncols, lg, c, pos);
-            work[kx0 + c + (long long) pos * H] = cur[c * LS + pos];
-        }
+        fx_col_fft<true>(r, ln, C, cur, oth, twf, sm_w[1]);
+#pragma unroll
+        for(int i = 0; i < E; i++)
+            if(active && i < L) work[off0 + i * dT] = r[i];
     }
 }
 
@@ -1451,7 +1352,7 @@ SpectralAdj *spectral_adj_create(SpectralState *s, std::string &err) {
         }
     }
     a->n_row_cta = (int) (((long long) s->g.bins / N) / s->row_rpc);
-    a->n_col_cta = (s->H + s->col_C - 1) / s->col_C;
+    a->n_col_cta = (s->H + (1 << s->lgC) - 1) >> s->lgC;
     bool ok = cudaMalloc(&a->tk, sizeof(double) * s->hat) == cudaSuccess &&
               cudaMalloc(&a->tm1, sizeof(double) * s->hat) == cudaSuccess &&
               cudaMalloc(&a->tm2, sizeof(double) * s->hat) == cudaSuccess &&
@@ -1465,12 +1366,10 @@ SpectralAdj *spectral_adj_create(SpectralState *s, std::string &err) {
          cudaMemcpy(a->tm2, tm2.data(), sizeof(double) * s->hat, cudaMemcpyHostToDevice) == cudaSuccess;
     if(ok) {
         size_t rs = s->row_smem, cs = s->col_smem;
-        if(rs > 48 * 1024) cudaFuncSetAttribute(row_adj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rs);
-        if(cs > 48 * 1024) {
-            cudaFuncSetAttribute(col_adj_kernel<ADJ_A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) cs);
-            cudaFuncSetAttribute(col_adj_kernel<ADJ_B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) cs);
-            cudaFuncSetAttribute(col_adj_kernel<ADJ_BA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) cs);
-        }
+        allow_smem((const void *) row_adj_kernel, rs);
+        allow_smem((const void *) col_adj_kernel<ADJ_A>, cs);
+        allow_smem((const void *) col_adj_kernel<ADJ_B>, cs);
+        allow_smem((const void *) col_adj_kernel<ADJ_BA>, cs);
         ok = cudaGetLastError() == cudaSuccess;
     }
     if(!ok) {
@@ -1518,8 +1417,8 @@ cudaError_t spectral_adj_col(SpectralAdj *a, SpectralState *s, int mode, const d
     const int N = s->g.N;
     dim3 grid((unsigned) a->n_col_cta);
 #define ADJ_COL_ARGS                                                                                                   \
-    a->work, a->lam, s->alpha, s->beta, a->tk, a->tm1, a->tm2, psi_next, psi_cur, N, ilog2(N), s->H, s->col_C,         \
-        s->col_tpl, s->twf, a->gk, a->gm
+    a->work, a->lam, s->alpha, s->beta, a->tk, a->tm1, a->tm2, psi_next, psi_cur, ilog2(N), s->H, s->lgC, s->twf,      \
+        a->gk, a->gm
     if(mode == ADJ_A) col_adj_kernel<ADJ_A><<<grid, s->col_threads, s->col_smem, st>>>(ADJ_COL_ARGS);
     else if(mode == ADJ_B) col_adj_kernel<ADJ_B><<<grid, s->col_threads, s->col_smem, st>>>(ADJ_COL_ARGS);
     else col_adj_kernel<ADJ_BA><<<grid, s->col_threads, s->col_smem, st>>>(ADJ_COL_ARGS);
@@ -1528,9 +1427,8 @@ cudaError_t spectral_adj_col(SpectralAdj *a, SpectralState *s, int mode, const d
 }
 
 cudaError_t spectral_adj_row(SpectralAdj *a, SpectralState *s, const double *psi_n, cudaStream_t st) {
-    const int M = s->g.N / 2;
-    row_adj_kernel<<<a->n_row_cta, s->row_threads, s->row_smem, st>>>(a->work, psi_n, s->g.N, M, ilog2(M), s->row_rpc,
-                                                                       s->row_tpl, s->twf, s->m.epsilon, a->geps);
+    row_adj_kernel<<<a->n_row_cta, s->row_threads, s->row_smem, st>>>(a->work, psi_n, ilog2(s->g.N) - 1, s->row_rpc,
+                                                                       s->twf, s->m.epsilon, a->geps);
     return cudaGetLastError();
 }
 

@@ -14,6 +14,8 @@ struct SpectralState;
 // Allocate the spectral state of one box (rho_hat, wave-vector tables, scratch).
 int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, SpectralState **out, std::string &err);
 void spectral_destroy(SpectralState *s);
+// Whether the passes are programmatic dependent launches (the default).
+void spectral_set_pdl(SpectralState *s, bool on);
 // rho_hat = FFT(rho) (src/integrators/PseudospectralCPU.cpp:95-101); rho is a device field.
 int spectral_set_rho(SpectralState *s, const double *d_rho, cudaStream_t st, int64_t *launches, std::string &err);
 // nsteps semi-implicit steps (src/integrators/PseudospectralCPU.cpp:112-136).
@@ -82,9 +84,9 @@ struct PsBatchRep {
     const double *alpha, *beta;
     const int4 *twf;        // fixed-point twiddles (bfp.cuh)
     ModelDev m;
-    int N, M, log2M, log2N, H;
-    int row_rpc, row_tpl;   // rows per CTA, threads per row line
-    int col_C, col_tpl;     // columns per CTA, threads per column line
+    int N, log2N, H;
+    int row_rpc;            // rows per CTA
+    int col_C, log2C;       // columns per CTA
     long long bins, hat;
 };
 constexpr int PS_BATCH_THREADS = 256;
