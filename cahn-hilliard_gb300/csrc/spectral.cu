@@ -57,7 +57,6 @@ namespace {
 // interleaved in groups of at most FX_MAX_INTERLEAVE.
 constexpr int FX_MAX_INTERLEAVE = 8;
 constexpr int FX_MAX_WARPS = 32;
-constexpr int FX_E_SMALL = 4;
 
 inline int fx_line_threads(int L, int E) { return L > E ? L / E : 1; }
 
@@ -381,7 +380,7 @@ __global__ void __launch_bounds__(256) row_batch_kernel(const PsBatchRep *__rest
     extern __shared__ fx2 sm2[];
     const int2 it = items[blockIdx.x];
     const PsBatchRep &r = reps[it.x];
-    row_body<KIND, FX_E_SMALL, ROW_IN_HAT, true, false, true>(r.work, nullptr, nullptr, r.log2N - 1, r.row_rpc, r.bins, r.hat,
+    row_body<KIND, PS_BATCH_ROW_E, ROW_IN_HAT, true, false, true>(r.work, nullptr, nullptr, r.log2N - 1, r.row_rpc, r.bins, r.hat,
                                                   r.twf, r.m, it.y, sm2);
 }
 
@@ -438,8 +437,7 @@ __device__ __forceinline__ void fx_col_fft(double2 (&r)[E], const FxLine &ln, in
 // The shared memory holds two buffers of C lines.
 template <int MODE, int E>
 __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
-                                         const double *__restrict__ alpha, const double *__restrict__ beta, int lgL,
-                                         int H, int lgC, long long elem_stride, long long plane_stride, long long hat,
+                                         const double2 *__restrict__ ab, int lgL, int H, int lgC, long long elem_stride, long long plane_stride, long long hat,
                                          const int4 *__restrict__ twf, double scale, int kx0, long long plane,
                                          long long species, fx2 *sm, const ColOps &ops = ColOps()) {
     __shared__ int sm_w[2][FX_MAX_WARPS * FX_MAX_INTERLEAVE];
@@ -497,9 +495,8 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
         for(int i = 0; i < E; i++) {
             const long long off = off0 + i * dT;
             if(!active || i >= L || !CHGB_BC(101, off - species * hat, hat)) continue;
-            const double2 ph = psi_hat[off];
-            const double al = alpha[off], be = beta[off];
-            const double2 nv = make_double2(fma(al, ph.x, -be * r[i].x), fma(al, ph.y, -be * r[i].y));
+            const double2 ph = psi_hat[off], c = ab[off];
+            const double2 nv = make_double2(fma(c.x, ph.x, -c.y * r[i].x), fma(c.x, ph.y, -c.y * r[i].y));
             psi_hat[off] = nv;
             r[i] = nv;
         }
@@ -547,31 +544,31 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
 
 template <int MODE, int E>
 __global__ void __launch_bounds__(512, E == 4 ? 2 : 1) col_kernel(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
-                                                  const double *__restrict__ alpha, const double *__restrict__ beta,
-                                                  int lgL, int H, int lgC, long long elem_stride,
+                                                  const double2 *__restrict__ ab, int lgL, int H, int lgC,
+                                                  long long elem_stride,
                                                   long long plane_stride, long long hat,
                                                   const int4 *__restrict__ twf, double scale, ColOps ops) {
     extern __shared__ fx2 sm2[];
     pdl_begin();
-    col_body<MODE, E>(work, psi_hat, alpha, beta, lgL, H, lgC, elem_stride, plane_stride, hat, twf, scale,
+    col_body<MODE, E>(work, psi_hat, ab, lgL, H, lgC, elem_stride, plane_stride, hat, twf, scale,
                    (int) blockIdx.x << lgC, blockIdx.y, blockIdx.z, sm2, ops);
 }
 
 // Batched 2D column pass (forward, update, inverse) of one time step:
 // CTA b takes columns items[b].z.. of species items[b].y of replica items[b].x.
-__global__ void __launch_bounds__(256) col_batch_kernel(const PsBatchRep *__restrict__ reps,
-                                                        const int4 *__restrict__ items) {
+template <int E>
+__global__ void __launch_bounds__(256, E == 4 ? 4 : 2) col_batch_kernel(const PsBatchRep *__restrict__ reps,
+                                                                       const int4 *__restrict__ items) {
     extern __shared__ fx2 sm2[];
     const int4 it = items[blockIdx.x];
     const PsBatchRep &r = reps[it.x];
-    col_body<COL_STEP, FX_E_SMALL>(r.work, r.psi_hat, r.alpha, r.beta, r.log2N, r.H, r.log2C, r.H, 0, r.hat, r.twf, 0.0, it.z, 0,
-                       it.y, sm2);
+    col_body<COL_STEP, E>(r.work, r.psi_hat, r.ab, r.log2N, r.H, r.log2C, r.H, 0, r.hat, r.twf, 0.0, it.z, 0, it.y,
+                          sm2);
 }
 
 // 1D: elementwise init (psi_t = F[rho] / N) or update on the half spectrum.
 __global__ void update1d_kernel(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
-                                const double *__restrict__ alpha, const double *__restrict__ beta, long long n,
-                                int init, double scale) {
+                                const double2 *__restrict__ ab, long long n, int init, double scale) {
     for(long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < n; i += (long long) gridDim.x * blockDim.x) {
         double2 f = work[i];
         if(init) {
@@ -579,8 +576,8 @@ __global__ void update1d_kernel(double2 *__restrict__ work, double2 *__restrict_
         }
         else {
             double2 ph = psi_hat[i];
-            double al = alpha[i], be = beta[i];
-            double2 nv = make_double2(fma(al, ph.x, -be * f.x), fma(al, ph.y, -be * f.y));
+            const double2 c = ab[i];
+            double2 nv = make_double2(fma(c.x, ph.x, -c.y * f.x), fma(c.x, ph.y, -c.y * f.y));
             psi_hat[i] = nv;
             work[i] = nv;
         }
@@ -595,6 +592,12 @@ int ilog2(int n) {
 
 }  // namespace
 
+// A column pass's launch shape: values per thread, log2 of the columns per CTA.
+struct ColShape {
+    int E = 8, lgC = 0, threads = 1;
+    size_t smem = 0;
+};
+
 struct SpectralState {
     chgb_params p;
     Geom g;
@@ -603,22 +606,21 @@ struct SpectralState {
     long long hat = 0;       // complex values per species
     double2 *psi_hat = nullptr, *work = nullptr;
     int4 *twf = nullptr;      // the twiddles in fixed point (bfp.cuh): limbs of round(w 2^62)
-    double *alpha = nullptr, *beta = nullptr;
+    double2 *ab = nullptr;    // the update's coefficients (alpha, beta) of every mode
     const double *real_buf = nullptr;  // the handle's real-space density buffer
     bool real_valid = false;  // the real buffer holds the current rho
     bool hat_valid = false;   // work holds the x-half-spectrum rows of the current rho
-    // launch shapes: rows per row CTA, log2 of the columns per column CTA
+    // launch shapes: rows per row CTA; the column passes, and COL_STEP's
     int row_rpc = 1, row_threads = 1;
     size_t row_smem = 0;
-    int lgC = 0, col_threads = 1;
-    size_t col_smem = 0;
+    ColShape col, step;
     bool pdl = true;          // programmatic dependent launch of the passes
-    int E = 8;                // values per thread of the line transforms
+    int row_E = 8;            // values per thread of the row transforms
 };
 
 // Wave-vector tables of src/integrators/PseudospectralCPU.cpp:32-86, folded
 // into the update coefficients.
-static void build_tables(const SpectralState &s, std::vector<double> &alpha, std::vector<double> &beta) {
+static void build_tables(const SpectralState &s, std::vector<double2> &ab) {
     const int N = s.g.N, dims = s.g.dims, S = s.g.S;
     const double dx = s.p.dx, dt = s.p.dt, M = s.p.M, Ssplit = s.p.splitting_S;
     const double bins = (double) s.g.bins;
@@ -659,16 +661,14 @@ static void build_tables(const SpectralState &s, std::vector<double> &alpha, std
             }
         }
     }
-    alpha.resize((size_t) S * s.hat);
-    beta.resize((size_t) S * s.hat);
+    ab.resize((size_t) S * s.hat);
     for(int sp = 0; sp < S; sp++) {
         for(long long i = 0; i < s.hat; i++) {
             double k2 = k2v[i], k4 = k2 * k2;
             double denom = 1.0 + dt * M * (Ssplit * k2 + 2.0 * s.p.k[sp] * k4);
             double c = dt * M * k2;
             double dm = s.p.use_dealias ? mask[i] : 1.0;
-            alpha[sp * s.hat + i] = (1.0 + c * Ssplit) / denom;
-            beta[sp * s.hat + i] = c * dm / denom / bins;
+            ab[sp * s.hat + i] = make_double2((1.0 + c * Ssplit) / denom, c * dm / denom / bins);
         }
     }
 }
@@ -732,15 +732,24 @@ static void tune_col_shape(SpectralState *s);
 // Values per thread of a box's line transforms: four where the box has too few
 // lines to fill the GPU's schedulers eight values to a thread (a shorter chain
 // for each warp), eight where it has not (fewer twiddle products and
-// exchanges).  Measured on GB300, us per pass: 2D N=256 Saleh (50 steps) 1406
-// with four, 1775 with eight; 3D N=128 (27 steps) 2618 with eight.
-static int fx_elems(const Geom &g) { return g.dims == 2 && g.N <= 1024 ? FX_E_SMALL : 8; }
+// exchanges).
+// GB300, us per pass of 2D N=1024: `pseudospectral` (100 steps), rows with four
+// and COL_STEP with eight 5694, both four 6170, both eight 5890; the
+// variable-mobility step (10 steps; three boxes at once), whose column passes
+// make one transform each, with four 2313, with eight 2459.  2D N=256 Saleh
+// (50 steps): 1406 with four, 1775 with eight.
+static int fx_row_elems(const Geom &g) { return g.dims == 2 && g.N <= 1024 ? 4 : 8; }
+static int fx_col_elems(const Geom &g) { return g.dims == 2 && g.N <= 1024 ? 4 : 8; }
+static int fx_step_elems(const Geom &g) { return g.dims == 2 && g.N <= 512 ? 4 : 8; }
 
-// Columns per CTA of the column passes.
-static void set_col_shape(SpectralState *s, int C) {
-    s->lgC = ilog2(C);
-    s->col_threads = C * fx_line_threads(s->g.N, s->E);
-    s->col_smem = sizeof(fx2) * 2 * (size_t) C * fx_line_size(s->g.N);
+// The shape with C columns per CTA.
+static ColShape col_shape(const Geom &g, int E, int C) {
+    ColShape c;
+    c.E = E;
+    c.lgC = ilog2(C);
+    c.threads = C * fx_line_threads(g.N, E);
+    c.smem = sizeof(fx2) * 2 * (size_t) C * fx_line_size(g.N);
+    return c;
 }
 
 // Let a kernel take `smem` bytes of dynamic shared memory.  The limit is one of
@@ -766,8 +775,7 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
     for(int d = 1; d < g.dims; d++) s->hat *= g.N;
     size_t hat_bytes = sizeof(double2) * (size_t) s->hat * g.S;
     bool ok = cudaMalloc(&s->psi_hat, hat_bytes) == cudaSuccess && cudaMalloc(&s->work, hat_bytes) == cudaSuccess &&
-              cudaMalloc(&s->alpha, sizeof(double) * (size_t) s->hat * g.S) == cudaSuccess &&
-              cudaMalloc(&s->beta, sizeof(double) * (size_t) s->hat * g.S) == cudaSuccess &&
+              cudaMalloc(&s->ab, hat_bytes) == cudaSuccess &&
               cudaMalloc(&s->twf, sizeof(int4) * g.N) == cudaSuccess;
     if(!ok) {
         cudaGetLastError();
@@ -775,19 +783,18 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
         err = "device allocation failed";
         return CHGB_ERR_ALLOC;
     }
-    std::vector<double> a, b;
-    build_tables(*s, a, b);
+    std::vector<double2> ab;
+    build_tables(*s, ab);
     std::vector<int4> wf;
     build_twiddles(g.N, wf);
-    ok = cudaMemcpy(s->alpha, a.data(), sizeof(double) * a.size(), cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(s->beta, b.data(), sizeof(double) * b.size(), cudaMemcpyHostToDevice) == cudaSuccess &&
+    ok = cudaMemcpy(s->ab, ab.data(), hat_bytes, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(s->twf, wf.data(), sizeof(int4) * wf.size(), cudaMemcpyHostToDevice) == cudaSuccess;
     if(!ok) {
         spectral_destroy(s);
         err = "table upload failed";
         return CHGB_ERR_CUDA;
     }
-    s->E = fx_elems(g);
+    s->row_E = fx_row_elems(g);
     s->pdl = g.dims == 3;
     // launch shapes.  A CTA takes at least a warp's worth of lines, then more up
     // to 128 threads while ~2 CTAs per SM are left: small boxes want their few
@@ -795,20 +802,23 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
     constexpr long long kSpreadCtas = 2 * 152;
     const int M = g.N / 2;
     const long long rows = (long long) g.bins / g.N;
-    const int row_T = fx_line_threads(M, s->E);
+    const int row_T = fx_line_threads(M, s->row_E);
     s->row_rpc = 1;
     while(s->row_rpc * 2 * row_T * g.S <= 128 && s->row_rpc * 2 <= rows &&
           (s->row_rpc * row_T * g.S < 32 || rows / (s->row_rpc * 2) >= kSpreadCtas))
         s->row_rpc *= 2;
     s->row_threads = s->row_rpc * g.S * row_T;
     s->row_smem = sizeof(fx2) * 2 * (size_t) (s->row_threads / row_T) * fx_line_size(M);
-    const int col_T = fx_line_threads(g.N, s->E);
     const long long col_lines = (long long) s->H * (g.dims == 3 ? g.N : 1) * g.S;
-    int C = 1;
-    while(C * 2 * col_T <= 256 && C * 2 <= FX_MAX_INTERLEAVE &&
-          (C * col_T < 32 || col_lines / (C * 2) >= kSpreadCtas))
-        C *= 2;
-    set_col_shape(s, C);
+    auto spread = [&](int E) {
+        const int T = fx_line_threads(g.N, E);
+        int C = 1;
+        while(C * 2 * T <= 256 && C * 2 <= FX_MAX_INTERLEAVE && (C * T < 32 || col_lines / (C * 2) >= kSpreadCtas))
+            C *= 2;
+        return col_shape(g, E, C);
+    };
+    s->col = spread(fx_col_elems(g));
+    s->step = spread(fx_step_elems(g));
     // shared-memory attributes, once
     auto setattr = [](const void *f, size_t smem) { allow_smem(f, smem); };
 #define SETROW(K, E)                                                                            \
@@ -850,8 +860,7 @@ void spectral_destroy(SpectralState *s) {
     if(!s) return;
     if(s->psi_hat) cudaFree(s->psi_hat);
     if(s->work) cudaFree(s->work);
-    if(s->alpha) cudaFree(s->alpha);
-    if(s->beta) cudaFree(s->beta);
+    if(s->ab) cudaFree(s->ab);
     if(s->twf) cudaFree(s->twf);
     delete s;
 }
@@ -882,7 +891,7 @@ dim3 row_grid(const SpectralState *s) { return dim3((unsigned) ((long long) s->g
 
 template <int KIND, int IN, bool FPRIME, bool WRITE_REAL, bool R2C>
 cudaError_t launch_row_kind(SpectralState *s, const double *real_in, double *real_out, cudaStream_t st) {
-    auto kernel = s->E == 8 ? row_kernel<KIND, 8, IN, FPRIME, WRITE_REAL, R2C>
+    auto kernel = s->row_E == 8 ? row_kernel<KIND, 8, IN, FPRIME, WRITE_REAL, R2C>
                             : row_kernel<KIND, 4, IN, FPRIME, WRITE_REAL, R2C>;
     return launch_pass(s, kernel, row_grid(s), s->row_threads, s->row_smem, st, s->work, real_in, real_out, ilog2(s->g.N) - 1, s->row_rpc, s->g.bins, s->hat, s->twf, s->m,
                        nullptr, nullptr);
@@ -891,7 +900,7 @@ cudaError_t launch_row_kind(SpectralState *s, const double *real_in, double *rea
 // Row pass of the variable-mobility flux: c2r of work's rows, the flux stage, r2c back into work.
 template <int KIND, int FLUX>
 cudaError_t launch_row_flux_kind(SpectralState *s, const double *mob, const double *M0, cudaStream_t st) {
-    auto kernel = s->E == 8 ? row_kernel<KIND, 8, ROW_IN_HAT, false, false, true, FLUX>
+    auto kernel = s->row_E == 8 ? row_kernel<KIND, 8, ROW_IN_HAT, false, false, true, FLUX>
                             : row_kernel<KIND, 4, ROW_IN_HAT, false, false, true, FLUX>;
     return launch_pass(s, kernel, row_grid(s), s->row_threads, s->row_smem, st, s->work, nullptr, nullptr, ilog2(s->g.N) - 1, s->row_rpc, s->g.bins, s->hat,
                        s->twf, s->m, mob, M0);
@@ -938,24 +947,51 @@ cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps
         plane_stride = H;
         planes = N;
     }
-    const int C = 1 << s->lgC;
-    auto kernel = s->E == 8 ? col_kernel<MODE, 8> : col_kernel<MODE, 4>;
-    return launch_pass(s, kernel, dim3((unsigned) ((H + C - 1) / C), (unsigned) planes, (unsigned) s->g.S),
-                       s->col_threads, s->col_smem, st, s->work, s->psi_hat, s->alpha, s->beta, ilog2(N), H, s->lgC,
-                       elem_stride, plane_stride, s->hat, s->twf, 1.0 / (double) s->g.bins, ops);
+    const ColShape &c = MODE == COL_STEP ? s->step : s->col;
+    const int C = 1 << c.lgC;
+    auto kernel = c.E == 8 ? col_kernel<MODE, 8> : col_kernel<MODE, 4>;
+    return launch_pass(s, kernel, dim3((unsigned) ((H + C - 1) / C), (unsigned) planes, (unsigned) s->g.S), c.threads,
+                       c.smem, st, s->work, s->psi_hat, s->ab, ilog2(N), H, c.lgC, elem_stride, plane_stride, s->hat,
+                       s->twf, 1.0 / (double) s->g.bins, ops);
 }
 
 }  // namespace
 
 // Columns per CTA of the column passes, timed at create.  Adjacent columns in
 // one CTA use whole 32-byte sectors of the strided column loads, while fewer,
-// larger CTAs spread the lines over fewer SMs; which wins depends on the box
-// (measured on GB300: 2 for 2D N=1024 and 3D N=128, 1 for 2D N=256 and
-// N=2048).  So boxes of 2^18 cells and more time one column step with 1, 2
-// and 4 columns per CTA (those that fit 1024 threads and the shared memory) on
-// a state filled with noise, and keep the fastest.  Every shape gives the same
-// bits: a line's transform does not depend on its CTA.  The state is zeroed
-// afterwards (an upload sets it).
+// larger CTAs spread the lines over fewer SMs; which wins depends on the box.
+// So boxes of 2^18 cells and more time one column step and one forward pass
+// with 1, 2, 4 and 8 columns per CTA (those that fit 512 threads and the shared
+// memory) on a state filled with noise, and keep the fastest of each.  Every
+// shape gives the same bits: a line's transform does not depend on its CTA.
+// The state is zeroed afterwards (an upload sets it).
+template <int MODE>
+static void tune_col_mode(SpectralState *s, ColShape &shape, cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1) {
+    const int axis = s->g.dims - 1;
+    ColShape pick = shape;
+    float best = 0.0f;
+    for(int C : {1, 2, 4, 8}) {
+        shape = col_shape(s->g, shape.E, C);
+        if(shape.threads > 512 || shape.threads < 32 || shape.smem > 224 * 1024) continue;
+        cudaError_t e = launch_col<MODE>(s, axis, st);   // warm-up
+        if(e == cudaSuccess) e = cudaEventRecord(ev0, st);
+        for(int r = 0; r < 5 && e == cudaSuccess; r++) e = launch_col<MODE>(s, axis, st);
+        if(e == cudaSuccess) e = cudaEventRecord(ev1, st);
+        if(e == cudaSuccess) e = cudaEventSynchronize(ev1);
+        float ms = 0.0f;
+        if(e == cudaSuccess) e = cudaEventElapsedTime(&ms, ev0, ev1);
+        if(e != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if(best == 0.0f || ms < best) {
+            best = ms;
+            pick = shape;
+        }
+    }
+    shape = pick;
+}
+
 static void tune_col_shape(SpectralState *s) {
     if(s->g.dims < 2 || (long long) s->g.bins < (1ll << 18)) return;
     cudaStream_t st = nullptr;
@@ -967,34 +1003,12 @@ static void tune_col_shape(SpectralState *s) {
         if(st) cudaStreamDestroy(st);
         return;
     }
-    const int axis = s->g.dims - 1;
     const long long nd = s->hat * s->g.S * 2;   // doubles of psi_hat / work
-    const int C0 = 1 << s->lgC;
-    int bestC = C0;
-    float best = 0.0f;
-    bool ok = launch_fill_noise(reinterpret_cast<double *>(s->psi_hat), 0.0, 1e-2, nd, st) == cudaSuccess &&
-              launch_fill_noise(reinterpret_cast<double *>(s->work), 0.0, 1e-2, nd, st) == cudaSuccess;
-    for(int C : {1, 2, 4, 8}) {
-        if(!ok) break;
-        set_col_shape(s, C);
-        if(s->col_threads > 512 || s->col_threads < 32 || s->col_smem > 224 * 1024) continue;
-        cudaError_t e = launch_col<COL_STEP>(s, axis, st);   // warm-up
-        if(e == cudaSuccess) e = cudaEventRecord(ev0, st);
-        for(int r = 0; r < 5 && e == cudaSuccess; r++) e = launch_col<COL_STEP>(s, axis, st);
-        if(e == cudaSuccess) e = cudaEventRecord(ev1, st);
-        if(e == cudaSuccess) e = cudaEventSynchronize(ev1);
-        float ms = 0.0f;
-        if(e == cudaSuccess) e = cudaEventElapsedTime(&ms, ev0, ev1);
-        if(e != cudaSuccess) {
-            cudaGetLastError();
-            continue;
-        }
-        if(best == 0.0f || ms < best) {
-            best = ms;
-            bestC = C;
-        }
+    if(launch_fill_noise(reinterpret_cast<double *>(s->psi_hat), 0.0, 1e-2, nd, st) == cudaSuccess &&
+       launch_fill_noise(reinterpret_cast<double *>(s->work), 0.0, 1e-2, nd, st) == cudaSuccess) {
+        tune_col_mode<COL_STEP>(s, s->step, st, ev0, ev1);
+        tune_col_mode<COL_FWD>(s, s->col, st, ev0, ev1);
     }
-    set_col_shape(s, bestC);
     cudaMemsetAsync(s->psi_hat, 0, sizeof(double) * nd, st);
     cudaMemsetAsync(s->work, 0, sizeof(double) * nd, st);
     cudaStreamSynchronize(st);
@@ -1009,7 +1023,7 @@ namespace {
 cudaError_t launch_update1d(SpectralState *s, int init, cudaStream_t st) {
     long long n = s->hat * s->g.S;
     int grid = (int) std::min<long long>((n + 255) / 256, 152 * 8);
-    update1d_kernel<<<grid, 256, 0, st>>>(s->work, s->psi_hat, s->alpha, s->beta, n, init, 1.0 / (double) s->g.bins);
+    update1d_kernel<<<grid, 256, 0, st>>>(s->work, s->psi_hat, s->ab, n, init, 1.0 / (double) s->g.bins);
     return cudaGetLastError();
 }
 
@@ -1110,8 +1124,7 @@ void spectral_batch_rep(const SpectralState *s, PsBatchRep *r, size_t *row_smem,
     const int N = s->g.N, M = N / 2, S = s->g.S;
     r->work = s->work;
     r->psi_hat = s->psi_hat;
-    r->alpha = s->alpha;
-    r->beta = s->beta;
+    r->ab = s->ab;
     r->twf = s->twf;
     r->m = s->m;
     r->N = N;
@@ -1119,7 +1132,8 @@ void spectral_batch_rep(const SpectralState *s, PsBatchRep *r, size_t *row_smem,
     r->H = s->H;
     r->bins = s->g.bins;
     r->hat = s->hat;
-    const int row_T = fx_line_threads(M, FX_E_SMALL), col_T = fx_line_threads(N, FX_E_SMALL);
+    r->col_E = s->step.E;
+    const int row_T = fx_line_threads(M, s->row_E), col_T = fx_line_threads(N, s->step.E);
     r->row_rpc = 1;
     while(r->row_rpc * 2 * row_T * S <= PS_BATCH_THREADS && r->row_rpc * 2 <= N) r->row_rpc *= 2;
     r->col_C = std::max(1, std::min(PS_BATCH_THREADS / col_T, 16));
@@ -1132,7 +1146,8 @@ namespace {
 template <int KIND>
 cudaError_t configure_kind(size_t row_smem, size_t col_smem) {
     cudaError_t e = allow_smem((const void *) row_batch_kernel<KIND>, row_smem);
-    if(e == cudaSuccess) e = allow_smem((const void *) col_batch_kernel, col_smem);
+    if(e == cudaSuccess) e = allow_smem((const void *) col_batch_kernel<4>, col_smem);
+    if(e == cudaSuccess) e = allow_smem((const void *) col_batch_kernel<8>, col_smem);
     return e;
 }
 }  // namespace
@@ -1146,7 +1161,7 @@ cudaError_t configure_ps2d_batch(int kind, size_t row_smem, size_t col_smem) {
 }
 
 cudaError_t launch_ps2d_batch(int kind, const PsBatchRep *reps, const int2 *row_items, int nrow, const int4 *col_items,
-                              int ncol, size_t row_smem, size_t col_smem, cudaStream_t st) {
+                              int ncol8, int ncol4, size_t row_smem, size_t col_smem, cudaStream_t st) {
     if(nrow > 0) {
         switch(kind) {
             case CHGB_MODEL_LANDAU:
@@ -1160,7 +1175,8 @@ cudaError_t launch_ps2d_batch(int kind, const PsBatchRep *reps, const int2 *row_
         cudaError_t e = cudaGetLastError();
         if(e != cudaSuccess) return e;
     }
-    if(ncol > 0) col_batch_kernel<<<ncol, PS_BATCH_THREADS, col_smem, st>>>(reps, col_items);
+    if(ncol8 > 0) col_batch_kernel<8><<<ncol8, PS_BATCH_THREADS, col_smem, st>>>(reps, col_items);
+    if(ncol4 > 0) col_batch_kernel<4><<<ncol4, PS_BATCH_THREADS, col_smem, st>>>(reps, col_items + ncol8);
     return cudaGetLastError();
 }
 
@@ -1217,7 +1233,7 @@ __global__ void __launch_bounds__(256) row_adj_kernel(double2 *__restrict__ work
     extern __shared__ fx2 sm2[];
     __shared__ double red[32];
     __shared__ int sm_w[2][FX_MAX_WARPS];
-    constexpr int E = FX_E_SMALL;
+    constexpr int E = 4;   // fx_row_elems of the adjoint's boxes, N <= 1024
     const FxLine ln = fx_line<E>(lgM, 0, false);
     const int M = 1 << lgM, N = 2 * M, LS = fx_line_size(M);
     const int li = threadIdx.x / ln.T, nl = blockDim.x / ln.T;
@@ -1247,8 +1263,8 @@ enum { ADJ_A = 1, ADJ_B = 2, ADJ_BA = 3 };
 // update) and/or A part (gradient sums with psi_next = psi_t_{n+1} and
 // psi_cur = psi_t_n, then beta * lam_hat and the inverse y FFT into work).
 template <int MODE>
-__global__ void __launch_bounds__(256) col_adj_kernel(double2 *__restrict__ work, double2 *__restrict__ lam,
-                                                     const double *__restrict__ alpha, const double *__restrict__ beta,
+__global__ void __launch_bounds__(512) col_adj_kernel(double2 *__restrict__ work, double2 *__restrict__ lam,
+                                                     const double2 *__restrict__ ab,
                                                      const double *__restrict__ tk, const double *__restrict__ tm1,
                                                      const double *__restrict__ tm2,
                                                      const double2 *__restrict__ psi_next,
@@ -1258,8 +1274,8 @@ __global__ void __launch_bounds__(256) col_adj_kernel(double2 *__restrict__ work
     extern __shared__ fx2 sm2[];
     __shared__ double red[32];
     __shared__ int sm_w[2][FX_MAX_WARPS * FX_MAX_INTERLEAVE];
+    constexpr int E = 4;   // fx_col_elems of the adjoint's boxes, N <= 1024
     const int C = 1 << lgC;   // at most FX_MAX_INTERLEAVE: one group
-    constexpr int E = FX_E_SMALL;
     const FxLine ln = fx_line<E>(lgL, lgC, false);
     const int L = 1 << lgL;
     const int kx = blockIdx.x * C + ln.c;
@@ -1277,7 +1293,7 @@ __global__ void __launch_bounds__(256) col_adj_kernel(double2 *__restrict__ work
             if(active && i < L) {
                 const long long off = off0 + i * dT;
                 const double2 l = lam[off];
-                const double al = alpha[off];
+                const double al = ab[off].x;
                 r[i] = make_double2(fma(al, l.x, -r[i].x), fma(al, l.y, -r[i].y));
                 lam[off] = r[i];
             }
@@ -1295,7 +1311,7 @@ __global__ void __launch_bounds__(256) col_adj_kernel(double2 *__restrict__ work
                 const double dc = fma(l.x, pc.x, l.y * pc.y);
                 ak = fma(w * tk[off], dn, ak);
                 am = fma(w, fma(tm1[off], dn, -tm2[off] * dc), am);
-                const double be = beta[off];
+                const double be = ab[off].y;
                 r[i] = make_double2(be * l.x, be * l.y);
             }
         }
@@ -1352,7 +1368,7 @@ SpectralAdj *spectral_adj_create(SpectralState *s, std::string &err) {
         }
     }
     a->n_row_cta = (int) (((long long) s->g.bins / N) / s->row_rpc);
-    a->n_col_cta = (s->H + (1 << s->lgC) - 1) >> s->lgC;
+    a->n_col_cta = (s->H + (1 << s->col.lgC) - 1) >> s->col.lgC;
     bool ok = cudaMalloc(&a->tk, sizeof(double) * s->hat) == cudaSuccess &&
               cudaMalloc(&a->tm1, sizeof(double) * s->hat) == cudaSuccess &&
               cudaMalloc(&a->tm2, sizeof(double) * s->hat) == cudaSuccess &&
@@ -1365,7 +1381,7 @@ SpectralAdj *spectral_adj_create(SpectralState *s, std::string &err) {
          cudaMemcpy(a->tm1, tm1.data(), sizeof(double) * s->hat, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(a->tm2, tm2.data(), sizeof(double) * s->hat, cudaMemcpyHostToDevice) == cudaSuccess;
     if(ok) {
-        size_t rs = s->row_smem, cs = s->col_smem;
+        size_t rs = s->row_smem, cs = s->col.smem;
         allow_smem((const void *) row_adj_kernel, rs);
         allow_smem((const void *) col_adj_kernel<ADJ_A>, cs);
         allow_smem((const void *) col_adj_kernel<ADJ_B>, cs);
@@ -1417,11 +1433,10 @@ cudaError_t spectral_adj_col(SpectralAdj *a, SpectralState *s, int mode, const d
     const int N = s->g.N;
     dim3 grid((unsigned) a->n_col_cta);
 #define ADJ_COL_ARGS                                                                                                   \
-    a->work, a->lam, s->alpha, s->beta, a->tk, a->tm1, a->tm2, psi_next, psi_cur, ilog2(N), s->H, s->lgC, s->twf,      \
+    a->work, a->lam, s->ab, a->tk, a->tm1, a->tm2, psi_next, psi_cur, ilog2(N), s->H, s->col.lgC, s->twf,      \
         a->gk, a->gm
-    if(mode == ADJ_A) col_adj_kernel<ADJ_A><<<grid, s->col_threads, s->col_smem, st>>>(ADJ_COL_ARGS);
-    else if(mode == ADJ_B) col_adj_kernel<ADJ_B><<<grid, s->col_threads, s->col_smem, st>>>(ADJ_COL_ARGS);
-    else col_adj_kernel<ADJ_BA><<<grid, s->col_threads, s->col_smem, st>>>(ADJ_COL_ARGS);
+    auto kernel = mode == ADJ_A ? col_adj_kernel<ADJ_A> : mode == ADJ_B ? col_adj_kernel<ADJ_B> : col_adj_kernel<ADJ_BA>;
+    kernel<<<grid, s->col.threads, s->col.smem, st>>>(ADJ_COL_ARGS);
 #undef ADJ_COL_ARGS
     return cudaGetLastError();
 }
