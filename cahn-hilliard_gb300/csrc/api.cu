@@ -460,7 +460,10 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
             h->variant = pick;
             cudaGetLastError();
         }
-        if(h->variant != 2 && !(h->variant == 5 && h->g.dims == 3)) {   // mu is stored by the split pairs only
+        // mu is stored by the split pairs only: variant 2, and variant 5 in 3D
+        // where it was asked for by number (launch_euler_bfp)
+        const bool bfp_pair = h->variant == 5 && h->g.dims == 3 && want == 5;
+        if(h->variant != 2 && !bfp_pair) {
             if(h->d_mu) cudaFree(h->d_mu);
             if(h->d_mobk) cudaFree(h->d_mobk);
             h->d_mu = h->d_mobk = nullptr;
@@ -551,7 +554,7 @@ static bool field_mobility(const chgb_handle *h) { return h->ec.mobf != nullptr;
 
 static int launches_per_step(const chgb_handle *h) {
     if(h->psm) return psmob_launches_per_step(h->psm) + (h->p.mobility_type != CHGB_MOBILITY_CONSTANT ? 1 : 0);
-    const bool pair = h->variant == 2 || (h->variant == 5 && h->g.dims == 3);   // 2D variant 5: one kernel
+    const bool pair = h->variant == 2 || (h->variant == 5 && h->d_mu);
     return (pair ? 2 : 1) + (field_mobility(h) ? 1 : 0);
 }
 
@@ -594,7 +597,7 @@ static cudaError_t one_step(chgb_handle *h) {
 static cudaError_t bfp_refresh(chgb_handle *h) {
     if(h->variant != 5) return cudaSuccess;
     h->launches += 1;
-    return launch_bfp_refresh(h->d_rho[h->cur], (long long) h->n, h->d_bfp, bfp_key_bank(h->g, h->cur), h->stream);
+    return launch_bfp_refresh(h->d_rho[h->cur], (long long) h->n, h->d_bfp, h->cur, h->stream);
 }
 
 // Queue `steps` time steps as chgb_step's graphs hold them (the timing at

@@ -53,7 +53,19 @@ constexpr int FX_TOP = 62;   // every complex magnitude stays below 2^FX_TOP
 // v = fx_hi(v) 2^32 + fx_lo(v), both signed.
 __device__ __forceinline__ int fx_hi(long long v) { return (int) (v >> 32) + (int) ((unsigned) v >> 31); }
 __device__ __forceinline__ int fx_lo(long long v) { return (int) v; }
-__device__ __forceinline__ long long wide(int a, int b) { return (long long) a * (long long) b; }
+// a b and a b + c, one IMAD.WIDE each.  In C++ a product of sign-extended low
+// words, (long long) (int) v * ..., is compiled as a full 64-bit product, five
+// instructions.
+__device__ __forceinline__ long long wide(int a, int b) {
+    long long r;
+    asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ long long wide(int a, int b, long long c) {
+    long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
 
 // a w / 2^62 (CONJ = false) or a conj(w) / 2^62 (CONJ = true), rounded;
 // w = {hx, lx, hy, ly}, the limbs of the twiddle's real and imaginary parts
@@ -65,10 +77,10 @@ __device__ __forceinline__ fx2 fx_cmul(fx2 a, int4 w) {
     const int rz = CONJ ? w.z : nz, rw = CONJ ? w.w : nw;   // Y's factor in the real part
     const int iz = CONJ ? nz : w.z, iw = CONJ ? nw : w.w;   // X's factor in the imaginary part
     const long long half = 1ll << 29;
-    const long long hx = wide(xh, w.x) + wide(yh, rz);
-    const long long mx = half + wide(xh, w.y) + wide(xl, w.x) + wide(yh, rw) + wide(yl, rz);
-    const long long hy = wide(yh, w.x) + wide(xh, iz);
-    const long long my = half + wide(yh, w.y) + wide(yl, w.x) + wide(xh, iw) + wide(xl, iz);
+    const long long hx = wide(xh, w.x, wide(yh, rz));
+    const long long mx = wide(xh, w.y, wide(xl, w.x, wide(yh, rw, wide(yl, rz, half))));
+    const long long hy = wide(yh, w.x, wide(xh, iz));
+    const long long my = wide(yh, w.y, wide(yl, w.x, wide(xh, iw, wide(xl, iz, half))));
     return fx2{4 * hx + (mx >> 30), 4 * hy + (my >> 30)};
 }
 
@@ -77,7 +89,7 @@ __device__ __forceinline__ long long fx_mul_sqrt_half(long long X) {
     constexpr long long C = 3260954456333195553ll;   // round(2^62 / sqrt(2))
     constexpr int Cl = (int) (C & 0xFFFFFFFFll), Ch = (int) ((C - Cl) >> 32);
     const int xh = fx_hi(X), xl = fx_lo(X);
-    const long long mid = (1ll << 29) + wide(xh, Cl) + wide(xl, Ch);
+    const long long mid = wide(xh, Cl, wide(xl, Ch, 1ll << 29));
     return 4 * wide(xh, Ch) + (mid >> 30);
 }
 
@@ -173,19 +185,19 @@ __device__ __forceinline__ double fx_out_fp(long long X, const FxScale &s) {
     const double d = __ll2double_rn(X);
     return X == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (s.sh << 20), __double2loint(d));
 }
-__device__ __forceinline__ double fx_out_int(long long X, const FxScale &s) {
+__device__ __forceinline__ double fx_nearest(long long X, int sh) {   // |X| < 2^63, a normal result
     const long long sg = X >> 63;
     const unsigned long long a = (unsigned long long) ((X ^ sg) - sg);
     const int lz = __clzll((long long) a);                     // 1 or more; 64 for 0
     const unsigned long long m = a << ((lz - 1) & 63);         // leading one at bit 62
     const unsigned long long q = (m + 0x1FF + ((m >> 10) & 1)) >> 10;   // 53 bits, or 2^53
     // the leading one adds 1 to the exponent field below it, a carry out of the mantissa 2
-    const unsigned long long bits = ((unsigned long long) (unsigned) (1085 - lz - s.sh) << 52) + q;
+    const unsigned long long bits = ((unsigned long long) (unsigned) (1085 - lz - sh) << 52) + q;
     const unsigned long long r = X == 0 ? 0ull : bits | ((unsigned long long) sg << 63);
     return __longlong_as_double((long long) r);
 }
 __device__ __forceinline__ double2 fx_out(fx2 v, const FxScale &s) {
-    return make_double2(fx_out_fp(v.x, s), fx_out_int(v.y, s));
+    return make_double2(fx_out_fp(v.x, s), fx_nearest(v.y, s.sh));
 }
 
 // v times f^3 where the line is `odd`.  The three products a value make the

@@ -21,6 +21,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "bfp.cuh"
 #include "bounds.cuh"
 #include "common.cuh"
 #include "fxsum.cuh"
@@ -1011,109 +1012,207 @@ __global__ void __launch_bounds__(256, (S == 1 && MOB == 0) ? 8 : 1) update_kern
 }
 
 // ---------------------------------------------------------------------------
-// Block fixed point (kernel_variant 5: Landau `euler`): the split pair in 3D
-// (mu_bfp_kernel, update_bfp_kernel), one kernel per step in 2D
-// (euler2d_bfp_kernel, below), the same arithmetic
+// Block fixed point (kernel_variant 5: Landau `euler`): one kernel per step
+// (euler2d_bfp_kernel, euler3d_bfp_kernel), and in 3D also a pair of kernels
+// (mu_bfp_kernel, update_bfp_kernel), the same arithmetic and bits
 // ---------------------------------------------------------------------------
 // The split pair above aligns the terms of each neighbour sum to the largest
 // exponent of that stencil: per cell a maximum over seven exponents and seven
 // variable shifts, about half of a step's integer work.  Here one exponent
 // serves the whole field for a step (block floating point, the field being the
-// block):
+// block), and mu is formed in integers throughout:
 //   - psi: emax, the largest biased exponent of |psi| over the field, is read
-//     from BfpState::key (below).  Each value becomes
-//     X = floor(psi 2^(1080 - emax)), |X| < 2^58, once, when it is staged, and
-//     a neighbour sum is a plain int64 sum.
-//   - mu: from emax and the model's constants follows a bound |mu| < 2^Emu,
-//     Emu = max(3 s, elin + s) + 2 with |psi| < 2^s and
-//     |lshift| + 2 D c2 < 2^elin (|psi|^3 + |lshift psi| + c2 |sum|, one bit
-//     spare).  mu goes to HBM in fixed point, M = floor(mu 2^(58 - Emu)),
-//     |M| <= 2^57 + 1, so the update's sums need no conversion.  Its two parts
-//     are formed apart and subtracted in integers: psi (psi^2 + lshift) in
-//     FP64 (the step's only two FP64 instructions of mu), truncated to M's
-//     unit, and c2 sum as the high half of the 64 x 64-bit product of the sum
-//     with c2's mantissa, shifted to M's unit.
+//     from BfpState::key (below); |psi| < 2^s, s = emax - 1022.  Each value
+//     becomes X = psi 2^(60-s) cut to an integer, |X| < 2^60, once, and a
+//     neighbour sum S is a plain int64 sum, |S| < 2^62.6.
+//   - mu = psi (psi^2 + lshift) - c2 sum.  With a = max(2 s, elin) (|lshift| +
+//     2 D |c2| < 2^elin), |mu| < 2^(a+s+2) (one bit spare), and mu is stored as
+//     M = mu 2^(56-a-s), |M| <= 2^57 + 1.  G = (psi^2 + lshift) 2^(61-a) =
+//     (X^2 >> 59 + a - 2 s) + lsi, |G| < 2^62, and M = (X G 2^-64 +
+//     S C 2^-64) >> 1, C = -c2 in the matching unit: the shifts do not depend
+//     on the cell, the scales drop out.  All factors are taken as signed 32-bit
+//     limbs (bfp.cuh), so the two products of M are eight IMAD.WIDE that
+//     accumulate; the products of two low limbs are left out.  No FP64
+//     instruction: FP64 issues at 1/64 of FP32's rate here, and the two that
+//     psi (psi^2 + lshift) took were the pipe's larger share of a step.  27
+//     instructions a cell; written as C++ products of sign-extended words they
+//     were 42 (bfp.cuh, `wide`).
 //   - the update: L = sum(M_nb) - 2 D M, exact (|L| < 2^61), and
-//     psi' = psi + c1 (L 2^(Emu - 58)): one int64 -> double rounding (on the
-//     FP64 pipe or in integers, see BFP_INT_ROUND_WARPS) and one FMA.  Each CTA
-//     folds the largest exponent of its psi' into the key.
-// Errors: the truncations of X, of psi (psi^2 + lshift) and of c2 sum, each
-// below 2^-56 of the field's largest value or of mu's bound, where the
-// reference's FP64 sums round relative to each cell's own terms.  The results
-// are not the other variants' bits; they agree with the reference far below
-// the parity tests' 1e-12 (relative to the field's largest value).
+//     psi' = psi + (c1 2^(a+s-56)) L: one int64 -> double rounding (on the FP64
+//     pipe, or in the 2D kernel and the pair for every other cell in integers:
+//     the same bits) and one FMA.
+//     Each CTA folds the largest exponent of its psi' into the key.
+// Errors, in units of M (mu's bound is 2^58 of them): X is cut 2^-60 below the
+// field's bound, which enters c2 sum and psi^3 at less than 2^-58 of theirs; G
+// drops at most 8 + 2 units of 2^-61 of its bound (X's low limb squared, the
+// shifts), half a unit of M; the products' low limbs and shifts 1 unit; C's
+// rounding 2^-4 unit.  So M is within 3 units of mu at the cut field, where the
+// reference's FP64 products and sums round each at 2^-53 of their own value:
+// at worst 2^-56 of mu's bound.  The results are not the other variants' bits.
 // The key is (generation << 16) | emax, the largest of BFP_SLOTS 64-bit slots.
-// A step's mu kernel reads generation g and publishes g + 1 (BfpState::gen)
-// with mu's exponent and the mode; the step's update kernel folds each CTA's
-// exponent into one slot as ((g + 1) << 16) | e by atomicMax, so the newer
-// generation supersedes the older with no reset between steps, and slots no
-// CTA wrote in this step fall behind.  Each chgb_step call first sets the key
+// A step reads generation g and folds each CTA's exponent into one slot of the
+// other bank as ((g + 1) << 16) | e by atomicMax, so the newer generation
+// supersedes the older with no reset between steps, and slots no CTA wrote in
+// this step fall behind.  (The pair's mu kernel publishes g + 1, mu's exponent
+// and the mode to its update kernel, BfpState::gen.)  Each chgb_step call first sets the key
 // from the field (a memset, then bfp_refresh_kernel).  A field whose emax is
-// 0 (zeros and subnormals only) or 2047 (inf, NaN), or so large or small that
-// mu's unit leaves [2^-1000, 2^900], takes plain FP64 sums in the reference's
-// neighbour order for that step (mode 0, mu stored as FP64).
+// below 128 or 2047 (zeros, values near the end of the double range, inf, NaN),
+// or so large or small that mu's unit leaves [2^-900, 2^900], takes plain FP64
+// sums in the reference's neighbour order for that step (mode 0).
 
-// floor(x 2^(1080 - u)) for a finite x whose biased exponent is at most u.
+// psi 2^(60-s) cut to an integer (`u` = emax, the biased exponent of 2^s's
+// binade): the mantissa at the top of a word, down by 4 or more; its one's
+// complement for negative values, the floor of all but whole ones.  Zeros and
+// subnormals (the implicit bit set here does not belong) shift out: u >= 128.
 __device__ __forceinline__ long long bfp_fixed(double x, int u) {
-    long long T;
-    int ek;
-    fx_term(x, T, ek);
-    return fx_sar(T, u - ek);
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned) __double2loint(x);
+    const unsigned mh = __funnelshift_l(lo, (unsigned) hi, 11) | 0x80000000u;
+    const unsigned long long m = fx_shr(((unsigned long long) mh << 32) | (lo << 11), u + 4 - ((hi >> 20) & 0x7FF));
+    return (long long) (m ^ (unsigned long long) (long long) (hi >> 31));
 }
 
-// In-plane offsets of the values a thread stages (the same for every plane of a
-// CTA's column): computed once instead of per plane.
-__device__ __forceinline__ void bfp_plane_offsets(int (&o)[SPF], const Geom &g, int x0, int y0, int tid) {
-#pragma unroll
-    for(int k = 0; k < SPF; k++) {
-        const int i = tid + k * STX * STY;
-        const int ly = i / SPX, lx = i - ly * SPX;
-        o[k] = ((x0 - 1 + lx) & g.mask) + (((y0 - 1 + ly) & g.mask) << g.log2N);
+// A step's scales, the same for every cell.
+struct BfpScale {
+    int emax, lmu, d;   // the field's exponent; M's unit is 2^lmu = 2^(a+s-56); a - 2 s
+    int ch, cl;         // the limbs of C
+    long long lsi;      // lshift in G's unit
+    bool fast;
+};
+
+template <int DIMS>
+__device__ __forceinline__ BfpScale bfp_scale(int emax, const EulerConsts &c, const BfpConsts &b) {
+    BfpScale t;
+    t.emax = emax;
+    const int s = emax - 1022, a = max(2 * s, b.elin);
+    t.lmu = a + s - 56;
+    t.fast = emax >= 128 && emax <= 2046 && t.lmu >= -900 && t.lmu <= 900;
+    t.d = a - 2 * s;
+    const double ls = c.lshift[DIMS - 1];
+    // 2^(61-a): elin is at least -800 where lshift is not zero
+    t.lsi = ls == 0.0 || !t.fast ? 0 : __double2ll_rn(ls * __hiloint2double((1023 + 61 - a) << 20, 0));
+    // -c2 S 2^(s-60) in half units of M: mc is c2's mantissa times 2^10 and
+    // 2^(1085-ec), so C = -mc 2^-(a+1024-ec), four or more places down
+    const int r = a + 1024 - b.ec;
+    const long long C = r > 62 ? 0 : -((b.mc + (1ll << (r - 1))) >> r);
+    t.ch = fx_hi(C);
+    t.cl = fx_lo(C);
+    return t;
+}
+
+// M of a cell from its X and neighbour sum.
+__device__ __forceinline__ long long bfp_mu(long long X, long long S, const BfpScale &t) {
+    const int xh = fx_hi(X), xl = fx_lo(X), sh = fx_hi(S), sl = fx_lo(S);
+    const long long G = (((wide(xh, xh) << 5) + (wide(xh, xl) >> 26)) >> t.d) + t.lsi;
+    const int gh = fx_hi(G), gl = fx_lo(G);
+    const long long hi = wide(xh, gh, wide(sh, t.ch));
+    const long long mid = wide(xh, gl, wide(xl, gh, wide(sh, t.cl, wide(sl, t.ch))));
+    return (hi + (mid >> 32)) >> 1;
+}
+
+// L 2^0 as the nearest double: FP64 pipe, or the same bits in integers.
+__device__ __forceinline__ double bfp_double_fp(long long L) { return __ll2double_rn(L); }
+__device__ __forceinline__ double bfp_double_int(long long L) { return fx_nearest(L, 0); }
+
+// Tiles of the 3D pair (taken where kernel_variant asks for 5 by number): 32 x
+// 16 cells per 256-thread CTA, two cells adjacent in x per thread, marching
+// over `zc` planes.  A thread keeps its own column of
+// three planes in registers; the planes in shared memory (two, one barrier a
+// plane) serve the x and y neighbours.  The tile's 96 halo cells are staged by
+// three of the eight warps, the plane after next being fetched meanwhile.  Per
+// cell this takes 2 + 2 shared loads of a pair's neighbours and half of each
+// global access, where a 32 x 8 tile with one cell a thread (and the whole
+// stencil in shared memory, 1.33 values staged a cell) took 7 and 1.33.
+constexpr int BTX = 32, BTY = 16, BPITCH = BTX + 4, BPLANE = BPITCH * (BTY + 2);
+constexpr int BHALO = 2 * BTX + 2 * BTY;
+
+struct BfpTile {
+    int own, halo;         // shared index of the own pair's left cell, of the halo cell (threads below BHALO)
+    unsigned gown, ghalo;  // their offsets in a plane
+    bool has_halo;
+};
+
+__device__ __forceinline__ BfpTile bfp_tile(const Geom &g, int tid) {
+    BfpTile t;
+    const int tx = tid & 15, ty = tid >> 4;
+    const int x0 = blockIdx.x * BTX, y0 = blockIdx.y * BTY;
+    t.own = (ty + 1) * BPITCH + 2 + 2 * tx;
+    t.gown = (unsigned) (x0 + 2 * tx) + ((unsigned) (y0 + ty) << g.log2N);
+    t.has_halo = tid < BHALO;
+    int lx, ly;            // tile coordinates of the halo cell
+    if(tid < 2 * BTX) {
+        lx = tid & (BTX - 1);
+        ly = tid < BTX ? -1 : BTY;
     }
-}
-
-template <int DIMS, typename T>
-__device__ __forceinline__ void bfp_fetch_plane(T (&v)[SPF], const T *__restrict__ src, const Geom &g,
-                                                const int (&o)[SPF], int z, int tid) {
-    const size_t zoff = (DIMS == 3) ? ((size_t) (z & g.mask) << (2 * g.log2N)) : 0;
-    const T *plane = src + zoff;
-#pragma unroll
-    for(int k = 0; k < SPF; k++)
-        if(tid + k * STX * STY < SPP && CHGB_BC(11, zoff + o[k], g.bins)) v[k] = plane[o[k]];
-}
-
-// The same with the offsets formed per plane: fewer registers, more integer work
-// (the update kernel, whose integer pipe has room and whose registers do not).
-template <int DIMS, typename T>
-__device__ __forceinline__ void bfp_fetch_plane_idx(T (&v)[SPF], const T *__restrict__ src, const Geom &g, int x0,
-                                                    int y0, int z, int tid) {
-    const T *plane = src + ((DIMS == 3) ? ((size_t) (z & g.mask) << (2 * g.log2N)) : 0);
-#pragma unroll
-    for(int k = 0; k < SPF; k++) {
-        const int i = tid + k * STX * STY;
-        if(i < SPP) {
-            const int ly = i / SPX, lx = i - ly * SPX;
-            const int o = ((x0 - 1 + lx) & g.mask) + (((y0 - 1 + ly) & g.mask) << g.log2N);
-            if(CHGB_BC(12, (size_t) (plane - src) + o, g.bins)) v[k] = plane[o];
-        }
+    else {
+        lx = tid < 2 * BTX + BTY ? -1 : BTX;
+        ly = (tid - 2 * BTX) & (BTY - 1);
     }
+    t.halo = (ly + 1) * BPITCH + 2 + lx;
+    t.ghalo = (unsigned) ((x0 + lx) & g.mask) + ((unsigned) ((y0 + ly) & g.mask) << g.log2N);
+    return t;
 }
 
-// The largest biased exponent of a block's per-thread values e, folded into
-// key slot `slot` as ((gen << 16) | e) by one atomicMax (256-thread blocks).
-// The CTAs of a launch spread over BFP_SLOTS slots, one 128-byte line each, so
-// that their atomics do not queue on one address.
-__device__ __forceinline__ void bfp_fold_key(int e, unsigned long long gen, unsigned long long *bank, int slot,
+// x and y neighbours of the thread's pair in a staged plane: the pair's partial sums.
+template <int PITCH>
+__device__ __forceinline__ void bfp_xy_sums(const long long *plane, int own, long long a, long long b, long long &sa,
+                                            long long &sb) {
+    const longlong2 up = *reinterpret_cast<const longlong2 *>(plane + own - PITCH);
+    const longlong2 dn = *reinterpret_cast<const longlong2 *>(plane + own + PITCH);
+    sa = (plane[own - 1] + b) + (up.x + dn.x);
+    sb = (a + plane[own + 2]) + (up.y + dn.y);
+}
+
+// Mode 0 (see above): the step of a w x h x d block of cells at (x0, y0, z0)
+// by a whole CTA, from global memory, in FP64 and the reference's order of
+// neighbours.  Returns the largest high word of the thread's |psi'|.  Not
+// inlined: its registers would be the integer path's.
+template <int DIMS>
+__device__ __noinline__ int bfp_slow_block(const double *__restrict__ in, double *__restrict__ out, int mask, int log2N,
+                                           double c1, double c2, double ls, int x0, int y0, int z0, int w, int h,
+                                           int d) {
+    auto index = [&](int X, int Y, int Z) {
+        return (size_t) (X & mask) + ((size_t) (Y & mask) << log2N) +
+               (DIMS == 3 ? ((size_t) (Z & mask) << (2 * log2N)) : 0);
+    };
+    auto psi = [&](int X, int Y, int Z) { return in[index(X, Y, Z)]; };
+    auto mu = [&](int X, int Y, int Z) {
+        const double r = psi(X, Y, Z);
+        const double sum = seq_sum(psi(X - 1, Y, Z), psi(X + 1, Y, Z), psi(X, Y - 1, Z), psi(X, Y + 1, Z),
+                                   DIMS == 3 ? psi(X, Y, Z - 1) : 0.0, DIMS == 3 ? psi(X, Y, Z + 1) : 0.0, 2 * DIMS);
+        return fma(-c2, sum, r * fma(r, r, ls));
+    };
+    int mag = 0;
+    for(int i = threadIdx.x; i < w * h * d; i += blockDim.x) {
+        const int x = x0 + i % w, y = y0 + i / w % h, z = z0 + i / (w * h);
+        const size_t gi = index(x, y, z);
+        if(!CHGB_BC(17, gi, (long long) 1 << (DIMS * log2N))) continue;
+        const double sum = seq_sum(mu(x - 1, y, z), mu(x + 1, y, z), mu(x, y - 1, z), mu(x, y + 1, z),
+                                   DIMS == 3 ? mu(x, y, z - 1) : 0.0, DIMS == 3 ? mu(x, y, z + 1) : 0.0, 2 * DIMS);
+        const double res = fma(c1, fma(-2.0 * DIMS, mu(x, y, z), sum), in[gi]);
+        out[gi] = res;
+        mag = max(mag, __double2hiint(res) & 0x7FFFFFFF);
+    }
+    return mag;
+}
+
+// The largest biased exponent of a block's per-thread values, given as the high
+// words of |values|, folded into key slot `slot` as ((gen << 16) | e) by one
+// atomicMax.  The CTAs of a launch spread over BFP_SLOTS
+// slots, one 128-byte line each, so that their atomics do not queue on one
+// address.
+template <int WARPS>
+__device__ __forceinline__ void bfp_fold_key(int mag, unsigned long long gen, unsigned long long *bank, int slot,
                                              int tid) {
-    __shared__ int wmax[8];
-    e = __reduce_max_sync(0xffffffffu, e);
+    __shared__ int wmax[WARPS];
+    const int e = __reduce_max_sync(0xffffffffu, mag);
     if((tid & 31) == 0) wmax[tid >> 5] = e;
     __syncthreads();
     if(tid == 0) {
         int m = wmax[0];
 #pragma unroll
-        for(int w = 1; w < 8; w++) m = wmax[w] > m ? wmax[w] : m;
-        atomicMax(&bank[(slot % BFP_SLOTS) * BFP_SLOT_STRIDE], (gen << 16) | (unsigned long long) m);
+        for(int w = 1; w < WARPS; w++) m = wmax[w] > m ? wmax[w] : m;
+        atomicMax(&bank[(slot % BFP_SLOTS) * BFP_SLOT_STRIDE], (gen << 16) | (unsigned long long) (m >> 20));
     }
 }
 
@@ -1135,212 +1234,66 @@ __device__ __forceinline__ unsigned long long bfp_read_key(const unsigned long l
     return s_key;
 }
 
-template <int DIMS, bool FAST>
-__device__ __forceinline__ void mu_bfp_run(const double *__restrict__ in, long long *__restrict__ mu, const Geom &g,
-                                           const EulerConsts &c, const BfpConsts &b, int emax, int lmu, int zc,
-                                           double (*ring)[SPP], long long (*ringX)[SPP]) {
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + STX * ty;
-    const int x0 = blockIdx.x * STX, y0 = blockIdx.y * STY;
-    const int z0 = (DIMS == 3) ? blockIdx.z * zc : 0;
-    const int nz = (DIMS == 3) ? zc : 1;
-    const int p = (ty + 1) * SPX + (tx + 1);
-    const int umu = lmu + 1080;                   // M = floor(mu 2^(1080 - umu))
-    const int rc = umu + 1021 - emax - b.ec;      // c2 sum: high product -> M's unit
-    const double ls = c.lshift[DIMS - 1];
-    auto commit = [&](int slot, const double (&v)[SPF]) {
-#pragma unroll
-        for(int k = 0; k < SPF; k++) {
-            const int i = tid + k * STX * STY;
-            if(i < SPP && CHGB_BC(13, slot, (DIMS == 3) ? 3 : 1)) {
-                ring[slot][i] = v[k];
-                if constexpr(FAST) ringX[slot][i] = bfp_fixed(v[k], emax);
-            }
-        }
-    };
-    int off[SPF];
-    bfp_plane_offsets(off, g, x0, y0, tid);
-    double pf[SPF];
-    if constexpr(DIMS == 3) {
-        bfp_fetch_plane<DIMS>(pf, in, g, off, z0 - 1, tid);
-        commit((z0 + 2) % 3, pf);
-        bfp_fetch_plane<DIMS>(pf, in, g, off, z0, tid);
-        commit(z0 % 3, pf);
-        bfp_fetch_plane<DIMS>(pf, in, g, off, z0 + 1, tid);
-    }
-    for(int z = z0; z < z0 + nz; z++) {
-        const int cz = (DIMS == 3) ? z % 3 : 0, zm = (z + 2) % 3, zp = (z + 1) % 3;
-        if constexpr(DIMS == 3) {
-            commit(zp, pf);
-            if(z + 1 < z0 + nz) bfp_fetch_plane<DIMS>(pf, in, g, off, z + 2, tid);
-        }
-        else {
-            bfp_fetch_plane<DIMS>(pf, in, g, off, 0, tid);
-            commit(0, pf);
-        }
-        __syncthreads();
-        const size_t gi = (size_t) (x0 + tx) + ((size_t) (y0 + ty) << g.log2N) +
-                          ((DIMS == 3) ? ((size_t) z << (2 * g.log2N)) : 0);
-        bool ok = CHGB_BC(14, p - SPX, SPP) && CHGB_BC(14, p + SPX, SPP) && CHGB_BC(15, gi, g.bins);
-        if constexpr(DIMS == 3) ok = ok && CHGB_BC(14, cz, 3) && CHGB_BC(14, zm, 3) && CHGB_BC(14, zp, 3);
-        if(ok) {
-            const double r = ring[cz][p];
-            if constexpr(FAST) {
-                const long long *q = &ringX[cz][p];
-                long long sum = (q[-1] + q[1]) + (q[-SPX] + q[SPX]);
-                if constexpr(DIMS == 3) sum += ringX[zm][p] + ringX[zp][p];
-                const long long F = bfp_fixed(r * fma(r, r, ls), umu);
-                mu[gi] = F - fx_sar(__mul64hi(sum, b.mc), rc);
-            }
-            else {
-                const double *q = &ring[cz][p];
-                double sum;
-                if constexpr(DIMS == 3) sum = seq_sum(q[-1], q[1], q[-SPX], q[SPX], ring[zm][p], ring[zp][p], 6);
-                else sum = seq_sum(q[-1], q[1], q[-SPX], q[SPX], 0.0, 0.0, 4);
-                reinterpret_cast<double *>(mu)[gi] = fma(-c.c2[0], sum, r * fma(r, r, ls));
-            }
-        }
-        __syncthreads();
-    }
-}
-
-template <int DIMS>
-__global__ void __launch_bounds__(256, 8) mu_bfp_kernel(const double *__restrict__ in, long long *__restrict__ mu,
-                                                        Geom g, EulerConsts c, BfpConsts b, BfpState *st, int zc) {
-    constexpr int R = (DIMS == 3) ? 3 : 1;
-    __shared__ double ring[R][SPP];
-    __shared__ long long ringX[R][SPP];
+__global__ void __launch_bounds__(256, 5) mu_bfp_kernel(const double *__restrict__ in, long long *__restrict__ mu,
+                                                        Geom g, EulerConsts c, BfpConsts b, BfpState *st, int parity,
+                                                        int zc) {
+    __shared__ __align__(16) long long ring[2][BPLANE];
+    const int tid = threadIdx.x;
     pdl_begin();
-    const unsigned long long key = bfp_read_key(st->key[0], threadIdx.x + STX * threadIdx.y);
-    const int emax = (int) (key & 0xFFFFu);
-    const int s = emax - 1022;                    // |psi| < 2^s
-    const int emu = max(3 * s, b.elin + s) + 2;   // |mu| < 2^emu
-    const int lmu = emu - 58;                     // M's unit is 2^lmu
-    const bool fast = emax >= 1 && emax <= 2046 && lmu >= -1000 && lmu <= 900;
-    if(blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+    const unsigned long long key = bfp_read_key(st->key[parity], tid);
+    const BfpScale sc = bfp_scale<3>((int) (key & 0xFFFFu), c, b);
+    if(blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0) {
         st->gen = (key >> 16) + 1;
-        st->lmu = lmu;
-        st->mode = fast ? 1 : 0;
+        st->lmu = sc.lmu;
+        st->mode = sc.fast ? 1 : 0;
     }
-    if(fast) mu_bfp_run<DIMS, true>(in, mu, g, c, b, emax, lmu, zc, ring, ringX);
-    else mu_bfp_run<DIMS, false>(in, mu, g, c, b, emax, lmu, zc, ring, ringX);
-}
-
-// Returns the largest biased exponent of the thread's psi'.
-// L 2^lmu (L != 0, |L| < 2^62) rounded to the nearest double, ties to even, in
-// integer arithmetic: the value of __ll2double_rn(L) scaled by 2^lmu.
-__device__ __forceinline__ double bfp_to_double_int(long long L, int lmu) {
-    const unsigned long long a = L < 0 ? 0ull - (unsigned long long) L : (unsigned long long) L;
-    const int top = 63 - __clzll((long long) a);   // the leading bit, <= 61
-    int E = top;
-    unsigned long long M;
-    if(top > 52) {
-        const int r = top - 52;
-        const unsigned long long rem = a & ((1ull << r) - 1), half = 1ull << (r - 1);
-        M = a >> r;
-        if(rem > half || (rem == half && (M & 1))) {
-            M++;
-            if(M >> 53) {
-                M >>= 1;
-                E++;
-            }
-        }
-    }
-    else {
-        M = a << (52 - top);
-    }
-    return __longlong_as_double((long long) (((unsigned long long) (L < 0) << 63) |
-                                             ((unsigned long long) (E + 1023 + lmu) << 52) |
-                                             (M & 0xFFFFFFFFFFFFFull)));
-}
-
-// Warps 0-3 of an update CTA round L with bfp_to_double_int, warps 4-7 with the
-// FP64-pipe conversion: the same bits, and the FP64 pipe, the update's busier
-// one, carries less (3D N=256 on GB300: 9.62e10 -> 9.69e10 cell-steps/s; 2 or 3
-// of the 8 warps gave 9.68e10 and 9.69e10).
-constexpr int BFP_INT_ROUND_WARPS = 4;
-
-template <int DIMS, bool FAST>
-__device__ __forceinline__ int update_bfp_run(const double *__restrict__ psi_in, const long long *__restrict__ mu,
-                                              double *__restrict__ out, const Geom &g, const EulerConsts &c, int lmu,
-                                              int zc, long long (*ringX)[SPP]) {
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + STX * ty;
-    const int x0 = blockIdx.x * STX, y0 = blockIdx.y * STY;
-    const int z0 = (DIMS == 3) ? blockIdx.z * zc : 0;
-    const int nz = (DIMS == 3) ? zc : 1;
-    const int p = (ty + 1) * SPX + (tx + 1);
-    const long long escale = (long long) lmu * (1ll << 52);   // 2^lmu through the exponent field
-    auto commit = [&](int slot, const long long (&v)[SPF]) {
-#pragma unroll
-        for(int k = 0; k < SPF; k++) {
-            const int i = tid + k * STX * STY;
-            if(i < SPP && CHGB_BC(16, slot, (DIMS == 3) ? 3 : 1)) ringX[slot][i] = v[k];
-        }
+    const BfpTile t = bfp_tile(g, tid);
+    const int z0 = blockIdx.z * zc;
+    if(!sc.fast) return;   // the update kernel does the whole step
+    auto plane = [&](int z) { return (unsigned) (z & g.mask) << (2 * g.log2N); };   // element offsets: below 2^30
+    auto pair = [&](int z) {
+        const unsigned gi = plane(z) + t.gown;
+        return CHGB_BC(11, gi + 1, g.bins) ? *reinterpret_cast<const double2 *>(in + gi) : make_double2(0.0, 0.0);
     };
-    int emx = 0;
-    long long pf[SPF];
-    if constexpr(DIMS == 3) {
-        bfp_fetch_plane_idx<DIMS>(pf, mu, g, x0, y0, z0 - 1, tid);
-        commit((z0 + 2) % 3, pf);
-        bfp_fetch_plane_idx<DIMS>(pf, mu, g, x0, y0, z0, tid);
-        commit(z0 % 3, pf);
-        bfp_fetch_plane_idx<DIMS>(pf, mu, g, x0, y0, z0 + 1, tid);
+    auto fixed = [&](double2 v) { return make_longlong2(bfp_fixed(v.x, sc.emax), bfp_fixed(v.y, sc.emax)); };
+    auto halo = [&](int z) {
+        return t.has_halo && CHGB_BC(12, plane(z) + t.ghalo, g.bins) ? in[plane(z) + t.ghalo] : 0.0;
+    };
+    auto stage = [&](int z, longlong2 X, double h) {
+        long long *p = ring[z & 1];
+        if(CHGB_BC(13, t.own + 1, BPLANE)) *reinterpret_cast<longlong2 *>(p + t.own) = X;
+        if(t.has_halo && CHGB_BC(13, t.halo, BPLANE)) p[t.halo] = bfp_fixed(h, sc.emax);
+    };
+    const longlong2 Xfirst = fixed(pair(z0 - 1));
+    longlong2 Xm = Xfirst, Xc = fixed(pair(z0));
+    stage(z0, Xc, halo(z0));
+    double2 next = pair(z0 + 1);
+    double hnext = zc > 1 ? halo(z0 + 1) : 0.0;
+    for(int z = z0; z < z0 + zc; z++) {
+        __syncthreads();   // plane z staged; plane z - 1 read by every warp
+        const longlong2 Xp = fixed(next);
+        if(z + 1 < z0 + zc) {
+            stage(z + 1, Xp, hnext);
+            next = pair(z + 2);
+            if(z + 2 < z0 + zc) hnext = halo(z + 2);
+        }
+        long long sa, sb;
+        bfp_xy_sums<BPITCH>(ring[z & 1], t.own, Xc.x, Xc.y, sa, sb);
+        const longlong2 M = make_longlong2(bfp_mu(Xc.x, sa + (Xm.x + Xp.x), sc), bfp_mu(Xc.y, sb + (Xm.y + Xp.y), sc));
+        const unsigned gi = t.gown + plane(z);
+        if(CHGB_BC(15, gi + 1, g.bins)) *reinterpret_cast<longlong2 *>(mu + gi) = M;
+        Xm = Xc;
+        Xc = Xp;
     }
-    for(int z = z0; z < z0 + nz; z++) {
-        const int cz = (DIMS == 3) ? z % 3 : 0, zm = (z + 2) % 3, zp = (z + 1) % 3;
-        const size_t gi = (size_t) (x0 + tx) + ((size_t) (y0 + ty) << g.log2N) +
-                          ((DIMS == 3) ? ((size_t) z << (2 * g.log2N)) : 0);
-        bool ok = CHGB_BC(17, gi, g.bins) && CHGB_BC(18, p - SPX, SPP) && CHGB_BC(18, p + SPX, SPP);
-        if constexpr(DIMS == 3) ok = ok && CHGB_BC(18, cz, 3) && CHGB_BC(18, zm, 3) && CHGB_BC(18, zp, 3);
-        const double psi0 = ok ? psi_in[gi] : 0.0;   // read before the staging barrier, to overlap its latency
-        if constexpr(DIMS == 3) {
-            commit(zp, pf);
-            if(z + 1 < z0 + nz) bfp_fetch_plane_idx<DIMS>(pf, mu, g, x0, y0, z + 2, tid);
-        }
-        else {
-            bfp_fetch_plane_idx<DIMS>(pf, mu, g, x0, y0, 0, tid);
-            commit(0, pf);
-        }
-        __syncthreads();
-        double res = 0.0;
-        if(!ok) {
-        }
-        else if constexpr(FAST) {
-            const long long *q = &ringX[cz][p];
-            long long L = (q[-1] + q[1]) + (q[-SPX] + q[SPX]);
-            if constexpr(DIMS == 3) L += ringX[zm][p] + ringX[zp][p];
-            L -= (long long) (2 * DIMS) * q[0];
-            const double ld = L == 0 ? 0.0
-                              : ((int) threadIdx.y < BFP_INT_ROUND_WARPS)
-                                  ? bfp_to_double_int(L, lmu)
-                                  : __longlong_as_double(__double_as_longlong(__ll2double_rn(L)) + escale);
-            res = fma(c.c1, ld, psi0);
-        }
-        else {
-            const double *u = reinterpret_cast<const double *>(&ringX[cz][p]);
-            double sum;
-            if constexpr(DIMS == 3)
-                sum = seq_sum(u[-1], u[1], u[-SPX], u[SPX], __longlong_as_double(ringX[zm][p]),
-                              __longlong_as_double(ringX[zp][p]), 6);
-            else sum = seq_sum(u[-1], u[1], u[-SPX], u[SPX], 0.0, 0.0, 4);
-            res = fma(c.c1, fma(-2.0 * DIMS, u[0], sum), psi0);
-        }
-        if(ok) out[gi] = res;
-        const int e = (int) ((unsigned long long) __double_as_longlong(res) >> 52) & 0x7FF;
-        emx = e > emx ? e : emx;
-        __syncthreads();
-    }
-    return emx;
 }
 
-template <int DIMS>
-__global__ void __launch_bounds__(256, 8) update_bfp_kernel(const double *__restrict__ psi_in,
+__global__ void __launch_bounds__(256, 5) update_bfp_kernel(const double *__restrict__ psi_in,
                                                             const long long *__restrict__ mu, double *__restrict__ out,
-                                                            Geom g, EulerConsts c, BfpState *st, int zc) {
-    constexpr int R = (DIMS == 3) ? 3 : 1;
-    __shared__ long long ringX[R][SPP];   // M (mode 1) or mu's FP64 bits (mode 0)
+                                                            Geom g, EulerConsts c, BfpState *st, int parity, int zc) {
+    __shared__ __align__(16) long long ring[2][BPLANE];
     __shared__ unsigned long long s_gen;
     __shared__ int s_lmu, s_mode;
-    const int tid = threadIdx.x + STX * threadIdx.y;
+    const int tid = threadIdx.x;
     pdl_begin();
     if(tid == 0) {   // one load per CTA of the step's state, shared
         s_gen = *(const volatile unsigned long long *) &st->gen;
@@ -1348,123 +1301,239 @@ __global__ void __launch_bounds__(256, 8) update_bfp_kernel(const double *__rest
         s_mode = *(const volatile int *) &st->mode;
     }
     __syncthreads();
-    const int lmu = s_lmu;
-    const int emx = s_mode ? update_bfp_run<DIMS, true>(psi_in, mu, out, g, c, lmu, zc, ringX)
-                           : update_bfp_run<DIMS, false>(psi_in, mu, out, g, c, lmu, zc, ringX);
-    bfp_fold_key(emx, s_gen, st->key[0], blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), tid);
+    const BfpTile t = bfp_tile(g, tid);
+    const int z0 = blockIdx.z * zc;
+    int mag = 0;
+    if(s_mode) {
+        const double c1 = c.c1 * __hiloint2double((1023 + s_lmu) << 20, 0);   // exact: |c1| is in [2^-100, 2^100] or 0
+        auto plane = [&](int z) { return (unsigned) (z & g.mask) << (2 * g.log2N); };
+        auto pair = [&](int z) {
+            const unsigned gi = plane(z) + t.gown;
+            return CHGB_BC(11, gi + 1, g.bins) ? *reinterpret_cast<const longlong2 *>(mu + gi) : make_longlong2(0, 0);
+        };
+        auto halo = [&](int z) {
+            return t.has_halo && CHGB_BC(12, plane(z) + t.ghalo, g.bins) ? mu[plane(z) + t.ghalo] : 0ll;
+        };
+        auto stage = [&](int z, longlong2 X, long long h) {
+            long long *p = ring[z & 1];
+            if(CHGB_BC(16, t.own + 1, BPLANE)) *reinterpret_cast<longlong2 *>(p + t.own) = X;
+            if(t.has_halo && CHGB_BC(16, t.halo, BPLANE)) p[t.halo] = h;
+        };
+        longlong2 Mm = pair(z0 - 1), Mc = pair(z0);
+        stage(z0, Mc, halo(z0));
+        longlong2 next = pair(z0 + 1);
+        long long hnext = zc > 1 ? halo(z0 + 1) : 0;
+        for(int z = z0; z < z0 + zc; z++) {
+            const unsigned gi = t.gown + plane(z);
+            const bool ok = CHGB_BC(17, gi + 1, g.bins);
+            const double2 psi = ok ? *reinterpret_cast<const double2 *>(psi_in + gi) : make_double2(0.0, 0.0);
+            __syncthreads();
+            const longlong2 Mp = next;
+            if(z + 1 < z0 + zc) {
+                stage(z + 1, Mp, hnext);
+                next = pair(z + 2);
+                if(z + 2 < z0 + zc) hnext = halo(z + 2);
+            }
+            long long sa, sb;
+            bfp_xy_sums<BPITCH>(ring[z & 1], t.own, Mc.x, Mc.y, sa, sb);
+            sa += (Mm.x + Mp.x) - 6 * Mc.x;
+            sb += (Mm.y + Mp.y) - 6 * Mc.y;
+            const double2 res = make_double2(fma(c1, bfp_double_fp(sa), psi.x), fma(c1, bfp_double_int(sb), psi.y));
+            if(ok) *reinterpret_cast<double2 *>(out + gi) = res;
+            mag = max(mag, max(__double2hiint(res.x) & 0x7FFFFFFF, __double2hiint(res.y) & 0x7FFFFFFF));
+            Mm = Mc;
+            Mc = Mp;
+        }
+    }
+    else {
+        mag = bfp_slow_block<3>(psi_in, out, g.mask, g.log2N, c.c1, c.c2[0], c.lshift[2], blockIdx.x * BTX,
+                                blockIdx.y * BTY, z0, BTX, BTY, zc);
+    }
+    bfp_fold_key<8>(mag, s_gen, st->key[parity ^ 1], blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), tid);
+}
+
+// 3D: one kernel per step.  A CTA owns a 32 x 16 tile and marches it through
+// `zc` planes: at plane z it stages X of plane z + 2, forms M of plane z + 1 on
+// the tile and a halo of 1, and updates plane z.  Each of 360 threads has one
+// pair of cells adjacent in x of the tile with a halo of 2 (18 pairs by 20
+// rows): its column of three X, and of three M, stays in registers, two planes
+// of X and two of M in shared memory serve the x and y neighbours, and there
+// is one barrier a plane.  All 360 convert their X, the first 324 form M, the
+// first 256 -- the tile -- update.  mu in integers made this the faster form: the
+// halo's M costs 1.27 x 27 integer instructions where it used to cost FP64
+// ones, and the step saves M's round trip through HBM (16 B a cell) and a
+// launch.  N = 256 on GB300, us a step: the pair with FP64 in mu 172, the pair
+// above 144, this kernel 116 (integer ALU 46 %, FP64 pipe 46 %, issue slots 59 %
+// busy; the barrier a plane and the shared loads are the larger stalls).
+constexpr int B3X = 32, B3Y = 16, B3P = B3X + 4, B3H = B3P / 2;   // tile, cells and pairs of a staged row
+constexpr int B3THREADS = 384, B3CTAS = 3;   // CTAs per SM: 56 registers a thread
+constexpr int B3OWN = B3X / 2 * B3Y, B3M = B3H * (B3Y + 2), B3ALL = B3H * (B3Y + 4);
+
+__global__ void __launch_bounds__(B3THREADS, B3CTAS) euler3d_bfp_kernel(const double *__restrict__ in,
+                                                                       double *__restrict__ out, Geom g, EulerConsts c,
+                                                                       BfpConsts b, BfpState *st, int parity, int zc) {
+    __shared__ __align__(16) long long sx[2][B3P * (B3Y + 4)], sm[2][B3P * (B3Y + 2)];
+    const int tid = threadIdx.x;
+    const int x0 = blockIdx.x * B3X, y0 = blockIdx.y * B3Y, z0 = blockIdx.z * zc;
+    const int z1 = min(z0 + zc, g.N);
+    pdl_begin();
+    const unsigned long long key = bfp_read_key(st->key[parity], tid);
+    const BfpScale sc = bfp_scale<3>((int) (key & 0xFFFFu), c, b);
+    int mag = 0;
+    if(sc.fast) {
+        int px, row;   // this thread's pair and row of the staged region
+        if(tid < B3OWN) {
+            px = 1 + tid % (B3X / 2);
+            row = 2 + tid / (B3X / 2);
+        }
+        else if(tid < B3OWN + 2 * B3H) {
+            const int k = tid - B3OWN;
+            px = k % B3H;
+            row = k < B3H ? 1 : B3Y + 2;
+        }
+        else if(tid < B3M) {
+            const int k = tid - (B3OWN + 2 * B3H);
+            px = k < B3Y ? 0 : B3H - 1;
+            row = 2 + k % B3Y;
+        }
+        else {
+            const int k = tid - B3M;
+            px = k % B3H;
+            row = k < B3H ? 0 : B3Y + 3;
+        }
+        const bool has = tid < B3ALL;
+        const int ix = row * B3P + 2 * px, im = ix - B3P;
+        const unsigned off = ((x0 - 2 + 2 * px) & g.mask) + ((unsigned) ((y0 - 2 + row) & g.mask) << g.log2N);
+        auto load = [&](int z) {
+            const unsigned gi = off + ((unsigned) (z & g.mask) << (2 * g.log2N));   // below 2^30
+            return has && CHGB_BC(11, gi + 1, g.bins) ? *reinterpret_cast<const double2 *>(in + gi) : make_double2(0.0, 0.0);
+        };
+        auto fixed = [&](double2 v) { return make_longlong2(bfp_fixed(v.x, sc.emax), bfp_fixed(v.y, sc.emax)); };
+        auto stage = [&](int z, longlong2 X) {
+            if(has && CHGB_BC(13, ix + 1, B3P * (B3Y + 4))) *reinterpret_cast<longlong2 *>(sx[z & 1] + ix) = X;
+        };
+        const double c1 = c.c1 * __hiloint2double((1023 + sc.lmu) << 20, 0);   // exact: |c1| is in [2^-100, 2^100] or 0
+        longlong2 Xa = fixed(load(z0 - 2)), Xb = fixed(load(z0 - 1));
+        stage(z0 - 1, Xb);
+        longlong2 Ma = make_longlong2(0, 0), Mb = Ma;
+        double2 next = load(z0), psi = make_double2(0.0, 0.0);
+#pragma unroll 3   // the columns' three planes turn without moves
+        for(int z = z0 - 2; z < z1; z++) {
+            __syncthreads();   // plane z + 1 of X and plane z of M staged; the planes before them read by every warp
+            const longlong2 Xc = fixed(next);
+            stage(z + 2, Xc);
+            if(z + 1 < z1) next = load(z + 3);
+            if(z >= z0 && tid < B3OWN) psi = load(z);   // in L2 (and L1): fetched three planes ago
+            longlong2 Mc = Ma;
+            if(tid < B3M && CHGB_BC(14, ix - B3P, B3P * (B3Y + 4)) && CHGB_BC(14, ix + B3P + 1, B3P * (B3Y + 4))) {
+                long long sa, sb;
+                bfp_xy_sums<B3P>(sx[(z + 1) & 1], ix, Xb.x, Xb.y, sa, sb);
+                Mc = make_longlong2(bfp_mu(Xb.x, sa + (Xa.x + Xc.x), sc), bfp_mu(Xb.y, sb + (Xa.y + Xc.y), sc));
+                *reinterpret_cast<longlong2 *>(sm[(z + 1) & 1] + im) = Mc;
+            }
+            if(z >= z0 && tid < B3OWN) {
+                const unsigned gi = off + ((unsigned) z << (2 * g.log2N));
+                long long sa, sb;
+                bfp_xy_sums<B3P>(sm[z & 1], im, Mb.x, Mb.y, sa, sb);
+                sa += (Ma.x + Mc.x) - 6 * Mb.x;
+                sb += (Ma.y + Mc.y) - 6 * Mb.y;
+                const double2 res = make_double2(fma(c1, bfp_double_fp(sa), psi.x), fma(c1, bfp_double_fp(sb), psi.y));
+                if(CHGB_BC(15, gi + 1, g.bins)) *reinterpret_cast<double2 *>(out + gi) = res;
+                mag = max(mag, max(__double2hiint(res.x) & 0x7FFFFFFF, __double2hiint(res.y) & 0x7FFFFFFF));
+            }
+            Xa = Xb;
+            Xb = Xc;
+            Ma = Mb;
+            Mb = Mc;
+        }
+    }
+    else {
+        mag = bfp_slow_block<3>(in, out, g.mask, g.log2N, c.c1, c.c2[0], c.lshift[2], x0, y0, z0, B3X, B3Y, z1 - z0);
+    }
+    bfp_fold_key<B3THREADS / 32>(mag, (key >> 16) + 1, st->key[parity ^ 1],
+                                 blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), tid);
 }
 
 // The key of the field psi (n values, n even): (0 << 16) | its largest biased
 // exponent, after the caller zeroed it.
 __global__ void __launch_bounds__(256) bfp_refresh_kernel(const double2 *__restrict__ psi, long long n2,
                                                           unsigned long long *bank) {
-    int e = 0;
+    int mag = 0;
     for(long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += (long long) gridDim.x * blockDim.x) {
         const double2 v = psi[i];
-        const int a = (int) ((unsigned long long) __double_as_longlong(v.x) >> 52) & 0x7FF;
-        const int b = (int) ((unsigned long long) __double_as_longlong(v.y) >> 52) & 0x7FF;
-        e = max(e, max(a, b));
+        mag = max(mag, max(__double2hiint(v.x) & 0x7FFFFFFF, __double2hiint(v.y) & 0x7FFFFFFF));
     }
-    bfp_fold_key(e, 0ull, bank, blockIdx.x, threadIdx.x);
+    bfp_fold_key<8>(mag, 0ull, bank, blockIdx.x, threadIdx.x);
 }
 
-// 2D: one kernel per step.  A CTA stages a 32 x 16 tile of psi with a halo of
-// 2 (and X of every staged value), forms M on the tile plus a halo of 1, then
-// updates the tile, two cells per thread.  The halo's M is formed by each CTA
-// that needs it from the same X, so the results are the pair's integers and
-// bits; what changes is one launch per step instead of two, and no M round
-// trip through memory.  The key is read from bank `parity` and the step's
-// exponents fold into the other bank (CTAs of one launch both read and fold).
-constexpr int F2X = 32;
-constexpr int F2SX = F2X + 4;                       // psi with a halo of 2: 36 x (F2Y + 4)
-constexpr int F2MX = F2X + 2;                       // M with a halo of 1: 34 x (F2Y + 2)
-template <int F2Y> struct F2Tile {
-    static constexpr int SP = F2SX * (F2Y + 4), MP = F2MX * (F2Y + 2);
-};
-
-template <int F2Y, bool FAST>
-__device__ __forceinline__ int euler2d_bfp_run(const double *__restrict__ in, double *__restrict__ out, const Geom &g,
-                                               const EulerConsts &c, const BfpConsts &b, int emax, int lmu,
-                                               double *sp, long long *sx, long long *sm) {
-    const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + STX * ty;
-    const int x0 = blockIdx.x * F2X, y0 = blockIdx.y * F2Y;
-    const int umu = lmu + 1080;                   // M = floor(mu 2^(1080 - umu))
-    const int rc = umu + 1021 - emax - b.ec;      // c2 sum: high product -> M's unit
-    const double ls = c.lshift[1];
-    const long long escale = (long long) lmu * (1ll << 52);
-    constexpr int F2SP = F2Tile<F2Y>::SP, F2MP = F2Tile<F2Y>::MP;
-    for(int i = tid; i < F2SP; i += STX * STY) {
-        const int ly = i / F2SX, lx = i - ly * F2SX;
-        const size_t gi = ((x0 - 2 + lx) & g.mask) + ((size_t) ((y0 - 2 + ly) & g.mask) << g.log2N);
-        const double v = CHGB_BC(21, gi, g.bins) ? in[gi] : 0.0;
-        sp[i] = v;
-        if constexpr(FAST) sx[i] = bfp_fixed(v, emax);
-    }
-    __syncthreads();
-    for(int j = tid; j < F2MP; j += STX * STY) {
-        const int my = j / F2MX, mx = j - my * F2MX;
-        const int q = (my + 1) * F2SX + mx + 1;
-        if(!CHGB_BC(22, q - F2SX, F2SP) || !CHGB_BC(22, q + F2SX, F2SP)) continue;
-        const double r = sp[q];
-        if constexpr(FAST) {
-            const long long sum = (sx[q - 1] + sx[q + 1]) + (sx[q - F2SX] + sx[q + F2SX]);
-            sm[j] = bfp_fixed(r * fma(r, r, ls), umu) - fx_sar(__mul64hi(sum, b.mc), rc);
-        }
-        else {
-            const double sum = seq_sum(sp[q - 1], sp[q + 1], sp[q - F2SX], sp[q + F2SX], 0.0, 0.0, 4);
-            reinterpret_cast<double *>(sm)[j] = fma(-c.c2[0], sum, r * fma(r, r, ls));
-        }
-    }
-    __syncthreads();
-    int emx = 0;
-#pragma unroll
-    for(int k = 0; k < F2Y / STY; k++) {
-        const int ly = ty + STY * k;
-        const int m = (ly + 1) * F2MX + tx + 1;
-        const size_t gi = (size_t) (x0 + tx) + ((size_t) (y0 + ly) << g.log2N);
-        if(!CHGB_BC(23, m - F2MX, F2MP) || !CHGB_BC(23, m + F2MX, F2MP) ||
-           !CHGB_BC(23, (ly + 2) * F2SX + tx + 2, F2SP) || !CHGB_BC(24, gi, g.bins))
-            continue;
-        const double psi0 = sp[(ly + 2) * F2SX + tx + 2];
-        double res;
-        if constexpr(FAST) {
-            long long L = (sm[m - 1] + sm[m + 1]) + (sm[m - F2MX] + sm[m + F2MX]);
-            L -= 4ll * sm[m];
-            const double ld = L == 0 ? 0.0
-                              : ((int) threadIdx.y < BFP_INT_ROUND_WARPS)
-                                  ? bfp_to_double_int(L, lmu)
-                                  : __longlong_as_double(__double_as_longlong(__ll2double_rn(L)) + escale);
-            res = fma(c.c1, ld, psi0);
-        }
-        else {
-            const double *u = reinterpret_cast<const double *>(sm);
-            res = fma(c.c1, fma(-4.0, u[m], seq_sum(u[m - 1], u[m + 1], u[m - F2MX], u[m + F2MX], 0.0, 0.0, 4)),
-                      psi0);
-        }
-        out[gi] = res;
-        const int e = (int) ((unsigned long long) __double_as_longlong(res) >> 52) & 0x7FF;
-        emx = e > emx ? e : emx;
-    }
-    return emx;
-}
-
-template <int F2Y>
-__global__ void __launch_bounds__(256, 8) euler2d_bfp_kernel(const double *__restrict__ in, double *__restrict__ out,
+// 2D: one kernel per step.  A CTA stages X of a TX x TY tile of psi with a halo
+// of 2, forms M on the tile plus a halo of 1, then updates the tile, everywhere
+// two cells adjacent in x at a time.  The halo's M is formed by each CTA that
+// needs it from the same X, so every CTA sees the same integers; there is one
+// launch per step and no M round trip through memory.  The key is read from
+// bank `parity` and the step's exponents fold into the other bank (CTAs of one
+// launch both read and fold).
+template <int TX, int TY>
+__global__ void __launch_bounds__(256, 4) euler2d_bfp_kernel(const double *__restrict__ in, double *__restrict__ out,
                                                              Geom g, EulerConsts c, BfpConsts b, BfpState *st,
                                                              int parity) {
-    __shared__ double sp[F2Tile<F2Y>::SP];
-    __shared__ long long sx[F2Tile<F2Y>::SP];
-    __shared__ long long sm[F2Tile<F2Y>::MP];   // M (mode 1) or mu's FP64 bits (mode 0)
-    const int tid = threadIdx.x + STX * threadIdx.y;
+    constexpr int P = TX + 4, H = P / 2;                // cells and pairs of a staged row
+    constexpr int NX = H * (TY + 4), NM = H * (TY + 2), NU = TX / 2 * TY;
+    // M is formed on whole pairs: the outermost cell of each row's ends reads
+    // into the neighbouring row and is not used
+    __shared__ __align__(16) long long sx[2 * NX], sm[2 * NM];
+    const int tid = threadIdx.x;
+    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     pdl_begin();
     const unsigned long long key = bfp_read_key(st->key[parity], tid);
-    const int emax = (int) (key & 0xFFFFu);
-    const int s = emax - 1022;                    // |psi| < 2^s
-    const int lmu = max(3 * s, b.elin + s) + 2 - 58;
-    const bool fast = emax >= 1 && emax <= 2046 && lmu >= -1000 && lmu <= 900;
-    const int emx = fast ? euler2d_bfp_run<F2Y, true>(in, out, g, c, b, emax, lmu, sp, sx, sm)
-                         : euler2d_bfp_run<F2Y, false>(in, out, g, c, b, emax, lmu, sp, sx, sm);
-    bfp_fold_key(emx, (key >> 16) + 1, st->key[parity ^ 1], blockIdx.x + gridDim.x * blockIdx.y, tid);
+    const BfpScale sc = bfp_scale<2>((int) (key & 0xFFFFu), c, b);
+    int mag = 0;
+    if(sc.fast) {
+#pragma unroll
+        for(int k = 0; k < (NX + 255) / 256; k++) {
+            const int i = tid + 256 * k;
+            if(i < NX) {
+                const int y = i / H, x = 2 * (i - y * H);
+                const unsigned gi = ((x0 - 2 + x) & g.mask) + ((unsigned) ((y0 - 2 + y) & g.mask) << g.log2N);
+                const double2 v = CHGB_BC(21, gi + 1, g.bins) ? *reinterpret_cast<const double2 *>(in + gi)
+                                                              : make_double2(0.0, 0.0);
+                *reinterpret_cast<longlong2 *>(sx + 2 * i) = make_longlong2(bfp_fixed(v.x, sc.emax), bfp_fixed(v.y, sc.emax));
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for(int k = 0; k < (NM + 255) / 256; k++) {
+            const int i = tid + 256 * k;
+            if(i < NM && CHGB_BC(22, 2 * i + 2 * P + 1, 2 * NX)) {
+                const longlong2 X = *reinterpret_cast<const longlong2 *>(sx + 2 * i + P);
+                long long sa, sb;
+                bfp_xy_sums<P>(sx, 2 * i + P, X.x, X.y, sa, sb);
+                *reinterpret_cast<longlong2 *>(sm + 2 * i) = make_longlong2(bfp_mu(X.x, sa, sc), bfp_mu(X.y, sb, sc));
+            }
+        }
+        __syncthreads();
+        const double c1 = c.c1 * __hiloint2double((1023 + sc.lmu) << 20, 0);   // exact: |c1| is in [2^-100, 2^100] or 0
+#pragma unroll
+        for(int k = 0; k < NU / 256; k++) {
+            const int i = tid + 256 * k;
+            const int y = i / (TX / 2), x = 2 * (i % (TX / 2));
+            const int m = (y + 1) * P + x + 2;
+            const unsigned gi = (unsigned) (x0 + x) + ((unsigned) (y0 + y) << g.log2N);
+            if(!CHGB_BC(23, m - P, 2 * NM) || !CHGB_BC(23, m + P + 1, 2 * NM) || !CHGB_BC(24, gi + 1, g.bins)) continue;
+            const double2 psi = *reinterpret_cast<const double2 *>(in + gi);
+            const longlong2 M = *reinterpret_cast<const longlong2 *>(sm + m);
+            long long sa, sb;
+            bfp_xy_sums<P>(sm, m, M.x, M.y, sa, sb);
+            const double2 res = make_double2(fma(c1, bfp_double_fp(sa - 4 * M.x), psi.x),
+                                             fma(c1, bfp_double_int(sb - 4 * M.y), psi.y));
+            *reinterpret_cast<double2 *>(out + gi) = res;
+            mag = max(mag, max(__double2hiint(res.x) & 0x7FFFFFFF, __double2hiint(res.y) & 0x7FFFFFFF));
+        }
+    }
+    else {
+        mag = bfp_slow_block<2>(in, out, g.mask, g.log2N, c.c1, c.c2[0], c.lshift[1], x0, y0, 0, TX, TY, 1);
+    }
+    bfp_fold_key<8>(mag, (key >> 16) + 1, st->key[parity ^ 1], blockIdx.x + gridDim.x * blockIdx.y, tid);
 }
 
 }  // namespace chgb
@@ -1777,58 +1846,86 @@ static BfpConsts bfp_consts(const EulerConsts &c, int dims) {
     b.ec = e ? e : 1;
     const double lin = std::fabs(c.lshift[dims - 1]) + 2.0 * dims * std::fabs(c2);
     b.elin = lin > 0.0 && std::isfinite(lin) ? std::ilogb(lin) + 1 : -4000;   // lin < 2^elin
+    // constants the integer step does not take (not finite, or so far from one
+    // that its scales would leave the exponent range) put every step in mode 0
+    const double a1 = std::fabs(c.c1);
+    const bool c1_ok = a1 == 0.0 || (a1 >= std::ldexp(1.0, -100) && a1 <= std::ldexp(1.0, 100));
+    if(!std::isfinite(lin) || (lin > 0.0 && b.elin < -800) || !c1_ok) b.elin = 100000;
     return b;
+}
+
+// Planes a CTA of the 3D step marches through: the chunk with the fewest plane
+// iterations (two of each chunk are its halo's) over the waves of CTAs that the
+// GPU holds.  Cell-steps/s on GB300: N = 256 37 planes (2 waves) 1.44e11, 32
+// (2.2 waves) 1.36e11, 16 1.25e11; N = 128 10 planes 1.03e11, 8 9.2e10, 16
+// 7.2e10; N = 512 64 planes 1.58e11, 32 1.52e11, 16 1.44e11.  N = 64, whose CTAs
+// never fill a wave, 4 planes 4.3e10, 2 3.2e10.
+static int bfp_zchunk(const Geom &g) {
+    if(g.N <= 64) return 4;
+    const long long tiles = (long long) (g.N / B3X) * (g.N / B3Y), slots = 152 * B3CTAS;
+    long long best = 0;
+    int pick = 8;
+    for(int zc = 8; zc <= 64; zc++) {
+        const long long ctas = tiles * ((g.N + zc - 1) / zc), cost = (ctas + slots - 1) / slots * (zc + 2);
+        if(best == 0 || cost < best) {
+            best = cost;
+            pick = zc;
+        }
+    }
+    return pick;
 }
 
 cudaError_t launch_euler_bfp(const Geom &g, const EulerConsts &c, const double *in, double *out, double *mu,
                              BfpState *st, int parity, cudaStream_t stream) {
     const BfpConsts b = bfp_consts(c, g.dims);
-    // z-chunk planes per CTA, measured on GB300 (cell-steps/s with 2, 4, 8, 16, 32
-    // planes): N=64 3.26, 3.07, 2.41, 1.43, 0.81e10; N=128 6.16, 7.27, 6.99,
-    // 6.91, 5.64e10; N=256 8.32e10 (4), 9.33e10 (8), 9.61e10 (16), 9.45e10 (32);
-    // N=512 7.07, 8.91, 10.1, 10.7, 11.0e10.  Small boxes want short columns
-    // (more CTAs, a shorter path through each), large ones long (fewer halo planes).
-    const int zc = (g.dims != 3) ? 1 : g.N <= 64 ? 2 : g.N == 128 ? 4 : g.N == 256 ? 16 : 32;
+    const int pair_zc = g.N <= 64 ? 2 : g.N == 128 ? 4 : g.N == 256 ? 16 : 32;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(g.N / STX, g.N / STY, (g.dims == 3) ? g.N / zc : 1);
-    cfg.blockDim = dim3(STX, STY);
+    cfg.blockDim = dim3(256);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    long long *m = reinterpret_cast<long long *>(mu);
     cudaError_t e;
     if(g.dims == 2) {
-        // one kernel per step; 32 x 16 tiles up to N = 1024, 32 x 32 above (2D
-        // on GB300, cell-steps/s: N=1024 8.29e10 against 8.12e10, N=2048
-        // 1.05e11 against 1.09e11, N=4096 1.12e11 against 1.16e11; the split
-        // pair ran 6.35e10, 7.49e10 and 7.50e10)
-        if(g.N >= 2048) {
-            cfg.gridDim = dim3(g.N / F2X, g.N / 32);
-            e = cudaLaunchKernelEx(&cfg, euler2d_bfp_kernel<32>, in, out, g, c, b, st, parity);
-        }
-        else {
-            cfg.gridDim = dim3(g.N / F2X, g.N / 16);
-            e = cudaLaunchKernelEx(&cfg, euler2d_bfp_kernel<16>, in, out, g, c, b, st, parity);
-        }
+        auto tile = [&](auto kernel, int tx, int ty) {
+            cfg.gridDim = dim3(g.N / tx, g.N / ty);
+            return cudaLaunchKernelEx(&cfg, kernel, in, out, g, c, b, st, parity);
+        };
+        // the largest tile that leaves every SM a CTA (halo work against
+        // CTAs).  Cell-steps/s on GB300 with 64 x 32, 32 x 32 and 64 x 16 tiles:
+        // N = 512 6.3e10 each, N = 1024 1.26, 1.18, 1.19e11; with 64 x 32
+        // and 64 x 16, N = 2048 1.78, 1.45e11, N = 4096 1.91, 1.48e11
+        if(g.N >= 1024) e = tile(euler2d_bfp_kernel<64, 32>, 64, 32);
+        else e = tile(euler2d_bfp_kernel<32, 32>, 32, 32);
     }
     else {
-        e = cudaLaunchKernelEx(&cfg, mu_bfp_kernel<3>, in, m, g, c, b, st, zc);
-        if(e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, update_bfp_kernel<3>, in, (const long long *) m, out, g, c, st, zc);
+        if(mu) {
+            cfg.gridDim = dim3(g.N / BTX, g.N / BTY, g.N / pair_zc);
+            long long *m = reinterpret_cast<long long *>(mu);
+            e = cudaLaunchKernelEx(&cfg, mu_bfp_kernel, in, m, g, c, b, st, parity, pair_zc);
+            if(e == cudaSuccess)
+                e = cudaLaunchKernelEx(&cfg, update_bfp_kernel, in, (const long long *) m, out, g, c, st, parity, pair_zc);
+        }
+        else {
+            const int zc = bfp_zchunk(g);
+            cfg.gridDim = dim3(g.N / B3X, g.N / B3Y, (g.N + zc - 1) / zc);
+            cfg.blockDim = dim3(B3THREADS);
+            e = cudaLaunchKernelEx(&cfg, euler3d_bfp_kernel, in, out, g, c, b, st, parity, zc);
+        }
     }
     return e;
 }
 
-cudaError_t launch_bfp_refresh(const double *psi, long long n, BfpState *st, int bank, cudaStream_t stream) {
+cudaError_t launch_bfp_refresh(const double *psi, long long n, BfpState *st, int parity, cudaStream_t stream) {
     // both banks: the 2D kernel folds into the other bank next, whose older
     // generations must not outrank the new sequence's
     cudaError_t e = cudaMemsetAsync(st->key, 0, sizeof st->key, stream);
     if(e != cudaSuccess) return e;
     const long long n2 = n / 2;
     const long long blocks = std::min<long long>((n2 + 255) / 256, 152 * 8);
-    bfp_refresh_kernel<<<(unsigned) blocks, 256, 0, stream>>>(reinterpret_cast<const double2 *>(psi), n2, st->key[bank]);
+    bfp_refresh_kernel<<<(unsigned) blocks, 256, 0, stream>>>(reinterpret_cast<const double2 *>(psi), n2, st->key[parity]);
     return cudaGetLastError();
 }
 

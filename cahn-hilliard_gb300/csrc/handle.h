@@ -46,10 +46,10 @@ struct chgb_handle {
     chgb::SpectralState *ps = nullptr;
     chgb::PsMob *psm = nullptr;            // pseudospectral_mobility state
     int variant = 1;               // 1 = fused kernel, 2 = split (mu stored once per cell), 3 = two steps per launch,
-                                   // 4 = the box resident in one cluster's shared memory, 5 = split in block fixed point
-    double *d_mu = nullptr;        // split variant: mu of every cell
+                                   // 4 = the box resident in one cluster's shared memory, 5 = block fixed point
+    double *d_mu = nullptr;        // split variants: mu of every cell (variant 5: its one-kernel steps have none)
     double *d_mobk = nullptr;      // split variant with the free-energy mobility: M of every cell
-    chgb::BfpState *d_bfp = nullptr;   // variant 5: the block-fixed-point key and this step's mu scale
+    chgb::BfpState *d_bfp = nullptr;   // variant 5: the block-fixed-point key, and the pair's mu scale
     chgb::SqPlan *sq = nullptr;            // S(q) shells, built on first use
     chgb::SpectralState *fft = nullptr;    // forward transform of euler boxes for S(q)
     std::string err;
