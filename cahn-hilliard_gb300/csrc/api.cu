@@ -53,15 +53,12 @@ static bool stream_is_capturing(cudaStream_t st) {
     return cs != cudaStreamCaptureStatusNone;
 }
 
-// The table of tab_log (common.cuh) on each device, made once per process and
-// kept for its lifetime (LOGTAB_N + 1 entries, 2 KB).  Entries are (1/c_j,
-// ln c_j) for c_j = 1 + (j + 1/2)/LOGTAB_N, rounded from long double, then
-// ln 2 split into a high part with eleven trailing zero bits (so that k times
-// it is exact for any double exponent k) and the rest.
+// The table of un_log (wertheim_fx.cuh) on each device, made once per process
+// and kept for its lifetime (4 KB).
 static std::mutex g_logtab_mutex;
-static std::map<int, double2 *> g_logtab;
+static std::map<int, UnLogEntry *> g_logtab;
 
-static const double2 *device_log_table(bool alloc) {
+static const UnLogEntry *device_log_table(bool alloc) {
     int dev = 0;
     if(cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
@@ -71,21 +68,16 @@ static const double2 *device_log_table(bool alloc) {
     auto it = g_logtab.find(dev);
     if(it != g_logtab.end()) return it->second;
     if(!alloc) return nullptr;
-    std::vector<double2> t(LOGTAB_N + 1);
-    for(int j = 0; j < LOGTAB_N; j++) {
-        const double c = 1.0 + (j + 0.5) / LOGTAB_N;   // exact
-        t[j] = make_double2(1.0 / c, (double) std::log((long double) c));
+    std::vector<UnLogEntry> t(UNLOG_N);
+    for(int j = 0; j < UNLOG_N; j++) {
+        const double c = 1.0 + (j + 0.5) / UNLOG_N;   // exact
+        t[j].inv = (uint32_t) std::llround(2147483648.0 / c);
+        t[j].pad = 0;
+        t[j].ln = (int64_t) std::llround(-std::log((long double) t[j].inv / 2147483648.0L) * 1152921504606846976.0L);
     }
-    const long double ln2 = std::log(2.0L);
-    double hi = (double) ln2;
-    uint64_t bits;
-    std::memcpy(&bits, &hi, sizeof bits);
-    bits &= ~((uint64_t) 0x7FF);
-    std::memcpy(&hi, &bits, sizeof bits);
-    t[LOGTAB_N] = make_double2(hi, (double) (ln2 - (long double) hi));
-    double2 *d = nullptr;
-    if(cudaMalloc(&d, sizeof(double2) * t.size()) != cudaSuccess ||
-       cudaMemcpy(d, t.data(), sizeof(double2) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    UnLogEntry *d = nullptr;
+    if(cudaMalloc(&d, sizeof(UnLogEntry) * t.size()) != cudaSuccess ||
+       cudaMemcpy(d, t.data(), sizeof(UnLogEntry) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
         if(d) cudaFree(d);
         return nullptr;
@@ -152,6 +144,7 @@ ModelDev make_model_dev(const chgb_model_params &mp, bool with_log_table) {
     m.dAA = mp.delta_AA;
     m.dBB = mp.delta_BB;
     m.dcf = mp.density_conversion_factor;
+    m.sw_fx = m.four_valence_delta > 0.0 && mp.valence >= 1 && mp.valence <= 64 && mp.regularisation_delta >= 0.0;
     m.logtab = mp.kind == CHGB_MODEL_LANDAU ? nullptr : device_log_table(with_log_table);
     return m;
 }

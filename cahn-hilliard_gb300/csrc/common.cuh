@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include "../../include/chgb.h"
+#include "wertheim_fx.cuh"
 
 namespace chgb {
 
@@ -30,12 +31,11 @@ struct ModelDev {
     double dAA, dBB;
     double dcf;                     // density conversion factor
     int ivalence;
-    // table of tab_log (LOGTAB_N entries (1/c_j, ln c_j), then (ln 2 high, low)),
-    // in device memory; nullptr: f' takes the library's log instead
-    const double2 *logtab;
+    int sw_fx;                      // simple_wertheim: the integer path (sw_cell) takes the constants
+    // table of un_log in device memory; nullptr: the FP64 formulas and the
+    // library's log instead
+    const UnLogEntry *logtab;
 };
-
-constexpr int LOGTAB_N = 128;
 
 // with_log_table = false never allocates (the table is used if an earlier
 // call made it for the current device).
@@ -122,39 +122,31 @@ __device__ __forceinline__ double div_known(double x, double d, double y) {
     return fma(r, y, q0);
 }
 
-// ln x by table lookup and a short polynomial, after P. T. P. Tang,
-// "Table-driven implementation of the logarithm function in IEEE
-// floating-point arithmetic", ACM TOMS 16 (1990): x = 2^k y with y in [1, 2),
-// c_j = 1 + (j + 1/2)/128 for the top seven mantissa bits j of y, and
-//     ln x = k ln 2 + ln c_j + ln(1 + r),  r = (y - c_j) / c_j,  |r| <= 2^-8,
-// y - c_j exact, ln(1 + r) by its Taylor polynomial to r^7 (truncation below
-// 2^-67).  13 FP64 instructions against 29 for the library's log (measured
-// with ncu on GB300).  The error stays below 2 ulp of the result, or of 1.0
-// where |ln x| < 1 (near x = 1 k ln 2 and ln c_j cancel; the f' terms fed are of
-// order 10).  Zero,
-// negative, subnormal, infinite and NaN arguments -- and a missing table --
-// take the library's log.
+// ln a in units of 2^-53 (wertheim_fx.cuh) through the device's table.
+__device__ __forceinline__ int64_t un_log_tab(Un a, const UnLogEntry *__restrict__ tab) {
+    return un_log(a, [tab](int j, uint32_t &inv, int64_t &ln) {
+        const int4 t = __ldg(reinterpret_cast<const int4 *>(tab + j));
+        inv = (uint32_t) t.x;
+        ln = (int64_t) (((uint64_t) (uint32_t) t.w << 32) | (uint32_t) t.z);
+    });
+}
+constexpr double UNLOG_UNIT = 1.1102230246251565e-16;   // 2^-53
+
+// A double the integer path takes: positive, finite, normal, its exponent far
+// from the range's ends (products of a few stay normal).
+__device__ __forceinline__ bool un_takes(double x) {
+    return (unsigned) (__double2hiint(x) >> 20) - 600u < 900u;   // 2^-423 .. 2^476; the sign bit fails it
+}
+__device__ __forceinline__ Un un_of(double x) { return un_from_bits((uint64_t) __double_as_longlong(x)); }
+
+// ln x: one FP64-pipe conversion and a product; 13 FP64 instructions in FP64
+// with a table, 29 in the library's log.  Within 2^-52 absolute, and half an
+// ulp of the rounding.
 __device__ __noinline__ static double log_fallback(double x) { return log(x); }
 
-__device__ __forceinline__ double tab_log(double x, const double2 *__restrict__ tab) {
-    const unsigned long long u = (unsigned long long) __double_as_longlong(x);
-    const unsigned se = (unsigned) (u >> 52);   // sign and biased exponent
-    if(tab == nullptr || se - 1u >= 2046u) return log_fallback(x);
-    const int j = (int) (u >> 45) & (LOGTAB_N - 1);
-    const double y = __longlong_as_double((long long) ((u & 0xFFFFFFFFFFFFFull) | 0x3FF0000000000000ull));
-    const double c = __longlong_as_double(
-        (long long) (0x3FF0000000000000ull | ((unsigned long long) j << 45) | (1ull << 44)));
-    const double2 t = __ldg(&tab[j]);
-    const double2 ln2 = __ldg(&tab[LOGTAB_N]);
-    const double r = (y - c) * t.x;
-    double q = fma(r, 1.0 / 7.0, -1.0 / 6.0);
-    q = fma(q, r, 1.0 / 5.0);
-    q = fma(q, r, -0.25);
-    q = fma(q, r, 1.0 / 3.0);
-    q = fma(q, r, -0.5);
-    const double p = fma(r * r, q, r);
-    const double k = (double) ((int) se - 1023);
-    return fma(k, ln2.x, t.y) + fma(k, ln2.y, p);
+__device__ __forceinline__ double fx_log(double x, const UnLogEntry *__restrict__ tab) {
+    if(tab == nullptr || !un_takes(x)) return log_fallback(x);
+    return (double) un_log_tab(un_of(x), tab) * UNLOG_UNIT;
 }
 
 // e^x by table lookup and a short polynomial, after P. T. P. Tang,
@@ -200,11 +192,20 @@ __device__ __forceinline__ double sw_X(const ModelDev &m, double rho) {
 }
 
 // X of one Saleh species pair, src/models/SalehWertheim.cpp:80-85; returns log X.
+__device__ __noinline__ static double saleh_log_X_fp(double rho_factor) {
+    const double X = (-1.0 + sqrt(1.0 + 4.0 * rho_factor)) * fast_rcp(2.0 * rho_factor);
+    return (rho_factor >= 0) ? log(X) : 0.0;
+}
+
 __device__ __forceinline__ double saleh_log_X(double delta, double v, double rho_s, double half, double rho_linker,
-                                              const double2 *tab) {
-    double rho_factor = delta * (v * rho_s + half * rho_linker);
-    double X = (-1.0 + sqrt(1.0 + 4.0 * rho_factor)) * fast_rcp(2.0 * rho_factor);
-    return (rho_factor >= 0) ? tab_log(X, tab) : 0.0;
+                                              const UnLogEntry *tab) {
+    const double rho_factor = delta * (v * rho_s + half * rho_linker);
+    // the exponent also bounds 4 rho_factor below 2^60
+    if(tab == nullptr || !un_takes(rho_factor) || rho_factor >= 0x1p57) return saleh_log_X_fp(rho_factor);
+    const double t = 4.0 * rho_factor;
+    Un X;
+    if(!un_X((uint64_t) __double_as_longlong(1.0 + t), un_of(t), X)) return saleh_log_X_fp(rho_factor);
+    return (double) un_log_tab(X, tab) * UNLOG_UNIT;
 }
 
 // f'(rho) of all S species of one cell: r[s] in, d[s] out.
@@ -218,23 +219,46 @@ __device__ __forceinline__ void der_bulk<CHGB_MODEL_LANDAU>(const ModelDev &m, c
     d[0] = op * fma(op, op, -m.epsilon);   // two FP64 instructions, two roundings
 }
 
-// f' of simple_wertheim for a given X(rho), src/models/SimpleWertheim.cpp:40-53
-__device__ __forceinline__ double sw_der_given_X(const ModelDev &m, double rho, double X) {
-    double der_f_ref = m.two_B2 * rho;
+// f' of a simple_wertheim cell (src/models/SimpleWertheim.cpp:40-53) and rho
+// X^v, which the free-energy mobility takes (:104-111).
+struct SwCell {
+    double der, rhoXv;
+};
+
+__device__ __noinline__ static SwCell sw_cell_fp(const ModelDev &m, double rho) {
+    const double X = sw_X(m, rho);
+    SwCell c;
+    c.rhoXv = rho * ipow(X, m.ivalence);
+    c.der = m.two_B2 * rho;
     if(rho < m.reg_delta) {
-        der_f_ref += m.log_delta + (rho - m.reg_delta) / m.reg_delta;
-        double der_f_bond = (rho > 0.) ? m.valence * log(X) : 0.0;
-        return der_f_ref + der_f_bond;
+        c.der += m.log_delta + (rho - m.reg_delta) / m.reg_delta;
+        c.der += (rho > 0.) ? m.valence * log(X) : 0.0;
     }
-    // log(rho) + valence log(X) as one logarithm, log(rho X^valence): the
-    // same value to round-off for one logarithm's FP64 work instead of two
-    return der_f_ref + tab_log(rho * ipow(X, m.ivalence), m.logtab);
+    else c.der += log(c.rhoXv);
+    return c;
+}
+
+// log(rho) + valence log(X) as one logarithm, log(rho X^valence).  In integers
+// (wertheim_fx.cuh) for densities at or above the regularisation that the path
+// takes: 5 FP64 instructions a cell instead of 40.
+__device__ __forceinline__ SwCell sw_cell(const ModelDev &m, double rho) {
+    const long long b = __double_as_longlong(rho);
+    if(!m.sw_fx || m.logtab == nullptr || !un_takes(rho) || b < __double_as_longlong(m.reg_delta)) return sw_cell_fp(m, rho);
+    const double t = m.four_valence_delta * rho;
+    Un X;
+    if(!un_takes(t) || t >= 0x1p59 || !un_X((uint64_t) __double_as_longlong(1.0 + t), un_of(t), X)) return sw_cell_fp(m, rho);
+    const Un P = un_mul(un_of(rho), un_pow(X, m.ivalence));
+    if(P.e < -1000) return sw_cell_fp(m, rho);
+    SwCell c;
+    c.rhoXv = __longlong_as_double((long long) un_to_bits(P));
+    c.der = fma((double) un_log_tab(P, m.logtab), UNLOG_UNIT, m.two_B2 * rho);
+    return c;
 }
 
 // src/models/SimpleWertheim.cpp:40-53
 template <>
 __device__ __forceinline__ void der_bulk<CHGB_MODEL_SIMPLE_WERTHEIM>(const ModelDev &m, const double *r, double *d) {
-    d[0] = sw_der_given_X(m, r[0], sw_X(m, r[0]));
+    d[0] = sw_cell(m, r[0]).der;
 }
 
 // src/models/SalehWertheim.cpp:87-109.  A species whose density is exactly
@@ -246,19 +270,14 @@ __device__ __forceinline__ void der_bulk<CHGB_MODEL_SALEH>(const ModelDev &m, co
     double b3 = 3.0 * m.B3 * (rho_tot * rho_tot);
     double lx0 = saleh_log_X(m.dAA, m.sv0, r[0], m.half, r[2], m.logtab);
     double lx1 = saleh_log_X(m.dBB, m.sv1, r[1], m.half, r[2], m.logtab);
-    d[0] = (r[0] != 0.) ? ((tab_log(r[0], m.logtab) + b2) + b3) + m.sv0 * lx0 : 0.0;
-    d[1] = (r[1] != 0.) ? ((tab_log(r[1], m.logtab) + b2) + b3) + m.sv1 * lx1 : 0.0;
-    d[2] = (r[2] != 0.) ? ((tab_log(r[2], m.logtab) + b2) + b3) + m.half * (lx0 + lx1) : 0.0;
+    d[0] = (r[0] != 0.) ? ((fx_log(r[0], m.logtab) + b2) + b3) + m.sv0 * lx0 : 0.0;
+    d[1] = (r[1] != 0.) ? ((fx_log(r[1], m.logtab) + b2) + b3) + m.sv1 * lx1 : 0.0;
+    d[2] = (r[2] != 0.) ? ((fx_log(r[2], m.logtab) + b2) + b3) + m.half * (lx0 + lx1) : 0.0;
 }
 
 // Free-energy mobility M0 * rho * X^valence, src/models/SimpleWertheim.cpp:104-111.
-__device__ __forceinline__ double sw_mobility_given_X(const ModelDev &m, double M0, double rho, double X) {
-    double D = M0 * ipow(X, m.ivalence);
-    return rho * D;
-}
-
 __device__ __forceinline__ double sw_mobility(const ModelDev &m, double M0, double rho) {
-    return sw_mobility_given_X(m, M0, rho, sw_X(m, rho));
+    return M0 * sw_cell(m, rho).rhoXv;
 }
 
 // Bulk free-energy density f(rho) of one cell (r[s] for all species).

@@ -44,13 +44,13 @@ int mobility_kind(int mobility_type) {
 }
 
 // f' of one cell; with the free-energy mobility of simple_wertheim it also
-// returns X(rho), which the mobility of the same cell reuses.
+// returns rho X^v, which the mobility of the same cell reuses.
 template <int KIND, int MOB>
 __device__ __forceinline__ double der_bulk_x(const ModelDev &m, const double *r, double *d) {
     if constexpr(KIND == CHGB_MODEL_SIMPLE_WERTHEIM && MOB == 2) {
-        const double X = sw_X(m, r[0]);
-        d[0] = sw_der_given_X(m, r[0], X);
-        return X;
+        const SwCell c = sw_cell(m, r[0]);
+        d[0] = c.der;
+        return c.rhoXv;
     }
     else {
         der_bulk<KIND>(m, r, d);
@@ -59,13 +59,13 @@ __device__ __forceinline__ double der_bulk_x(const ModelDev &m, const double *r,
 }
 
 // The mobility of one cell for the template mobility kind: 1 constant, 2 the
-// free-energy mobility of the cell's density (X from der_bulk_x), 3 the field
+// free-energy mobility of the cell's density (rho X^v from der_bulk_x), 3 the field
 // computed before the step (regularised / gel; `gi` is the cell's index in one
 // species' field).
 template <int MOB>
-__device__ __forceinline__ double cell_mobility(const ModelDev &m, const EulerConsts &c, int s, double r, double X,
+__device__ __forceinline__ double cell_mobility(const ModelDev &m, const EulerConsts &c, int s, double r, double rhoXv,
                                                 size_t bins, size_t gi) {
-    if constexpr(MOB == 2) return sw_mobility_given_X(m, c.M, r, X);
+    if constexpr(MOB == 2) return c.M * rhoXv;
     else if constexpr(MOB == 3) return CHGB_BC(40, gi, bins) ? c.mobf[s * bins + gi] : 0.0;
     else return c.M;
 }
@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(256, (KIND == CHGB_MODEL_LANDAU && MOB == 0) ?
                 sum = (DIMS == 3) ? nb_sum6(q[-1], q[1], q[-SPX], q[SPX], ring[(z + 2) % 3][s][p], ring[(z + 1) % 3][s][p])
                                   : nb_sum4(q[-1], q[1], q[-SPX], q[SPX]);
             if(CHGB_BC(4, gi, bins)) mu[s * bins + gi] = mu_cell<KIND, DIMS>(m, c, s, r[s], d[s], sum);
-            if(MOB == 2) mob[s * bins + gi] = sw_mobility_given_X(m, c.M, r[s], xsw);
+            if(MOB == 2) mob[s * bins + gi] = c.M * xsw;
         }
         __syncthreads();
     }

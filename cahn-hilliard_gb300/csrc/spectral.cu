@@ -278,7 +278,7 @@ __device__ __forceinline__ void row_fprime(double2 (&r)[E], const ModelDev &m, c
                         const double rho_tot = ((0. + (h ? r0.y : r0.x)) + (h ? r1.y : r1.x)) + (h ? r2.y : r2.x);
                         const double b2 = m.two_B2 * rho_tot, b3 = 3.0 * m.B3 * (rho_tot * rho_tot);
                         const double own = h ? o.y : o.x;
-                        const double f = (own != 0.) ? ((tab_log(own, m.logtab) + b2) + b3) + v * (h ? l.y : l.x) : 0.0;
+                        const double f = (own != 0.) ? ((fx_log(own, m.logtab) + b2) + b3) + v * (h ? l.y : l.x) : 0.0;
                         if(h) d.y = f;
                         else d.x = f;
                     }
