@@ -86,14 +86,12 @@ static const UnLogEntry *device_log_table(bool alloc) {
     return d;
 }
 
-// The table of tab_exp (common.cuh) on each device, made once per process
-// and kept for its lifetime (EXPTAB_N + 2 entries, 1 KB): (lead, trail) of
-// 2^(j/64) rounded from long double, then ln2/64 split into L1 (37
-// significant bits) and L2, then 64/ln2.
+// The table of un_expneg (wertheim_fx.cuh) on each device, made once per
+// process and kept for its lifetime (2 KB).
 static std::mutex g_exptab_mutex;
-static std::map<int, double2 *> g_exptab;
+static std::map<int, uint64_t *> g_exptab;
 
-static const double2 *device_exp_table() {
+static const uint64_t *device_exp_table() {
     int dev = 0;
     if(cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
@@ -102,19 +100,12 @@ static const double2 *device_exp_table() {
     std::lock_guard<std::mutex> lock(g_exptab_mutex);
     auto it = g_exptab.find(dev);
     if(it != g_exptab.end()) return it->second;
-    std::vector<double2> t(EXPTAB_N + 2);
-    for(int j = 0; j < EXPTAB_N; j++) {
-        const long double v = std::exp2((long double) j / EXPTAB_N);
-        const double lead = (double) v;
-        t[j] = make_double2(lead, (double) (v - (long double) lead));
-    }
-    const long double L = std::log(2.0L) / EXPTAB_N;              // in [2^-7, 2^-6)
-    const long double L1 = std::floor(std::ldexp(L, 43)) / std::ldexp(1.0L, 43);   // 37 significant bits
-    t[EXPTAB_N] = make_double2((double) L1, (double) (L - L1));
-    t[EXPTAB_N + 1] = make_double2((double) (EXPTAB_N / std::log(2.0L)), 0.0);
-    double2 *d = nullptr;
-    if(cudaMalloc(&d, sizeof(double2) * t.size()) != cudaSuccess ||
-       cudaMemcpy(d, t.data(), sizeof(double2) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    std::vector<uint64_t> t(UNEXP_N);
+    for(int j = 0; j < UNEXP_N; j++)
+        t[j] = (uint64_t) (std::exp2(-(long double) j / UNEXP_N) * 9223372036854775808.0L + 0.5L);
+    uint64_t *d = nullptr;
+    if(cudaMalloc(&d, sizeof(uint64_t) * t.size()) != cudaSuccess ||
+       cudaMemcpy(d, t.data(), sizeof(uint64_t) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
         if(d) cudaFree(d);
         return nullptr;
@@ -309,19 +300,23 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
     h->md.type = params->mobility_type;
     h->md.M = params->M;
     h->md.rho_min = params->rho_min;
-    {
-        // src/mobility/GelMobility.h:20-27
-        const double e = std::exp(params->gel_beta_delta_F);
-        h->md.p_gel = e / (1.0 + e);
-    }
-    h->md.phi_critical = params->gel_phi_critical;
     h->md.c0 = params->gel_c0;
-    h->md.M_c = params->gel_M_c;
-    h->md.dt = params->dt;
-    h->md.one_m_phic = 1.0 - params->gel_phi_critical;
-    h->md.inv_one_m_phic = 1.0 / h->md.one_m_phic;
-    h->md.inv_c0 = 1.0 / params->gel_c0;
-    h->md.exptab = params->mobility_type == CHGB_MOBILITY_GEL ? device_exp_table() : nullptr;
+    if(params->mobility_type == CHGB_MOBILITY_GEL) {
+        // src/mobility/GelMobility.h:20-27, 41-58: phi = (rho + 1) / 2, g = (p phi -
+        // phi_c) / (1 - phi_c), c += dt M_c (g c - c^2), M = exp(-c / c_0)
+        const long double ex = std::exp((long double) params->gel_beta_delta_F);
+        const long double p = std::isinf(ex) ? 1.0L : ex / (1.0L + ex), q = 1.0L - params->gel_phi_critical;
+        h->md.g_a = (double) (0.5L * p / q);
+        h->md.g_b = (double) ((0.5L * p - params->gel_phi_critical) / q);
+        h->md.Mdt = params->gel_M_c * params->dt;
+        const long double K = 1.0L / ((long double) params->gel_c0 * std::log(2.0L));
+        if(K > 1e-100L && K < 1e100L) {
+            int x;
+            const long double f = std::frexp(K, &x);   // [1/2, 1)
+            h->md.K = Un{(uint64_t) (f * 18446744073709551616.0L), x - 1};
+            h->md.exptab = device_exp_table();
+        }
+    }
 
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if(e != cudaSuccess) {

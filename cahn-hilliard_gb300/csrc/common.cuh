@@ -64,18 +64,17 @@ struct EulerConsts {
 struct MobilityDev {
     int type;                       // CHGB_MOBILITY_REGULARISED or CHGB_MOBILITY_GEL
     double M, rho_min;              // regularised
-    double p_gel, phi_critical, c0, M_c, dt;   // gel
-    double one_m_phic, inv_one_m_phic, inv_c0;  // 1 - phi_c and the reciprocals of the gel's two divisors
-    const double2 *exptab;          // table of tab_exp (null: the library's exp)
+    double c0;                      // gel
+    // gel, folded: g = g_a rho + g_b is (p phi - phi_c) / (1 - phi_c) with phi =
+    // (rho + 1) / 2, the order parameter's step c + Mdt c (g - c)
+    double g_a, g_b, Mdt;
+    Un K;                           // 1 / (c0 ln 2)
+    const uint64_t *exptab;         // table of un_expneg (null: the library's exp)
 };
 
-constexpr int EXPTAB_N = 64;   // tab_exp: 2^(j/64) for j < 64, then two rows of constants
-
-// (0 + i k) z, as std::complex<double> evaluates it: the wave-vector factor of
-// a spectral derivative (src/integrators/PseudospectralMobilityCPU.cpp:258-263)
-__device__ __forceinline__ double2 mul_ik(double k, double2 z) {
-    return make_double2(0.0 * z.x - k * z.y, 0.0 * z.y + k * z.x);
-}
+// i k z: the wave-vector factor of a spectral derivative
+// (src/integrators/PseudospectralMobilityCPU.cpp:258-263)
+__device__ __forceinline__ double2 mul_ik(double k, double2 z) { return make_double2(-k * z.y, k * z.x); }
 
 // ---------------------------------------------------------------------------
 // Models.  Each formula follows the reference's CPU code (the oracle); the
@@ -109,13 +108,13 @@ __device__ __forceinline__ double fast_rcp(double x) {
     return fma(y, e, y);
 }
 
-// x / d for a divisor d known in advance, y = RN(1/d): q0 = RN(x y), the
-// remainder x - q0 d exact by one FMA, then q = RN(q0 + r y) -- division by a
-// constant with one correction step (P. Markstein, "IA-64 and Elementary
-// Functions", 2000; N. Brisebarre, J.-M. Muller and S. K. Raina, IEEE Trans.
-// Computers 53 (2004)).  The correctly rounded quotient for all but rare
-// (x, d) pairs, and within 1 ulp of it always, for three FP64 instructions
-// against about ten for a division.  x infinite gives NaN, not infinity.
+// x / d by the reciprocal y of d (within 2 ulp): q0 = RN(x y), the remainder x -
+// q0 d exact by one FMA, then q = RN(q0 + r y) -- a division with one
+// correction step (P. Markstein, "IA-64 and Elementary Functions", 2000;
+// N. Brisebarre, J.-M. Muller and S. K. Raina, IEEE Trans. Computers 53
+// (2004)).  The correctly rounded quotient for all but rare (x, d) pairs, and
+// within 1 ulp of it always, for three FP64 instructions against about ten
+// for a division.  x infinite gives NaN, not infinity.
 __device__ __forceinline__ double div_known(double x, double d, double y) {
     const double q0 = x * y;
     const double r = fma(-q0, d, x);
@@ -149,40 +148,18 @@ __device__ __forceinline__ double fx_log(double x, const UnLogEntry *__restrict_
     return (double) un_log_tab(un_of(x), tab) * UNLOG_UNIT;
 }
 
-// e^x by table lookup and a short polynomial, after P. T. P. Tang,
-// "Table-driven implementation of the exponential function in IEEE
-// floating-point arithmetic", ACM TOMS 15 (1989), with 64 table entries:
-//     x = (64 m + j) ln2/64 + r,  |r| <= ln2/128 (plus rounding),
-//     e^x = 2^m 2^(j/64) (1 + p(r)),  p(r) = e^r - 1 by its Taylor polynomial
-// to r^6 (truncation below 2^-64).  n = 64 m + j comes from adding 1.5 2^52 to
-// x 64/ln2 (round to nearest); r = x - n L1 - n L2 with ln2/64 = L1 + L2, L1
-// of 37 significant bits, so that x - n L1 is exact (Sterbenz).  2^(j/64) is
-// a pair (lead, trail); e^x = 2^m (lead + (trail + lead p)), and 2^m enters
-// through the exponent field.  12 FP64 instructions; the error stays below
-// 0.52 ulp plus the table's rounding (checked against an exact model on the
-// CPU).  |x| > 700 (the result near the ends of the normal range or beyond),
-// NaN and a missing table take the library's exp.  Table: EXPTAB_N entries
-// (lead, trail), then (L1, L2), then (64/ln2, 0).
+// e^(-c/c0) of the gel mobility: in integers (wertheim_fx.cuh) up to c/c0 of
+// at least 177 (t below 512 by its exponent, so at most 354), 1 where |c/c0| is below 2^-59, the
+// library's exp for the rest: larger ones, negative c, NaN.
 __device__ __noinline__ static double exp_fallback(double x) { return exp(x); }
 
-__device__ __forceinline__ double tab_exp(double x, const double2 *__restrict__ tab) {
-    const unsigned long long a = (unsigned long long) __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
-    if(tab == nullptr || a > 0x4085E00000000000ull) return exp_fallback(x);   // |x| > 700 or NaN
-    const double2 L = __ldg(&tab[EXPTAB_N]);
-    const double2 K = __ldg(&tab[EXPTAB_N + 1]);
-    constexpr double SHIFT = 6755399441055744.0;   // 1.5 2^52
-    const double t = fma(x, K.x, SHIFT);
-    const int n = (int) __double2loint(t);
-    const double nd = t - SHIFT;
-    const double r = fma(-nd, L.y, fma(-nd, L.x, x));
-    double q = fma(r, 1.0 / 720.0, 1.0 / 120.0);
-    q = fma(q, r, 1.0 / 24.0);
-    q = fma(q, r, 1.0 / 6.0);
-    q = fma(q, r, 0.5);
-    const double p = fma(r * r, q, r);
-    const double2 sj = __ldg(&tab[n & (EXPTAB_N - 1)]);
-    const double v = sj.x + fma(sj.x, p, sj.y);
-    return __longlong_as_double(__double_as_longlong(v) + ((long long) (n >> 6) << 52));
+__device__ __forceinline__ double gel_exp(const MobilityDev &md, double c) {
+    const uint64_t *tab = md.exptab;
+    const int e = ((__double2hiint(c) >> 20) & 0x7FF) - 1023 + md.K.e;   // c/c0 < 2^(e+2) ln 2
+    if(tab != nullptr && un_takes(c) && e <= 7)
+        return __longlong_as_double((long long) un_to_bits(un_expneg(un_of(c), md.K, [tab](int j) { return __ldg(tab + j); })));
+    if(tab != nullptr && e < -60) return 1.0;
+    return exp_fallback(-(c / md.c0));
 }
 
 // X(rho) of src/models/SimpleWertheim.cpp:88-90 (the division by the fast

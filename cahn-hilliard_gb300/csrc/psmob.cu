@@ -17,9 +17,10 @@
 // r2c's row pass, mu on its last column pass, i k_d on the first inverse column
 // pass of a flux's c2r, the flux itself between the c2r and r2c of one row
 // pass, the divergence on the last forward column pass, the update on the
-// final c2r's first column pass -- 2D: 12 launches a step instead of 22.  1D
-// uses the elementwise kernels below.  Both are written in the reference's
-// order of operations and give the same bits.  A constant mobility makes every
+// final c2r's first column pass -- 2D: 12 launches a step instead of 22.  The
+// passes contract their products and sums and divide through one reciprocal;
+// 1D uses the elementwise kernels below, in the reference's order of
+// operations (the two agree to rounding).  A constant mobility makes every
 // flux exactly zero, so those stages are skipped.
 #include <cmath>
 #include <vector>
@@ -315,7 +316,7 @@ cudaError_t psmob_set_rho(PsMob *s, const double *rho, cudaStream_t st, int64_t 
 PsmobTables psmob_tables(const PsMob *s) { return PsmobTables{s->q2, s->dealias, s->p.use_dealias ? 1 : 0}; }
 
 // 2D and 3D: the pointwise stages ride on the transforms' column and row passes
-// (spectral_psmob_*), the same arithmetic in the same order.
+// (spectral_psmob_*).
 static cudaError_t psmob_step_fused(PsMob *s, const double *mob, double *rho, cudaStream_t st, int64_t *launches) {
     const PsmobTables t = psmob_tables(s);
     int nl = 0;

@@ -152,11 +152,11 @@ __device__ __forceinline__ void fx_row_c2r(double2 (&r)[E], const double2 *__res
 // r2c of one packed real row r[i] to its half spectrum dst[0..M], the
 // post-processing X[k] = (a + t) / 2, X[M-k] = conj(a - t) / 2 with
 // a = Z[k] + conj Z[M-k], t = w^k (-i) (Z[k] - conj Z[M-k]), two modes to a
-// product as above; the halving is folded into the output scale.
+// product as above; the halving is folded into the output scale, and 2^-down.
 template <int E>
 __device__ __forceinline__ void fx_row_r2c(double2 (&r)[E], double2 *__restrict__ dst, bool active,
                                            const FxLine &ln, fx2 *&cur, fx2 *&oth, const int4 *__restrict__ twf,
-                                           int *sm_w) {
+                                           int *sm_w, int down = 0) {
     const int M = 1 << ln.lg, np = min(E, M) / 2;
     int mag = 0;
 #pragma unroll
@@ -174,7 +174,7 @@ __device__ __forceinline__ void fx_row_r2c(double2 (&r)[E], double2 *__restrict_
     for(int i = 0; i < E; i++)
         if(i < M) cur[a0 + i * ln.step(ln.T)] = v[i];
     ln.sync();
-    s.sh += 1;
+    s.sh += 1 + down;
     double2 x[E + 1];
 #pragma unroll
     for(int i = 0; i < E / 2; i++) {
@@ -337,20 +337,21 @@ __device__ __forceinline__ void row_body(double2 *__restrict__ work, const doubl
     }
     if constexpr(FLUX != FLUX_NONE) {
         const double2 *mrow = reinterpret_cast<const double2 *>(mob + s * bins + row * N);
-        const double inv_bins = 1.0 / (double) bins;   // exact: N^d is a power of two
         const double m0 = (FLUX == FLUX_DM && active) ? M0[s] : 0.0;
 #pragma unroll
         for(int i = 0; i < E; i++) {
             if(active && i < M) {
                 const double2 mm = mrow[ln.lane + i * ln.T];
-                const double g0 = r[i].x * inv_bins, g1 = r[i].y * inv_bins;
-                if(FLUX == FLUX_DM) r[i] = make_double2((mm.x - m0) * g0, (mm.y - m0) * g1);
-                else r[i] = make_double2(mm.x * g0, mm.y * g1);
+                if(FLUX == FLUX_DM) r[i] = make_double2((mm.x - m0) * r[i].x, (mm.y - m0) * r[i].y);
+                else r[i] = make_double2(mm.x * r[i].x, mm.y * r[i].y);
             }
         }
     }
     if constexpr(FPRIME) row_fprime<KIND, E>(r, m, ln, cur, oth, s, LS, active);
-    if constexpr(R2C) fx_row_r2c(r, work + s * hat + row * H, active, ln, cur, oth, twf, sm_w[1]);
+    // the flux's division by N^d, a power of two, is one of the scale
+    if constexpr(R2C)
+        fx_row_r2c(r, work + s * hat + row * H, active, ln, cur, oth, twf, sm_w[1],
+                   FLUX != FLUX_NONE ? 63 - __clzll(bins) : 0);
 }
 
 // Threads of a row CTA: at most 256 a line (E = 8: N = 4096; E = 4: N = 2048).
@@ -388,9 +389,8 @@ enum { COL_FWD = 0, COL_INV = 1, COL_STEP = 2, COL_INIT = 3, COL_GRAD_INV = 4, C
        COL_UPD_INV = 7 };
 
 // The pointwise stages of the variable-mobility step that ride on a column
-// pass (src/integrators/PseudospectralMobilityCPU.cpp:249-306), each in the
-// order of operations of the matching psmob.cu kernel, so either path gives
-// the same bits.  All arrays share the half-spectrum layout (species-major);
+// pass (src/integrators/PseudospectralMobilityCPU.cpp:249-306).  All arrays
+// share the half-spectrum layout (species-major);
 // fields a mode does not use stay null.
 //   COL_GRAD_INV (load):  D i k_d src                            (:258-263)
 //   COL_FWD_DIV (store):  div (= if first, += otherwise) i k_d D f (:284-293)
@@ -402,21 +402,22 @@ struct ColOps {
     const double2 *src, *fder, *div_in;
     double2 *out, *rho;
     int use_dealias, first, with_div;
-    double two_k, dt, Ssplit, k0, inv_bins;   // inv_bins = 1 / N^d, exact (a power of two)
+    int log2_bins;
+    double two_k, dt, Ssplit;
 };
 
 // One transform of a column line: r[i] = values at positions lane + i T, INV
-// the unnormalised inverse.  Headroom G = log2 L + 1.
+// the unnormalised inverse, times 2^-down.  Headroom G = log2 L + 1.
 template <bool INV, int E>
 __device__ __forceinline__ void fx_col_fft(double2 (&r)[E], const FxLine &ln, int C, fx2 *&cur, fx2 *&oth,
-                                           const int4 *__restrict__ twf, int *sm_w) {
+                                           const int4 *__restrict__ twf, int *sm_w, int down = 0) {
     const int L = 1 << ln.lg;
     int mag = 0;
 #pragma unroll
     for(int i = 0; i < E; i++)
         if(i < L) mag = max(mag, max(fx_mag(r[i].x), fx_mag(r[i].y)));
     mag = fx_line_max(mag, C, ln.T * C, sm_w);
-    const FxScale s = fx_line_scale(mag, ln.lg + 1);
+    FxScale s = fx_line_scale(mag, ln.lg + 1);
     fx_scale_by(r, s.odd, s.pre);
     fx2 v[E];
 #pragma unroll
@@ -425,6 +426,7 @@ __device__ __forceinline__ void fx_col_fft(double2 (&r)[E], const FxLine &ln, in
         if(INV) v[i] = fx_swap(v[i]);
     }
     fx_fft(v, ln, cur, oth, twf, ln.lg);
+    s.sh += down;
 #pragma unroll
     for(int i = 0; i < E; i++) r[i] = fx_out(INV ? fx_swap(v[i]) : v[i], s);
     fx_scale_by(r, s.odd, s.post);
@@ -451,6 +453,7 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
     const long long off0 = species * hat + plane * plane_stride + kx + ln.lane * elem_stride;
     const long long dT = ln.T * elem_stride;
     double2 r[E];
+    const double dtm0 = MODE == COL_UPD_INV ? ops.dt * ops.M0[species] : 0.0;
 #pragma unroll
     for(int i = 0; i < E; i++) {
         r[i] = make_double2(0.0, 0.0);
@@ -466,22 +469,21 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
             }
         }
         else if(MODE == COL_UPD_INV) {
+            // 20 FP64 instructions a mode (40 as written in the reference, with
+            // two divisions): the products and sums contracted, one reciprocal
             const double k2 = ops.q2[off];
-            const double k4 = k2 * k2;
-            const double m0 = ops.M0[species];
-            const double denom = 1.0 + ops.dt * m0 * (ops.Ssplit * k2 + 2.0 * ops.k0 * k4);
-            const double cc = ops.dt * m0 * k2;
+            const double denom = fma(dtm0, fma(ops.two_k, k2 * k2, ops.Ssplit * k2), 1.0);
+            const double inv = fast_rcp(denom), cc = dtm0 * k2;
             const double2 q = ops.rho[off], f = ops.fder[off];
             double ar = q.x, ai = q.y;
             if(ops.with_div) {
                 const double2 d = ops.div_in[off];
-                ar = q.x + ops.dt * d.x;
-                ai = q.y + ops.dt * d.y;
+                ar = fma(ops.dt, d.x, q.x);
+                ai = fma(ops.dt, d.y, q.y);
             }
-            const double nr = (ar - cc * (f.x - ops.Ssplit * q.x)) / denom;
-            const double ni = (ai - cc * (f.y - ops.Ssplit * q.y)) / denom;
-            ops.rho[off] = make_double2(nr, ni);
-            v = make_double2(nr * ops.inv_bins, ni * ops.inv_bins);
+            v.x = div_known(fma(-cc, fma(-ops.Ssplit, q.x, f.x), ar), denom, inv);
+            v.y = div_known(fma(-cc, fma(-ops.Ssplit, q.y, f.y), ai), denom, inv);
+            ops.rho[off] = v;
         }
         else {
             v = work[off];
@@ -489,7 +491,7 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
         r[i] = v;
     }
     constexpr bool INV = MODE == COL_INV || MODE == COL_GRAD_INV || MODE == COL_UPD_INV;
-    fx_col_fft<INV>(r, ln, I, cur, oth, twf, sm_w[0]);
+    fx_col_fft<INV>(r, ln, I, cur, oth, twf, sm_w[0], MODE == COL_UPD_INV ? ops.log2_bins : 0);
     if constexpr(MODE == COL_STEP) {
 #pragma unroll
         for(int i = 0; i < E; i++) {
@@ -516,13 +518,13 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
                 f.x *= D;
                 f.y *= D;
             }
-            const double2 t = mul_ik(ops.kd[off], f);
+            const double k = ops.kd[off];
             if(ops.first) {
-                ops.out[off] = make_double2(0.0 + t.x, 0.0 + t.y);
+                ops.out[off] = mul_ik(k, f);
             }
             else {
                 const double2 d = ops.out[off];
-                ops.out[off] = make_double2(d.x + t.x, d.y + t.y);
+                ops.out[off] = make_double2(fma(-k, f.y, d.x), fma(k, f.x, d.y));
             }
         }
         else {
@@ -530,7 +532,7 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
             if(MODE == COL_FWD_MU) {
                 const double t = ops.two_k * ops.q2[off];
                 const double2 q = ops.rho[off];
-                double2 v = make_double2(f.x + t * q.x, f.y + t * q.y);
+                double2 v = make_double2(fma(t, q.x, f.x), fma(t, q.y, f.y));
                 if(ops.use_dealias) {
                     const double D = ops.dealias[off];
                     v.x *= D;
@@ -1630,8 +1632,8 @@ cudaError_t spectral_psmob_update(SpectralState *s, double2 *rho_hat, const doub
     o.with_div = div_hat ? 1 : 0;
     o.dt = dt;
     o.Ssplit = Ssplit;
-    o.k0 = k0;
-    o.inv_bins = 1.0 / (double) s->g.bins;
+    o.two_k = 2.0 * k0;
+    o.log2_bins = s->g.dims * s->g.log2N;
     cudaError_t e = launch_col<COL_UPD_INV>(s, s->g.dims - 1, st, o);
     int n = 1;
     if(e == cudaSuccess && s->g.dims == 3) {

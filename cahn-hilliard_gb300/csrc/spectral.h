@@ -33,8 +33,8 @@ cudaError_t spectral_c2r(SpectralState *s, double2 *hat, double *real, cudaStrea
 long long spectral_hat_size(const SpectralState *s);   // complex values per species
 
 // ---- the variable-mobility step's transforms with its pointwise stages fused
-// (psmob.cu; dims >= 2).  Each gives the same bits as the plain transform plus
-// the matching elementwise stage of src/integrators/PseudospectralMobilityCPU.cpp.
+// (psmob.cu; dims >= 2).  Each is the plain transform plus the matching
+// elementwise stage, to rounding, of src/integrators/PseudospectralMobilityCPU.cpp.
 struct PsmobTables {
     const double *q2, *dealias;   // |k|^2 and the dealiasing mask, half-spectrum layout
     int use_dealias;

@@ -1,6 +1,7 @@
 // wertheim_fx.cuh — X, X^v, logarithms and their products for the Wertheim
-// models in 64-bit integers (device code; also compiles on the host, where the
-// CPU test runs it against extended precision).
+// models, and the gel mobility's exponential, in 64-bit integers (device code;
+// also compiles on the host, where the CPU tests run it against extended
+// precision).
 //
 // On GB300 an FP64 instruction takes the pipe time of 32 integer-ALU ones, and a
 // simple_wertheim cell took 51 of them for mu (a square root, a reciprocal, a
@@ -19,6 +20,9 @@
 //   un_X      relative 2^-58 of (-1 + sqrt(1 + t)) / (t / 2) with the sum and
 //             the square root rounded to double
 //   un_log    absolute 1.1 2^-53, and |log2 a| 2^-64 of ln 2's last place
+//   un_expneg relative 2^-58 + t 2^-61.5
+// Measured, 3D N=128 euler_mobility: the mu kernel 180 -> 59 us (FP64 pipe 64 %
+// busy from the interface's conversions and sums), a step 265 -> 116 us.
 #pragma once
 
 #include <stdint.h>
@@ -208,6 +212,31 @@ CHGB_FX int64_t un_log(Un a, Entry entry) {
     const int64_t p = (r >> 2) - (r2 >> 21) + (fxws(r3, s) >> 29);
     // e ln 2: ln 2 = 0x58B90BFC 2^-31 - 0x1718432A 2^-63
     return (int64_t) ((uint64_t) fxws(a.e, 0x58B90BFC) << 22) - (fxws(a.e, 0x1718432A) >> 10) + ((lnc + p) >> 7);
+}
+
+// e^(-c/c0) = 2^(-t), t = c K < 512 with K = 1 / (c0 ln 2): t = n + j / 256 +
+// r, 2^(-j/256) from a table (units of 2^-63, UNEXP_N entries), 2^(-r) by its
+// Taylor polynomial in w = r ln 2 < 2^-8.5 to w^5.
+constexpr int UNEXP_N = 256;
+template <typename Entry>
+CHGB_FX Un un_expneg(Un c, Un K, Entry entry) {
+    const Un t = un_mul(c, K);
+    const int n = t.e < 0 ? 0 : (int) (t.m >> (63 - t.e));
+    const uint64_t F = t.e < 0 ? fx_down(t.m, -1 - t.e) : t.m << (t.e + 1);   // the fraction, units of 2^-64
+    const uint64_t q = entry((int) (F >> 56));
+    const uint32_t rh = (uint32_t) (F >> 32) & 0xFFFFFFu, rl = (uint32_t) F;
+    // w in units of 2^-62, w^2 in 2^-80, w^3 in 2^-57; ln 2 = 0xB17217F7 2^-32 + 0xD1CF79AC 2^-64
+    const uint64_t w = (fxw(rh, 0xB17217F7u) >> 2) + (fxw(rh, 0xD1CF79ACu) >> 34) + (fxw(rl, 0xB17217F7u) >> 34);
+    const uint32_t wh = (uint32_t) (w >> 22), wl = (uint32_t) w & 0x3FFFFFu;
+    const uint64_t w2 = fxw(wh, wh) + (fxw(wh, wl) >> 21);
+    const uint32_t w2h = (uint32_t) (w2 >> 31);
+    const uint32_t w3 = (uint32_t) (fxw(w2h, wh) >> 32);
+    // 1/6 - w/24 + w^2/120 in units of 2^-34
+    const uint32_t s = 2863311531u - (wh >> 6) / 24u + (w2h >> 15) / 120u;
+    const uint64_t p = (1ull << 62) - w + (w2 >> 19) - (fxw(w3, s) >> 29);
+    const uint64_t h = un_high(q, p << 1);   // in (2^61, 2^62]
+    const int z = fx_lead((uint32_t) (h >> 32));
+    return Un{h << z, 1 - z - n};
 }
 
 }  // namespace chgb
