@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(256) row_batch_kernel(const PsBatchRep *__rest
 }
 
 enum { COL_FWD = 0, COL_INV = 1, COL_STEP = 2, COL_INIT = 3, COL_GRAD_INV = 4, COL_FWD_DIV = 5, COL_FWD_MU = 6,
-       COL_UPD_INV = 7 };
+       COL_UPD_INV = 7, COL_LOAD_INV = 8 };
 
 // The pointwise stages of the variable-mobility step that ride on a column
 // pass (src/integrators/PseudospectralMobilityCPU.cpp:249-306).  All arrays
@@ -452,6 +452,8 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
     fx2 *cur = sm + group * LS, *oth = sm + (blockDim.x / (ln.T << lgI) + group) * LS;
     const long long off0 = species * hat + plane * plane_stride + kx + ln.lane * elem_stride;
     const long long dT = ln.T * elem_stride;
+    // the same mode in a spectrum that is kept column by column
+    const long long line0 = species * hat + ((plane * H + kx) << lgL) + ln.lane;
     double2 r[E];
     const double dtm0 = MODE == COL_UPD_INV ? ops.dt * ops.M0[species] : 0.0;
 #pragma unroll
@@ -460,7 +462,10 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
         const long long off = off0 + i * dT;
         if(!active || i >= L || !CHGB_BC(101, off - species * hat, hat)) continue;
         double2 v;
-        if(MODE == COL_GRAD_INV) {
+        if(MODE == COL_LOAD_INV) {
+            v = psi_hat[line0 + i * ln.T];
+        }
+        else if(MODE == COL_GRAD_INV) {
             v = mul_ik(ops.kd[off], ops.src[off]);
             if(ops.use_dealias) {
                 const double D = ops.dealias[off];
@@ -490,12 +495,12 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
         }
         r[i] = v;
     }
-    constexpr bool INV = MODE == COL_INV || MODE == COL_GRAD_INV || MODE == COL_UPD_INV;
+    constexpr bool INV = MODE == COL_INV || MODE == COL_LOAD_INV || MODE == COL_GRAD_INV || MODE == COL_UPD_INV;
     fx_col_fft<INV>(r, ln, I, cur, oth, twf, sm_w[0], MODE == COL_UPD_INV ? ops.log2_bins : 0);
     if constexpr(MODE == COL_STEP) {
 #pragma unroll
         for(int i = 0; i < E; i++) {
-            const long long off = off0 + i * dT;
+            const long long off = line0 + i * ln.T;
             if(!active || i >= L || !CHGB_BC(101, off - species * hat, hat)) continue;
             const double2 ph = psi_hat[off], c = ab[off];
             const double2 nv = make_double2(fma(c.x, ph.x, -c.y * r[i].x), fma(c.x, ph.y, -c.y * r[i].y));
@@ -510,7 +515,7 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
         if(!active || i >= L || !CHGB_BC(101, off - species * hat, hat)) continue;
         double2 f = r[i];
         if(MODE == COL_INIT) {
-            psi_hat[off] = make_double2(f.x * scale, f.y * scale);
+            psi_hat[line0 + i * ln.T] = make_double2(f.x * scale, f.y * scale);
         }
         else if(MODE == COL_FWD_DIV) {
             if(ops.use_dealias) {
@@ -620,6 +625,21 @@ struct SpectralState {
     int row_E = 8;            // values per thread of the row transforms
 };
 
+// Where a mode stands in the spectra kept column by column (psi_hat, ab and the
+// adjoint's), by its place in the rows' order.  The transforms' own buffer
+// `work` is written by rows; the arrays that only the last axis' column pass
+// touches lie along its columns, where a warp reads 512 contiguous bytes instead
+// of 16 from each of 32 rows.
+static std::vector<long long> line_index(const SpectralState &s) {
+    const int N = s.g.N, H = s.H;
+    std::vector<long long> at(s.hat);
+    for(long long i = 0; i < s.hat; i++) {
+        const long long last = s.g.dims == 1 ? 0 : i / (s.hat / N), rest = s.g.dims == 1 ? i : i % (s.hat / N);
+        at[i] = s.g.dims == 1 ? i : rest * N + last;
+    }
+    return at;
+}
+
 // Wave-vector tables of src/integrators/PseudospectralCPU.cpp:32-86, folded
 // into the update coefficients.
 static void build_tables(const SpectralState &s, std::vector<double2> &ab) {
@@ -664,13 +684,14 @@ static void build_tables(const SpectralState &s, std::vector<double2> &ab) {
         }
     }
     ab.resize((size_t) S * s.hat);
+    const std::vector<long long> line = line_index(s);
     for(int sp = 0; sp < S; sp++) {
         for(long long i = 0; i < s.hat; i++) {
             double k2 = k2v[i], k4 = k2 * k2;
             double denom = 1.0 + dt * M * (Ssplit * k2 + 2.0 * s.p.k[sp] * k4);
             double c = dt * M * k2;
             double dm = s.p.use_dealias ? mask[i] : 1.0;
-            ab[sp * s.hat + i] = make_double2((1.0 + c * Ssplit) / denom, c * dm / denom / bins);
+            ab[sp * s.hat + line[i]] = make_double2((1.0 + c * Ssplit) / denom, c * dm / denom / bins);
         }
     }
 }
@@ -842,6 +863,7 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
                          (const void *) col_kernel<COL_STEP, 8>, (const void *) col_kernel<COL_INIT, 8>,
                          (const void *) col_kernel<COL_GRAD_INV, 8>, (const void *) col_kernel<COL_FWD_DIV, 8>,
                          (const void *) col_kernel<COL_FWD_MU, 8>, (const void *) col_kernel<COL_UPD_INV, 8>,
+                         (const void *) col_kernel<COL_LOAD_INV, 8>, (const void *) col_kernel<COL_LOAD_INV, 4>,
                          (const void *) col_kernel<COL_FWD, 4>, (const void *) col_kernel<COL_INV, 4>,
                          (const void *) col_kernel<COL_STEP, 4>, (const void *) col_kernel<COL_INIT, 4>,
                          (const void *) col_kernel<COL_GRAD_INV, 4>, (const void *) col_kernel<COL_FWD_DIV, 4>,
@@ -930,7 +952,8 @@ cudaError_t launch_row(SpectralState *s, const double *real_in, double *real_out
 
 // axis: 1 = y, 2 = z (3D only).  planes/strides follow the [z][y][kx] layout.
 template <int MODE>
-cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps &ops = ColOps()) {
+cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps &ops = ColOps(),
+                       const double2 *load = nullptr) {
     const int N = s->g.N, H = s->H;
     long long elem_stride, plane_stride;
     int planes;
@@ -953,7 +976,7 @@ cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps
     const int C = 1 << c.lgC;
     auto kernel = c.E == 8 ? col_kernel<MODE, 8> : col_kernel<MODE, 4>;
     return launch_pass(s, kernel, dim3((unsigned) ((H + C - 1) / C), (unsigned) planes, (unsigned) s->g.S), c.threads,
-                       c.smem, st, s->work, s->psi_hat, s->ab, ilog2(N), H, c.lgC, elem_stride, plane_stride, s->hat,
+                       c.smem, st, s->work, load ? const_cast<double2 *>(load) : s->psi_hat, s->ab, ilog2(N), H, c.lgC, elem_stride, plane_stride, s->hat,
                        s->twf, 1.0 / (double) s->g.bins, ops);
 }
 
@@ -1283,17 +1306,19 @@ __global__ void __launch_bounds__(512) col_adj_kernel(double2 *__restrict__ work
     const int kx = blockIdx.x * C + ln.c;
     const bool active = kx < H;
     fx2 *cur = sm2, *oth = sm2 + (fx_line_size(L) << lgC);
+    // work by rows, lam, psi and the tables by columns
     const long long off0 = kx + (long long) ln.lane * H, dT = (long long) ln.T * H;
+    const long long line0 = ((long long) kx << lgL) + ln.lane;
     double2 r[E];
 #pragma unroll
     for(int i = 0; i < E; i++)
-        r[i] = (active && i < L) ? ((MODE & ADJ_B) ? work : lam)[off0 + i * dT] : make_double2(0.0, 0.0);
+        r[i] = (!active || i >= L) ? make_double2(0.0, 0.0) : (MODE & ADJ_B) ? work[off0 + i * dT] : lam[line0 + i * ln.T];
     if(MODE & ADJ_B) {
         fx_col_fft<false>(r, ln, C, cur, oth, twf, sm_w[0]);
 #pragma unroll
         for(int i = 0; i < E; i++) {
             if(active && i < L) {
-                const long long off = off0 + i * dT;
+                const long long off = line0 + i * ln.T;
                 const double2 l = lam[off];
                 const double al = ab[off].x;
                 r[i] = make_double2(fma(al, l.x, -r[i].x), fma(al, l.y, -r[i].y));
@@ -1307,7 +1332,7 @@ __global__ void __launch_bounds__(512) col_adj_kernel(double2 *__restrict__ work
 #pragma unroll
         for(int i = 0; i < E; i++) {
             if(active && i < L) {
-                const long long off = off0 + i * dT;
+                const long long off = line0 + i * ln.T;
                 const double2 l = r[i], pn = psi_next[off], pc = psi_cur[off];
                 const double dn = fma(l.x, pn.x, l.y * pn.y);
                 const double dc = fma(l.x, pc.x, l.y * pc.y);
@@ -1354,19 +1379,19 @@ SpectralAdj *spectral_adj_create(SpectralState *s, std::string &err) {
     const int N = s->g.N;
     const double dx = s->p.dx, dt = s->p.dt, M = s->p.M, Ssplit = s->p.splitting_S, k = s->p.k[0];
     std::vector<double> tk(s->hat), tm1(s->hat), tm2(s->hat);
-    long long idx = 0;
     // the same wave vectors as build_tables (src/integrators/PseudospectralCPU.cpp:44-57)
     for(int kx_idx = 0; kx_idx < N; kx_idx++) {
         int kx = (kx_idx < N / 2) ? kx_idx : N - kx_idx;
-        for(int ky = 0; ky < N / 2 + 1; ky++, idx++) {
+        for(int ky = 0; ky < N / 2 + 1; ky++) {
             double kk = 2.0 * M_PI * std::sqrt((double) (kx * kx + ky * ky)) / (N * dx);
             double k2 = kk * kk, k4 = k2 * k2;
             double denom = 1.0 + dt * M * (Ssplit * k2 + 2.0 * k * k4);
             double c = dt * M * k2;
             double alpha = (1.0 + c * Ssplit) / denom;
-            tk[idx] = -2.0 * dt * M * k4 / denom;
-            tm1[idx] = 1.0 / (M * denom);
-            tm2[idx] = 2.0 * k * k4 * dt / (denom * denom) + alpha / (M * denom);
+            const long long at = (long long) ky * N + kx_idx;
+            tk[at] = -2.0 * dt * M * k4 / denom;
+            tm1[at] = 1.0 / (M * denom);
+            tm2[at] = 2.0 * k * k4 * dt / (denom * denom) + alpha / (M * denom);
         }
     }
     a->n_row_cta = (int) (((long long) s->g.bins / N) / s->row_rpc);
@@ -1471,8 +1496,7 @@ cudaError_t spectral_load_hat(SpectralState *s, const double2 *hat, cudaStream_t
     size_t bytes = sizeof(double2) * (size_t) s->hat * s->g.S;
     cudaError_t e = cudaSuccess;
     if(hat != s->psi_hat) e = cudaMemcpyAsync(s->psi_hat, hat, bytes, cudaMemcpyDeviceToDevice, st);
-    if(e == cudaSuccess) e = cudaMemcpyAsync(s->work, hat, bytes, cudaMemcpyDeviceToDevice, st);
-    if(e == cudaSuccess) e = launch_col<COL_INV>(s, 1, st);
+    if(e == cudaSuccess) e = launch_col<COL_LOAD_INV>(s, 1, st, ColOps(), s->psi_hat);
     s->hat_valid = true;
     s->real_valid = false;
     return e;
@@ -1489,9 +1513,7 @@ cudaError_t spectral_step_record(SpectralState *s, double *real_out, cudaStream_
 
 // real_out = C2R(hat_scaled) (unnormalised: a scaled state gives the field).
 cudaError_t spectral_inverse(SpectralState *s, const double2 *hat_scaled, double *real_out, cudaStream_t st) {
-    size_t bytes = sizeof(double2) * (size_t) s->hat * s->g.S;
-    cudaError_t e = cudaMemcpyAsync(s->work, hat_scaled, bytes, cudaMemcpyDeviceToDevice, st);
-    if(e == cudaSuccess) e = launch_col<COL_INV>(s, 1, st);
+    cudaError_t e = launch_col<COL_LOAD_INV>(s, 1, st, ColOps(), hat_scaled);
     if(e == cudaSuccess) e = launch_row<ROW_IN_HAT, false, true, false>(s, nullptr, real_out, st);
     s->hat_valid = false;
     return e;

@@ -23,11 +23,13 @@ int spectral_step(SpectralState *s, int64_t nsteps, cudaStream_t st, int64_t *la
 // Real-space density of the current state into d_rho.
 int spectral_real(SpectralState *s, double *d_rho, cudaStream_t st, int64_t *launches, std::string &err);
 
-// Scaled half spectrum psi_t = rho_hat / N^dims of one species (the master state).
+// Scaled half spectrum psi_t = rho_hat / N^dims of one species (the master
+// state), column by column: mode (kx, ky) of a 2D box at kx N + ky, (kx, ky, kz)
+// at (ky H + kx) N + kz, H = N/2 + 1.  The adjoint's spectra lie the same way.
 const double2 *spectral_psi_hat(const SpectralState *s, int species);
 double2 *spectral_psi_hat_mut(SpectralState *s);
 // FFTW-style unnormalised transforms of S-species fields on caller buffers
-// (the half spectrum in the state's layout); c2r overwrites `hat`.
+// (the half spectrum row by row, kx fastest); c2r overwrites `hat`.
 cudaError_t spectral_r2c(SpectralState *s, const double *real, double2 *hat, cudaStream_t st, int *launches);
 cudaError_t spectral_c2r(SpectralState *s, double2 *hat, double *real, cudaStream_t st, int *launches);
 long long spectral_hat_size(const SpectralState *s);   // complex values per species

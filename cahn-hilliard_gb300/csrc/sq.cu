@@ -86,7 +86,7 @@ SqPlan *sq_plan_create(int N, std::string &err) {
     for(int yi = 0; yi < N; yi++) {
         int ky = (yi < N / 2) ? yi : yi - N;
         for(int kx = 0; kx < H; kx++) {
-            long long m = (long long) yi * H + kx;
+            long long m = (long long) kx * N + yi;   // psi_t lies column by column
             int b = sq_shell_of(kx, ky);
             bool twice = (kx != 0 && kx != N / 2);
             shell[m] = b;
