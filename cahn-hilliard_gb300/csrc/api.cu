@@ -553,7 +553,8 @@ static cudaError_t one_step_psm(chgb_handle *h) {
     if(h->p.mobility_type == CHGB_MOBILITY_FREE_ENERGY)
         e = launch_set_mobility(h->m, rho, h->p.M, h->d_mob, (long long) h->n, h->stream);
     else if(h->p.mobility_type != CHGB_MOBILITY_CONSTANT)
-        e = launch_mobility_update(h->md, rho, h->d_gel, h->d_mob, h->g.S, (long long) h->g.bins, h->stream);
+        e = launch_mobility_update(h->md, rho, h->d_gel, h->d_mob, h->g.S, (long long) h->g.bins, h->stream,
+                                   psmob_m0_sink(h->psm));
     int64_t n = 0;
     if(e == cudaSuccess) e = psmob_step(h->psm, h->d_mob, rho, h->stream, &n);
     // the GMRES path launches as many kernels as its iterations need; the

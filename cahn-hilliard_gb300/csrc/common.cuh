@@ -72,6 +72,47 @@ struct MobilityDev {
     const uint64_t *exptab;         // table of un_expneg (null: the library's exp)
 };
 
+// Maximum of a mobility field per species, max(0, max M): the values' bits in
+// order as unsigned integers (M > 0; negative ones and NaN are passed over, as
+// m < v ? v : m from m = 0 does).  Each block adds its maximum to acc; the last
+// one, counted per species, hands it to M0 and clears both for the next launch.
+struct M0Sink {
+    unsigned long long *acc;
+    unsigned *count;
+    double *M0;                     // null: no maximum is wanted
+};
+
+__device__ __forceinline__ void m0_take(unsigned long long &m, double v) {
+    const long long b = __double_as_longlong(v);
+    if(b > (long long) m && b <= 0x7FF0000000000000ll) m = (unsigned long long) b;
+}
+
+// All threads of a block; species s0 .. s1 - 1 share the value.
+__device__ __forceinline__ void m0_commit(unsigned long long m, const M0Sink &sink, int s0, int s1) {
+    __shared__ unsigned long long red[32];
+#pragma unroll
+    for(int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xFFFFFFFFu, m, o);
+        m = m < v ? v : m;
+    }
+    if((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if(threadIdx.x == 0) {
+        for(int w = 1; w < (int) (blockDim.x + 31) / 32; w++) m = m < red[w] ? red[w] : m;
+        for(int s = s0; s < s1; s++) {
+            atomicMax(&sink.acc[s], m);
+            __threadfence();   // the maximum is in before the count says so
+            if(atomicAdd(&sink.count[s], 1u) == gridDim.x - 1) {
+                __threadfence();
+                sink.M0[s] = __longlong_as_double((long long) __ldcg(&sink.acc[s]));
+                sink.acc[s] = 0;
+                sink.count[s] = 0;
+            }
+        }
+    }
+    __syncthreads();   // red is free again
+}
+
 // i k z: the wave-vector factor of a spectral derivative
 // (src/integrators/PseudospectralMobilityCPU.cpp:258-263)
 __device__ __forceinline__ double2 mul_ik(double k, double2 z) { return make_double2(-k * z.y, k * z.x); }

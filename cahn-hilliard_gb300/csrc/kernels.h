@@ -89,7 +89,7 @@ cudaError_t launch_fill_noise(double *p, double mean, double amp, long long n, c
 // `bins` cells): mob = M rho / (rho + rho_min) per species, or the gel order
 // parameter advanced one explicit step and mob = exp(-c / c_0) for every species.
 cudaError_t launch_mobility_update(const MobilityDev &md, const double *rho, double *gel, double *mob, int S,
-                                   long long bins, cudaStream_t st);
+                                   long long bins, cudaStream_t st, const M0Sink &sink = M0Sink{});
 // euler_mobility kernels' mobility kind (1 constant, 2 free energy, 3 field) of a CHGB_MOBILITY_* type.
 int mobility_kind(int mobility_type);
 // Partial sums of mass and free energy into `partials` (2 * nblocks doubles),

@@ -33,57 +33,17 @@ namespace chgb {
 
 namespace {
 
-constexpr int M0_BLOCKS = 4 * 152;   // most partial maxima per species (4 blocks per SM)
+constexpr int M0_BLOCKS = 4 * 152;   // most blocks per species (4 blocks per SM)
 
-// M0 = max(0, max M) per species in one launch (PseudospectralMobilityCPU.cpp:
-// 434-442): each block reduces a grid-stride share of the species' mobility
-// into part[s * nblk + b]; the last block to finish, counted per species,
-// reduces the partials and resets its counter for the next launch.  A maximum
-// is exact, so the grouping does not change the result; every comparison is
-// the reference's m < v ? v : m from m = 0, which passes over NaN.
-__device__ __forceinline__ double m0_block_max(double m, double *red) {
-    red[threadIdx.x] = m;
-    __syncthreads();
-    for(int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if(threadIdx.x < o) red[threadIdx.x] = (red[threadIdx.x] < red[threadIdx.x + o]) ? red[threadIdx.x + o]
-                                                                                      : red[threadIdx.x];
-        __syncthreads();
-    }
-    return red[0];
-}
-
-__global__ void __launch_bounds__(256) m0_kernel(const double *__restrict__ mob, long long bins,
-                                                 double *__restrict__ part, unsigned *__restrict__ count,
-                                                 double *__restrict__ M0) {
+// M0 = max(0, max M) per species (PseudospectralMobilityCPU.cpp:434-442) where
+// the mobility's own update does not reduce it (m0_commit, common.cuh).
+__global__ void __launch_bounds__(256) m0_kernel(const double *__restrict__ mob, long long bins, M0Sink sink) {
     const int s = blockIdx.y;
-    __shared__ double red[256];
-    __shared__ bool last;
-    double m = 0.0;
+    unsigned long long m = 0;
     for(long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x; i < bins;
-        i += (long long) gridDim.x * blockDim.x) {
-        const double v = mob[s * bins + i];
-        m = (m < v) ? v : m;
-    }
-    m = m0_block_max(m, red);
-    if(threadIdx.x == 0) {
-        part[s * gridDim.x + blockIdx.x] = m;
-        __threadfence();   // the partial is visible before the count says so
-        last = atomicAdd(&count[s], 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if(!last) return;
-    __threadfence();
-    m = 0.0;
-    for(int b = threadIdx.x; b < (int) gridDim.x; b += blockDim.x) {
-        const double v = __ldcg(&part[s * gridDim.x + b]);
-        m = (m < v) ? v : m;
-    }
-    __syncthreads();   // red is reused
-    m = m0_block_max(m, red);
-    if(threadIdx.x == 0) {
-        M0[s] = m;
-        count[s] = 0;
-    }
+        i += (long long) gridDim.x * blockDim.x)
+        m0_take(m, mob[s * bins + i]);
+    m0_commit(m, sink, s, s + 1);
 }
 
 // mu_hat = f'_hat + 2 k q^2 rho_hat (:249-254)
@@ -187,7 +147,8 @@ void psmob_destroy(PsMob *s) {
     if(!s) return;
     if(s->eng) spectral_destroy(s->eng);
     for(double2 *p : {s->rho_hat, s->fder_hat, s->mu_hat, s->tmp_hat, s->div_hat}) cudaFree(p);
-    for(double *p : {s->q2, s->dealias, s->kc[0], s->kc[1], s->kc[2], s->fder, s->tmp, s->M0, s->part}) cudaFree(p);
+    for(double *p : {s->q2, s->dealias, s->kc[0], s->kc[1], s->kc[2], s->fder, s->tmp, s->M0}) cudaFree(p);
+    cudaFree(s->m0_acc);
     cudaFree(s->m0_count);
     psmob_gmres_release(s);
     delete s;
@@ -213,6 +174,7 @@ int psmob_create(const chgb_params &p, const Geom &g, const ModelDev &m, PsMob *
     s->hat = spectral_hat_size(s->eng);
     s->hall = s->hat * s->S;
     s->constant = p.mobility_type == CHGB_MOBILITY_CONSTANT;
+    s->m0_by_update = p.mobility_type == CHGB_MOBILITY_REGULARISED || p.mobility_type == CHGB_MOBILITY_GEL;
     // wave vectors and dealiaser, PseudospectralMobilityCPU.cpp:56-118
     const int N = g.N, dims = g.dims;
     const double dx = p.dx;
@@ -223,10 +185,11 @@ int psmob_create(const chgb_params &p, const Geom &g, const ModelDev &m, PsMob *
     for(int sp = 0; sp < s->S; sp++) {
         if(dims == 1) {
             for(long long i = 0; i < s->hat; i++, k_idx++) {
+                const long long at = k_idx;
                 double kx = 2.0 * M_PI * i / (N * dx);
-                dl[k_idx] = (std::abs(kx) <= k_cut) ? 1.0 : 0.0;
-                kc[0][k_idx] = kx;
-                q2[k_idx] = kx * kx;
+                dl[at] = (std::abs(kx) <= k_cut) ? 1.0 : 0.0;
+                kc[0][at] = kx;
+                q2[at] = kx * kx;
             }
         }
         else if(dims == 2) {
@@ -234,12 +197,13 @@ int psmob_create(const chgb_params &p, const Geom &g, const ModelDev &m, PsMob *
                 int ai = (a < N / 2) ? a : (a - N);
                 double kx = 2.0 * M_PI * ai / (N * dx);
                 for(int b = 0; b < N / 2 + 1; b++, k_idx++) {
+                    const long long at = sp * s->hat + spectral_line_index(g, k_idx - sp * s->hat);
                     double ky = 2.0 * M_PI * b / (N * dx);
                     double k2 = kx * kx + ky * ky;
-                    dl[k_idx] = (std::sqrt(k2) <= k_cut) ? 1.0 : 0.0;
-                    kc[0][k_idx] = kx;
-                    kc[1][k_idx] = ky;
-                    q2[k_idx] = k2;
+                    dl[at] = (std::sqrt(k2) <= k_cut) ? 1.0 : 0.0;
+                    kc[0][at] = kx;
+                    kc[1][at] = ky;
+                    q2[at] = k2;
                 }
             }
         }
@@ -251,18 +215,23 @@ int psmob_create(const chgb_params &p, const Geom &g, const ModelDev &m, PsMob *
                     int bi = (b < N / 2) ? b : (b - N);
                     double ky = 2.0 * M_PI * bi / (N * dx);
                     for(int c = 0; c < N / 2 + 1; c++, k_idx++) {
+                        const long long at = sp * s->hat + spectral_line_index(g, k_idx - sp * s->hat);
                         double kz = 2.0 * M_PI * c / (N * dx);
                         double k2 = kx * kx + ky * ky + kz * kz;
-                        dl[k_idx] = (std::sqrt(k2) <= k_cut) ? 1.0 : 0.0;
-                        kc[0][k_idx] = kx;
-                        kc[1][k_idx] = ky;
-                        kc[2][k_idx] = kz;
-                        q2[k_idx] = k2;
+                        dl[at] = (std::sqrt(k2) <= k_cut) ? 1.0 : 0.0;
+                        kc[0][at] = kx;
+                        kc[1][at] = ky;
+                        kc[2][at] = kz;
+                        q2[at] = k2;
                     }
                 }
             }
         }
     }
+    // i k_d is only ever taken of modes that dealiasing keeps
+    if(p.use_dealias)
+        for(int d = 0; d < dims; d++)
+            for(long long i = 0; i < s->hall; i++) kc[d][i] *= dl[i];
     const size_t hb = sizeof(double2) * (size_t) s->hall, tb = sizeof(double) * (size_t) s->hall;
     const size_t rb = sizeof(double) * (size_t) s->bins * s->S;
     bool ok = cudaMalloc(&s->rho_hat, hb) == cudaSuccess && cudaMalloc(&s->fder_hat, hb) == cudaSuccess &&
@@ -270,7 +239,8 @@ int psmob_create(const chgb_params &p, const Geom &g, const ModelDev &m, PsMob *
               cudaMalloc(&s->div_hat, hb) == cudaSuccess && cudaMalloc(&s->q2, tb) == cudaSuccess &&
               cudaMalloc(&s->dealias, tb) == cudaSuccess && cudaMalloc(&s->fder, rb) == cudaSuccess &&
               cudaMalloc(&s->tmp, rb) == cudaSuccess && cudaMalloc(&s->M0, sizeof(double) * s->S) == cudaSuccess &&
-              cudaMalloc(&s->part, sizeof(double) * s->S * M0_BLOCKS) == cudaSuccess &&
+              cudaMalloc(&s->m0_acc, sizeof(unsigned long long) * s->S) == cudaSuccess &&
+              cudaMemset(s->m0_acc, 0, sizeof(unsigned long long) * s->S) == cudaSuccess &&
               cudaMalloc(&s->m0_count, sizeof(unsigned) * s->S) == cudaSuccess &&
               cudaMemset(s->m0_count, 0, sizeof(unsigned) * s->S) == cudaSuccess;
     for(int d = 0; d < dims && ok; d++) ok = cudaMalloc(&s->kc[d], tb) == cudaSuccess;
@@ -287,9 +257,12 @@ int psmob_create(const chgb_params &p, const Geom &g, const ModelDev &m, PsMob *
     return CHGB_OK;
 }
 
+M0Sink psmob_m0_sink(const PsMob *s) { return M0Sink{s->m0_acc, s->m0_count, s->M0}; }
+
 int psmob_m0(PsMob *s, const double *mob, cudaStream_t st) {
+    if(s->m0_by_update) return 0;
     const int nblk = (int) std::min<long long>(M0_BLOCKS, std::max<long long>(1, (s->bins + 2047) / 2048));
-    m0_kernel<<<dim3(nblk, s->S), 256, 0, st>>>(mob, s->bins, s->part, s->m0_count, s->M0);
+    m0_kernel<<<dim3(nblk, s->S), 256, 0, st>>>(mob, s->bins, psmob_m0_sink(s));
     return 1;
 }
 
@@ -313,21 +286,18 @@ cudaError_t psmob_set_rho(PsMob *s, const double *rho, cudaStream_t st, int64_t 
     return e;
 }
 
-PsmobTables psmob_tables(const PsMob *s) { return PsmobTables{s->q2, s->dealias, s->p.use_dealias ? 1 : 0}; }
-
 // 2D and 3D: the pointwise stages ride on the transforms' column and row passes
 // (spectral_psmob_*).
 static cudaError_t psmob_step_fused(PsMob *s, const double *mob, double *rho, cudaStream_t st, int64_t *launches) {
-    const PsmobTables t = psmob_tables(s);
     int nl = 0;
     nl += psmob_m0(s, mob, st);
-    cudaError_t e = spectral_psmob_fprime(s->eng, rho, s->fder_hat, s->constant ? nullptr : s->mu_hat, s->rho_hat, t,
+    cudaError_t e = spectral_psmob_fprime(s->eng, rho, s->fder_hat, s->constant ? nullptr : s->mu_hat, s->rho_hat, s->q2,
                                           2.0 * s->p.k[0], st, &nl);
     for(int d = 0; d < s->g.dims && e == cudaSuccess && !s->constant; d++)
-        e = spectral_psmob_flux(s->eng, s->mu_hat, s->kc[d], t, mob, s->M0, s->div_hat, d == 0, s->tmp_hat, st, &nl);
+        e = spectral_psmob_flux(s->eng, s->mu_hat, s->kc[d], mob, s->M0, s->div_hat, d == 0, st, &nl);
     if(e == cudaSuccess)
         e = spectral_psmob_update(s->eng, s->rho_hat, s->fder_hat, s->constant ? nullptr : s->div_hat, s->q2, s->M0,
-                                  s->p.dt, s->p.splitting_S, s->p.k[0], s->tmp_hat, rho, st, &nl);
+                                  s->p.dt, s->p.splitting_S, s->p.k[0], rho, st, &nl);
     *launches += nl;
     return e;
 }
@@ -385,12 +355,12 @@ cudaError_t psmob_step(PsMob *s, const double *mob, double *rho, cudaStream_t st
 
 int psmob_launches_per_step(const PsMob *s) {
     const int t = s->g.dims;   // kernels per transform: row pass + one column pass per further axis
-    if(t >= 2) {               // M0, f' + r2c (+ mu), update + c2r, per axis a c2r and r2c sharing the row pass
-        int n = 1 + t + t;
+    if(t >= 2) {               // M0 (or with the mobility's update), f' + r2c (+ mu), update + c2r, per axis a c2r and r2c sharing the row pass
+        int n = (s->m0_by_update ? 0 : 1) + t + t;
         if(!s->constant) n += s->g.dims * (2 * t - 1);
         return n;
     }
-    int n = 1 + 1 + t + 1 + t;  // M0, f', r2c, update, c2r
+    int n = (s->m0_by_update ? 0 : 1) + 1 + t + 1 + t;  // M0, f', r2c, update, c2r
     if(!s->constant) n += 1 + s->g.dims * (1 + t + 1 + t + 1);
     return n;
 }

@@ -388,23 +388,31 @@ __global__ void __launch_bounds__(256) row_batch_kernel(const PsBatchRep *__rest
 enum { COL_FWD = 0, COL_INV = 1, COL_STEP = 2, COL_INIT = 3, COL_GRAD_INV = 4, COL_FWD_DIV = 5, COL_FWD_MU = 6,
        COL_UPD_INV = 7, COL_LOAD_INV = 8 };
 
-// The pointwise stages of the variable-mobility step that ride on a column
-// pass (src/integrators/PseudospectralMobilityCPU.cpp:249-306).  All arrays
-// share the half-spectrum layout (species-major);
-// fields a mode does not use stay null.
-//   COL_GRAD_INV (load):  D i k_d src                            (:258-263)
-//   COL_FWD_DIV (store):  div (= if first, += otherwise) i k_d D f (:284-293)
-//   COL_FWD_MU (store):   work = f, mu = D (f + two_k q2 rho_hat)  (:249-254)
-//   COL_UPD_INV (load):   the semi-implicit update of rho_hat, inverse
-//                         transform of rho_hat / N^d               (:296-306)
+// The pointwise stages of the variable-mobility step that ride on the last
+// axis' column pass (src/integrators/PseudospectralMobilityCPU.cpp:249-306).
+// Their spectra and tables lie column by column (species-major), `work` by rows;
+// kd holds 0 for the modes that dealiasing drops; fields a mode does not use
+// stay null.
+//   COL_GRAD_INV (load):  i k_d src                                    (:258-263)
+//   COL_FWD_DIV (store):  div (= if first, += otherwise) i k_d f       (:284-293)
+//   COL_FWD_MU (store):   psi_hat = f'_hat; out = f'_hat + two_k q2 rho (:249-254)
+//   COL_UPD_INV (load):   rho <- the semi-implicit update with f'_hat = psi_hat; rho N^-d (:296-306)
 struct ColOps {
-    const double *kd, *dealias, *q2, *M0;
-    const double2 *src, *fder, *div_in;
+    const double *kd, *q2, *M0;
+    const double2 *src, *div_in;
     double2 *out, *rho;
-    int use_dealias, first, with_div;
+    int first, with_div;
     int log2_bins;
     double two_k, dt, Ssplit;
 };
+
+// dt / x: the reciprocal in integers (relative 2^-58, then one rounding) where
+// both are in its range.
+__device__ __noinline__ static double div_fallback(double a, double x) { return a / x; }
+__device__ __forceinline__ double dt_over(double dt, double x) {
+    if(!un_takes(x) || !un_takes(dt)) return div_fallback(dt, x);
+    return __longlong_as_double((long long) un_to_bits(un_mul(un_of(dt), un_rcp(un_of(x)))));
+}
 
 // One transform of a column line: r[i] = values at positions lane + i T, INV
 // the unnormalised inverse, times 2^-down.  Headroom G = log2 L + 1.
@@ -455,7 +463,7 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
     // the same mode in a spectrum that is kept column by column
     const long long line0 = species * hat + ((plane * H + kx) << lgL) + ln.lane;
     double2 r[E];
-    const double dtm0 = MODE == COL_UPD_INV ? ops.dt * ops.M0[species] : 0.0;
+    const double m0 = MODE == COL_UPD_INV ? ops.M0[species] : 0.0;
 #pragma unroll
     for(int i = 0; i < E; i++) {
         r[i] = make_double2(0.0, 0.0);
@@ -466,29 +474,22 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
             v = psi_hat[line0 + i * ln.T];
         }
         else if(MODE == COL_GRAD_INV) {
-            v = mul_ik(ops.kd[off], ops.src[off]);
-            if(ops.use_dealias) {
-                const double D = ops.dealias[off];
-                v.x *= D;
-                v.y *= D;
-            }
+            v = mul_ik(ops.kd[line0 + i * ln.T], ops.src[line0 + i * ln.T]);
         }
         else if(MODE == COL_UPD_INV) {
-            // 20 FP64 instructions a mode (40 as written in the reference, with
-            // two divisions): the products and sums contracted, one reciprocal
-            const double k2 = ops.q2[off];
-            const double denom = fma(dtm0, fma(ops.two_k, k2 * k2, ops.Ssplit * k2), 1.0);
-            const double inv = fast_rcp(denom), cc = dtm0 * k2;
-            const double2 q = ops.rho[off], f = ops.fder[off];
-            double ar = q.x, ai = q.y;
-            if(ops.with_div) {
-                const double2 d = ops.div_in[off];
-                ar = fma(ops.dt, d.x, q.x);
-                ai = fma(ops.dt, d.y, q.y);
-            }
-            v.x = div_known(fma(-cc, fma(-ops.Ssplit, q.x, f.x), ar), denom, inv);
-            v.y = div_known(fma(-cc, fma(-ops.Ssplit, q.y, f.y), ai), denom, inv);
-            ops.rho[off] = v;
+            // the reference's (rho + dt div - c (f' - S rho)) / (1 + c (S + 2 k q^2)), c =
+            // dt M0 q^2, with its numerator less rho times its denominator: rho + dt / (1
+            // + ...) (div - M0 q^2 (f' + 2 k q^2 rho)), whose rounding is rho's alone.  12
+            // FP64 instructions a mode and a reciprocal in integers, against 22 with a
+            // corrected division of each part
+            const long long lo = line0 + i * ln.T;
+            const double k2 = ops.q2[lo], t = ops.two_k * k2, mk = m0 * k2;
+            const double g = dt_over(ops.dt, fma(ops.dt * mk, ops.Ssplit + t, 1.0));
+            const double2 q = ops.rho[lo], f = psi_hat[lo];
+            const double2 d = ops.with_div ? ops.div_in[lo] : make_double2(0.0, 0.0);
+            v.x = fma(g, fma(-mk, fma(t, q.x, f.x), d.x), q.x);
+            v.y = fma(g, fma(-mk, fma(t, q.y, f.y), d.y), q.y);
+            ops.rho[lo] = v;
         }
         else {
             v = work[off];
@@ -517,34 +518,26 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
         if(MODE == COL_INIT) {
             psi_hat[line0 + i * ln.T] = make_double2(f.x * scale, f.y * scale);
         }
+        else if(MODE == COL_FWD_MU) {
+            const long long lo = line0 + i * ln.T;
+            psi_hat[lo] = f;
+            const double t = ops.two_k * ops.q2[lo];
+            const double2 q = ops.rho[lo];
+            ops.out[lo] = make_double2(fma(t, q.x, f.x), fma(t, q.y, f.y));
+        }
         else if(MODE == COL_FWD_DIV) {
-            if(ops.use_dealias) {
-                const double D = ops.dealias[off];
-                f.x *= D;
-                f.y *= D;
-            }
-            const double k = ops.kd[off];
+            const long long lo = line0 + i * ln.T;
+            const double k = ops.kd[lo];
             if(ops.first) {
-                ops.out[off] = mul_ik(k, f);
+                ops.out[lo] = mul_ik(k, f);
             }
             else {
-                const double2 d = ops.out[off];
-                ops.out[off] = make_double2(fma(-k, f.y, d.x), fma(k, f.x, d.y));
+                const double2 d = ops.out[lo];
+                ops.out[lo] = make_double2(fma(-k, f.y, d.x), fma(k, f.x, d.y));
             }
         }
         else {
             work[off] = f;
-            if(MODE == COL_FWD_MU) {
-                const double t = ops.two_k * ops.q2[off];
-                const double2 q = ops.rho[off];
-                double2 v = make_double2(fma(t, q.x, f.x), fma(t, q.y, f.y));
-                if(ops.use_dealias) {
-                    const double D = ops.dealias[off];
-                    v.x *= D;
-                    v.y *= D;
-                }
-                ops.out[off] = v;
-            }
         }
     }
 }
@@ -630,14 +623,10 @@ struct SpectralState {
 // `work` is written by rows; the arrays that only the last axis' column pass
 // touches lie along its columns, where a warp reads 512 contiguous bytes instead
 // of 16 from each of 32 rows.
-static std::vector<long long> line_index(const SpectralState &s) {
-    const int N = s.g.N, H = s.H;
-    std::vector<long long> at(s.hat);
-    for(long long i = 0; i < s.hat; i++) {
-        const long long last = s.g.dims == 1 ? 0 : i / (s.hat / N), rest = s.g.dims == 1 ? i : i % (s.hat / N);
-        at[i] = s.g.dims == 1 ? i : rest * N + last;
-    }
-    return at;
+long long spectral_line_index(const Geom &g, long long mode) {
+    if(g.dims == 1) return mode;
+    const long long lines = (long long) (g.N / 2 + 1) * (g.dims == 3 ? g.N : 1);
+    return mode % lines * g.N + mode / lines;
 }
 
 // Wave-vector tables of src/integrators/PseudospectralCPU.cpp:32-86, folded
@@ -684,14 +673,13 @@ static void build_tables(const SpectralState &s, std::vector<double2> &ab) {
         }
     }
     ab.resize((size_t) S * s.hat);
-    const std::vector<long long> line = line_index(s);
     for(int sp = 0; sp < S; sp++) {
         for(long long i = 0; i < s.hat; i++) {
             double k2 = k2v[i], k4 = k2 * k2;
             double denom = 1.0 + dt * M * (Ssplit * k2 + 2.0 * s.p.k[sp] * k4);
             double c = dt * M * k2;
             double dm = s.p.use_dealias ? mask[i] : 1.0;
-            ab[sp * s.hat + line[i]] = make_double2((1.0 + c * Ssplit) / denom, c * dm / denom / bins);
+            ab[sp * s.hat + spectral_line_index(s.g, i)] = make_double2((1.0 + c * Ssplit) / denom, c * dm / denom / bins);
         }
     }
 }
@@ -951,9 +939,11 @@ cudaError_t launch_row(SpectralState *s, const double *real_in, double *real_out
 }
 
 // axis: 1 = y, 2 = z (3D only).  planes/strides follow the [z][y][kx] layout.
+// `spec`: the spectrum, column by column, that the pass loads or stores in place
+// of the state's psi (COL_INIT then keeps the transform unscaled).
 template <int MODE>
 cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps &ops = ColOps(),
-                       const double2 *load = nullptr) {
+                       double2 *spec = nullptr) {
     const int N = s->g.N, H = s->H;
     long long elem_stride, plane_stride;
     int planes;
@@ -976,8 +966,8 @@ cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps
     const int C = 1 << c.lgC;
     auto kernel = c.E == 8 ? col_kernel<MODE, 8> : col_kernel<MODE, 4>;
     return launch_pass(s, kernel, dim3((unsigned) ((H + C - 1) / C), (unsigned) planes, (unsigned) s->g.S), c.threads,
-                       c.smem, st, s->work, load ? const_cast<double2 *>(load) : s->psi_hat, s->ab, ilog2(N), H, c.lgC, elem_stride, plane_stride, s->hat,
-                       s->twf, 1.0 / (double) s->g.bins, ops);
+                       c.smem, st, s->work, spec ? spec : s->psi_hat, s->ab, ilog2(N), H, c.lgC, elem_stride, plane_stride, s->hat,
+                       s->twf, spec ? 1.0 : 1.0 / (double) s->g.bins, ops);
 }
 
 }  // namespace
@@ -1513,7 +1503,7 @@ cudaError_t spectral_step_record(SpectralState *s, double *real_out, cudaStream_
 
 // real_out = C2R(hat_scaled) (unnormalised: a scaled state gives the field).
 cudaError_t spectral_inverse(SpectralState *s, const double2 *hat_scaled, double *real_out, cudaStream_t st) {
-    cudaError_t e = launch_col<COL_LOAD_INV>(s, 1, st, ColOps(), hat_scaled);
+    cudaError_t e = launch_col<COL_LOAD_INV>(s, 1, st, ColOps(), const_cast<double2 *>(hat_scaled));   // read only in this mode
     if(e == cudaSuccess) e = launch_row<ROW_IN_HAT, false, true, false>(s, nullptr, real_out, st);
     s->hat_valid = false;
     return e;
@@ -1521,47 +1511,30 @@ cudaError_t spectral_inverse(SpectralState *s, const double2 *hat_scaled, double
 
 double2 *spectral_psi_hat_mut(SpectralState *s) { return s->psi_hat; }
 
-// Plain transforms on caller buffers, FFTW's unnormalised r2c / c2r in the
-// half-spectrum layout, S species: the row and column passes of a step without
-// the model or the update.  `hat` stands in for the state's work array for the
-// duration of the call (the kernels take it as an argument at launch).
+// Plain transforms on caller buffers, FFTW's unnormalised r2c / c2r, S species:
+// the row and column passes of a step without the model or the update.  The
+// passes run in the state's work array; the last axis' stores and loads the
+// spectrum column by column.  1D: `hat` is the work array.
 cudaError_t spectral_r2c(SpectralState *s, const double *real, double2 *hat, cudaStream_t st, int *launches) {
     double2 *saved = s->work;
-    s->work = hat;
+    if(s->g.dims == 1) s->work = hat;
     cudaError_t e = launch_row<ROW_IN_REAL, false, false, true>(s, real, nullptr, st);
-    int n = 1;
-    if(e == cudaSuccess && s->g.dims >= 2) {
-        e = launch_col<COL_FWD>(s, 1, st);
-        n++;
-    }
-    if(e == cudaSuccess && s->g.dims == 3) {
-        e = launch_col<COL_FWD>(s, 2, st);
-        n++;
-    }
+    if(e == cudaSuccess && s->g.dims == 3) e = launch_col<COL_FWD>(s, 1, st);
+    if(e == cudaSuccess && s->g.dims >= 2) e = launch_col<COL_INIT>(s, s->g.dims - 1, st, ColOps(), hat);
     s->work = saved;
-    *launches += n;
+    *launches += s->g.dims;
     return e;
 }
 
 cudaError_t spectral_c2r(SpectralState *s, double2 *hat, double *real, cudaStream_t st, int *launches) {
     double2 *saved = s->work;
-    s->work = hat;
+    if(s->g.dims == 1) s->work = hat;
     cudaError_t e = cudaSuccess;
-    int n = 0;
-    if(s->g.dims == 3) {
-        e = launch_col<COL_INV>(s, 2, st);
-        n++;
-    }
-    if(e == cudaSuccess && s->g.dims >= 2) {
-        e = launch_col<COL_INV>(s, 1, st);
-        n++;
-    }
-    if(e == cudaSuccess) {
-        e = launch_row<ROW_IN_HAT, false, true, false>(s, nullptr, real, st);
-        n++;
-    }
+    if(s->g.dims >= 2) e = launch_col<COL_LOAD_INV>(s, s->g.dims - 1, st, ColOps(), hat);
+    if(e == cudaSuccess && s->g.dims == 3) e = launch_col<COL_INV>(s, 1, st);
+    if(e == cudaSuccess) e = launch_row<ROW_IN_HAT, false, true, false>(s, nullptr, real, st);
     s->work = saved;
-    *launches += n;
+    *launches += s->g.dims;
     return e;
 }
 long long spectral_hat_size(const SpectralState *s) { return s->hat; }
@@ -1569,105 +1542,60 @@ long long spectral_hat_size(const SpectralState *s) { return s->hat; }
 // ---- the variable-mobility step with its pointwise stages on the passes -----
 // dims >= 2.  The stage rides on the slowest axis's column pass (y in 2D, z in
 // 3D): the first inverse pass of a c2r loads through it, the last forward pass
-// of an r2c stores through it.  `scratch` stands in for the state's work array.
+// of an r2c stores through it.
 
 cudaError_t spectral_psmob_fprime(SpectralState *s, const double *rho, double2 *fder_hat, double2 *mu,
-                                  const double2 *rho_hat, const PsmobTables &t, double two_k, cudaStream_t st,
+                                  const double2 *rho_hat, const double *q2, double two_k, cudaStream_t st,
                                   int *launches) {
-    double2 *saved = s->work;
-    s->work = fder_hat;
     const int last = s->g.dims - 1;
     cudaError_t e = launch_row<ROW_IN_REAL, true, false, true>(s, rho, nullptr, st);
-    int n = 1;
-    if(e == cudaSuccess && s->g.dims == 3) {
-        e = launch_col<COL_FWD>(s, 1, st);
-        n++;
-    }
-    if(e == cudaSuccess) {
-        if(mu) {
-            ColOps o{};
-            o.q2 = t.q2;
-            o.dealias = t.dealias;
-            o.use_dealias = t.use_dealias;
-            o.rho = const_cast<double2 *>(rho_hat);   // read only in this mode
-            o.out = mu;
-            o.two_k = two_k;
-            e = launch_col<COL_FWD_MU>(s, last, st, o);
-        }
-        else {
-            e = launch_col<COL_FWD>(s, last, st);
-        }
-        n++;
-    }
-    s->work = saved;
-    *launches += n;
+    if(e == cudaSuccess && s->g.dims == 3) e = launch_col<COL_FWD>(s, 1, st);
+    ColOps o{};
+    o.q2 = q2;
+    o.rho = const_cast<double2 *>(rho_hat);   // read only in this mode
+    o.out = mu;
+    o.two_k = two_k;
+    if(e == cudaSuccess)
+        e = mu ? launch_col<COL_FWD_MU>(s, last, st, o, fder_hat) : launch_col<COL_INIT>(s, last, st, o, fder_hat);
+    *launches += s->g.dims;
     return e;
 }
 
-cudaError_t spectral_psmob_flux(SpectralState *s, const double2 *src, const double *kd, const PsmobTables &t,
-                                const double *mob, const double *M0, double2 *div, bool first, double2 *scratch,
-                                cudaStream_t st, int *launches) {
-    double2 *saved = s->work;
-    s->work = scratch;
+cudaError_t spectral_psmob_flux(SpectralState *s, const double2 *src, const double *kd, const double *mob,
+                                const double *M0, double2 *div, bool first, cudaStream_t st, int *launches) {
     const int last = s->g.dims - 1;
     ColOps o{};
     o.kd = kd;
-    o.dealias = t.dealias;
-    o.use_dealias = t.use_dealias;
     o.src = src;
     o.out = div;
     o.first = first ? 1 : 0;
     cudaError_t e = launch_col<COL_GRAD_INV>(s, last, st, o);
-    int n = 1;
-    if(e == cudaSuccess && s->g.dims == 3) {
-        e = launch_col<COL_INV>(s, 1, st);
-        n++;
-    }
-    if(e == cudaSuccess) {
+    if(e == cudaSuccess && s->g.dims == 3) e = launch_col<COL_INV>(s, 1, st);
+    if(e == cudaSuccess)
         e = M0 ? launch_row_flux<FLUX_DM>(s, mob, M0, st) : launch_row_flux<FLUX_M>(s, mob, nullptr, st);
-        n++;
-    }
-    if(e == cudaSuccess && s->g.dims == 3) {
-        e = launch_col<COL_FWD>(s, 1, st);
-        n++;
-    }
-    if(e == cudaSuccess) {
-        e = launch_col<COL_FWD_DIV>(s, last, st, o);
-        n++;
-    }
-    s->work = saved;
-    *launches += n;
+    if(e == cudaSuccess && s->g.dims == 3) e = launch_col<COL_FWD>(s, 1, st);
+    if(e == cudaSuccess) e = launch_col<COL_FWD_DIV>(s, last, st, o);
+    *launches += 2 * s->g.dims - 1;
     return e;
 }
 
 cudaError_t spectral_psmob_update(SpectralState *s, double2 *rho_hat, const double2 *fder_hat, const double2 *div_hat,
                                   const double *q2, const double *M0, double dt, double Ssplit, double k0,
-                                  double2 *scratch, double *rho, cudaStream_t st, int *launches) {
-    double2 *saved = s->work;
-    s->work = scratch;
+                                  double *rho, cudaStream_t st, int *launches) {
     ColOps o{};
     o.q2 = q2;
     o.M0 = M0;
     o.rho = rho_hat;
-    o.fder = fder_hat;
     o.div_in = div_hat;
     o.with_div = div_hat ? 1 : 0;
     o.dt = dt;
     o.Ssplit = Ssplit;
     o.two_k = 2.0 * k0;
     o.log2_bins = s->g.dims * s->g.log2N;
-    cudaError_t e = launch_col<COL_UPD_INV>(s, s->g.dims - 1, st, o);
-    int n = 1;
-    if(e == cudaSuccess && s->g.dims == 3) {
-        e = launch_col<COL_INV>(s, 1, st);
-        n++;
-    }
-    if(e == cudaSuccess) {
-        e = launch_row<ROW_IN_HAT, false, true, false>(s, nullptr, rho, st);
-        n++;
-    }
-    s->work = saved;
-    *launches += n;
+    cudaError_t e = launch_col<COL_UPD_INV>(s, s->g.dims - 1, st, o, const_cast<double2 *>(fder_hat));   // read only
+    if(e == cudaSuccess && s->g.dims == 3) e = launch_col<COL_INV>(s, 1, st);
+    if(e == cudaSuccess) e = launch_row<ROW_IN_HAT, false, true, false>(s, nullptr, rho, st);
+    *launches += s->g.dims;
     return e;
 }
 

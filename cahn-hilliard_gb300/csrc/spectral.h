@@ -29,31 +29,29 @@ int spectral_real(SpectralState *s, double *d_rho, cudaStream_t st, int64_t *lau
 const double2 *spectral_psi_hat(const SpectralState *s, int species);
 double2 *spectral_psi_hat_mut(SpectralState *s);
 // FFTW-style unnormalised transforms of S-species fields on caller buffers
-// (the half spectrum row by row, kx fastest); c2r overwrites `hat`.
+// (column by column as above; 1D: c2r overwrites `hat`).
 cudaError_t spectral_r2c(SpectralState *s, const double *real, double2 *hat, cudaStream_t st, int *launches);
 cudaError_t spectral_c2r(SpectralState *s, double2 *hat, double *real, cudaStream_t st, int *launches);
+// Place of a mode in those spectra, by its place in the order kx fastest, then ky, then kz.
+long long spectral_line_index(const Geom &g, long long mode);
 long long spectral_hat_size(const SpectralState *s);   // complex values per species
 
 // ---- the variable-mobility step's transforms with its pointwise stages fused
 // (psmob.cu; dims >= 2).  Each is the plain transform plus the matching
-// elementwise stage, to rounding, of src/integrators/PseudospectralMobilityCPU.cpp.
-struct PsmobTables {
-    const double *q2, *dealias;   // |k|^2 and the dealiasing mask, half-spectrum layout
-    int use_dealias;
-};
-// fder_hat = R2C(f'(rho)); with mu non-null also mu = D (fder_hat + two_k q2 rho_hat) (:245-254).
+// elementwise stage, to rounding, of src/integrators/PseudospectralMobilityCPU.cpp;
+// spectra and tables column by column.
+// fder_hat = R2C(f'(rho)); with mu non-null also mu = fder_hat + two_k q2 rho_hat (:245-254).
 cudaError_t spectral_psmob_fprime(SpectralState *s, const double *rho, double2 *fder_hat, double2 *mu,
-                                  const double2 *rho_hat, const PsmobTables &t, double two_k, cudaStream_t st,
+                                  const double2 *rho_hat, const double *q2, double two_k, cudaStream_t st,
                                   int *launches);
-// One axis of the flux divergence (:258-293): g = C2R(D i k_d src), g <- (M - M0) g / N^d
-// (M g / N^d when M0 is null), div (= if first, += otherwise) i k_d D R2C(g).  scratch: a half spectrum.
-cudaError_t spectral_psmob_flux(SpectralState *s, const double2 *src, const double *kd, const PsmobTables &t,
-                                const double *mob, const double *M0, double2 *div, bool first, double2 *scratch,
-                                cudaStream_t st, int *launches);
+// One axis of the flux divergence (:258-293): g = C2R(i k_d src), g <- (M - M0) g / N^d (M g / N^d when
+// M0 is null), div (= if first, += otherwise) i k_d R2C(g).  kd: k_d, 0 for the modes dealiasing drops.
+cudaError_t spectral_psmob_flux(SpectralState *s, const double2 *src, const double *kd, const double *mob,
+                                const double *M0, double2 *div, bool first, cudaStream_t st, int *launches);
 // The semi-implicit update of rho_hat (:296-306; div_hat null: constant mobility) and rho = C2R(rho_hat / N^d).
 cudaError_t spectral_psmob_update(SpectralState *s, double2 *rho_hat, const double2 *fder_hat, const double2 *div_hat,
                                   const double *q2, const double *M0, double dt, double Ssplit, double k0,
-                                  double2 *scratch, double *rho, cudaStream_t st, int *launches);
+                                  double *rho, cudaStream_t st, int *launches);
 
 // ---- adjoint support (adjoint.cu) -------------------------------------------
 // psi_hat <- hat and the transformed rows a step starts from.
