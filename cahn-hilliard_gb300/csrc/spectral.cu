@@ -740,18 +740,16 @@ static void build_twiddles(int N, std::vector<int4> &wf) {
 
 static void tune_col_shape(SpectralState *s);
 
-// Values per thread of a box's line transforms: four where the box has too few
-// lines to fill the GPU's schedulers eight values to a thread (a shorter chain
-// for each warp), eight where it has not (fewer twiddle products and
-// exchanges).
-// GB300, us per pass of 2D N=1024: `pseudospectral` (100 steps), rows with four
-// and COL_STEP with eight 5694, both four 6170, both eight 5890; the
-// variable-mobility step (10 steps; three boxes at once), whose column passes
-// make one transform each, with four 2313, with eight 2459.  2D N=256 Saleh
-// (50 steps): 1406 with four, 1775 with eight.
-static int fx_row_elems(const Geom &g) { return g.dims == 2 && g.N <= 1024 ? 4 : 8; }
-static int fx_col_elems(const Geom &g) { return g.dims == 2 && g.N <= 1024 ? 4 : 8; }
-static int fx_step_elems(const Geom &g) { return g.dims == 2 && g.N <= 512 ? 4 : 8; }
+// Values per thread of a box's line transforms: four up to N = 1024 (twice the
+// warps, each with half the chain of products, hide the latencies of loads and
+// exchanges), eight for longer lines, whose 512 threads of four would leave two
+// CTAs to an SM and whose extra exchange costs more than it hides.
+// GB300, us per `pseudospectral` step of one box alone / of three at once:
+//            2D N=512      N=1024      N=2048      3D N=64     N=128       N=256
+//   four   19.7 / 10.7   45.4 / 35.1   196 / 183   34.7/14.6   91.2/75.2   675/649
+//   eight  24.8 / 11.4   47.2 / 36.3   196 / 173   46.1/21.2   108 /83.1   778/718
+static int fx_row_elems(const Geom &g) { return g.N <= 1024 ? 4 : 8; }
+static int fx_col_elems(const Geom &g) { return g.N <= 1024 ? 4 : 8; }
 
 // The shape with C columns per CTA.
 static ColShape col_shape(const Geom &g, int E, int C) {
@@ -829,7 +827,7 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
         return col_shape(g, E, C);
     };
     s->col = spread(fx_col_elems(g));
-    s->step = spread(fx_step_elems(g));
+    s->step = spread(fx_col_elems(g));
     // shared-memory attributes, once
     auto setattr = [](const void *f, size_t smem) { allow_smem(f, smem); };
 #define SETROW(K, E)                                                                            \
