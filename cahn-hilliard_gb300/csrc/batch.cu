@@ -50,7 +50,7 @@ struct PsGroup {
     PsBatchRep *d_reps = nullptr;
     int2 *d_rows = nullptr;
     int4 *d_cols = nullptr;
-    int nrows = 0, ncols8 = 0, ncols4 = 0;   // column items by their values per thread
+    int nrows = 0, ncols = 0;
     size_t row_smem = 0, col_smem = 0;
 };
 
@@ -152,13 +152,9 @@ static cudaError_t ps_group_upload(chgb_batch *b, PsGroup &g) {
     std::vector<int2> r2;
     for(auto &w : rows) r2.push_back(make_int2(w.v.x, w.v.y));
     std::vector<int4> c4;
-    for(int E : {8, 4}) {
-        for(auto &w : cols)
-            if(reps[w.v.x].col_E == E) c4.push_back(w.v);
-        if(E == 8) g.ncols8 = (int) c4.size();
-    }
+    for(auto &w : cols) c4.push_back(w.v);
     g.nrows = (int) r2.size();
-    g.ncols4 = (int) c4.size() - g.ncols8;
+    g.ncols = (int) c4.size();
     cudaError_t e = cudaMalloc(&g.d_reps, sizeof(PsBatchRep) * reps.size());
     if(e == cudaSuccess) e = cudaMalloc(&g.d_rows, sizeof(int2) * r2.size());
     if(e == cudaSuccess) e = cudaMalloc(&g.d_cols, sizeof(int4) * c4.size());
@@ -177,7 +173,7 @@ static cudaError_t batched_step(chgb_batch *b, int parity, bool ps_batched) {
     }
     if(ps_batched) {
         for(auto &g : b->pg) {
-            cudaError_t e = launch_ps2d_batch(g.kind, g.d_reps, g.d_rows, g.nrows, g.d_cols, g.ncols8, g.ncols4,
+            cudaError_t e = launch_ps2d_batch(g.kind, g.d_reps, g.d_rows, g.nrows, g.d_cols, g.ncols,
                                               g.row_smem, g.col_smem, b->stream);
             if(e != cudaSuccess) return e;
         }
@@ -188,7 +184,7 @@ static cudaError_t batched_step(chgb_batch *b, int parity, bool ps_batched) {
 static int launches_per_batched_step(const chgb_batch *b) {
     int n = 0;
     for(auto &g : b->eg) n += g.nitems > 0 ? 1 : 0;
-    for(auto &g : b->pg) n += (g.nrows > 0 ? 1 : 0) + (g.ncols8 > 0 ? 1 : 0) + (g.ncols4 > 0 ? 1 : 0);
+    for(auto &g : b->pg) n += (g.nrows > 0 ? 1 : 0) + (g.ncols > 0 ? 1 : 0);
     return n;
 }
 

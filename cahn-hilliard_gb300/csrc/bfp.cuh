@@ -214,12 +214,12 @@ __device__ __forceinline__ void fx_scale_by(double2 (&v)[E], bool odd, double f)
 
 // ---------------------------------------------------------------------------
 // One line's forward Stockham FFT of length 2^lg on T = max(1, 2^lg / E)
-// threads, E = 4 or 8 values a thread: v[i] is position lane + i T, on the way
+// threads, E = 2, 4 or 8 values a thread: v[i] is position lane + i T, on the way
 // in and on the way out (2^lg < E: the first 2^lg entries).  The inverse
 // transform is the same with real and imaginary parts swapped on both ways.
 //
-// E = 4: radix 4, after one radix-2 pass (two butterflies a thread) where lg is
-// odd.  E = 8: radix 8, with one radix-4 pass (two butterflies) where lg is 2
+// E = 2: radix 2.  E = 4: radix 4, after one radix-2 pass (two butterflies a
+// thread) where lg is odd.  E = 8: radix 8, with one radix-4 pass (two butterflies) where lg is 2
 // modulo 3 and two where it is 1.  Values stay in registers; between two passes
 // they cross through shared memory, which the line's loads and stores do not
 // touch.
@@ -261,7 +261,8 @@ template <int E>
 __device__ __forceinline__ void fx_fft(fx2 (&v)[E], const FxLine &ln, fx2 *&cur, fx2 *&oth,
                                        const int4 *__restrict__ tw, int lgtab) {
     const int lg = ln.lg, lane = ln.lane;
-    if(lg < (E == 8 ? 3 : 2)) {   // one thread per line
+    if(lg < (E == 8 ? 3 : E == 4 ? 2 : 1)) {   // one thread per line
+        if(E == 2) return;
         if(E == 8 && lg == 2) fx_dft4(v[0], v[1], v[2], v[3]);
         else {
             const fx2 s = fx_add(v[0], v[1]);
@@ -282,6 +283,17 @@ __device__ __forceinline__ void fx_fft(fx2 (&v)[E], const FxLine &ln, fx2 *&cur,
 #pragma unroll
                 for(int m = 0; m < 8; m++) cur[o + (m << ln.lgC)] = v[m];
             }
+        }
+    }
+    else if(E == 2) {
+        const fx2 s = fx_add(v[0], v[1]);
+        v[1] = fx_sub(v[0], v[1]);
+        v[0] = s;
+        ns = 1;
+        if(lg > 1) {
+            const int o = ln.at(lane << 1);
+            cur[o] = v[0];
+            cur[o + (1 << ln.lgC)] = v[1];
         }
     }
     else if(lg & 1) {
@@ -327,9 +339,22 @@ __device__ __forceinline__ void fx_fft(fx2 (&v)[E], const FxLine &ln, fx2 *&cur,
                 continue;
             }
         }
-        constexpr int B = E / 4;   // butterflies a thread
+        if constexpr(E == 2) {
+            const int k = lane & ((1 << ns) - 1);
+            const fx2 t = fx_cmul<false>(v[1], __ldg(&tw[k << (lgtab - ns - 1)])), s = fx_add(v[0], t);
+            v[1] = fx_sub(v[0], t);
+            v[0] = s;
+            if(left > 1) {
+                const int p = ((lane - k) << 1) + k;
+                cur[ln.at(p)] = v[0];
+                cur[ln.at(p + (1 << ns))] = v[1];
+            }
+            ns += 1;
+            continue;
+        }
+        constexpr int B = E >= 4 ? E / 4 : 1;   // butterflies a thread
 #pragma unroll
-        for(int b = 0; b < B; b++) {
+        for(int b = 0; b < (E >= 4 ? B : 0); b++) {
             const int j = lane + b * ln.T;
             const int k = j & ((1 << ns) - 1);
             const int q = k << (lgtab - ns - 2);

@@ -62,7 +62,7 @@ inline int fx_line_threads(int L, int E) { return L > E ? L / E : 1; }
 
 template <int E>
 __device__ __forceinline__ FxLine fx_line(int lg, int lgC, bool whole_block) {
-    constexpr int lgE = E == 8 ? 3 : 2;
+    constexpr int lgE = E == 8 ? 3 : E == 4 ? 2 : 1;
     FxLine ln;
     ln.lg = lg;
     ln.lgC = lgC;
@@ -381,8 +381,12 @@ __global__ void __launch_bounds__(256) row_batch_kernel(const PsBatchRep *__rest
     extern __shared__ fx2 sm2[];
     const int2 it = items[blockIdx.x];
     const PsBatchRep &r = reps[it.x];
-    row_body<KIND, PS_BATCH_ROW_E, ROW_IN_HAT, true, false, true>(r.work, nullptr, nullptr, r.log2N - 1, r.row_rpc, r.bins, r.hat,
-                                                  r.twf, r.m, it.y, sm2);
+    if(r.E == 2)
+        row_body<KIND, 2, ROW_IN_HAT, true, false, true>(r.work, nullptr, nullptr, r.log2N - 1, r.row_rpc, r.bins, r.hat,
+                                                         r.twf, r.m, it.y, sm2);
+    else
+        row_body<KIND, 4, ROW_IN_HAT, true, false, true>(r.work, nullptr, nullptr, r.log2N - 1, r.row_rpc, r.bins, r.hat,
+                                                         r.twf, r.m, it.y, sm2);
 }
 
 enum { COL_FWD = 0, COL_INV = 1, COL_STEP = 2, COL_INIT = 3, COL_GRAD_INV = 4, COL_FWD_DIV = 5, COL_FWD_MU = 6,
@@ -543,7 +547,7 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
 }
 
 template <int MODE, int E>
-__global__ void __launch_bounds__(512, E == 4 ? 2 : 1) col_kernel(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
+__global__ void __launch_bounds__(512, E == 8 ? 1 : 2) col_kernel(double2 *__restrict__ work, double2 *__restrict__ psi_hat,
                                                   const double2 *__restrict__ ab, int lgL, int H, int lgC,
                                                   long long elem_stride,
                                                   long long plane_stride, long long hat,
@@ -556,14 +560,15 @@ __global__ void __launch_bounds__(512, E == 4 ? 2 : 1) col_kernel(double2 *__res
 
 // Batched 2D column pass (forward, update, inverse) of one time step:
 // CTA b takes columns items[b].z.. of species items[b].y of replica items[b].x.
-template <int E>
-__global__ void __launch_bounds__(256, E == 4 ? 4 : 2) col_batch_kernel(const PsBatchRep *__restrict__ reps,
-                                                                       const int4 *__restrict__ items) {
+__global__ void __launch_bounds__(256, 4) col_batch_kernel(const PsBatchRep *__restrict__ reps,
+                                                           const int4 *__restrict__ items) {
     extern __shared__ fx2 sm2[];
     const int4 it = items[blockIdx.x];
     const PsBatchRep &r = reps[it.x];
-    col_body<COL_STEP, E>(r.work, r.psi_hat, r.ab, r.log2N, r.H, r.log2C, r.H, 0, r.hat, r.twf, 0.0, it.z, 0, it.y,
-                          sm2);
+    if(r.E == 2)
+        col_body<COL_STEP, 2>(r.work, r.psi_hat, r.ab, r.log2N, r.H, r.log2C, r.H, 0, r.hat, r.twf, 0.0, it.z, 0, it.y, sm2);
+    else
+        col_body<COL_STEP, 4>(r.work, r.psi_hat, r.ab, r.log2N, r.H, r.log2C, r.H, 0, r.hat, r.twf, 0.0, it.z, 0, it.y, sm2);
 }
 
 // 1D: elementwise init (psi_t = F[rho] / N) or update on the half spectrum.
@@ -740,16 +745,20 @@ static void build_twiddles(int N, std::vector<int4> &wf) {
 
 static void tune_col_shape(SpectralState *s);
 
-// Values per thread of a box's line transforms: four up to N = 1024 (twice the
-// warps, each with half the chain of products, hide the latencies of loads and
-// exchanges), eight for longer lines, whose 512 threads of four would leave two
-// CTAs to an SM and whose extra exchange costs more than it hides.
+// Values per thread of a box's line transforms.  The fewer, the more warps and
+// the shorter each one's chain of products, which hides the latencies of loads
+// and exchanges; the more, the fewer exchanges and twiddle products.  Two where
+// one box leaves most of the GPU's schedulers idle (2D N <= 256, 3D N <= 64),
+// four up to N = 1024, eight for longer lines, whose 512 threads of four would
+// leave two CTAs to an SM.
 // GB300, us per `pseudospectral` step of one box alone / of three at once:
-//            2D N=512      N=1024      N=2048      3D N=64     N=128       N=256
-//   four   19.7 / 10.7   45.4 / 35.1   196 / 183   34.7/14.6   91.2/75.2   675/649
-//   eight  24.8 / 11.4   47.2 / 36.3   196 / 173   46.1/21.2   108 /83.1   778/718
-static int fx_row_elems(const Geom &g) { return g.N <= 1024 ? 4 : 8; }
-static int fx_col_elems(const Geom &g) { return g.N <= 1024 ? 4 : 8; }
+//          2D N=64     N=256      N=512      N=1024     N=2048     3D N=32    N=64       N=128      N=256
+//   two    10.7/4.1   13.6/5.8   22.6/12.1                         18.0/6.7   33.0/13.5  92.0/74.8
+//   four   14.9/5.2   14.8/5.7   19.7/10.7  45.4/35.1  196/183     22.0/8.3   34.5/14.6  91.2/75.2  675/649
+//   eight                        24.8/11.4  47.2/36.3  196/173                46.1/21.2  108 /83.1  778/718
+// (2D N=256 with two: the adjoint's 200 steps 9080 -> 7685 us, two GMRES steps
+// 2062 -> 1715; a batch of 33 boxes up to N=512 2742 -> 2778.)
+static int fx_line_elems(const Geom &g) { return g.N <= (g.dims == 3 ? 64 : 256) ? 2 : g.N <= 1024 ? 4 : 8; }
 
 // The shape with C columns per CTA.
 static ColShape col_shape(const Geom &g, int E, int C) {
@@ -803,7 +812,7 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
         err = "table upload failed";
         return CHGB_ERR_CUDA;
     }
-    s->row_E = fx_row_elems(g);
+    s->row_E = fx_line_elems(g);
     s->pdl = g.dims == 3;
     // launch shapes.  A CTA takes at least a warp's worth of lines, then more up
     // to 128 threads while ~2 CTAs per SM are left: small boxes want their few
@@ -826,8 +835,8 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
             C *= 2;
         return col_shape(g, E, C);
     };
-    s->col = spread(fx_col_elems(g));
-    s->step = spread(fx_col_elems(g));
+    s->col = spread(fx_line_elems(g));
+    s->step = spread(fx_line_elems(g));
     // shared-memory attributes, once
     auto setattr = [](const void *f, size_t smem) { allow_smem(f, smem); };
 #define SETROW(K, E)                                                                            \
@@ -844,17 +853,21 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
     SETROW(CHGB_MODEL_LANDAU, 4)
     SETROW(CHGB_MODEL_SIMPLE_WERTHEIM, 4)
     SETROW(CHGB_MODEL_SALEH, 4)
+    SETROW(CHGB_MODEL_LANDAU, 2)
+    SETROW(CHGB_MODEL_SIMPLE_WERTHEIM, 2)
+    SETROW(CHGB_MODEL_SALEH, 2)
 #undef SETROW
-    for(const void *f : {(const void *) col_kernel<COL_FWD, 8>, (const void *) col_kernel<COL_INV, 8>,
-                         (const void *) col_kernel<COL_STEP, 8>, (const void *) col_kernel<COL_INIT, 8>,
-                         (const void *) col_kernel<COL_GRAD_INV, 8>, (const void *) col_kernel<COL_FWD_DIV, 8>,
-                         (const void *) col_kernel<COL_FWD_MU, 8>, (const void *) col_kernel<COL_UPD_INV, 8>,
-                         (const void *) col_kernel<COL_LOAD_INV, 8>, (const void *) col_kernel<COL_LOAD_INV, 4>,
-                         (const void *) col_kernel<COL_FWD, 4>, (const void *) col_kernel<COL_INV, 4>,
-                         (const void *) col_kernel<COL_STEP, 4>, (const void *) col_kernel<COL_INIT, 4>,
-                         (const void *) col_kernel<COL_GRAD_INV, 4>, (const void *) col_kernel<COL_FWD_DIV, 4>,
-                         (const void *) col_kernel<COL_FWD_MU, 4>, (const void *) col_kernel<COL_UPD_INV, 4>})
+#define SETCOL(E)                                                                                                  \
+    for(const void *f : {(const void *) col_kernel<COL_FWD, E>, (const void *) col_kernel<COL_INV, E>,             \
+                         (const void *) col_kernel<COL_STEP, E>, (const void *) col_kernel<COL_INIT, E>,           \
+                         (const void *) col_kernel<COL_GRAD_INV, E>, (const void *) col_kernel<COL_FWD_DIV, E>,    \
+                         (const void *) col_kernel<COL_FWD_MU, E>, (const void *) col_kernel<COL_UPD_INV, E>,      \
+                         (const void *) col_kernel<COL_LOAD_INV, E>})                                              \
         setattr(f, 224 * 1024);   // whatever shape the timing below picks
+    SETCOL(8)
+    SETCOL(4)
+    SETCOL(2)
+#undef SETCOL
     cudaError_t e = cudaGetLastError();
     if(e != cudaSuccess) {
         spectral_destroy(s);
@@ -901,8 +914,9 @@ dim3 row_grid(const SpectralState *s) { return dim3((unsigned) ((long long) s->g
 
 template <int KIND, int IN, bool FPRIME, bool WRITE_REAL, bool R2C>
 cudaError_t launch_row_kind(SpectralState *s, const double *real_in, double *real_out, cudaStream_t st) {
-    auto kernel = s->row_E == 8 ? row_kernel<KIND, 8, IN, FPRIME, WRITE_REAL, R2C>
-                            : row_kernel<KIND, 4, IN, FPRIME, WRITE_REAL, R2C>;
+    auto kernel = s->row_E == 8   ? row_kernel<KIND, 8, IN, FPRIME, WRITE_REAL, R2C>
+                  : s->row_E == 4 ? row_kernel<KIND, 4, IN, FPRIME, WRITE_REAL, R2C>
+                                  : row_kernel<KIND, 2, IN, FPRIME, WRITE_REAL, R2C>;
     return launch_pass(s, kernel, row_grid(s), s->row_threads, s->row_smem, st, s->work, real_in, real_out, ilog2(s->g.N) - 1, s->row_rpc, s->g.bins, s->hat, s->twf, s->m,
                        nullptr, nullptr);
 }
@@ -910,8 +924,9 @@ cudaError_t launch_row_kind(SpectralState *s, const double *real_in, double *rea
 // Row pass of the variable-mobility flux: c2r of work's rows, the flux stage, r2c back into work.
 template <int KIND, int FLUX>
 cudaError_t launch_row_flux_kind(SpectralState *s, const double *mob, const double *M0, cudaStream_t st) {
-    auto kernel = s->row_E == 8 ? row_kernel<KIND, 8, ROW_IN_HAT, false, false, true, FLUX>
-                            : row_kernel<KIND, 4, ROW_IN_HAT, false, false, true, FLUX>;
+    auto kernel = s->row_E == 8   ? row_kernel<KIND, 8, ROW_IN_HAT, false, false, true, FLUX>
+                  : s->row_E == 4 ? row_kernel<KIND, 4, ROW_IN_HAT, false, false, true, FLUX>
+                                  : row_kernel<KIND, 2, ROW_IN_HAT, false, false, true, FLUX>;
     return launch_pass(s, kernel, row_grid(s), s->row_threads, s->row_smem, st, s->work, nullptr, nullptr, ilog2(s->g.N) - 1, s->row_rpc, s->g.bins, s->hat,
                        s->twf, s->m, mob, M0);
 }
@@ -962,7 +977,7 @@ cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps
     }
     const ColShape &c = MODE == COL_STEP ? s->step : s->col;
     const int C = 1 << c.lgC;
-    auto kernel = c.E == 8 ? col_kernel<MODE, 8> : col_kernel<MODE, 4>;
+    auto kernel = c.E == 8 ? col_kernel<MODE, 8> : c.E == 4 ? col_kernel<MODE, 4> : col_kernel<MODE, 2>;
     return launch_pass(s, kernel, dim3((unsigned) ((H + C - 1) / C), (unsigned) planes, (unsigned) s->g.S), c.threads,
                        c.smem, st, s->work, spec ? spec : s->psi_hat, s->ab, ilog2(N), H, c.lgC, elem_stride, plane_stride, s->hat,
                        s->twf, spec ? 1.0 : 1.0 / (double) s->g.bins, ops);
@@ -1145,7 +1160,7 @@ void spectral_batch_rep(const SpectralState *s, PsBatchRep *r, size_t *row_smem,
     r->H = s->H;
     r->bins = s->g.bins;
     r->hat = s->hat;
-    r->col_E = s->step.E;
+    r->E = s->row_E;   // the columns' as well
     const int row_T = fx_line_threads(M, s->row_E), col_T = fx_line_threads(N, s->step.E);
     r->row_rpc = 1;
     while(r->row_rpc * 2 * row_T * S <= PS_BATCH_THREADS && r->row_rpc * 2 <= N) r->row_rpc *= 2;
@@ -1159,8 +1174,7 @@ namespace {
 template <int KIND>
 cudaError_t configure_kind(size_t row_smem, size_t col_smem) {
     cudaError_t e = allow_smem((const void *) row_batch_kernel<KIND>, row_smem);
-    if(e == cudaSuccess) e = allow_smem((const void *) col_batch_kernel<4>, col_smem);
-    if(e == cudaSuccess) e = allow_smem((const void *) col_batch_kernel<8>, col_smem);
+    if(e == cudaSuccess) e = allow_smem((const void *) col_batch_kernel, col_smem);
     return e;
 }
 }  // namespace
@@ -1174,7 +1188,7 @@ cudaError_t configure_ps2d_batch(int kind, size_t row_smem, size_t col_smem) {
 }
 
 cudaError_t launch_ps2d_batch(int kind, const PsBatchRep *reps, const int2 *row_items, int nrow, const int4 *col_items,
-                              int ncol8, int ncol4, size_t row_smem, size_t col_smem, cudaStream_t st) {
+                              int ncol, size_t row_smem, size_t col_smem, cudaStream_t st) {
     if(nrow > 0) {
         switch(kind) {
             case CHGB_MODEL_LANDAU:
@@ -1188,8 +1202,7 @@ cudaError_t launch_ps2d_batch(int kind, const PsBatchRep *reps, const int2 *row_
         cudaError_t e = cudaGetLastError();
         if(e != cudaSuccess) return e;
     }
-    if(ncol8 > 0) col_batch_kernel<8><<<ncol8, PS_BATCH_THREADS, col_smem, st>>>(reps, col_items);
-    if(ncol4 > 0) col_batch_kernel<4><<<ncol4, PS_BATCH_THREADS, col_smem, st>>>(reps, col_items + ncol8);
+    if(ncol > 0) col_batch_kernel<<<ncol, PS_BATCH_THREADS, col_smem, st>>>(reps, col_items);
     return cudaGetLastError();
 }
 
@@ -1240,13 +1253,13 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
 
 // Row pass of the adjoint step: work rows (x half spectrum of beta lam_hat after
 // the inverse y transform) -> C2R -> B lam; geps += <B lam, psi_n>; * f''(psi_n) -> R2C.
+template <int E>
 __global__ void __launch_bounds__(256) row_adj_kernel(double2 *__restrict__ work, const double *__restrict__ psi_n,
                                                      int lgM, int rows_per_cta, const int4 *__restrict__ twf,
                                                      double eps, double *__restrict__ geps) {
     extern __shared__ fx2 sm2[];
     __shared__ double red[32];
     __shared__ int sm_w[2][FX_MAX_WARPS];
-    constexpr int E = 4;   // fx_row_elems of the adjoint's boxes, N <= 1024
     const FxLine ln = fx_line<E>(lgM, 0, false);
     const int M = 1 << lgM, N = 2 * M, LS = fx_line_size(M);
     const int li = threadIdx.x / ln.T, nl = blockDim.x / ln.T;
@@ -1275,7 +1288,7 @@ enum { ADJ_A = 1, ADJ_B = 2, ADJ_BA = 3 };
 // Column pass of the adjoint: B part (forward y FFT of the row result, lam_hat
 // update) and/or A part (gradient sums with psi_next = psi_t_{n+1} and
 // psi_cur = psi_t_n, then beta * lam_hat and the inverse y FFT into work).
-template <int MODE>
+template <int MODE, int E>
 __global__ void __launch_bounds__(512) col_adj_kernel(double2 *__restrict__ work, double2 *__restrict__ lam,
                                                      const double2 *__restrict__ ab,
                                                      const double *__restrict__ tk, const double *__restrict__ tm1,
@@ -1287,7 +1300,6 @@ __global__ void __launch_bounds__(512) col_adj_kernel(double2 *__restrict__ work
     extern __shared__ fx2 sm2[];
     __shared__ double red[32];
     __shared__ int sm_w[2][FX_MAX_WARPS * FX_MAX_INTERLEAVE];
-    constexpr int E = 4;   // fx_col_elems of the adjoint's boxes, N <= 1024
     const int C = 1 << lgC;   // at most FX_MAX_INTERLEAVE: one group
     const FxLine ln = fx_line<E>(lgL, lgC, false);
     const int L = 1 << lgL;
@@ -1397,10 +1409,11 @@ SpectralAdj *spectral_adj_create(SpectralState *s, std::string &err) {
          cudaMemcpy(a->tm2, tm2.data(), sizeof(double) * s->hat, cudaMemcpyHostToDevice) == cudaSuccess;
     if(ok) {
         size_t rs = s->row_smem, cs = s->col.smem;
-        allow_smem((const void *) row_adj_kernel, rs);
-        allow_smem((const void *) col_adj_kernel<ADJ_A>, cs);
-        allow_smem((const void *) col_adj_kernel<ADJ_B>, cs);
-        allow_smem((const void *) col_adj_kernel<ADJ_BA>, cs);
+        for(const void *f : {(const void *) row_adj_kernel<2>, (const void *) row_adj_kernel<4>}) allow_smem(f, rs);
+        for(const void *f : {(const void *) col_adj_kernel<ADJ_A, 2>, (const void *) col_adj_kernel<ADJ_A, 4>,
+                             (const void *) col_adj_kernel<ADJ_B, 2>, (const void *) col_adj_kernel<ADJ_B, 4>,
+                             (const void *) col_adj_kernel<ADJ_BA, 2>, (const void *) col_adj_kernel<ADJ_BA, 4>})
+            allow_smem(f, cs);
         ok = cudaGetLastError() == cudaSuccess;
     }
     if(!ok) {
@@ -1450,14 +1463,18 @@ cudaError_t spectral_adj_col(SpectralAdj *a, SpectralState *s, int mode, const d
 #define ADJ_COL_ARGS                                                                                                   \
     a->work, a->lam, s->ab, a->tk, a->tm1, a->tm2, psi_next, psi_cur, ilog2(N), s->H, s->col.lgC, s->twf,      \
         a->gk, a->gm
-    auto kernel = mode == ADJ_A ? col_adj_kernel<ADJ_A> : mode == ADJ_B ? col_adj_kernel<ADJ_B> : col_adj_kernel<ADJ_BA>;
+    // the adjoint's boxes (N <= 1024) have two or four values a thread
+    auto kernel = s->col.E == 2
+                      ? (mode == ADJ_A ? col_adj_kernel<ADJ_A, 2> : mode == ADJ_B ? col_adj_kernel<ADJ_B, 2> : col_adj_kernel<ADJ_BA, 2>)
+                      : (mode == ADJ_A ? col_adj_kernel<ADJ_A, 4> : mode == ADJ_B ? col_adj_kernel<ADJ_B, 4> : col_adj_kernel<ADJ_BA, 4>);
     kernel<<<grid, s->col.threads, s->col.smem, st>>>(ADJ_COL_ARGS);
 #undef ADJ_COL_ARGS
     return cudaGetLastError();
 }
 
 cudaError_t spectral_adj_row(SpectralAdj *a, SpectralState *s, const double *psi_n, cudaStream_t st) {
-    row_adj_kernel<<<a->n_row_cta, s->row_threads, s->row_smem, st>>>(a->work, psi_n, ilog2(s->g.N) - 1, s->row_rpc,
+    auto kernel = s->row_E == 2 ? row_adj_kernel<2> : row_adj_kernel<4>;
+    kernel<<<a->n_row_cta, s->row_threads, s->row_smem, st>>>(a->work, psi_n, ilog2(s->g.N) - 1, s->row_rpc,
                                                                        s->twf, s->m.epsilon, a->geps);
     return cudaGetLastError();
 }

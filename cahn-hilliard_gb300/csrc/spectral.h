@@ -87,10 +87,10 @@ struct PsBatchRep {
     int N, log2N, H;
     int row_rpc;            // rows per CTA
     int col_C, log2C;       // columns per CTA
-    int col_E;              // values per thread of a column line (a row line has PS_BATCH_ROW_E)
+    int E;                  // values per thread of a line, 2 or 4
     long long bins, hat;
 };
-constexpr int PS_BATCH_THREADS = 256, PS_BATCH_ROW_E = 4;
+constexpr int PS_BATCH_THREADS = 256;
 // 2D, N in [8, 1024]: the state can join a batch.
 bool spectral_batchable(const SpectralState *s);
 // Fill the descriptor; returns the dynamic shared memory its row and column CTAs need.
@@ -100,8 +100,7 @@ bool spectral_hat_valid(const SpectralState *s);
 // Record `nsteps` steps taken by batched kernels.
 void spectral_mark_stepped(SpectralState *s);
 cudaError_t configure_ps2d_batch(int kind, size_t row_smem, size_t col_smem);
-// The column items of the replicas with eight values per thread come first (ncol8), then the others' (ncol4).
 cudaError_t launch_ps2d_batch(int kind, const PsBatchRep *reps, const int2 *row_items, int nrow, const int4 *col_items,
-                              int ncol8, int ncol4, size_t row_smem, size_t col_smem, cudaStream_t st);
+                              int ncol, size_t row_smem, size_t col_smem, cudaStream_t st);
 
 }  // namespace chgb
