@@ -240,6 +240,11 @@ static float time_variant(chgb_handle *h, int nsteps);
 // Wertheim models' number densities are of order 1e-5 in internal units.
 static double m_kind_density_scale(const ModelDev &m) { return m.kind == CHGB_MODEL_LANDAU ? 0.0 : 1e-5; }
 
+// euler_mobility in block fixed point by rule, where it measured fastest (us a
+// step, simple_wertheim with the free-energy mobility: 2D N=256 9.3 against 7.3 of
+// the best other variant, N=512 14.1 against 16.5; 3D N=32 20.1 against 35.2).
+static bool fx_mob_measured(const Geom &g) { return g.dims == 2 ? g.N >= 512 : g.N >= 32; }
+
 static void release(chgb_handle *h) {
     if(!h) return;
     for(int i = 0; i < 2; i++) {
@@ -252,6 +257,7 @@ static void release(chgb_handle *h) {
     if(h->d_mu) cudaFree(h->d_mu);
     if(h->d_mobk) cudaFree(h->d_mobk);
     if(h->d_bfp) cudaFree(h->d_bfp);
+    if(h->d_mobkey) cudaFree(h->d_mobkey);
     if(h->d_partials) cudaFree(h->d_partials);
     if(h->d_obs) cudaFree(h->d_obs);
     if(h->d_pressure) cudaFree(h->d_pressure);
@@ -408,7 +414,11 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
                    params->mobility_type == CHGB_MOBILITY_FREE_ENERGY;
         const bool bfp_ok = (want == 0 || want == 5) &&
                             euler_bfp_supported(params->integrator, params->model.kind, h->g);
+        const bool mob_fx = want == 0 && euler_mob_fx_supported(params->integrator, params->model.kind,
+                                                                params->mobility_type, h->g) && fx_mob_measured(h->g);
         ok = cudaMalloc(&h->d_mu, bytes) == cudaSuccess && (!mob || cudaMalloc(&h->d_mobk, bytes) == cudaSuccess) &&
+             (!mob_fx || (cudaMalloc(&h->d_mobkey, 4 * sizeof(unsigned)) == cudaSuccess &&
+                          cudaMemset(h->d_mobkey, 0, 4 * sizeof(unsigned)) == cudaSuccess)) &&
              (!bfp_ok || cudaMalloc(&h->d_bfp, sizeof(BfpState)) == cudaSuccess);
         if(!ok) {
             cudaGetLastError();
@@ -419,6 +429,9 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
         }
         else if(want >= 2) {
             h->variant = want;
+        }
+        else if(mob_fx) {
+            h->variant = 5;   // by a fixed rule, as below
         }
         else if(bfp_ok && ((h->g.dims == 2 && h->g.N >= 512) || (h->g.dims == 3 && h->g.N >= 64))) {
             // block fixed point where it was measured fastest on GB300, by a fixed
@@ -451,7 +464,7 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
         // mu is stored by the split pairs only: variant 2, and variant 5 in 3D
         // where it was asked for by number (launch_euler_bfp)
         const bool bfp_pair = h->variant == 5 && h->g.dims == 3 && want == 5;
-        if(h->variant != 2 && !bfp_pair) {
+        if(h->variant != 2 && !bfp_pair && !(h->variant == 5 && h->d_mobkey)) {
             if(h->d_mu) cudaFree(h->d_mu);
             if(h->d_mobk) cudaFree(h->d_mobk);
             h->d_mu = h->d_mobk = nullptr;
@@ -459,6 +472,10 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
         if(h->variant != 5 && h->d_bfp) {
             cudaFree(h->d_bfp);
             h->d_bfp = nullptr;
+        }
+        if(h->variant != 5 && h->d_mobkey) {
+            cudaFree(h->d_mobkey);
+            h->d_mobkey = nullptr;
         }
         h->launches = 0;
         h->cur = 0;
@@ -574,6 +591,8 @@ static cudaError_t one_step(chgb_handle *h) {
         if(e != cudaSuccess) return e;
     }
     if(h->variant == 2) e = launch_euler_split(h->p.integrator, h->g, h->m, h->ec, in, outp, h->d_mu, h->d_mobk, h->stream);
+    else if(h->d_mobkey)
+        e = launch_euler_split(h->p.integrator, h->g, h->m, h->ec, in, outp, h->d_mu, h->d_mobk, h->stream, h->d_mobkey, h->cur);
     else if(h->variant == 5) e = launch_euler_bfp(h->g, h->ec, in, outp, h->d_mu, h->d_bfp, h->cur, h->stream);
     else e = launch_euler_step(h->p.integrator, h->g, h->m, h->ec, in, outp, h->stream);
     h->cur ^= 1;
@@ -584,7 +603,7 @@ static cudaError_t one_step(chgb_handle *h) {
 // Variant 5: set the block-fixed-point key from the current field, before the
 // first step of a sequence (the steps keep it up to date from then on).
 static cudaError_t bfp_refresh(chgb_handle *h) {
-    if(h->variant != 5) return cudaSuccess;
+    if(h->variant != 5 || h->d_mobkey) return cudaSuccess;   // euler_mobility's key is each step's own
     h->launches += 1;
     return launch_bfp_refresh(h->d_rho[h->cur], (long long) h->n, h->d_bfp, h->cur, h->stream);
 }

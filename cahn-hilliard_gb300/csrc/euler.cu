@@ -793,12 +793,14 @@ __device__ __forceinline__ double split_lap_fx(const double (*ring)[SPP], const 
 
 template <int KIND, int MOB, int DIMS>
 __global__ void __launch_bounds__(256, (KIND == CHGB_MODEL_LANDAU && MOB == 0) ? 8 : 1) mu_kernel(const double *__restrict__ in, double *__restrict__ mu,
-                                                 double *__restrict__ mob, Geom g, ModelDev m, EulerConsts c, int zc) {
+                                                 double *__restrict__ mob, Geom g, ModelDev m, EulerConsts c, int zc,
+                                                 unsigned *__restrict__ key) {
     constexpr int S = NSpecies<KIND>::value;
     constexpr int R = (DIMS == 3) ? 3 : 1;
     // single species: each staged value's fixed-point form is computed once,
     // at staging, instead of at each of its seven uses
     constexpr bool PRE = S == 1;
+    constexpr bool KEYED = S == 1 && (MOB == 1 || MOB == 2);   // the forms update_mob_fx_kernel follows
     __shared__ double ring[R][S][SPP];
     __shared__ long long ringT[PRE ? R : 1][PRE ? SPP : 1];
     __shared__ int ringE[PRE ? R : 1][PRE ? SPP : 1];
@@ -813,6 +815,7 @@ __global__ void __launch_bounds__(256, (KIND == CHGB_MODEL_LANDAU && MOB == 0) ?
         else split_load_plane<DIMS, S>(ring[slot], in, g, x0, y0, z, bins, tid);
     };
     pdl_begin();
+    unsigned top_mu = 0, top_mob = 0;   // with a key: the largest high words of |mu| and |M|
     double pf[SPF];   // plane z + 1, fetched during the previous plane (3D single species)
     if constexpr(DIMS == 3) {
         stage((z0 + 2) % 3, z0 - 1);
@@ -848,10 +851,33 @@ __global__ void __launch_bounds__(256, (KIND == CHGB_MODEL_LANDAU && MOB == 0) ?
             else
                 sum = (DIMS == 3) ? nb_sum6(q[-1], q[1], q[-SPX], q[SPX], ring[(z + 2) % 3][s][p], ring[(z + 1) % 3][s][p])
                                   : nb_sum4(q[-1], q[1], q[-SPX], q[SPX]);
-            if(CHGB_BC(4, gi, bins)) mu[s * bins + gi] = mu_cell<KIND, DIMS>(m, c, s, r[s], d[s], sum);
-            if(MOB == 2) mob[s * bins + gi] = c.M * xsw;
+            const double mv = mu_cell<KIND, DIMS>(m, c, s, r[s], d[s], sum);
+            if(CHGB_BC(4, gi, bins)) mu[s * bins + gi] = mv;
+            if(KEYED) top_mu = max(top_mu, (unsigned) fx_mag(mv));
+            if(MOB == 2) {
+                const double Mv = c.M * xsw;
+                mob[s * bins + gi] = Mv;
+                top_mob = max(top_mob, (unsigned) fx_mag(Mv));
+            }
         }
         __syncthreads();
+    }
+    if constexpr(KEYED) {
+        if(key) {
+            __shared__ unsigned top[2][STY];
+            top_mu = __reduce_max_sync(0xFFFFFFFFu, top_mu);
+            top_mob = __reduce_max_sync(0xFFFFFFFFu, top_mob);
+            if(tx == 0) {
+                top[0][ty] = top_mu;
+                top[1][ty] = top_mob;
+            }
+            __syncthreads();
+            if(tid < 2) {
+                unsigned v = top[tid][0];
+                for(int w = 1; w < STY; w++) v = max(v, top[tid][w]);
+                atomicMax(&key[tid], v);
+            }
+        }
     }
 }
 
@@ -1008,6 +1034,173 @@ __global__ void __launch_bounds__(256, (S == 1 && MOB == 0) ? 8 : 1) update_kern
             if(CHGB_BC(6, gi, bins)) out[s * bins + gi] = res;
         }
         __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The update of euler_mobility in block fixed point (kernel_variant 5,
+// one species, constant or free-energy mobility): mu_kernel writes mu and M and
+// folds their largest magnitudes into a key; here one exponent for each serves
+// the field, U = mu 2^(60-su) and W = M 2^(60-sm) are integers below 2^60, a
+// face's flux (W_a + W_b)(U_b - U_a) is the upper part, in units of 2^62, of one
+// product on IMAD.WIDE (a constant M: the difference itself, |U| < 2^59), and
+// the divergence an int64 sum -- the same integer for both cells of a face, so
+// the fluxes cancel exactly.  A cell takes two FP64 instructions (a conversion
+// and the final FMA) where update_kernel takes 16, which bound it (75 % of that
+// pipe).  simple_wertheim with the free-energy mobility on GB300, us a step (mu
+// and update), the FP64 update and this one: 3D N=64 41.8 and 30.5, N=128 133.8
+// and 78.4, N=256 949 and 538; 2D N=512 16.5 and 14.1, N=1024 48.4 and 33.2.
+//
+// A CTA of 128 threads has a tile of 32 x 16 cells, a warp each of four rows
+// of it: a thread's four cells lie above one another, so that their y faces are
+// formed once but for the warps' borders and the z faces carried from plane to
+// plane; x faces come from the lane to the left, the tile's left ones from one
+// extra product of lanes 0-3.  One barrier a plane, the next plane's values in
+// flight during it.
+// ---------------------------------------------------------------------------
+constexpr int MTX = 32, MTY = 16, MTHR = 128, MPX = MTX + 2, MPP = MPX * (MTY + 2);
+constexpr int MPF = (MPP + MTHR - 1) / MTHR;
+
+// a b 2^-62, |a| and |b| below 2^61 (within 2 units, the same way for every pair).
+__device__ __forceinline__ long long face_flux(long long a, long long b) {
+    const int ah = (int) (a >> 31), al = (int) a & 0x7FFFFFFF, bh = (int) (b >> 31), bl = (int) b & 0x7FFFFFFF;
+    return wide(ah, bh) + (wide(ah, bl, wide(al, bh)) >> 31);
+}
+
+// The step in FP64, for fields outside the integer path's range (zeros, NaN,
+// infinities, exponents near the ends): a w x h x d block by a whole CTA.
+template <int DIMS, bool CONST>
+__device__ __noinline__ void mob_slow_block(const double *__restrict__ psi, const double *__restrict__ mu,
+                                            const double *__restrict__ mob, double *__restrict__ out, int mask,
+                                            int log2N, double M, double k, int x0, int y0, int z0, int d) {
+    auto index = [&](int X, int Y, int Z) {
+        return (size_t) (X & mask) + ((size_t) (Y & mask) << log2N) +
+               (DIMS == 3 ? ((size_t) (Z & mask) << (2 * log2N)) : 0);
+    };
+    for(int i = threadIdx.x; i < MTX * MTY * d; i += MTHR) {
+        const int x = x0 + i % MTX, y = y0 + i / MTX % MTY, z = z0 + i / (MTX * MTY);
+        const size_t c = index(x, y, z);
+        auto face = [&](size_t a, size_t b) { return (CONST ? M + M : mob[a] + mob[b]) * (mu[b] - mu[a]); };
+        double div = (face(c, index(x + 1, y, z)) - face(index(x - 1, y, z), c)) +
+                     (face(c, index(x, y + 1, z)) - face(index(x, y - 1, z), c));
+        if(DIMS == 3) div = div + (face(c, index(x, y, z + 1)) - face(index(x, y, z - 1), c));
+        if(CHGB_BC(20, c, (long long) 1 << (DIMS * log2N))) out[c] = fma(k, div, psi[c]);
+    }
+}
+
+template <int DIMS, bool CONST>
+__global__ void __launch_bounds__(MTHR) update_mob_fx_kernel(const double *__restrict__ psi_in,
+                                                             const double *__restrict__ mu,
+                                                             const double *__restrict__ mob, double *__restrict__ out,
+                                                             Geom g, EulerConsts c, int zc, unsigned *__restrict__ key,
+                                                             int parity) {
+    constexpr int R = DIMS == 3 ? 3 : 1;
+    constexpr int WR = CONST ? 1 : R, WP = CONST ? 1 : MPP;
+    __shared__ long long rU[R][MPP], rW[WR][WP];
+    const int tid = threadIdx.x, tx = tid & 31, row0 = (tid >> 5) * 4;
+    const int x0 = blockIdx.x * MTX, y0 = blockIdx.y * MTY, z0 = DIMS == 3 ? blockIdx.z * zc : 0;
+    const int nz = DIMS == 3 ? zc : 1;
+    pdl_begin();
+    const int eu = (int) (__ldcg(&key[2 * parity]) >> 20), ew = CONST ? 1022 : (int) (__ldcg(&key[2 * parity + 1]) >> 20);
+    if(tid < 2 && blockIdx.x + blockIdx.y + blockIdx.z == 0) key[2 * (parity ^ 1) + tid] = 0;   // the next step's
+    // the flux's unit is 2^(62 + (su - 60) + (sm - 60)), s = e - 1022, or with a
+    // constant M, whose sum of two goes into k, 2^(su - 59)
+    const int ek = CONST ? eu - 1022 - 59 : eu + ew - 2 * 1022 - 58;
+    const double kd = c.dt * c.half_inv_dx2;
+    if(eu < 300 || eu > 1700 || ew < 300 || ew > 1700 || ek < -800 || ek > 800) {
+        mob_slow_block<DIMS, CONST>(psi_in, mu, mob, out, g.mask, g.log2N, c.M, kd, x0, y0, z0, nz);
+        return;
+    }
+    const double k = (CONST ? kd * (c.M + c.M) : kd) * __hiloint2double((1023 + ek) << 20, 0);
+    FxScale su, sw;
+    su.sh = (CONST ? 59 : 60) - (eu - 1022);
+    sw.sh = 60 - (ew - 1022);
+    // this thread's cells of a staged plane
+    int off[MPF];
+#pragma unroll
+    for(int i = 0; i < MPF; i++) {
+        const int q = tid + i * MTHR, ly = q / MPX, lx = q - ly * MPX;
+        off[i] = ((x0 - 1 + lx) & g.mask) + (((y0 - 1 + ly) & g.mask) << g.log2N);
+    }
+    auto plane = [&](int z) { return DIMS == 3 ? (size_t) (z & g.mask) << (2 * g.log2N) : 0; };
+    double fu[MPF], fw[MPF];
+    auto fetch = [&](int z) {
+        const size_t b = plane(z);
+#pragma unroll
+        for(int i = 0; i < MPF; i++) {
+            const bool in = tid + i * MTHR < MPP && CHGB_BC(18, b + off[i], g.bins);
+            fu[i] = in ? mu[b + off[i]] : 0.0;
+            if(!CONST) fw[i] = in ? mob[b + off[i]] : 0.0;
+        }
+    };
+    auto commit = [&](int slot) {
+#pragma unroll
+        for(int i = 0; i < MPF; i++) {
+            const int q = tid + i * MTHR;
+            if(q < MPP) {
+                rU[slot][q] = fx_in(fu[i], su);
+                if(!CONST) rW[slot][q] = fx_in(fw[i], sw);
+            }
+        }
+    };
+    auto flux = [&](long long wa, long long wb, long long d) { return CONST ? d : face_flux(wa + wb, d); };
+    auto W = [&](int slot, int p) { return CONST ? 0 : rW[CONST ? 0 : slot][CONST ? 0 : p]; };
+    const int p0 = (row0 + 1) * MPX + tx + 1;   // the thread's first cell in a staged plane
+    const size_t c0 = (size_t) (x0 + tx) + ((size_t) (y0 + row0) << g.log2N);
+    long long jz[4] = {0, 0, 0, 0};
+    fetch(z0);
+    commit(DIMS == 3 ? z0 % 3 : 0);
+    if constexpr(DIMS == 3) {
+        fetch(z0 + 1);
+        // the lowest z faces: the plane below is needed at the thread's own cells only
+        __syncthreads();
+        const size_t b = plane(z0 - 1) + c0;
+#pragma unroll
+        for(int r = 0; r < 4; r++) {
+            const size_t gi = b + ((size_t) r << g.log2N);
+            const bool in = CHGB_BC(19, gi, g.bins);
+            const long long u = fx_in(in ? mu[gi] : 0.0, su), w = CONST ? 0 : fx_in(in ? mob[gi] : 0.0, sw);
+            const int p = p0 + r * MPX;
+            jz[r] = flux(w, W(z0 % 3, p), rU[z0 % 3][p] - u);
+        }
+    }
+    for(int z = z0; z < z0 + nz; z++) {
+        const int cz = DIMS == 3 ? z % 3 : 0, zp = DIMS == 3 ? (z + 1) % 3 : 0;
+        const size_t b = plane(z) + c0;
+        double psi[4];
+#pragma unroll
+        for(int r = 0; r < 4; r++) {
+            const size_t gi = b + ((size_t) r << g.log2N);
+            psi[r] = CHGB_BC(19, gi, g.bins) ? psi_in[gi] : 0.0;
+        }
+        if constexpr(DIMS == 3) {
+            commit(zp);
+            if(z + 1 < z0 + nz) fetch(z + 2);
+        }
+        __syncthreads();
+        const long long *U = rU[cz];
+        const int pe = (row0 + 1 + (tx & 3)) * MPX + 1;   // lanes 0-3: the tile's left faces of the four rows
+        const long long edge = flux(W(cz, pe - 1), W(cz, pe), U[pe] - U[pe - 1]);
+        long long u = U[p0], w = W(cz, p0);
+        long long jym = flux(W(cz, p0 - MPX), w, u - U[p0 - MPX]);
+#pragma unroll
+        for(int r = 0; r < 4; r++) {
+            const int p = p0 + r * MPX;
+            const long long un = U[p + MPX], wn = W(cz, p + MPX);
+            const long long jxp = flux(w, W(cz, p + 1), U[p + 1] - u), jyp = flux(w, wn, un - u);
+            const long long left = __shfl_up_sync(0xFFFFFFFFu, jxp, 1), first = __shfl_sync(0xFFFFFFFFu, edge, r);
+            long long D = (jxp - (tx == 0 ? first : left)) + (jyp - jym);
+            if constexpr(DIMS == 3) {
+                const long long jzp = flux(w, W(zp, p), rU[zp][p] - u);
+                D += jzp - jz[r];
+                jz[r] = jzp;
+            }
+            jym = jyp;
+            u = un;
+            w = wn;
+            const size_t gi = b + ((size_t) r << g.log2N);
+            if(CHGB_BC(19, gi, g.bins)) out[gi] = fma(k, (double) D, psi[r]);
+        }
     }
 }
 
@@ -1658,14 +1851,19 @@ cudaError_t launch_mob(int mob, const Geom &g, const ModelDev &m, const EulerCon
 
 namespace {
 
+constexpr int SPLIT_CTAS = 2 * 152;
+
 template <int KIND, int MOB, int DIMS>
 cudaError_t launch_split_kind(const Geom &g, const ModelDev &m, const EulerConsts &c, const double *in, double *out,
-                              double *mu, double *mob, cudaStream_t st) {
+                              double *mu, double *mob, cudaStream_t st, unsigned *key,
+                              int parity) {
     constexpr int S = NSpecies<KIND>::value;
     // 8-plane z-chunks: the extra halo planes per chunk are cheap L2 loads,
     // and the many small CTAs keep every SM's FP64 pipe fed to the end of the
-    // launch (N=256: 8192 CTAs, 7% faster than 32-plane chunks on GB300)
+    // launch (N=256: 8192 CTAs, 7% faster than 32-plane chunks on GB300); fewer
+    // planes where those would not give every SM two CTAs (N <= 64)
     int zc = (DIMS == 3) ? 8 : 1;
+    while(zc > 1 && (g.N / STX) * (g.N / STY) * (g.N / zc) < SPLIT_CTAS) zc /= 2;
     dim3 grid(g.N / STX, g.N / STY, (DIMS == 3) ? g.N / zc : 1);
     dim3 block(STX, STY);
     cudaLaunchConfig_t cfg = {};
@@ -1677,27 +1875,42 @@ cudaError_t launch_split_kind(const Geom &g, const ModelDev &m, const EulerConst
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, mu_kernel<KIND, MOB, DIMS>, in, mu, mob, g, m, c, zc);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, mu_kernel<KIND, MOB, DIMS>, in, mu, mob, g, m, c, zc, key);
     if(e != cudaSuccess) return e;
+    if constexpr(S == 1 && (MOB == 1 || MOB == 2))
+        if(key) {
+            // z chunks of 16 planes where that gives 1,000 CTAs (two and a half on each
+            // SM at a time), of four below, fewer yet for every SM to have two.  3D N=128:
+            // 4 planes 78.4 us a step, 8 planes 86.9, 2 planes 79.2; N=256: 16 538, 32 553
+            const int tiles = (g.N / MTX) * (g.N / MTY);
+            int uz = DIMS == 2 ? 1 : tiles * (g.N / 16) >= 1000 ? 16 : 4;
+            while(uz > 1 && tiles * (g.N / uz) < SPLIT_CTAS) uz /= 2;
+            cfg.gridDim = dim3(g.N / MTX, g.N / MTY, DIMS == 3 ? g.N / uz : 1);
+            cfg.blockDim = dim3(MTHR);
+            return cudaLaunchKernelEx(&cfg, update_mob_fx_kernel<DIMS, MOB == 1>, in, (const double *) mu,
+                                      (const double *) mob, out, g, c, uz, key - 2 * parity, parity);
+        }
     return cudaLaunchKernelEx(&cfg, update_kernel<S, MOB, DIMS>, in, (const double *) mu, (const double *) mob, out, g,
                               c, zc);
 }
 
 template <int KIND, int MOB>
 cudaError_t launch_split_mob(const Geom &g, const ModelDev &m, const EulerConsts &c, const double *in, double *out,
-                             double *mu, double *mob, cudaStream_t st) {
-    if(g.dims == 2) return launch_split_kind<KIND, MOB, 2>(g, m, c, in, out, mu, mob, st);
-    return launch_split_kind<KIND, MOB, 3>(g, m, c, in, out, mu, mob, st);
+                             double *mu, double *mob, cudaStream_t st, unsigned *key,
+                              int parity) {
+    if(g.dims == 2) return launch_split_kind<KIND, MOB, 2>(g, m, c, in, out, mu, mob, st, key, parity);
+    return launch_split_kind<KIND, MOB, 3>(g, m, c, in, out, mu, mob, st, key, parity);
 }
 
 template <int KIND>
 cudaError_t launch_split_model(int mob_kind, const Geom &g, const ModelDev &m, const EulerConsts &c,
-                               const double *in, double *out, double *mu, double *mob, cudaStream_t st) {
-    if(mob_kind == 0) return launch_split_mob<KIND, 0>(g, m, c, in, out, mu, mob, st);
-    if(mob_kind == 1) return launch_split_mob<KIND, 1>(g, m, c, in, out, mu, mob, st);
+                               const double *in, double *out, double *mu, double *mob, cudaStream_t st, unsigned *key,
+                              int parity) {
+    if(mob_kind == 0) return launch_split_mob<KIND, 0>(g, m, c, in, out, mu, mob, st, key, parity);
+    if(mob_kind == 1) return launch_split_mob<KIND, 1>(g, m, c, in, out, mu, mob, st, key, parity);
     // kind 3 reads the given field; mu_kernel writes `mob` only for kind 2
-    if(mob_kind == 3) return launch_split_mob<KIND, 3>(g, m, c, in, out, mu, const_cast<double *>(c.mobf), st);
-    if constexpr(KIND == CHGB_MODEL_SIMPLE_WERTHEIM) return launch_split_mob<KIND, 2>(g, m, c, in, out, mu, mob, st);
+    if(mob_kind == 3) return launch_split_mob<KIND, 3>(g, m, c, in, out, mu, const_cast<double *>(c.mobf), st, key, parity);
+    if constexpr(KIND == CHGB_MODEL_SIMPLE_WERTHEIM) return launch_split_mob<KIND, 2>(g, m, c, in, out, mu, mob, st, key, parity);
     return cudaErrorInvalidValue;
 }
 
@@ -1930,15 +2143,23 @@ cudaError_t launch_bfp_refresh(const double *psi, long long n, BfpState *st, int
 }
 
 cudaError_t launch_euler_split(int integrator, const Geom &g, const ModelDev &m, const EulerConsts &c,
-                               const double *in, double *out, double *mu, double *mob, cudaStream_t st) {
+                               const double *in, double *out, double *mu, double *mob, cudaStream_t st, unsigned *key,
+                               int parity) {
+    if(key) key += 2 * parity;   // the entries mu_kernel folds into
     int mob_kind = 0;
     if(integrator == CHGB_INTEGRATOR_EULER_MOBILITY) mob_kind = mobility_kind(c.mobility_type);
     switch(m.kind) {
-        case CHGB_MODEL_LANDAU: return launch_split_model<CHGB_MODEL_LANDAU>(mob_kind, g, m, c, in, out, mu, mob, st);
+        case CHGB_MODEL_LANDAU: return launch_split_model<CHGB_MODEL_LANDAU>(mob_kind, g, m, c, in, out, mu, mob, st, key, parity);
         case CHGB_MODEL_SIMPLE_WERTHEIM:
-            return launch_split_model<CHGB_MODEL_SIMPLE_WERTHEIM>(mob_kind, g, m, c, in, out, mu, mob, st);
-        default: return launch_split_model<CHGB_MODEL_SALEH>(mob_kind, g, m, c, in, out, mu, mob, st);
+            return launch_split_model<CHGB_MODEL_SIMPLE_WERTHEIM>(mob_kind, g, m, c, in, out, mu, mob, st, key, parity);
+        default: return launch_split_model<CHGB_MODEL_SALEH>(mob_kind, g, m, c, in, out, mu, mob, st, key, parity);
     }
+}
+
+bool euler_mob_fx_supported(int integrator, int model, int mobility_type, const Geom &g) {
+    return integrator == CHGB_INTEGRATOR_EULER_MOBILITY && model != CHGB_MODEL_SALEH && g.dims >= 2 && g.N >= 32 &&
+           (mobility_type == CHGB_MOBILITY_CONSTANT ||
+            (mobility_type == CHGB_MOBILITY_FREE_ENERGY && model == CHGB_MODEL_SIMPLE_WERTHEIM));
 }
 
 cudaError_t launch_euler_step(int integrator, const Geom &g, const ModelDev &m, const EulerConsts &c,

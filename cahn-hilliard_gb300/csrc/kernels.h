@@ -32,7 +32,13 @@ bool euler_cluster_supported(int integrator, const Geom &g);
 cudaError_t launch_euler_cluster(const Geom &g, const ModelDev &m, const EulerConsts &c, const double *in,
                                  double *out, int nsteps, cudaStream_t st, bool configure = false);
 cudaError_t launch_euler_split(int integrator, const Geom &g, const ModelDev &m, const EulerConsts &c,
-                               const double *in, double *out, double *mu, double *mob, cudaStream_t st);
+                               const double *in, double *out, double *mu, double *mob, cudaStream_t st,
+                               unsigned *key = nullptr, int parity = 0);
+// With `key` (four zeroed words in device memory; two for each parity of the
+// step): euler_mobility's pair, of one species with a constant or the
+// free-energy mobility, whose update is in block fixed point -- not the other
+// variants' bits (within a few units of 2^-57 of the largest flux).
+bool euler_mob_fx_supported(int integrator, int model, int mobility_type, const Geom &g);
 
 // Block fixed point (kernel_variant 5; euler.cu): plain `euler` with the
 // Landau model, dims >= 2, N >= 32; one kernel per step, or in 3D, with `mu` not
