@@ -419,7 +419,8 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
         ok = cudaMalloc(&h->d_mu, bytes) == cudaSuccess && (!mob || cudaMalloc(&h->d_mobk, bytes) == cudaSuccess) &&
              (!mob_fx || (cudaMalloc(&h->d_mobkey, 4 * sizeof(unsigned)) == cudaSuccess &&
                           cudaMemset(h->d_mobkey, 0, 4 * sizeof(unsigned)) == cudaSuccess)) &&
-             (!bfp_ok || cudaMalloc(&h->d_bfp, sizeof(BfpState)) == cudaSuccess);
+             (!bfp_ok || (cudaMalloc(&h->d_bfp, sizeof(BfpState)) == cudaSuccess &&
+                         cudaMemset(h->d_bfp, 0, sizeof(BfpState)) == cudaSuccess));
         if(!ok) {
             cudaGetLastError();
             if(want == 2 || want == 5) {
@@ -601,11 +602,13 @@ static cudaError_t one_step(chgb_handle *h) {
 }
 
 // Variant 5: set the block-fixed-point key from the current field, before the
-// first step of a sequence (the steps keep it up to date from then on).
-static cudaError_t bfp_refresh(chgb_handle *h) {
+// first of `steps` steps (which keep it up to date from then on).
+static cudaError_t bfp_refresh(chgb_handle *h, int64_t steps) {
     if(h->variant != 5 || h->d_mobkey) return cudaSuccess;   // euler_mobility's key is each step's own
     h->launches += 1;
-    return launch_bfp_refresh(h->d_rho[h->cur], (long long) h->n, h->d_bfp, h->cur, h->stream);
+    const unsigned long long gen = h->bfp_gen + 1;
+    h->bfp_gen = gen + (unsigned long long) steps;
+    return launch_bfp_refresh(h->d_rho[h->cur], (long long) h->n, h->d_bfp, h->cur, gen, h->stream);
 }
 
 // Queue `steps` time steps as chgb_step's graphs hold them (the timing at
@@ -653,7 +656,6 @@ static float time_variant(chgb_handle *h, int nsteps) {
     if(graph) cudaGraphDestroy(graph);
     cudaEvent_t a = nullptr, b = nullptr;
     ok = ok && cudaEventCreate(&a) == cudaSuccess && cudaEventCreate(&b) == cudaSuccess;
-    ok = ok && bfp_refresh(h) == cudaSuccess;
     ok = ok && cudaGraphLaunch(exec, h->stream) == cudaSuccess;   // warm-up
     float best = -1.f;
     for(int rep = 0; rep < 2 && ok; rep++) {
@@ -739,7 +741,7 @@ int chgb_step(chgb_handle *h, int64_t nsteps) {
         return CHGB_OK;
     }
     const bool no_parity = h->ps || h->psm;
-    CK(h, bfp_refresh(h), "block fixed point key");
+    CK(h, bfp_refresh(h, left), "block fixed point key");
     while(left > 0) {
         int lg = GRAPH_LOG2;
         while(((int64_t) 1 << lg) > left) lg--;

@@ -1248,7 +1248,7 @@ __global__ void __launch_bounds__(MTHR) update_mob_fx_kernel(const double *__res
 // supersedes the older with no reset between steps, and slots no CTA wrote in
 // this step fall behind.  (The pair's mu kernel publishes g + 1, mu's exponent
 // and the mode to its update kernel, BfpState::gen.)  Each chgb_step call first sets the key
-// from the field (a memset, then bfp_refresh_kernel).  A field whose emax is
+// from the field (bfp_refresh_kernel, with a generation above all before it).  A field whose emax is
 // below 128 or 2047 (zeros, values near the end of the double range, inf, NaN),
 // or so large or small that mu's unit leaves [2^-900, 2^900], takes plain FP64
 // sums in the reference's neighbour order for that step (mode 0).
@@ -1647,16 +1647,15 @@ __global__ void __launch_bounds__(B3THREADS, B3CTAS) euler3d_bfp_kernel(const do
                                  blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), tid);
 }
 
-// The key of the field psi (n values, n even): (0 << 16) | its largest biased
-// exponent, after the caller zeroed it.
+// The key of the field psi (n values, n even): (gen << 16) | its largest biased exponent.
 __global__ void __launch_bounds__(256) bfp_refresh_kernel(const double2 *__restrict__ psi, long long n2,
-                                                          unsigned long long *bank) {
+                                                          unsigned long long *bank, unsigned long long gen) {
     int mag = 0;
     for(long long i = (long long) blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += (long long) gridDim.x * blockDim.x) {
         const double2 v = psi[i];
         mag = max(mag, max(__double2hiint(v.x) & 0x7FFFFFFF, __double2hiint(v.y) & 0x7FFFFFFF));
     }
-    bfp_fold_key<8>(mag, 0ull, bank, blockIdx.x, threadIdx.x);
+    bfp_fold_key<8>(mag, gen, bank, blockIdx.x, threadIdx.x);
 }
 
 // 2D: one kernel per step.  A CTA stages X of a TX x TY tile of psi with a halo
@@ -2131,14 +2130,11 @@ cudaError_t launch_euler_bfp(const Geom &g, const EulerConsts &c, const double *
     return e;
 }
 
-cudaError_t launch_bfp_refresh(const double *psi, long long n, BfpState *st, int parity, cudaStream_t stream) {
-    // both banks: the 2D kernel folds into the other bank next, whose older
-    // generations must not outrank the new sequence's
-    cudaError_t e = cudaMemsetAsync(st->key, 0, sizeof st->key, stream);
-    if(e != cudaSuccess) return e;
+cudaError_t launch_bfp_refresh(const double *psi, long long n, BfpState *st, int parity, unsigned long long gen,
+                               cudaStream_t stream) {
     const long long n2 = n / 2;
     const long long blocks = std::min<long long>((n2 + 255) / 256, 152 * 8);
-    bfp_refresh_kernel<<<(unsigned) blocks, 256, 0, stream>>>(reinterpret_cast<const double2 *>(psi), n2, st->key[parity]);
+    bfp_refresh_kernel<<<(unsigned) blocks, 256, 0, stream>>>(reinterpret_cast<const double2 *>(psi), n2, st->key[parity], gen);
     return cudaGetLastError();
 }
 

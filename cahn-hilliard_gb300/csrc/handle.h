@@ -50,6 +50,7 @@ struct chgb_handle {
     double *d_mu = nullptr;        // split variants: mu of every cell (variant 5: its one-kernel steps have none)
     double *d_mobk = nullptr;      // split variant with the free-energy mobility: M of every cell
     unsigned *d_mobkey = nullptr;  // variant 5 of euler_mobility: the largest |mu| and |M| of the step, by parity
+    unsigned long long bfp_gen = 0;    // variant 5: no key in d_bfp has a newer generation
     chgb::BfpState *d_bfp = nullptr;   // variant 5: the block-fixed-point key, and the pair's mu scale
     chgb::SqPlan *sq = nullptr;            // S(q) shells, built on first use
     chgb::SpectralState *fft = nullptr;    // forward transform of euler boxes for S(q)

@@ -45,8 +45,9 @@ bool euler_mob_fx_supported(int integrator, int model, int mobility_type, const 
 // null, the split pair (mu stored there as integers) -- the same bits.  One
 // exponent for the whole field per step; not the other variants' bits (within a few units of
 // 2^-56 of the field's largest value per step).  BfpState lives in device
-// memory and must hold the field's key before the first step of a sequence:
-// launch_bfp_refresh (a memset and one kernel) sets it from psi.
+// memory, zeroed once, and must hold the field's key before the first step of
+// a sequence: launch_bfp_refresh sets it from psi with a generation above any
+// before it (a step's is one above its predecessor's), so that no key is cleared.
 constexpr int BFP_SLOTS = 32, BFP_SLOT_STRIDE = 16;   // key slots, one per 128-byte line
 struct BfpState {
     // (generation << 16) | largest biased exponent of |psi|, over the slots
@@ -69,7 +70,8 @@ bool euler_bfp_supported(int integrator, int model_kind, const Geom &g);
 cudaError_t launch_euler_bfp(const Geom &g, const EulerConsts &c, const double *in, double *out, double *mu,
                              BfpState *st, int parity, cudaStream_t stream);
 // The key of psi into the bank of its ping-pong parity.
-cudaError_t launch_bfp_refresh(const double *psi, long long n, BfpState *st, int parity, cudaStream_t stream);
+cudaError_t launch_bfp_refresh(const double *psi, long long n, BfpState *st, int parity, unsigned long long gen,
+                               cudaStream_t stream);
 
 // One 2D `euler` replica of a batch (batch.cu): buffers 0 and 1 and its constants.
 struct EulerBatchRep {
