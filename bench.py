@@ -44,7 +44,7 @@ FLUSH_BYTES = 256 << 20  # L2 flush buffer (L2 is 129 MB)
 #   bytes_per_cell  the compulsory FP64 state read + write (16 B);
 #   fp64_per_cell   instructions of the FP64 pipe per cell and time step for
 #                   each kernel variant (1 fused, 2 split, 3 two steps per
-#                   launch, 4 cluster-resident, 5 split in block fixed point),
+#                   launch, 4 cluster-resident, 5 block fixed point),
 #                   halo recomputation included:
 #                   ncu's sm__inst_executed_pipe_fp64 x 32 per cell (the
 #                   explicit steps' neighbour sums run on the integer pipe, so
@@ -57,19 +57,20 @@ FLUSH_BYTES = 256 << 20  # L2 flush buffer (L2 is 129 MB)
 #                   from one ncu capture, per variant (profiles/).
 WORKLOADS = {
     "euler3d_N256": dict(dims=3, N=256, integrator="euler", dt=0.005, bytes_per_cell=16.0,
-                         fp64_per_cell={1: 7.31, 2: 6.0, 5: 2.0 + 1.5}, alu_per_cell={2: 173.8, 5: 69.3 + 55.4},
-                         ncu_traffic={2: 135.3e6 + 94.9e6 + 269.6e6 + 115.9e6,
-                                      5: 135.4e6 + 94.7e6 + 274.4e6 + 107.1e6},
+                         # 5: the one-kernel form that variant 0 takes
+                         fp64_per_cell={1: 7.31, 2: 6.0, 5: 2.08}, alu_per_cell={2: 173.8, 5: 72.3},
+                         ncu_traffic={2: 135.3e6 + 94.9e6 + 269.6e6 + 115.9e6, 5: 145.7e6 + 141.7e6},
                          desc="3D Landau euler N=256, dt=0.005, k=1, M=1, eps=0.9, psi0=U(-0.01,0.01)"),
     "euler2d_N1024": dict(dims=2, N=1024, integrator="euler", dt=0.01, bytes_per_cell=16.0,
-                          fp64_per_cell={1: 4 * (34 * 34) / (32 * 32) + 2, 2: 5.0, 5: 4.25},
-                          alu_per_cell={2: 177.6, 5: 114.6},
-                          ncu_traffic={2: 8.39e6 + 16.78e6, 5: 8.41e6},
+                          fp64_per_cell={1: 4 * (34 * 34) / (32 * 32) + 2, 2: 5.0, 5: 2.0},
+                          alu_per_cell={2: 177.6, 5: 63.5},
+                          ncu_traffic={2: 8.39e6 + 16.78e6, 5: 0.73e6},   # 5: L2-resident, caches kept
                           desc="2D Landau euler N=1024, dt=0.01, k=1, M=1, eps=0.9, psi0=U(-0.01,0.01)"),
     "pseudospectral2d_N1024": dict(dims=2, N=1024, integrator="pseudospectral", dt=0.05, bytes_per_cell=16.0,
-                                   # fixed-point transforms: FP64 only in f' and the mode update
-                                   fp64_per_cell={1: 5.9, 2: 5.9}, alu_per_cell={1: 637.0, 2: 637.0},
-                                   ncu_traffic={1: 8.50e6 + 25.34e6, 2: 8.50e6 + 25.34e6},
+                                   # fixed-point transforms: FP64 in f', the mode update and half the
+                                   # conversions back
+                                   fp64_per_cell={1: 6.0, 2: 6.0}, alu_per_cell={1: 355.6, 2: 355.6},
+                                   ncu_traffic={1: 3.9e6, 2: 3.9e6},   # L2-resident, caches kept
                                    desc="2D Landau pseudospectral N=1024, dt=0.05, k=1, M=1, eps=0.9, "
                                         "psi0=U(-0.01,0.01)"),
 }
@@ -82,7 +83,8 @@ WORKLOADS["euler2d_N64"] = dict(
          "CPU-runnable case, launch-latency bound on one box (many such boxes belong in the batch)")
 WORKLOADS["wertheim3d_N128"] = dict(
     dims=3, N=128, integrator="euler_mobility", model="simple_wertheim", dt=1e-4, rho_mean=1.107e-5,
-    bytes_per_cell=16.0, fp64_per_cell={2: 51.25 + 16.25}, alu_per_cell={2: 134.6 + 81.4}, ncu_traffic={},
+    bytes_per_cell=16.0, fp64_per_cell={2: 10.0 + 16.25, 5: 10.0 + 2.1}, alu_per_cell={2: 256.0 + 81.4, 5: 256.0 + 114.2},
+    ncu_traffic={},
     desc="3D simple_wertheim euler_mobility N=128, free-energy mobility M0 rho X^4, dt=1e-4, dx=10, k=1e6, "
          "rho0=1.107e-5 (about half the sites bonded) with 1% relative noise")
 HEADLINE = "euler3d_N256"

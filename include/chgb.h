@@ -133,8 +133,11 @@ typedef struct chgb_params {
                                          field's largest value per step), not bit for bit.
                                          Variant 0 picks it by a fixed rule, without timing,
                                          for 2D N >= 512 and 3D N >= 64 (in 3D as one kernel
-                                         per step, the pair's bits), and times 1-4
-                                         elsewhere, so a configuration always runs the same
+                                         per step, the pair's bits), and its form for
+                                         `euler_mobility` (landau or simple_wertheim, constant
+                                         or free-energy mobility; two kernels per step) for
+                                         2D N >= 512 and 3D N >= 32; it times 1-4 elsewhere,
+                                         so a configuration always runs the same
                                          arithmetic. */
     chgb_model_params model;
     /* `regularised` mobility: mobility.rho_min / user_to_internal (M is `M` above). */
