@@ -791,8 +791,18 @@ __device__ __forceinline__ double split_lap_fx(const double (*ring)[SPP], const 
     return fx_total<K>(T, ek, emax, -(long long) K * Tv, ekv);
 }
 
+// CTAs an SM: eight for plain Landau; the integer Wertheim models, whose chains
+// are long, five in 3D and six in 2D (48 and 40 registers; simple_wertheim with
+// the free-energy mobility, us a step with the compiler's choice, 4, 5, 6: 3D
+// N=64 19.4 17.4 18.9 21.0, N=128 77.7 73.5 72.8 75.4, N=256 536 506 490 492;
+// 2D N=2048 118.1 118.0 117.7 113.7).
 template <int KIND, int MOB, int DIMS>
-__global__ void __launch_bounds__(256, (KIND == CHGB_MODEL_LANDAU && MOB == 0) ? 8 : 1) mu_kernel(const double *__restrict__ in, double *__restrict__ mu,
+constexpr int MU_CTAS = KIND == CHGB_MODEL_LANDAU && MOB == 0 ? 8
+                        : KIND == CHGB_MODEL_SIMPLE_WERTHEIM  ? (DIMS == 3 ? 5 : 6)
+                                                              : 1;
+
+template <int KIND, int MOB, int DIMS>
+__global__ void __launch_bounds__(256, MU_CTAS<KIND, MOB, DIMS>) mu_kernel(const double *__restrict__ in, double *__restrict__ mu,
                                                  double *__restrict__ mob, Geom g, ModelDev m, EulerConsts c, int zc,
                                                  unsigned *__restrict__ key) {
     constexpr int S = NSpecies<KIND>::value;
@@ -1048,8 +1058,9 @@ __global__ void __launch_bounds__(256, (S == 1 && MOB == 0) ? 8 : 1) update_kern
 // the fluxes cancel exactly.  A cell takes two FP64 instructions (a conversion
 // and the final FMA) where update_kernel takes 16, which bound it (75 % of that
 // pipe).  simple_wertheim with the free-energy mobility on GB300, us a step (mu
-// and update), the FP64 update and this one: 3D N=64 41.8 and 30.5, N=128 133.8
-// and 78.4, N=256 949 and 538; 2D N=512 16.5 and 14.1, N=1024 48.4 and 33.2.
+// and update), the FP64 update and this one: 3D N=32 8.6 and 7.0, N=64 28.6 and
+// 17.2, N=128 128.8 and 71.6, N=256 901 and 490; 2D N=512 16.4 and 12.0, N=1024
+// 47.8 and 31.9.
 //
 // A CTA of 128 threads has a tile of 32 x 16 cells, a warp each of four rows
 // of it: a thread's four cells lie above one another, so that their y faces are
@@ -1088,8 +1099,10 @@ __device__ __noinline__ void mob_slow_block(const double *__restrict__ psi, cons
     }
 }
 
+// 2D: eight CTAs an SM lets the compiler take 64 registers (2D N=512 14.1 -> 11.9
+// us a step); in 3D the same bound costs (N=128 72.8 -> 74.2, N=256 490 -> 534).
 template <int DIMS, bool CONST>
-__global__ void __launch_bounds__(MTHR) update_mob_fx_kernel(const double *__restrict__ psi_in,
+__global__ void __launch_bounds__(MTHR, DIMS == 2 ? 8 : 1) update_mob_fx_kernel(const double *__restrict__ psi_in,
                                                              const double *__restrict__ mu,
                                                              const double *__restrict__ mob, double *__restrict__ out,
                                                              Geom g, EulerConsts c, int zc, unsigned *__restrict__ key,
