@@ -556,15 +556,11 @@ int chgb_adjoint_backward(chgb_adjoint *a, const double *dl_dsq, const double *d
             ACK(a, cudaStreamWaitEvent(s2, a->ev_adj[b], 0), "wait");
             ACK(a, spectral_load_hat(ps, a->ckpt_hat[j], s2), "segment start");
             ACK(a, run_graph(a, gkey(G_PS_REC, nsteps, b << 1), s2, [&]() -> cudaError_t {
-                    cudaError_t e = cudaSuccess;
-                    for(int i = 0; i < nsteps && e == cudaSuccess; i++) {
-                        e = cudaMemcpyAsync(sh + (size_t) i * hs, spectral_psi_hat(ps, 0), sizeof(double2) * hs,
-                                            cudaMemcpyDeviceToDevice, s2);
-                        if(e == cudaSuccess) e = spectral_step_record(ps, sr + (size_t) i * a->n, s2);
-                    }
-                    if(e == cudaSuccess)
-                        e = cudaMemcpyAsync(sh + (size_t) nsteps * hs, spectral_psi_hat(ps, 0), sizeof(double2) * hs,
-                                            cudaMemcpyDeviceToDevice, s2);
+                    // the first spectrum is a copy, the others come from the column pass
+                    cudaError_t e = cudaMemcpyAsync(sh, spectral_psi_hat(ps, 0), sizeof(double2) * hs,
+                                                    cudaMemcpyDeviceToDevice, s2);
+                    for(int i = 0; i < nsteps && e == cudaSuccess; i++)
+                        e = spectral_step_record(ps, sr + (size_t) i * a->n, sh + (size_t) (i + 1) * hs, s2);
                     return e;
                 }), "segment recompute");
             ACK(a, cudaEventRecord(a->ev_rec[b], s2), "event");

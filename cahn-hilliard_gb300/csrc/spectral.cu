@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(256) row_batch_kernel(const PsBatchRep *__rest
 }
 
 enum { COL_FWD = 0, COL_INV = 1, COL_STEP = 2, COL_INIT = 3, COL_GRAD_INV = 4, COL_FWD_DIV = 5, COL_FWD_MU = 6,
-       COL_UPD_INV = 7, COL_LOAD_INV = 8 };
+       COL_UPD_INV = 7, COL_LOAD_INV = 8, COL_STEP_REC = 9 };
 
 // The pointwise stages of the variable-mobility step that ride on the last
 // axis' column pass (src/integrators/PseudospectralMobilityCPU.cpp:249-306).
@@ -502,7 +502,7 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
     }
     constexpr bool INV = MODE == COL_INV || MODE == COL_LOAD_INV || MODE == COL_GRAD_INV || MODE == COL_UPD_INV;
     fx_col_fft<INV>(r, ln, I, cur, oth, twf, sm_w[0], MODE == COL_UPD_INV ? ops.log2_bins : 0);
-    if constexpr(MODE == COL_STEP) {
+    if constexpr(MODE == COL_STEP || MODE == COL_STEP_REC) {
 #pragma unroll
         for(int i = 0; i < E; i++) {
             const long long off = line0 + i * ln.T;
@@ -510,6 +510,9 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
             const double2 ph = psi_hat[off], c = ab[off];
             const double2 nv = make_double2(fma(c.x, ph.x, -c.y * r[i].x), fma(c.x, ph.y, -c.y * r[i].y));
             psi_hat[off] = nv;
+            // a trajectory's record (a mode of its own: as a test of the pointer it cost the
+            // plain step 2 %)
+            if(MODE == COL_STEP_REC) ops.out[off] = nv;
             r[i] = nv;
         }
         fx_col_fft<true>(r, ln, I, cur, oth, twf, sm_w[1]);
@@ -862,7 +865,7 @@ int spectral_create(const chgb_params &p, const Geom &g, const ModelDev &m, Spec
                          (const void *) col_kernel<COL_STEP, E>, (const void *) col_kernel<COL_INIT, E>,           \
                          (const void *) col_kernel<COL_GRAD_INV, E>, (const void *) col_kernel<COL_FWD_DIV, E>,    \
                          (const void *) col_kernel<COL_FWD_MU, E>, (const void *) col_kernel<COL_UPD_INV, E>,      \
-                         (const void *) col_kernel<COL_LOAD_INV, E>})                                              \
+                         (const void *) col_kernel<COL_LOAD_INV, E>, (const void *) col_kernel<COL_STEP_REC, E>})  \
         setattr(f, 224 * 1024);   // whatever shape the timing below picks
     SETCOL(8)
     SETCOL(4)
@@ -975,7 +978,7 @@ cudaError_t launch_col(SpectralState *s, int axis, cudaStream_t st, const ColOps
         plane_stride = H;
         planes = N;
     }
-    const ColShape &c = MODE == COL_STEP ? s->step : s->col;
+    const ColShape &c = MODE == COL_STEP || MODE == COL_STEP_REC ? s->step : s->col;
     const int C = 1 << c.lgC;
     auto kernel = c.E == 8 ? col_kernel<MODE, 8> : c.E == 4 ? col_kernel<MODE, 4> : col_kernel<MODE, 2>;
     return launch_pass(s, kernel, dim3((unsigned) ((H + C - 1) / C), (unsigned) planes, (unsigned) s->g.S), c.threads,
@@ -1507,10 +1510,13 @@ cudaError_t spectral_load_hat(SpectralState *s, const double2 *hat, cudaStream_t
     return e;
 }
 
-// One forward step from the half-spectrum state that also writes rho_n (real) to real_out.
-cudaError_t spectral_step_record(SpectralState *s, double *real_out, cudaStream_t st) {
+// One forward step from the half-spectrum state that also writes rho_n (real) to
+// real_out and psi_{n+1} to hat_out.
+cudaError_t spectral_step_record(SpectralState *s, double *real_out, double2 *hat_out, cudaStream_t st) {
     cudaError_t e = launch_row<ROW_IN_HAT, true, true, true>(s, nullptr, real_out, st);
-    if(e == cudaSuccess) e = launch_col<COL_STEP>(s, 1, st);
+    ColOps o{};
+    o.out = hat_out;
+    if(e == cudaSuccess) e = launch_col<COL_STEP_REC>(s, 1, st, o);
     s->hat_valid = true;
     s->real_valid = false;
     return e;

@@ -56,8 +56,9 @@ cudaError_t spectral_psmob_update(SpectralState *s, double2 *rho_hat, const doub
 // ---- adjoint support (adjoint.cu) -------------------------------------------
 // psi_hat <- hat and the transformed rows a step starts from.
 cudaError_t spectral_load_hat(SpectralState *s, const double2 *hat, cudaStream_t st);
-// One forward step from the half spectrum, also writing rho_n (real) to real_out.
-cudaError_t spectral_step_record(SpectralState *s, double *real_out, cudaStream_t st);
+// One forward step from the half spectrum, also writing rho_n (real) to real_out
+// and psi_{n+1} to hat_out.
+cudaError_t spectral_step_record(SpectralState *s, double *real_out, double2 *hat_out, cudaStream_t st);
 // real_out = C2R(hat_scaled), unnormalised (a scaled state gives the field).
 cudaError_t spectral_inverse(SpectralState *s, const double2 *hat_scaled, double *real_out, cudaStream_t st);
 
