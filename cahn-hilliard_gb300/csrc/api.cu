@@ -240,11 +240,6 @@ static float time_variant(chgb_handle *h, int nsteps);
 // Wertheim models' number densities are of order 1e-5 in internal units.
 static double m_kind_density_scale(const ModelDev &m) { return m.kind == CHGB_MODEL_LANDAU ? 0.0 : 1e-5; }
 
-// euler_mobility in block fixed point by rule, where it measured fastest (us a
-// step, simple_wertheim with the free-energy mobility: 2D N=256 9.3 against 7.3 of
-// the best other variant, N=512 14.1 against 16.5; 3D N=32 20.1 against 35.2).
-static bool fx_mob_measured(const Geom &g) { return g.dims == 2 ? g.N >= 512 : g.N >= 32; }
-
 static void release(chgb_handle *h) {
     if(!h) return;
     for(int i = 0; i < 2; i++) {
@@ -414,8 +409,12 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
                    params->mobility_type == CHGB_MOBILITY_FREE_ENERGY;
         const bool bfp_ok = (want == 0 || want == 5) &&
                             euler_bfp_supported(params->integrator, params->model.kind, h->g);
+        // euler_mobility in block fixed point wherever its kernels run: faster at
+        // every size than the best of variants 1 and 2 (us a step, simple_wertheim with
+        // the free-energy mobility: 2D N=32 4.6 against 4.9, N=128 4.9 and 5.5, N=256 6.2
+        // and 7.1, N=512 12.0 and 16.4; 3D N=32 7.0 and 8.6, N=256 490 and 901)
         const bool mob_fx = want == 0 && euler_mob_fx_supported(params->integrator, params->model.kind,
-                                                                params->mobility_type, h->g) && fx_mob_measured(h->g);
+                                                                params->mobility_type, h->g);
         ok = cudaMalloc(&h->d_mu, bytes) == cudaSuccess && (!mob || cudaMalloc(&h->d_mobk, bytes) == cudaSuccess) &&
              (!mob_fx || (cudaMalloc(&h->d_mobkey, 4 * sizeof(unsigned)) == cudaSuccess &&
                           cudaMemset(h->d_mobkey, 0, 4 * sizeof(unsigned)) == cudaSuccess)) &&
@@ -432,7 +431,7 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
             h->variant = want;
         }
         else if(mob_fx) {
-            h->variant = 5;   // by a fixed rule, as below
+            h->variant = 5;   // by rule, as below
         }
         else if(bfp_ok && ((h->g.dims == 2 && h->g.N >= 512) || (h->g.dims == 3 && h->g.N >= 64))) {
             // block fixed point where it was measured fastest on GB300, by a fixed
@@ -546,6 +545,8 @@ int chgb_upload(chgb_handle *h, const double *rho, const double *mobility) {
     CK(h, cudaMemcpyAsync(h->d_rho[0], rho, h->n * sizeof(double), cudaMemcpyHostToDevice, h->stream),
        "upload rho");
     h->cur = 0;
+    // the last step cleared the other parity's entries only
+    if(h->d_mobkey) CK(h, cudaMemsetAsync(h->d_mobkey, 0, 4 * sizeof(unsigned), h->stream), "mobility key");
     h->steps_done = 0;
     if(h->ps) {
         int r = spectral_set_rho(h->ps, h->d_rho[0], h->stream, &h->launches, h->err);

@@ -136,9 +136,8 @@ typedef struct chgb_params {
                                          per step, the pair's bits), and its form for
                                          `euler_mobility` (landau or simple_wertheim, constant
                                          or free-energy mobility; two kernels per step) for
-                                         2D N >= 512 and 3D N >= 32; it times 1-4 elsewhere,
-                                         so a configuration always runs the same
-                                         arithmetic. */
+                                         2D and 3D N >= 32; it times 1-4 elsewhere, so a
+                                         configuration always runs the same arithmetic. */
     chgb_model_params model;
     /* `regularised` mobility: mobility.rho_min / user_to_internal (M is `M` above). */
     double rho_min;
