@@ -385,7 +385,8 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
     // recomputation), two fused steps per launch (small 2D boxes), or the box
     // resident in one cluster's shared memory (N = 32, 64).  All give
     // bit-identical fields; with kernel_variant = 0 each candidate is timed
-    // once on the zeroed buffers and the fastest is kept.
+    // once on a noise field and the fastest is kept, but where block fixed
+    // point is taken by rule (variant 5, the bits its own).
     h->variant = 1;
     int want = params->kernel_variant;
     const bool two_ok = !h->ps && !h->psm && euler_two_supported(params->integrator, h->g);

@@ -17,7 +17,8 @@
 // r2c's row pass, mu on its last column pass, i k_d on the first inverse column
 // pass of a flux's c2r, the flux itself between the c2r and r2c of one row
 // pass, the divergence on the last forward column pass, the update on the
-// final c2r's first column pass -- 2D: 12 launches a step instead of 22.  The
+// final c2r's first column pass -- 2D: 12 launches a step instead
+// of 22, 11 where the mobility's update reduces M0.  The
 // passes contract their products and sums and divide through one reciprocal;
 // 1D uses the elementwise kernels below, in the reference's order of
 // operations (the two agree to rounding).  A constant mobility makes every

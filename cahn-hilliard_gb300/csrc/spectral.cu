@@ -4,9 +4,10 @@
 // per-mode update) and its CUDA mirror src/CUDA/integrators/PseudospectralCUDA.cu
 // (single-precision cuFFT for f'; not followed).
 //
-// State.  The master copy is the half spectrum psi_t = rho_hat / N^dims in the
-// reference's layout [species][n0]..[n_{d-2}][N/2+1] (the last, fastest axis x
-// halved, as FFTW's r2c).  Storing it pre-divided by N^dims makes the inverse
+// State.  The master copy is the half spectrum psi_t = rho_hat / N^dims (axis x
+// halved, as FFTW's r2c), along the last transformed axis (spectral_line_index);
+// the transforms' work array has the reference's layout
+// [species][n0]..[n_{d-2}][N/2+1].  Storing psi_t pre-divided by N^dims makes the inverse
 // transform produce rho directly, so the per-mode update of
 // PseudospectralCPU.cpp:119-131 folds to
 //     psi_t' = alpha * psi_t - beta * F[f'(rho)],
@@ -29,9 +30,9 @@
 // sweep.  The transforms run in 64-bit block floating point (bfp.cuh): each
 // line is converted to fixed point with one exponent, transformed with integer
 // arithmetic and converted back; the state, f' and the mode update stay FP64.
-// A line's values live in registers, four or eight to a thread, from the load
+// A line's values live in registers, two, four or eight to a thread, from the load
 // of the row or column to the store of its transform; they cross between
-// threads through shared memory once per radix-4 or radix-8 pass.
+// threads through shared memory once per radix-2, -4 or -8 pass.
 #include <cmath>
 #include <vector>
 
@@ -354,7 +355,7 @@ __device__ __forceinline__ void row_body(double2 *__restrict__ work, const doubl
                    FLUX != FLUX_NONE ? 63 - __clzll(bins) : 0);
 }
 
-// Threads of a row CTA: at most 256 a line (E = 8: N = 4096; E = 4: N = 2048).
+// Threads of a row CTA: at most 256 a line (E = 8: N = 4096).
 template <int KIND>
 struct RowThreads {
     static constexpr int value = 256 * NSpecies<KIND>::value;
