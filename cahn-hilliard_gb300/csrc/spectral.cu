@@ -1143,7 +1143,14 @@ int spectral_real(SpectralState *s, double *d_rho, cudaStream_t st, int64_t *lau
 // ---------------------------------------------------------------------------
 namespace chgb {
 
-bool spectral_batchable(const SpectralState *s) { return s->g.dims == 2 && s->g.N >= 8 && s->g.N <= 1024; }
+// A batch CTA takes at least one whole row of every species, and one whole
+// column.  (Three species need 384 threads a row at N = 1024: such a box runs on
+// its own, where it fills the GPU alone.)
+bool spectral_batchable(const SpectralState *s) {
+    return s->g.dims == 2 && s->g.N >= 8 && s->g.N <= 1024 &&
+           fx_line_threads(s->g.N / 2, s->row_E) * s->g.S <= PS_BATCH_THREADS &&
+           fx_line_threads(s->g.N, s->step.E) <= PS_BATCH_THREADS;
+}
 
 bool spectral_hat_valid(const SpectralState *s) { return s->hat_valid; }
 

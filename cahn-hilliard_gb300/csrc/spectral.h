@@ -92,7 +92,7 @@ struct PsBatchRep {
     long long bins, hat;
 };
 constexpr int PS_BATCH_THREADS = 256;
-// 2D, N in [8, 1024]: the state can join a batch.
+// 2D, N in [8, 1024], a row of every species in one CTA: the state can join a batch.
 bool spectral_batchable(const SpectralState *s);
 // Fill the descriptor; returns the dynamic shared memory its row and column CTAs need.
 void spectral_batch_rep(const SpectralState *s, PsBatchRep *r, size_t *row_smem, size_t *col_smem);
