@@ -2,7 +2,7 @@
 // (chgb_adjoint_*).  No counterpart in the reference.
 //
 // Scope: 2D Landau boxes, `euler` (N >= 32, a multiple of 32) and
-// `pseudospectral` (8 <= N <= 1024).  The loss is given by its gradient with
+// `pseudospectral` (8 <= N <= 4096).  The loss is given by its gradient with
 // respect to the radially averaged S(q) of the final state (see
 // chgb_structure_factor) and/or with respect to the final field itself.
 // Gradients come back for the initial field and for (epsilon, k, M) in
@@ -397,7 +397,7 @@ int chgb_adjoint_create(const chgb_params *params, int64_t nsteps, int32_t check
     a->spectral = h->ps != nullptr;
     if(a->spectral && !spectral_adjoint_supported(h->ps)) {
         adj_release(a);
-        return afail(nullptr, CHGB_ERR_UNSUPPORTED, "the pseudospectral adjoint needs 8 <= N <= 1024");
+        return afail(nullptr, CHGB_ERR_UNSUPPORTED, "the pseudospectral adjoint needs 8 <= N <= 4096");
     }
     a->n = (size_t) h->g.bins;
     bool ok = true;

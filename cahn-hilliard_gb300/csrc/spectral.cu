@@ -1381,6 +1381,20 @@ struct SpectralAdj {
     int n_row_cta = 0, n_col_cta = 0;
 };
 
+// The kernels for the state's values per thread.
+static auto row_adj_kernel_of(const SpectralState *s) {
+    return s->row_E == 8 ? row_adj_kernel<8> : s->row_E == 4 ? row_adj_kernel<4> : row_adj_kernel<2>;
+}
+
+template <int E>
+static auto col_adj_kernel_of(int mode) {
+    return mode == ADJ_A ? col_adj_kernel<ADJ_A, E> : mode == ADJ_B ? col_adj_kernel<ADJ_B, E> : col_adj_kernel<ADJ_BA, E>;
+}
+
+static auto col_adj_kernel_of(const SpectralState *s, int mode) {
+    return s->col.E == 8 ? col_adj_kernel_of<8>(mode) : s->col.E == 4 ? col_adj_kernel_of<4>(mode) : col_adj_kernel_of<2>(mode);
+}
+
 bool spectral_adjoint_supported(const SpectralState *s) {
     return s->g.dims == 2 && s->g.S == 1 && s->m.kind == CHGB_MODEL_LANDAU && s->g.N >= 8;
 }
@@ -1420,11 +1434,8 @@ SpectralAdj *spectral_adj_create(SpectralState *s, std::string &err) {
          cudaMemcpy(a->tm2, tm2.data(), sizeof(double) * s->hat, cudaMemcpyHostToDevice) == cudaSuccess;
     if(ok) {
         size_t rs = s->row_smem, cs = s->col.smem;
-        for(const void *f : {(const void *) row_adj_kernel<2>, (const void *) row_adj_kernel<4>}) allow_smem(f, rs);
-        for(const void *f : {(const void *) col_adj_kernel<ADJ_A, 2>, (const void *) col_adj_kernel<ADJ_A, 4>,
-                             (const void *) col_adj_kernel<ADJ_B, 2>, (const void *) col_adj_kernel<ADJ_B, 4>,
-                             (const void *) col_adj_kernel<ADJ_BA, 2>, (const void *) col_adj_kernel<ADJ_BA, 4>})
-            allow_smem(f, cs);
+        allow_smem((const void *) row_adj_kernel_of(s), rs);
+        for(int mode : {ADJ_A, ADJ_B, ADJ_BA}) allow_smem((const void *) col_adj_kernel_of(s, mode), cs);
         ok = cudaGetLastError() == cudaSuccess;
     }
     if(!ok) {
@@ -1474,19 +1485,14 @@ cudaError_t spectral_adj_col(SpectralAdj *a, SpectralState *s, int mode, const d
 #define ADJ_COL_ARGS                                                                                                   \
     a->work, a->lam, s->ab, a->tk, a->tm1, a->tm2, psi_next, psi_cur, ilog2(N), s->H, s->col.lgC, s->twf,      \
         a->gk, a->gm
-    // the adjoint's boxes (N <= 1024) have two or four values a thread
-    auto kernel = s->col.E == 2
-                      ? (mode == ADJ_A ? col_adj_kernel<ADJ_A, 2> : mode == ADJ_B ? col_adj_kernel<ADJ_B, 2> : col_adj_kernel<ADJ_BA, 2>)
-                      : (mode == ADJ_A ? col_adj_kernel<ADJ_A, 4> : mode == ADJ_B ? col_adj_kernel<ADJ_B, 4> : col_adj_kernel<ADJ_BA, 4>);
-    kernel<<<grid, s->col.threads, s->col.smem, st>>>(ADJ_COL_ARGS);
+    col_adj_kernel_of(s, mode)<<<grid, s->col.threads, s->col.smem, st>>>(ADJ_COL_ARGS);
 #undef ADJ_COL_ARGS
     return cudaGetLastError();
 }
 
 cudaError_t spectral_adj_row(SpectralAdj *a, SpectralState *s, const double *psi_n, cudaStream_t st) {
-    auto kernel = s->row_E == 2 ? row_adj_kernel<2> : row_adj_kernel<4>;
-    kernel<<<a->n_row_cta, s->row_threads, s->row_smem, st>>>(a->work, psi_n, ilog2(s->g.N) - 1, s->row_rpc,
-                                                                       s->twf, s->m.epsilon, a->geps);
+    row_adj_kernel_of(s)<<<a->n_row_cta, s->row_threads, s->row_smem, st>>>(a->work, psi_n, ilog2(s->g.N) - 1, s->row_rpc,
+                                                                            s->twf, s->m.epsilon, a->geps);
     return cudaGetLastError();
 }
 

@@ -308,7 +308,7 @@ int chgb_structure_factor(chgb_handle *h, int32_t species, double *sq, int32_t n
  * after `nsteps` steps with respect to the initial field and to
  * (epsilon, k, M) in internal units, for 2D Landau boxes with constant
  * mobility, `euler` (N >= 32, multiple of 32) or `pseudospectral`
- * (8 <= N <= 1024).  The forward pass stores a checkpoint every
+ * (8 <= N <= 4096).  The forward pass stores a checkpoint every
  * `checkpoint_every` steps (<= 0: ceil(sqrt(nsteps))); the backward pass
  * recomputes one segment at a time and runs the hand-written adjoint steps.
  * The pseudospectral trajectory here starts from the transformed initial
