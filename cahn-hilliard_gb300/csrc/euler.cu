@@ -1298,9 +1298,10 @@ __device__ __forceinline__ BfpScale bfp_scale(int emax, const EulerConsts &c, co
     // 2^(61-a): elin is at least -800 where lshift is not zero
     t.lsi = ls == 0.0 || !t.fast ? 0 : __double2ll_rn(ls * __hiloint2double((1023 + 61 - a) << 20, 0));
     // -c2 S 2^(s-60) in half units of M: mc is c2's mantissa times 2^10 and
-    // 2^(1085-ec), so C = -mc 2^-(a+1024-ec), four or more places down
+    // 2^(1085-ec), so C = -mc 2^-(a+1024-ec), four or more places down, rounded:
+    // the half is added in its own place, mc being up to 2^63 - 1024
     const int r = a + 1024 - b.ec;
-    const long long C = r > 62 ? 0 : -((b.mc + (1ll << (r - 1))) >> r);
+    const long long C = r > 62 ? 0 : -(((b.mc >> (r - 1)) + 1) >> 1);
     t.ch = fx_hi(C);
     t.cl = fx_lo(C);
     return t;
