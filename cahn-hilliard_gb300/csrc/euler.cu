@@ -1293,7 +1293,7 @@ __device__ __forceinline__ BfpScale bfp_scale(int emax, const EulerConsts &c, co
     const int s = emax - 1022, a = max(2 * s, b.elin);
     t.lmu = a + s - 56;
     t.fast = emax >= 128 && emax <= 2046 && t.lmu >= -900 && t.lmu <= 900;
-    t.d = a - 2 * s;
+    t.d = min(a - 2 * s, 63);   // X^2 2^-59 is below 2^61: nothing is left of it from 62 on
     const double ls = c.lshift[DIMS - 1];
     // 2^(61-a): elin is at least -800 where lshift is not zero
     t.lsi = ls == 0.0 || !t.fast ? 0 : __double2ll_rn(ls * __hiloint2double((1023 + 61 - a) << 20, 0));
