@@ -418,9 +418,9 @@ int chgb_create(const chgb_params *params, chgb_handle **out) {
                                                                 params->mobility_type, h->g);
         ok = cudaMalloc(&h->d_mu, bytes) == cudaSuccess && (!mob || cudaMalloc(&h->d_mobk, bytes) == cudaSuccess) &&
              (!mob_fx || (cudaMalloc(&h->d_mobkey, 4 * sizeof(unsigned)) == cudaSuccess &&
-                          cudaMemset(h->d_mobkey, 0, 4 * sizeof(unsigned)) == cudaSuccess)) &&
+                          cudaMemsetAsync(h->d_mobkey, 0, 4 * sizeof(unsigned), h->stream) == cudaSuccess)) &&
              (!bfp_ok || (cudaMalloc(&h->d_bfp, sizeof(BfpState)) == cudaSuccess &&
-                         cudaMemset(h->d_bfp, 0, sizeof(BfpState)) == cudaSuccess));
+                         cudaMemsetAsync(h->d_bfp, 0, sizeof(BfpState), h->stream) == cudaSuccess));
         if(!ok) {
             cudaGetLastError();
             if(want == 2 || want == 5) {
