@@ -186,7 +186,8 @@ CHGB_FX int64_t un_sqrt(uint64_t abits, int &k) {
 // t < 2^60.  Returns false where sqrt(a) = 1.
 CHGB_FX bool un_X(uint64_t abits, Un t, Un &X) {
     int k;
-    const int64_t z = un_sqrt(abits, k) - (int64_t) ((1ull << 52) >> k);   // y - 1, exact
+    const int64_t y = un_sqrt(abits, k);                     // sets k, which the next line reads
+    const int64_t z = y - (int64_t) ((1ull << 52) >> k);     // y - 1, exact
     if(z == 0) return false;
     const uint32_t zh = (uint32_t) ((uint64_t) z >> 32);
     const int s = zh ? fx_lead(zh) : 32 + fx_lead((uint32_t) z);
