@@ -1055,12 +1055,19 @@ __global__ void __launch_bounds__(256, (S == 1 && MOB == 0) ? 8 : 1) update_kern
 // face's flux (W_a + W_b)(U_b - U_a) is the upper part, in units of 2^62, of one
 // product on IMAD.WIDE (a constant M: the difference itself, |U| < 2^59), and
 // the divergence an int64 sum -- the same integer for both cells of a face, so
-// the fluxes cancel exactly.  A cell takes two FP64 instructions (a conversion
+// the fluxes cancel exactly.  Per face the integers are off by one unit with a
+// constant M (half a one for each U) and by three else (half a one each for W and
+// the difference, two for the product's upper part).  They are taken where all
+// that stays below 2^-56 of psi, an eighth of its last place; a block with a
+// density for which it does not, many decades below the field's largest, does the
+// step in FP64.  (A Landau field passes through zero, where its value does not
+// tell the scale of what is summed there: its largest value in the block stands
+// for it.)  A cell takes two FP64 instructions (a conversion
 // and the final FMA) where update_kernel takes 16, which bound it (75 % of that
 // pipe).  simple_wertheim with the free-energy mobility on GB300, us a step (mu
-// and update), the FP64 update and this one: 3D N=32 8.6 and 7.0, N=64 28.6 and
-// 17.2, N=128 128.8 and 71.6, N=256 901 and 490; 2D N=512 16.4 and 12.0, N=1024
-// 47.8 and 31.9.
+// and update), the FP64 update and this one: 3D N=32 8.6 and 7.2, N=64 28.6 and
+// 17.1, N=128 128.8 and 71.6, N=256 901 and 491; 2D N=512 16.4 and 12.1, N=1024
+// 47.8 and 31.8.  Where every block falls back, N=128 157.
 //
 // A CTA of 128 threads has a tile of 32 x 16 cells, a warp each of four rows
 // of it: a thread's four cells lie above one another, so that their y faces are
@@ -1079,7 +1086,8 @@ __device__ __forceinline__ long long face_flux(long long a, long long b) {
 }
 
 // The step in FP64, for fields outside the integer path's range (zeros, NaN,
-// infinities, exponents near the ends): a w x h x d block by a whole CTA.
+// infinities, exponents near the ends) and blocks outside its precision: 32 x
+// 16 x d cells by a whole CTA.
 template <int DIMS, bool CONST>
 __device__ __noinline__ void mob_slow_block(const double *__restrict__ psi, const double *__restrict__ mu,
                                             const double *__restrict__ mob, double *__restrict__ out, int mask,
@@ -1101,7 +1109,7 @@ __device__ __noinline__ void mob_slow_block(const double *__restrict__ psi, cons
 
 // 2D: eight CTAs an SM lets the compiler take 64 registers (2D N=512 14.1 -> 11.9
 // us a step); in 3D the same bound costs (N=128 72.8 -> 74.2, N=256 490 -> 534).
-template <int DIMS, bool CONST>
+template <int DIMS, bool CONST, bool DENSITY>
 __global__ void __launch_bounds__(MTHR, DIMS == 2 ? 8 : 1) update_mob_fx_kernel(const double *__restrict__ psi_in,
                                                              const double *__restrict__ mu,
                                                              const double *__restrict__ mob, double *__restrict__ out,
@@ -1120,101 +1128,107 @@ __global__ void __launch_bounds__(MTHR, DIMS == 2 ? 8 : 1) update_mob_fx_kernel(
     // constant M, whose sum of two goes into k, 2^(su - 59)
     const int ek = CONST ? eu - 1022 - 59 : eu + ew - 2 * 1022 - 58;
     const double kd = c.dt * c.half_inv_dx2;
-    if(eu < 300 || eu > 1700 || ew < 300 || ew > 1700 || ek < -800 || ek > 800) {
-        mob_slow_block<DIMS, CONST>(psi_in, mu, mob, out, g.mask, g.log2N, c.M, kd, x0, y0, z0, nz);
-        return;
-    }
-    const double k = (CONST ? kd * (c.M + c.M) : kd) * __hiloint2double((1023 + ek) << 20, 0);
-    FxScale su, sw;
-    su.sh = (CONST ? 59 : 60) - (eu - 1022);
-    sw.sh = 60 - (ew - 1022);
-    // this thread's cells of a staged plane
-    int off[MPF];
-#pragma unroll
-    for(int i = 0; i < MPF; i++) {
-        const int q = tid + i * MTHR, ly = q / MPX, lx = q - ly * MPX;
-        off[i] = ((x0 - 1 + lx) & g.mask) + (((y0 - 1 + ly) & g.mask) << g.log2N);
-    }
-    auto plane = [&](int z) { return DIMS == 3 ? (size_t) (z & g.mask) << (2 * g.log2N) : 0; };
-    double fu[MPF], fw[MPF];
-    auto fetch = [&](int z) {
-        const size_t b = plane(z);
+    bool safe = eu >= 300 && eu <= 1700 && ew >= 300 && ew <= 1700 && ek >= -800 && ek <= 800;
+    if(safe) {
+        const double k = (CONST ? kd * (c.M + c.M) : kd) * __hiloint2double((1023 + ek) << 20, 0);
+        // psi above this (by its high word) is safe from the integers' error
+        const int least = fx_mag(k * ((CONST ? 2.0 : 6.0) * DIMS * 0x1p56));
+        int seen = DENSITY ? 0x7FFFFFFF : 0;   // the least, or the largest, of the thread's |psi|
+        FxScale su, sw;
+        su.sh = (CONST ? 59 : 60) - (eu - 1022);
+        sw.sh = 60 - (ew - 1022);
+        // this thread's cells of a staged plane
+        int off[MPF];
 #pragma unroll
         for(int i = 0; i < MPF; i++) {
-            const bool in = tid + i * MTHR < MPP && CHGB_BC(18, b + off[i], g.bins);
-            fu[i] = in ? mu[b + off[i]] : 0.0;
-            if(!CONST) fw[i] = in ? mob[b + off[i]] : 0.0;
+            const int q = tid + i * MTHR, ly = q / MPX, lx = q - ly * MPX;
+            off[i] = ((x0 - 1 + lx) & g.mask) + (((y0 - 1 + ly) & g.mask) << g.log2N);
         }
-    };
-    auto commit = [&](int slot) {
+        auto plane = [&](int z) { return DIMS == 3 ? (size_t) (z & g.mask) << (2 * g.log2N) : 0; };
+        double fu[MPF], fw[MPF];
+        auto fetch = [&](int z) {
+            const size_t b = plane(z);
 #pragma unroll
-        for(int i = 0; i < MPF; i++) {
-            const int q = tid + i * MTHR;
-            if(q < MPP) {
-                rU[slot][q] = fx_in(fu[i], su);
-                if(!CONST) rW[slot][q] = fx_in(fw[i], sw);
+            for(int i = 0; i < MPF; i++) {
+                const bool in = tid + i * MTHR < MPP && CHGB_BC(18, b + off[i], g.bins);
+                fu[i] = in ? mu[b + off[i]] : 0.0;
+                if(!CONST) fw[i] = in ? mob[b + off[i]] : 0.0;
             }
-        }
-    };
-    auto flux = [&](long long wa, long long wb, long long d) { return CONST ? d : face_flux(wa + wb, d); };
-    auto W = [&](int slot, int p) { return CONST ? 0 : rW[CONST ? 0 : slot][CONST ? 0 : p]; };
-    const int p0 = (row0 + 1) * MPX + tx + 1;   // the thread's first cell in a staged plane
-    const size_t c0 = (size_t) (x0 + tx) + ((size_t) (y0 + row0) << g.log2N);
-    long long jz[4] = {0, 0, 0, 0};
-    fetch(z0);
-    commit(DIMS == 3 ? z0 % 3 : 0);
-    if constexpr(DIMS == 3) {
-        fetch(z0 + 1);
-        // the lowest z faces: the plane below is needed at the thread's own cells only
-        __syncthreads();
-        const size_t b = plane(z0 - 1) + c0;
+        };
+        auto commit = [&](int slot) {
 #pragma unroll
-        for(int r = 0; r < 4; r++) {
-            const size_t gi = b + ((size_t) r << g.log2N);
-            const bool in = CHGB_BC(19, gi, g.bins);
-            const long long u = fx_in(in ? mu[gi] : 0.0, su), w = CONST ? 0 : fx_in(in ? mob[gi] : 0.0, sw);
-            const int p = p0 + r * MPX;
-            jz[r] = flux(w, W(z0 % 3, p), rU[z0 % 3][p] - u);
-        }
-    }
-    for(int z = z0; z < z0 + nz; z++) {
-        const int cz = DIMS == 3 ? z % 3 : 0, zp = DIMS == 3 ? (z + 1) % 3 : 0;
-        const size_t b = plane(z) + c0;
-        double psi[4];
-#pragma unroll
-        for(int r = 0; r < 4; r++) {
-            const size_t gi = b + ((size_t) r << g.log2N);
-            psi[r] = CHGB_BC(19, gi, g.bins) ? psi_in[gi] : 0.0;
-        }
+            for(int i = 0; i < MPF; i++) {
+                const int q = tid + i * MTHR;
+                if(q < MPP) {
+                    rU[slot][q] = fx_in(fu[i], su);
+                    if(!CONST) rW[slot][q] = fx_in(fw[i], sw);
+                }
+            }
+        };
+        auto flux = [&](long long wa, long long wb, long long d) { return CONST ? d : face_flux(wa + wb, d); };
+        auto W = [&](int slot, int p) { return CONST ? 0 : rW[CONST ? 0 : slot][CONST ? 0 : p]; };
+        const int p0 = (row0 + 1) * MPX + tx + 1;   // the thread's first cell in a staged plane
+        const size_t c0 = (size_t) (x0 + tx) + ((size_t) (y0 + row0) << g.log2N);
+        long long jz[4] = {0, 0, 0, 0};
+        fetch(z0);
+        commit(DIMS == 3 ? z0 % 3 : 0);
         if constexpr(DIMS == 3) {
-            commit(zp);
-            if(z + 1 < z0 + nz) fetch(z + 2);
-        }
-        __syncthreads();
-        const long long *U = rU[cz];
-        const int pe = (row0 + 1 + (tx & 3)) * MPX + 1;   // lanes 0-3: the tile's left faces of the four rows
-        const long long edge = flux(W(cz, pe - 1), W(cz, pe), U[pe] - U[pe - 1]);
-        long long u = U[p0], w = W(cz, p0);
-        long long jym = flux(W(cz, p0 - MPX), w, u - U[p0 - MPX]);
+            fetch(z0 + 1);
+            // the lowest z faces: the plane below is needed at the thread's own cells only
+            __syncthreads();
+            const size_t b = plane(z0 - 1) + c0;
 #pragma unroll
-        for(int r = 0; r < 4; r++) {
-            const int p = p0 + r * MPX;
-            const long long un = U[p + MPX], wn = W(cz, p + MPX);
-            const long long jxp = flux(w, W(cz, p + 1), U[p + 1] - u), jyp = flux(w, wn, un - u);
-            const long long left = __shfl_up_sync(0xFFFFFFFFu, jxp, 1), first = __shfl_sync(0xFFFFFFFFu, edge, r);
-            long long D = (jxp - (tx == 0 ? first : left)) + (jyp - jym);
-            if constexpr(DIMS == 3) {
-                const long long jzp = flux(w, W(zp, p), rU[zp][p] - u);
-                D += jzp - jz[r];
-                jz[r] = jzp;
+            for(int r = 0; r < 4; r++) {
+                const size_t gi = b + ((size_t) r << g.log2N);
+                const bool in = CHGB_BC(19, gi, g.bins);
+                const long long u = fx_in(in ? mu[gi] : 0.0, su), w = CONST ? 0 : fx_in(in ? mob[gi] : 0.0, sw);
+                const int p = p0 + r * MPX;
+                jz[r] = flux(w, W(z0 % 3, p), rU[z0 % 3][p] - u);
             }
-            jym = jyp;
-            u = un;
-            w = wn;
-            const size_t gi = b + ((size_t) r << g.log2N);
-            if(CHGB_BC(19, gi, g.bins)) out[gi] = fma(k, (double) D, psi[r]);
         }
+        for(int z = z0; z < z0 + nz; z++) {
+            const int cz = DIMS == 3 ? z % 3 : 0, zp = DIMS == 3 ? (z + 1) % 3 : 0;
+            const size_t b = plane(z) + c0;
+            double psi[4];
+#pragma unroll
+            for(int r = 0; r < 4; r++) {
+                const size_t gi = b + ((size_t) r << g.log2N);
+                psi[r] = CHGB_BC(19, gi, g.bins) ? psi_in[gi] : 0.0;
+            }
+            if constexpr(DIMS == 3) {
+                commit(zp);
+                if(z + 1 < z0 + nz) fetch(z + 2);
+            }
+            __syncthreads();
+            const long long *U = rU[cz];
+            const int pe = (row0 + 1 + (tx & 3)) * MPX + 1;   // lanes 0-3: the tile's left faces of the four rows
+            const long long edge = flux(W(cz, pe - 1), W(cz, pe), U[pe] - U[pe - 1]);
+            long long u = U[p0], w = W(cz, p0);
+            long long jym = flux(W(cz, p0 - MPX), w, u - U[p0 - MPX]);
+#pragma unroll
+            for(int r = 0; r < 4; r++) {
+                const int p = p0 + r * MPX;
+                const long long un = U[p + MPX], wn = W(cz, p + MPX);
+                const long long jxp = flux(w, W(cz, p + 1), U[p + 1] - u), jyp = flux(w, wn, un - u);
+                const long long left = __shfl_up_sync(0xFFFFFFFFu, jxp, 1), first = __shfl_sync(0xFFFFFFFFu, edge, r);
+                long long D = (jxp - (tx == 0 ? first : left)) + (jyp - jym);
+                if constexpr(DIMS == 3) {
+                    const long long jzp = flux(w, W(zp, p), rU[zp][p] - u);
+                    D += jzp - jz[r];
+                    jz[r] = jzp;
+                }
+                jym = jyp;
+                u = un;
+                w = wn;
+                const size_t gi = b + ((size_t) r << g.log2N);
+                if(CHGB_BC(19, gi, g.bins)) out[gi] = fma(k, (double) D, psi[r]);
+                seen = DENSITY ? min(seen, fx_mag(psi[r])) : max(seen, fx_mag(psi[r]));
+            }
+        }
+        safe = seen > least;
     }
+    if(!(DENSITY ? __syncthreads_and(safe) : __syncthreads_or(safe)))
+        mob_slow_block<DIMS, CONST>(psi_in, mu, mob, out, g.mask, g.log2N, c.M, kd, x0, y0, z0, nz);
 }
 
 // ---------------------------------------------------------------------------
@@ -1900,7 +1914,7 @@ cudaError_t launch_split_kind(const Geom &g, const ModelDev &m, const EulerConst
             while(uz > 1 && tiles * (g.N / uz) < SPLIT_CTAS) uz /= 2;
             cfg.gridDim = dim3(g.N / MTX, g.N / MTY, DIMS == 3 ? g.N / uz : 1);
             cfg.blockDim = dim3(MTHR);
-            return cudaLaunchKernelEx(&cfg, update_mob_fx_kernel<DIMS, MOB == 1>, in, (const double *) mu,
+            return cudaLaunchKernelEx(&cfg, update_mob_fx_kernel<DIMS, MOB == 1, KIND == CHGB_MODEL_SIMPLE_WERTHEIM>, in, (const double *) mu,
                                       (const double *) mob, out, g, c, uz, key - 2 * parity, parity);
         }
     return cudaLaunchKernelEx(&cfg, update_kernel<S, MOB, DIMS>, in, (const double *) mu, (const double *) mob, out, g,
