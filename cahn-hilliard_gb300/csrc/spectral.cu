@@ -408,7 +408,7 @@ struct ColOps {
     double2 *out, *rho;
     int first, with_div;
     int log2_bins;
-    double two_k, dt, Ssplit;
+    double two_k, dt, inv_dt, Ssplit;
 };
 
 // dt / x: the reciprocal in integers (relative 2^-58, then one rounding) where
@@ -483,17 +483,28 @@ __device__ __forceinline__ void col_body(double2 *__restrict__ work, double2 *__
         }
         else if(MODE == COL_UPD_INV) {
             // the reference's (rho + dt div - c (f' - S rho)) / (1 + c (S + 2 k q^2)), c =
-            // dt M0 q^2, with its numerator less rho times its denominator: rho + dt / (1
-            // + ...) (div - M0 q^2 (f' + 2 k q^2 rho)), whose rounding is rho's alone.  12
-            // FP64 instructions a mode and a reciprocal in integers, against 22 with a
-            // corrected division of each part
+            // dt M0 q^2, with its numerator less rho times its denominator where that is
+            // below 2: rho + dt / (1 + ...) (div - M0 q^2 (f' + 2 k q^2 rho)), whose
+            // rounding is rho's alone.  A mode that is damped further would keep the
+            // rounding of the larger value it had: there as it stands, dt taken out.  12
+            // FP64 instructions a mode either way and a reciprocal in integers, against 22
+            // with a corrected division of each part.  The two forms against the first
+            // alone, us a step: 2D N=1024 176.6 -> 177.6, 3D N=128 428.6 -> 432.5 (as
+            // operands selected for the same FMAs 179.6 and 433.5)
             const long long lo = line0 + i * ln.T;
             const double k2 = ops.q2[lo], t = ops.two_k * k2, mk = m0 * k2;
-            const double g = dt_over(ops.dt, fma(ops.dt * mk, ops.Ssplit + t, 1.0));
+            const double den = fma(ops.dt * mk, ops.Ssplit + t, 1.0), g = dt_over(ops.dt, den);
             const double2 q = ops.rho[lo], f = psi_hat[lo];
             const double2 d = ops.with_div ? ops.div_in[lo] : make_double2(0.0, 0.0);
-            v.x = fma(g, fma(-mk, fma(t, q.x, f.x), d.x), q.x);
-            v.y = fma(g, fma(-mk, fma(t, q.y, f.y), d.y), q.y);
+            if(den < 2.0) {
+                v.x = fma(g, fma(-mk, fma(t, q.x, f.x), d.x), q.x);
+                v.y = fma(g, fma(-mk, fma(t, q.y, f.y), d.y), q.y);
+            }
+            else {
+                const double a = fma(mk, ops.Ssplit, ops.inv_dt);
+                v.x = g * fma(a, q.x, fma(-mk, f.x, d.x));
+                v.y = g * fma(a, q.y, fma(-mk, f.y, d.y));
+            }
             ops.rho[lo] = v;
         }
         else {
@@ -1624,6 +1635,7 @@ cudaError_t spectral_psmob_update(SpectralState *s, double2 *rho_hat, const doub
     o.div_in = div_hat;
     o.with_div = div_hat ? 1 : 0;
     o.dt = dt;
+    o.inv_dt = 1.0 / dt;
     o.Ssplit = Ssplit;
     o.two_k = 2.0 * k0;
     o.log2_bins = s->g.dims * s->g.log2N;
