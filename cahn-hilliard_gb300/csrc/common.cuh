@@ -149,19 +149,6 @@ __device__ __forceinline__ double fast_rcp(double x) {
     return fma(y, e, y);
 }
 
-// x / d by the reciprocal y of d (within 2 ulp): q0 = RN(x y), the remainder x -
-// q0 d exact by one FMA, then q = RN(q0 + r y) -- a division with one
-// correction step (P. Markstein, "IA-64 and Elementary Functions", 2000;
-// N. Brisebarre, J.-M. Muller and S. K. Raina, IEEE Trans. Computers 53
-// (2004)).  The correctly rounded quotient for all but rare (x, d) pairs, and
-// within 1 ulp of it always, for three FP64 instructions against about ten
-// for a division.  x infinite gives NaN, not infinity.
-__device__ __forceinline__ double div_known(double x, double d, double y) {
-    const double q0 = x * y;
-    const double r = fma(-q0, d, x);
-    return fma(r, y, q0);
-}
-
 // ln a in units of 2^-53 (wertheim_fx.cuh) through the device's table.
 __device__ __forceinline__ int64_t un_log_tab(Un a, const UnLogEntry *__restrict__ tab) {
     return un_log(a, [tab](int j, uint32_t &inv, int64_t &ln) {
