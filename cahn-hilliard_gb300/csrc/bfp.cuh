@@ -222,7 +222,10 @@ __device__ __forceinline__ void fx_scale_by(double2 (&v)[E], bool odd, double f)
 // thread) where lg is odd.  E = 8: radix 8, with one radix-4 pass (two butterflies) where lg is 2
 // modulo 3 and two where it is 1.  Values stay in registers; between two passes
 // they cross through shared memory, which the line's loads and stores do not
-// touch.
+// touch.  The boxes' lines are of 64 values and more with E = 4 and of 1024 and more
+// with E = 8 (fx_line_elems, spectral.cu).  The tests for shorter ones stay: without
+// them the compiler takes 128 registers for the rows with E = 8 instead of 100 (2D
+// N = 2048 197.9 -> 201.6 us a step).
 //
 // The lines of a CTA lie in groups of C = 2^lgC interleaved lines (adjacent
 // columns: a warp's loads then take whole sectors): element p of line c is at
