@@ -1058,16 +1058,16 @@ __global__ void __launch_bounds__(256, (S == 1 && MOB == 0) ? 8 : 1) update_kern
 // the fluxes cancel exactly.  Per face the integers are off by one unit with a
 // constant M (half a one for each U) and by three else (half a one each for W and
 // the difference, two for the product's upper part).  They are taken where all
-// that stays below 2^-56 of psi, an eighth of its last place; a block with a
-// density for which it does not, many decades below the field's largest, does the
-// step in FP64.  (A Landau field passes through zero, where its value does not
-// tell the scale of what is summed there: its largest value in the block stands
-// for it.)  A cell takes two FP64 instructions (a conversion
+// that stays below 2^-56 of psi, an eighth of its last place; a warp (32 x 4 cells
+// of each plane) with a density for which it does not, many decades below the
+// field's largest, does the step in FP64.  (A Landau field passes through zero,
+// where its value does not tell the scale of what is summed there: the warp's
+// largest value stands for it.)  A cell takes two FP64 instructions (a conversion
 // and the final FMA) where update_kernel takes 16, which bound it (75 % of that
 // pipe).  simple_wertheim with the free-energy mobility on GB300, us a step (mu
 // and update), the FP64 update and this one: 3D N=32 8.6 and 7.2, N=64 28.6 and
-// 17.1, N=128 128.8 and 71.6, N=256 901 and 491; 2D N=512 16.4 and 12.1, N=1024
-// 47.8 and 31.8.  Where every block falls back, N=128 157.
+// 17.1, N=128 128.8 and 71.6, N=256 901 and 491; 2D N=512 16.4 and 11.9, N=1024
+// 47.8 and 31.7.  Where every warp falls back, N=128 156.
 //
 // A CTA of 128 threads has a tile of 32 x 16 cells, a warp each of four rows
 // of it: a thread's four cells lie above one another, so that their y faces are
@@ -1085,19 +1085,19 @@ __device__ __forceinline__ long long face_flux(long long a, long long b) {
     return wide(ah, bh) + (wide(ah, bl, wide(al, bh)) >> 31);
 }
 
-// The step in FP64, for fields outside the integer path's range (zeros, NaN,
-// infinities, exponents near the ends) and blocks outside its precision: 32 x
-// 16 x d cells by a whole CTA.
+// The step of a thread's cells (four rows of `d` planes) in FP64, for fields outside
+// the integer path's range (zeros, NaN, infinities, exponents near the ends) and
+// warps outside its precision.
 template <int DIMS, bool CONST>
-__device__ __noinline__ void mob_slow_block(const double *__restrict__ psi, const double *__restrict__ mu,
+__device__ __noinline__ void mob_slow_cells(const double *__restrict__ psi, const double *__restrict__ mu,
                                             const double *__restrict__ mob, double *__restrict__ out, int mask,
-                                            int log2N, double M, double k, int x0, int y0, int z0, int d) {
+                                            int log2N, double M, double k, int x, int y0, int z0, int d) {
     auto index = [&](int X, int Y, int Z) {
         return (size_t) (X & mask) + ((size_t) (Y & mask) << log2N) +
                (DIMS == 3 ? ((size_t) (Z & mask) << (2 * log2N)) : 0);
     };
-    for(int i = threadIdx.x; i < MTX * MTY * d; i += MTHR) {
-        const int x = x0 + i % MTX, y = y0 + i / MTX % MTY, z = z0 + i / (MTX * MTY);
+    for(int i = 0; i < 4 * d; i++) {
+        const int y = y0 + (i & 3), z = z0 + (i >> 2);
         const size_t c = index(x, y, z);
         auto face = [&](size_t a, size_t b) { return (CONST ? M + M : mob[a] + mob[b]) * (mu[b] - mu[a]); };
         double div = (face(c, index(x + 1, y, z)) - face(index(x - 1, y, z), c)) +
@@ -1227,8 +1227,8 @@ __global__ void __launch_bounds__(MTHR, DIMS == 2 ? 8 : 1) update_mob_fx_kernel(
         }
         safe = seen > least;
     }
-    if(!(DENSITY ? __syncthreads_and(safe) : __syncthreads_or(safe)))
-        mob_slow_block<DIMS, CONST>(psi_in, mu, mob, out, g.mask, g.log2N, c.M, kd, x0, y0, z0, nz);
+    if(!(DENSITY ? __all_sync(0xFFFFFFFFu, safe) : __any_sync(0xFFFFFFFFu, safe)))
+        mob_slow_cells<DIMS, CONST>(psi_in, mu, mob, out, g.mask, g.log2N, c.M, kd, x0 + tx, y0 + row0, z0, nz);
 }
 
 // ---------------------------------------------------------------------------
