@@ -74,22 +74,24 @@ cudaError_t launch_der_bulk(const ModelDev &m, const double *rho, double *der, l
 namespace {
 
 // src/mobility/RegularisedMobility.h:26-33 and src/mobility/GelMobility.h:41-58;
-// with sink.M0 set also the field's maximum per species.  Gel: 4 FP64
-// instructions a cell and the exponential in integers (28 FP64 ones with two
-// corrected divisions by constants and a table-driven exponential); 2D N=1024
-// 62.9 -> 14.3 us, and a reduction pass of 11 us saved.
+// MAX: also the field's maximum per species.  A kernel each: in one, without MAX,
+// a regularised euler_mobility step took 0.1 us longer (2D N=128 6.52, 6.42 now).
+// Gel: 4 FP64 instructions a cell and the exponential in integers (28 FP64 ones
+// with two corrected divisions by constants and a table-driven exponential); 2D
+// N=1024 62.9 -> 14.3 us, and a reduction pass of 11 us saved.
+template <bool GEL, bool MAX>
 __global__ void mobility_update_kernel(MobilityDev md, const double *__restrict__ rho, double *__restrict__ gel,
                                        double *__restrict__ mob, int S, long long bins, M0Sink sink) {
     const long long i0 = blockIdx.x * (long long) blockDim.x + threadIdx.x, di = (long long) gridDim.x * blockDim.x;
-    if(md.type == CHGB_MOBILITY_REGULARISED) {
+    if constexpr(!GEL) {
         for(int s = 0; s < S; s++) {
             unsigned long long m = 0;
             for(long long i = i0; i < bins; i += di) {
                 const double r = rho[s * bins + i], M = md.M * r / (r + md.rho_min);
                 mob[s * bins + i] = M;
-                m0_take(m, M);
+                if constexpr(MAX) m0_take(m, M);
             }
-            if(sink.M0) m0_commit(m, sink, s, s + 1);
+            if constexpr(MAX) m0_commit(m, sink, s, s + 1);
         }
     }
     else {
@@ -102,9 +104,9 @@ __global__ void mobility_update_kernel(MobilityDev md, const double *__restrict_
             gel[i] = c;
             const double M = gel_exp(md, c);
             for(int s = 0; s < S; s++) mob[s * bins + i] = M;
-            m0_take(m, M);
+            if constexpr(MAX) m0_take(m, M);
         }
-        if(sink.M0) m0_commit(m, sink, 0, S);
+        if constexpr(MAX) m0_commit(m, sink, 0, S);
     }
 }
 
@@ -112,7 +114,10 @@ __global__ void mobility_update_kernel(MobilityDev md, const double *__restrict_
 
 cudaError_t launch_mobility_update(const MobilityDev &md, const double *rho, double *gel, double *mob, int S,
                                    long long bins, cudaStream_t st, const M0Sink &sink) {
-    mobility_update_kernel<<<grid_for(bins), 256, 0, st>>>(md, rho, gel, mob, S, bins, sink);
+    auto kernel = md.type == CHGB_MOBILITY_GEL
+                      ? (sink.M0 ? mobility_update_kernel<true, true> : mobility_update_kernel<true, false>)
+                      : (sink.M0 ? mobility_update_kernel<false, true> : mobility_update_kernel<false, false>);
+    kernel<<<grid_for(bins), 256, 0, st>>>(md, rho, gel, mob, S, bins, sink);
     return cudaGetLastError();
 }
 
