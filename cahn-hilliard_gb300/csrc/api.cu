@@ -129,6 +129,8 @@ ModelDev make_model_dev(const chgb_model_params &mp, bool with_log_table) {
     m.two_B2 = 2.0 * mp.B2;
     m.reg_delta = mp.regularisation_delta;
     m.log_delta = std::log(mp.regularisation_delta);        // src/models/SimpleWertheim.cpp:32
+    m.reg_slope = 2.0 * mp.B2 + 1.0 / mp.regularisation_delta;
+    m.reg_base = m.log_delta - 1.0;
     m.sv0 = (double) mp.saleh_valence[0];
     m.sv1 = (double) mp.saleh_valence[1];
     m.half = (double) (mp.saleh_valence[2] / 2);            // src/models/SalehWertheim.cpp:28

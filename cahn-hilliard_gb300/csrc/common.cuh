@@ -27,6 +27,7 @@ struct ModelDev {
     double four_valence_delta;      // 2 * two_valence_delta (exact: a power-of-two multiple)
     double two_B2;                  // 2 * B2 (exact)
     double reg_delta, log_delta;    // regularisation_delta and log(regularisation_delta)
+    double reg_slope, reg_base;     // below it f' is reg_slope rho + reg_base + valence log X
     double sv0, sv1, half;          // saleh valences of A and B, linker half valence
     double dAA, dBB;
     double dcf;                     // density conversion factor
@@ -230,9 +231,33 @@ struct SwCell {
     double der, rhoXv;
 };
 
-__device__ __noinline__ static SwCell sw_cell_fp(const ModelDev &m, double rho) {
-    const double X = sw_X(m, rho);
+// The cell in integers (wertheim_fx.cuh) where the path takes the density: 5 FP64
+// instructions instead of 40.  log(rho) + valence log(X) as one logarithm,
+// log(rho X^valence); BELOW the regularisation log(X) alone.
+template <bool BELOW>
+__device__ __forceinline__ bool sw_cell_fx(const ModelDev &m, double rho, SwCell &c) {
+    const double t = m.four_valence_delta * rho;
+    Un X;
+    if(!un_takes(t) || t >= 0x1p59 || !un_X((uint64_t) __double_as_longlong(1.0 + t), un_of(t), X)) return false;
+    const Un P = un_mul(un_of(rho), un_pow(X, m.ivalence));
+    if(P.e < -1000) return false;
+    c.rhoXv = __longlong_as_double((long long) un_to_bits(P));
+    if constexpr(BELOW)
+        c.der = fma((double) un_log_tab(X, m.logtab), m.valence * UNLOG_UNIT, fma(m.reg_slope, rho, m.reg_base));
+    else c.der = fma((double) un_log_tab(P, m.logtab), UNLOG_UNIT, m.two_B2 * rho);
+    return true;
+}
+
+// Cells below the regularisation and those in FP64, out of the others' way: with
+// the ones below in the inlined path, as operands selected, a 3D N=128
+// euler_mobility step that has none took 75.8 us instead of 72.2.  In FP64 they
+// made `euler` boxes slower than FP64 for every cell did: 2D N=32 with half of
+// them below 7.1 -> 8.4 us a step, here 5.9; N=1024 with all below 135 -> 148,
+// here 31.
+__device__ __noinline__ static SwCell sw_cell_other(const ModelDev &m, double rho) {
     SwCell c;
+    if(m.sw_fx && m.logtab != nullptr && un_takes(rho) && rho < m.reg_delta && sw_cell_fx<true>(m, rho, c)) return c;
+    const double X = sw_X(m, rho);
     c.rhoXv = rho * ipow(X, m.ivalence);
     c.der = m.two_B2 * rho;
     if(rho < m.reg_delta) {
@@ -243,20 +268,11 @@ __device__ __noinline__ static SwCell sw_cell_fp(const ModelDev &m, double rho) 
     return c;
 }
 
-// log(rho) + valence log(X) as one logarithm, log(rho X^valence).  In integers
-// (wertheim_fx.cuh) for densities at or above the regularisation that the path
-// takes: 5 FP64 instructions a cell instead of 40.
 __device__ __forceinline__ SwCell sw_cell(const ModelDev &m, double rho) {
-    const long long b = __double_as_longlong(rho);
-    if(!m.sw_fx || m.logtab == nullptr || !un_takes(rho) || b < __double_as_longlong(m.reg_delta)) return sw_cell_fp(m, rho);
-    const double t = m.four_valence_delta * rho;
-    Un X;
-    if(!un_takes(t) || t >= 0x1p59 || !un_X((uint64_t) __double_as_longlong(1.0 + t), un_of(t), X)) return sw_cell_fp(m, rho);
-    const Un P = un_mul(un_of(rho), un_pow(X, m.ivalence));
-    if(P.e < -1000) return sw_cell_fp(m, rho);
     SwCell c;
-    c.rhoXv = __longlong_as_double((long long) un_to_bits(P));
-    c.der = fma((double) un_log_tab(P, m.logtab), UNLOG_UNIT, m.two_B2 * rho);
+    if(!m.sw_fx || m.logtab == nullptr || !un_takes(rho) ||
+       __double_as_longlong(rho) < __double_as_longlong(m.reg_delta) || !sw_cell_fx<false>(m, rho, c))
+        return sw_cell_other(m, rho);
     return c;
 }
 
