@@ -1067,7 +1067,7 @@ __global__ void __launch_bounds__(256, (S == 1 && MOB == 0) ? 8 : 1) update_kern
 // pipe).  simple_wertheim with the free-energy mobility on GB300, us a step (mu
 // and update), the FP64 update and this one: 3D N=32 8.6 and 7.2, N=64 28.6 and
 // 17.1, N=128 128.8 and 71.6, N=256 901 and 491; 2D N=512 16.4 and 11.9, N=1024
-// 47.8 and 31.7.  Where every warp falls back, N=128 156.
+// 47.8 and 31.7.  A field of twelve decades, N=128: 287 and 122.
 //
 // A CTA of 128 threads has a tile of 32 x 16 cells, a warp each of four rows
 // of it: a thread's four cells lie above one another, so that their y faces are
@@ -1085,25 +1085,48 @@ __device__ __forceinline__ long long face_flux(long long a, long long b) {
     return wide(ah, bh) + (wide(ah, bl, wide(al, bh)) >> 31);
 }
 
-// The step of a thread's cells (four rows of `d` planes) in FP64, for fields outside
-// the integer path's range (zeros, NaN, infinities, exponents near the ends) and
-// warps outside its precision.
+// The step of a warp's cells (32 x 4 of each of `d` planes; a thread has a column of
+// four) in FP64, for fields outside the integer path's range (zeros, NaN,
+// infinities, exponents near the ends) and warps outside its precision.  A thread
+// forms the y faces between its cells and the z faces between planes once (N=128, a
+// field of twelve decades, 142 -> 122 us a step; one with a Landau spot 110 -> 98).
 template <int DIMS, bool CONST>
 __device__ __noinline__ void mob_slow_cells(const double *__restrict__ psi, const double *__restrict__ mu,
                                             const double *__restrict__ mob, double *__restrict__ out, int mask,
                                             int log2N, double M, double k, int x, int y0, int z0, int d) {
-    auto index = [&](int X, int Y, int Z) {
-        return (size_t) (X & mask) + ((size_t) (Y & mask) << log2N) +
-               (DIMS == 3 ? ((size_t) (Z & mask) << (2 * log2N)) : 0);
+    const unsigned xm = (x - 1) & mask, xp = (x + 1) & mask;
+    auto row = [&](int Y, int Z) {   // below 2^30
+        return ((unsigned) (Y & mask) << log2N) + (DIMS == 3 ? (unsigned) (Z & mask) << (2 * log2N) : 0u);
     };
-    for(int i = 0; i < 4 * d; i++) {
-        const int y = y0 + (i & 3), z = z0 + (i >> 2);
-        const size_t c = index(x, y, z);
-        auto face = [&](size_t a, size_t b) { return (CONST ? M + M : mob[a] + mob[b]) * (mu[b] - mu[a]); };
-        double div = (face(c, index(x + 1, y, z)) - face(index(x - 1, y, z), c)) +
-                     (face(c, index(x, y + 1, z)) - face(index(x, y - 1, z), c));
-        if(DIMS == 3) div = div + (face(c, index(x, y, z + 1)) - face(index(x, y, z - 1), c));
-        if(CHGB_BC(20, c, (long long) 1 << (DIMS * log2N))) out[c] = fma(k, div, psi[c]);
+    auto W = [&](unsigned c) { return CONST ? M : mob[c]; };
+    double jz[4] = {0.0, 0.0, 0.0, 0.0};
+    if constexpr(DIMS == 3)
+#pragma unroll
+        for(int r = 0; r < 4; r++) {
+            const unsigned c = row(y0 + r, z0) + x, b = row(y0 + r, z0 - 1) + x;
+            jz[r] = (W(b) + W(c)) * (mu[c] - mu[b]);
+        }
+    for(int z = z0; z < z0 + d; z++) {
+        const unsigned below = row(y0 - 1, z) + x;
+        double u = mu[row(y0, z) + x], w = W(row(y0, z) + x);
+        double jym = (W(below) + w) * (u - mu[below]);
+#pragma unroll
+        for(int r = 0; r < 4; r++) {
+            const unsigned line = row(y0 + r, z), c = line + x, n = row(y0 + r + 1, z) + x;
+            const double un = mu[n], wn = W(n), jyp = (w + wn) * (un - u);
+            const double jxp = (w + W(line + xp)) * (mu[line + xp] - u), jxm = (W(line + xm) + w) * (u - mu[line + xm]);
+            double div = (jxp - jxm) + (jyp - jym);
+            if constexpr(DIMS == 3) {
+                const unsigned a = row(y0 + r, z + 1) + x;
+                const double jzp = (w + W(a)) * (mu[a] - u);
+                div = div + (jzp - jz[r]);
+                jz[r] = jzp;
+            }
+            if(CHGB_BC(20, c, (long long) 1 << (DIMS * log2N))) out[c] = fma(k, div, psi[c]);
+            jym = jyp;
+            u = un;
+            w = wn;
+        }
     }
 }
 
