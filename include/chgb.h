@@ -264,7 +264,8 @@ int64_t chgb_launch_count(const chgb_handle *h);
 int chgb_bounds_report(unsigned long long *first);
 
 /* Kernel variant the handle runs: 1 fused, 2 split, 3 two steps per launch, 4 cluster-resident,
- * 5 split in block fixed point (see kernel_variant);
+ * 5 block fixed point (see kernel_variant; `euler_mobility` boxes report it under
+ * kernel_variant 0 and do not take it by number);
  * 1 for the pseudospectral integrators. */
 int chgb_kernel_variant(const chgb_handle *h);
 
@@ -341,7 +342,8 @@ int64_t chgb_adjoint_launch_count(const chgb_adjoint *a);
  * all differ).  2D `euler` and 2D `pseudospectral` replicas are stepped by
  * shared work-list kernels (one launch per phase for the whole group, replayed
  * from a CUDA graph); any other replica runs on its own stream alongside.
- * A replica gives the same bits stepped in a batch as stepped alone.
+ * A replica gives the same bits stepped in a batch as stepped alone (a 2D `euler`
+ * one: as alone with kernel_variant 1, whose arithmetic the shared kernel has).
  */
 typedef struct chgb_batch chgb_batch;
 
