@@ -1066,7 +1066,7 @@ __global__ void __launch_bounds__(256, (S == 1 && MOB == 0) ? 8 : 1) update_kern
 // and the final FMA) where update_kernel takes 16, which bound it (75 % of that
 // pipe).  simple_wertheim with the free-energy mobility on GB300, us a step (mu
 // and update), the FP64 update and this one: 3D N=32 8.6 and 7.2, N=64 28.6 and
-// 17.1, N=128 128.8 and 71.6, N=256 901 and 491; 2D N=512 16.4 and 11.9, N=1024
+// 17.1, N=128 128.8 and 71.6, N=256 901 and 483; 2D N=512 16.4 and 11.9, N=1024
 // 47.8 and 31.7.  A field of twelve decades, N=128: 287 and 122.
 //
 // A CTA of 128 threads has a tile of 32 x 16 cells, a warp each of four rows
@@ -1130,10 +1130,13 @@ __device__ __noinline__ void mob_slow_cells(const double *__restrict__ psi, cons
     }
 }
 
-// 2D: eight CTAs an SM lets the compiler take 64 registers (2D N=512 14.1 -> 11.9
-// us a step); in 3D the same bound costs (N=128 72.8 -> 74.2, N=256 490 -> 534).
-template <int DIMS, bool CONST, bool DENSITY>
-__global__ void __launch_bounds__(MTHR, DIMS == 2 ? 8 : 1) update_mob_fx_kernel(const double *__restrict__ psi_in,
+// CTAs an SM the registers are limited for.  2D: eight, 64 registers (2D N=512 14.1
+// -> 11.9 us a step).  3D: five (96 registers instead of 112) where the launch has
+// as many CTAs, none for the small boxes (free-energy mobility, us a step without and
+// with the limit: N=256 491 and 483, N=128 72.4 and 72.2, with three boxes at once
+// 61.2 and 59.9; N=64 17.4 and 18.1, N=32 7.6 and 8.6).
+template <int DIMS, bool CONST, bool DENSITY, int CTAS>
+__global__ void __launch_bounds__(MTHR, CTAS) update_mob_fx_kernel(const double *__restrict__ psi_in,
                                                              const double *__restrict__ mu,
                                                              const double *__restrict__ mob, double *__restrict__ out,
                                                              Geom g, EulerConsts c, int zc, unsigned *__restrict__ key,
@@ -1937,7 +1940,10 @@ cudaError_t launch_split_kind(const Geom &g, const ModelDev &m, const EulerConst
             while(uz > 1 && tiles * (g.N / uz) < SPLIT_CTAS) uz /= 2;
             cfg.gridDim = dim3(g.N / MTX, g.N / MTY, DIMS == 3 ? g.N / uz : 1);
             cfg.blockDim = dim3(MTHR);
-            return cudaLaunchKernelEx(&cfg, update_mob_fx_kernel<DIMS, MOB == 1, KIND == CHGB_MODEL_SIMPLE_WERTHEIM>, in, (const double *) mu,
+            constexpr bool CONST = MOB == 1, DENSITY = KIND == CHGB_MODEL_SIMPLE_WERTHEIM;
+            auto kernel = tiles * (g.N / uz) >= 5 * 152 ? update_mob_fx_kernel<DIMS, CONST, DENSITY, DIMS == 2 ? 8 : 5>
+                                                        : update_mob_fx_kernel<DIMS, CONST, DENSITY, DIMS == 2 ? 8 : 1>;
+            return cudaLaunchKernelEx(&cfg, kernel, in, (const double *) mu,
                                       (const double *) mob, out, g, c, uz, key - 2 * parity, parity);
         }
     return cudaLaunchKernelEx(&cfg, update_kernel<S, MOB, DIMS>, in, (const double *) mu, (const double *) mob, out, g,
